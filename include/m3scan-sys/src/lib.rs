@@ -81,7 +81,8 @@ pub struct m3_scan_desc {
     pub path: i32,
     /// the last `reverse_heads` heads walk time right to left (bidirectional mixer, models/mamba3.rs:97-112)
     pub reverse_heads: i32,
-    pub reserved0: i32,
+    /// elements between consecutive tokens of theta and its gradient; 0 = dense
+    pub theta_stride: i32,
     pub x: *const c_void,
     pub b: *const c_void,
     pub c: *const c_void,
@@ -288,6 +289,55 @@ pub struct m3_gate_norm_desc {
     pub eps: f32,
 }
 
+/// The mixer between its two projections (src/models/mamba3.rs:340-461, :475-484).
+#[repr(C)]
+#[derive(Clone, Copy)]
+pub struct m3_mixer_desc {
+    pub batch: i32,
+    pub seq: i32,
+    pub heads: i32,
+    pub head_dim: i32,
+    pub d_state: i32,
+    pub rank: i32,
+    pub groups: i32,
+    pub chunk: i32,
+    pub dtype: i32,
+    pub discretization: i32,
+    pub dynamics: i32,
+    pub conv_kernel: i32,
+    pub has_norm: i32,
+    pub post_norm: i32,
+    pub path: i32,
+    pub reverse_heads: i32,
+    pub eps: f32,
+    pub reserved0: i32,
+    pub proj: *const c_void,
+    pub conv_weight: *const f32,
+    pub conv_bias: *const f32,
+    pub dt_bias: *const f32,
+    pub a_log: *const f32,
+    pub d_skip: *const f32,
+    pub b_bias: *const f32,
+    pub c_bias: *const f32,
+    pub norm_weight: *const f32,
+    pub post_weight: *const f32,
+}
+
+/// The carried cache of an inference window, in and out (src/models/mamba3.rs:486-560).
+#[repr(C)]
+#[derive(Clone, Copy)]
+pub struct m3_mixer_window_io {
+    pub conv_in: *const c_void,
+    pub h_in: *const f32,
+    pub last_u_in: *const f32,
+    pub angle_in: *const f32,
+    pub out: *mut c_void,
+    pub conv_out: *mut c_void,
+    pub h_out: *mut f32,
+    pub last_u_out: *mut f32,
+    pub angle_out: *mut f32,
+}
+
 extern "C" {
     pub fn m3_version() -> *const c_char;
 
@@ -348,4 +398,9 @@ extern "C" {
     pub fn m3_gate_norm_forward(ctx: *mut m3_ctx, desc: *const m3_gate_norm_desc, out: *mut c_void) -> c_int;
     pub fn m3_gate_norm_backward(ctx: *mut m3_ctx, desc: *const m3_gate_norm_desc, dout: *const c_void, dy: *mut c_void,
                                  dz: *mut c_void, dweight: *mut f32) -> c_int;
+
+    /// Mamba3Mixer::apply_with_state between the projections: a prefill window or one decoding step.
+    pub fn m3_mixer_window_bytes(desc: *const m3_mixer_desc, io: *const m3_mixer_window_io) -> usize;
+    pub fn m3_mixer_window(ctx: *mut m3_ctx, desc: *const m3_mixer_desc, io: *const m3_mixer_window_io,
+                           workspace: *mut c_void) -> c_int;
 }

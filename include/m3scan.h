@@ -75,7 +75,8 @@ typedef struct {
                            * outputs and gradients all stay in ordinary time.  0 = none; heads/2 for
                            * the bidirectional mixer.  The carried state of such a head enters at the
                            * last token and the returned one is the state after token 0. */
-  int32_t reserved0;      /* must be 0 */
+  int32_t theta_stride;   /* elements between consecutive tokens of theta and of its gradient: theta may be a
+                           * column band of the input projection.  0 = dense (heads * d_state/2) */
   const void *x;          /* [batch, seq, heads, head_dim, rank] */
   const void *b;          /* [batch, seq, heads, d_state, rank]  */
   const void *c;          /* [batch, seq, heads, d_state, rank]  */
@@ -374,6 +375,45 @@ typedef struct {
 int m3_gate_norm_forward(m3_ctx *ctx, const m3_gate_norm_desc *desc, void *out);
 int m3_gate_norm_backward(m3_ctx *ctx, const m3_gate_norm_desc *desc, const void *dout, void *dy, void *dz,
                           float *dweight);
+
+/* The mixer between its two projections (Mamba3Mixer::project / finish around mamba3_scan,
+ * src/models/mamba3.rs:340-461, :475-484), described once for the calls below.  proj is the input
+ * projection's output [batch, seq, width], width = 2 d_inner + 2 bc + heads + (heads when lambda is
+ * learned) + (heads * d_state/2 when rotational), d_inner = heads * head_dim * rank and bc = groups *
+ * d_state * rank, cut into z | x B C | dt | lambda | theta; every step reads its band in place. */
+typedef struct {
+  int32_t batch, seq, heads, head_dim, d_state, rank, groups;
+  int32_t chunk, dtype, discretization, dynamics;
+  int32_t conv_kernel;        /* taps of the convolution, 1..8 */
+  int32_t has_norm;           /* bc_norm */
+  int32_t post_norm;          /* post_gate_norm */
+  int32_t path, reverse_heads;
+  float eps;
+  int32_t reserved0;
+  const void *proj;
+  const float *conv_weight;   /* [conv_kernel, d_inner + 2 bc] */
+  const float *conv_bias;     /* [d_inner + 2 bc] or NULL */
+  const float *dt_bias;       /* [heads] or NULL */
+  const float *a_log;         /* [heads] */
+  const float *d_skip;        /* [heads] or NULL */
+  const float *b_bias, *c_bias; /* [heads, d_state] or NULL */
+  const float *norm_weight;   /* [d_state] or NULL */
+  const float *post_weight;   /* [d_inner] or NULL */
+} m3_mixer_desc;
+
+/* Inference with a carried cache (apply_with_state, src/models/mamba3.rs:486-560): a prefill window, or a
+ * decoding step when seq is 1.  The new cache goes to buffers of its own (inputs are never written). */
+typedef struct {
+  const void *conv_in;        /* [batch, conv_kernel-1, d_inner + 2 bc]: the convolution's last inputs */
+  const float *h_in, *last_u_in, *angle_in;   /* the scan's state; angle may be NULL (zero) */
+  void *out;                  /* [batch, seq, d_inner]: the gated output */
+  void *conv_out;
+  float *h_out, *last_u_out, *angle_out;
+} m3_mixer_window_io;
+/* workspace: m3_mixer_window_bytes bytes of device memory, 256-byte aligned; NULL when that is 0 (a decoding
+ * step of a shape that runs as one launch). */
+size_t m3_mixer_window_bytes(const m3_mixer_desc *desc, const m3_mixer_window_io *io);
+int m3_mixer_window(m3_ctx *ctx, const m3_mixer_desc *desc, const m3_mixer_window_io *io, void *workspace);
 
 /* Bytes of device scratch a forward with this descriptor allocates (kept until
  * m3_saved_free when `saved` is requested). */

@@ -6,6 +6,7 @@ library has not been built: there is no CPU or eager fallback behind this module
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from pathlib import Path
 
 _LIB_PATH = Path(__file__).resolve().parent / "libm3scan.so"
@@ -26,7 +27,7 @@ NOALLOC_SCRATCH_BYTES = 16 << 20   # M3_NOALLOC_SCRATCH_BYTES
 class ScanDesc(C.Structure):
     _fields_ = [(n, C.c_int32) for n in (
         "batch", "seq", "heads", "head_dim", "d_state", "rank", "chunk", "dtype",
-        "discretization", "dynamics", "want_state", "path", "reverse_heads", "reserved0")] + [
+        "discretization", "dynamics", "want_state", "path", "reverse_heads", "theta_stride")] + [
         (n, C.c_void_p) for n in (
             "x", "b", "c", "dt", "lambda_", "theta", "a_log", "d_skip", "h0", "last_u0", "angle0",
             "a_raw", "g_raw", "w_raw")]
@@ -84,6 +85,25 @@ class GateNormDesc(C.Structure):
         (n, C.c_void_p) for n in ("y", "z", "weight")] + [("eps", C.c_float)]
 
 
+class MixerDesc(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in (
+        "batch", "seq", "heads", "head_dim", "d_state", "rank", "groups", "chunk", "dtype", "discretization", "dynamics",
+        "conv_kernel", "has_norm", "post_norm", "path", "reverse_heads")] + [("eps", C.c_float), ("reserved0", C.c_int32)] + [
+        (n, C.c_void_p) for n in ("proj", "conv_weight", "conv_bias", "dt_bias", "a_log", "d_skip", "b_bias", "c_bias",
+                                  "norm_weight", "post_weight")]
+
+
+class MixerWindowIo(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("conv_in", "h_in", "last_u_in", "angle_in", "out", "conv_out", "h_out",
+                                          "last_u_out", "angle_out")]
+
+
+# The mixer calls sit on latency-bound paths, where filling a ctypes structure field by field is a large part of
+# the call: these lay the same bytes out in one pack (0 for a NULL pointer).
+PACK_MIXER_DESC = struct.Struct("@16ifi10P")
+PACK_MIXER_WINDOW_IO = struct.Struct("@9P")
+
+
 class HostIn(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("x", "b", "c", "dt", "lambda_", "theta", "dy")]
 
@@ -123,6 +143,8 @@ SYMBOLS = {
     "m3_gate_backward": (C.c_int, [C.c_void_p, C.POINTER(GateDesc), C.c_void_p, C.c_void_p, C.c_void_p]),
     "m3_gate_norm_forward": (C.c_int, [C.c_void_p, C.POINTER(GateNormDesc), C.c_void_p]),
     "m3_gate_norm_backward": (C.c_int, [C.c_void_p, C.POINTER(GateNormDesc), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "m3_mixer_window_bytes": (C.c_size_t, [C.c_char_p, C.c_char_p]),
+    "m3_mixer_window": (C.c_int, [C.c_void_p, C.c_char_p, C.c_char_p, C.c_void_p]),
     "m3_host_alloc": (C.c_int, [C.c_size_t, C.POINTER(C.c_void_p)]),
     "m3_host_free": (C.c_int, [C.c_void_p]),
     "m3_host_pipe_create": (C.c_int, [C.c_void_p, C.POINTER(ScanDesc), C.c_int, C.POINTER(C.c_void_p)]),

@@ -104,6 +104,8 @@ int make_dims(m3_ctx* ctx, const m3_scan_desc& s, m3::Dims* out) {
   d.LR = L * s.rank;
   d.raw = raw ? 1 : 0;
   d.rev = s.reverse_heads;
+  d.ths = s.theta_stride ? s.theta_stride : d.H * d.NH;
+  if (d.rot && d.ths < d.H * d.NH) return fail(ctx, M3_ERR_SHAPE, "theta_stride %d below heads * d_state / 2", d.ths);
   *out = d;
   return M3_OK;
 }
@@ -213,7 +215,7 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
   p.dlu0 = (has_state && want(M3_GRAD_LAST_U0, g->dlast_u0)) ? g->dlast_u0 : nullptr;
   p.dangle0 = (d.rot && desc.angle0 && want(M3_GRAD_ANGLE0, g->dangle0)) ? g->dangle0 : nullptr;
   p.err = ctx->dev_err;
-  p.B = d.B; p.T = d.T; p.H = d.H; p.R = d.R; p.disc = d.disc; p.rev = d.rev;
+  p.B = d.B; p.T = d.T; p.H = d.H; p.R = d.R; p.disc = d.disc; p.rev = d.rev; p.ths = d.ths;
   p.wait_limit = ctx->wait_limit ? ctx->wait_limit : (1u << 18);
   if (!m3::tc_aligned(p.dy) || !m3::tc_aligned(p.dx) || !m3::tc_aligned(p.db) || !m3::tc_aligned(p.dc) ||
       !m3::tc_aligned(p.dtheta)) {
@@ -231,7 +233,7 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
         !m3::tc_make_row_map(&p.tm_c, p.c, d.B, d.T, d.H, 128 * d.R, steps, true) ||
         !m3::tc_make_row_map(&p.tm_x, p.x, d.B, d.T, d.H, 64 * d.R, steps, true) ||
         !m3::tc_make_row_map(&p.tm_dy, p.dy, d.B, d.T, d.H, 64 * d.R, steps, true) ||
-        (d.rot && !m3::tc_make_row_map(&p.tm_th, p.theta, d.B, d.T, d.H, 64, steps, false))) {
+        (d.rot && !m3::tc_make_row_map(&p.tm_th, p.theta, d.B, d.T, d.H, 64, steps, false, d.ths))) {
       cudaFreeAsync(base, ctx->stream);
       return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs 16-byte aligned b, c, x, dy and theta");
     }
@@ -446,7 +448,7 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     p.lu_out = desc->want_state ? out->last_u : nullptr;
     p.angle_out = (desc->want_state && d.rot) ? out->angle : nullptr;
     p.err = ctx->dev_err;
-    p.B = d.B; p.T = d.T; p.H = d.H; p.R = d.R; p.disc = d.disc; p.rev = d.rev;
+    p.B = d.B; p.T = d.T; p.H = d.H; p.R = d.R; p.disc = d.disc; p.rev = d.rev; p.ths = d.ths;
     p.wait_limit = ctx->wait_limit ? ctx->wait_limit : (1u << 18);
     // Rank 1 with real dynamics needs no conversion of its rows: bulk tensor copies land them in
     // operand layout (every head left to right, T a multiple of 8, 16-byte aligned tensors).
@@ -459,7 +461,7 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
       if (!m3::tc_make_row_map(&p.tm_b, p.b, d.B, d.T, d.H, 128 * d.R, steps, true) ||
           !m3::tc_make_row_map(&p.tm_c, p.c, d.B, d.T, d.H, 128 * d.R, steps, true))
         return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs 16-byte aligned b and c");
-      if (d.rot && !m3::tc_make_row_map(&p.tm_th, p.theta, d.B, d.T, d.H, 64, steps, false))
+      if (d.rot && !m3::tc_make_row_map(&p.tm_th, p.theta, d.B, d.T, d.H, 64, steps, false, d.ths))
         return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs a 16-byte aligned theta");
       // y leaves by bulk tensor stores where it can (a 16-byte aligned tensor); by plain stores otherwise
       p.out_maps = m3::tc_make_row_map(&p.tm_y, p.y, d.B, d.T, d.H, 64 * d.R, steps, true) ? 1 : 0;

@@ -18,6 +18,7 @@ struct Dims {
   int LR;        // L * R rows per chunk
   int raw;       // 1: a, g, w come from the caller (the ssd_chunked form)
   int rev;       // the last `rev` heads walk time right to left (bidirectional mixer)
+  int ths;       // elements between consecutive tokens of theta and its gradient (a band of a wider row)
 };
 
 // Token-head index (row of a [B, T, H, ...] tensor) of scan position t of head h: heads that
@@ -25,6 +26,12 @@ struct Dims {
 __host__ __device__ __forceinline__ size_t tok_index(const Dims& d, int b, int t, int h) {
   const int tm = (h >= d.H - d.rev) ? d.T - 1 - t : t;
   return ((size_t)b * d.T + tm) * d.H + h;
+}
+
+// Where theta's (and d theta's) planes of that position start.
+__host__ __device__ __forceinline__ size_t theta_index(const Dims& d, int b, int t, int h) {
+  const int tm = (h >= d.H - d.rev) ? d.T - 1 - t : t;
+  return ((size_t)b * d.T + tm) * d.ths + (size_t)h * d.NH;
 }
 
 __device__ __forceinline__ float ldf(const float* p, size_t i) { return p[i]; }
@@ -54,6 +61,15 @@ __device__ __forceinline__ float lambda_at(const TIn* lam, int disc, size_t i) {
   if (disc == 1) return 0.5f;
   return ldf(lam, i);
 }
+
+// Activations of the mixer's steps.  Fast-math exponentials and divisions (2 ulp): the kernels that use them are
+// bound by instruction issue, and their results are rounded to the element type at once.
+__device__ __forceinline__ float softplus(float v) { return v > 20.0f ? v : log1pf(__expf(v)); }
+__device__ __forceinline__ float sigmoid(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
+
+// A float rounded to the element type, as storing and reading it back would.
+__device__ __forceinline__ float round_to(const float*, float v) { return v; }
+__device__ __forceinline__ float round_to(const __nv_bfloat16*, float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 // ---------------------------------------------------------------------------
 // 64x64 block GEMM on CUDA cores, 256 threads, 4x4 outputs per thread.

@@ -182,7 +182,7 @@ __global__ void kb_dstep(Dims d, const T* __restrict__ dt, const T* __restrict__
       bw.dphi[o] = run;  // dstep
       if (t < d.T && dtheta) {
         const size_t i = tok_index(d, b, t, h);
-        stf(dtheta, i * NH + m, run * ldf(dt, i));
+        stf(dtheta, theta_index(d, b, t, h) + m, run * ldf(dt, i));
       }
     }
   }
@@ -191,8 +191,8 @@ __global__ void kb_dstep(Dims d, const T* __restrict__ dt, const T* __restrict__
     const int t = t0 + l;
     float s = 0.0f;
     if (t < d.T) {
-      const size_t i = tok_index(d, b, t, h);
-      for (int m = 0; m < NH; ++m) s += bw.dphi[((size_t)bh * d.Tp + t) * NH + m] * ldf(theta, i * NH + m);
+      const size_t i = theta_index(d, b, t, h);
+      for (int m = 0; m < NH; ++m) s += bw.dphi[((size_t)bh * d.Tp + t) * NH + m] * ldf(theta, i + m);
     }
     bw.ddt_rot[(size_t)bh * d.Tp + t] = s;
   }

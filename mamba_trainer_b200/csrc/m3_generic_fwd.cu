@@ -21,7 +21,7 @@ __global__ void k_angle_sum(Dims d, const T* __restrict__ dt, const T* __restric
       const int t = k * d.L + l;
       if (t >= d.T) break;
       const size_t i = tok_index(d, b, t, h);
-      s += ldf(dt, i) * ldf(theta, i * d.NH + m);
+      s += ldf(dt, i) * ldf(theta, theta_index(d, b, t, h) + m);
     }
     abase[((size_t)bh * d.C + k) * d.NH + m] = s;
   }
@@ -99,8 +99,7 @@ __global__ void k_prep(Dims d, const T* __restrict__ x, const T* __restrict__ bm
         const int t = t0 + l;
         float ph = 0.0f;
         if (t < d.T) {
-          const size_t i = tok_index(d, b, t, h);
-          run += s_dt[l] * ldf(theta, i * d.NH + m);
+          run += s_dt[l] * ldf(theta, theta_index(d, b, t, h) + m);
           ph = wrap_angle(run);
           if (angle_out && t == d.T - 1) angle_out[(size_t)bh * d.NH + m] = ph;
         }

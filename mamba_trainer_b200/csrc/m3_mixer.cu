@@ -23,6 +23,8 @@
 namespace {
 
 using m3::ldf;
+using m3::sigmoid;
+using m3::softplus;
 using m3::stf;
 
 constexpr int kBcWarps = 8;      // warps per block
@@ -341,9 +343,6 @@ __global__ void __launch_bounds__(kBcWarps * 32)
 }
 
 // ---- dt / lambda ---------------------------------------------------------------------------------------
-__device__ __forceinline__ float softplus(float v) { return v > 20.0f ? v : log1pf(__expf(v)); }
-__device__ __forceinline__ float sigmoid(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
-
 template <class T>
 __global__ void k_act_fwd(int ntok, int H, long long stride, const T* __restrict__ dt_raw, const T* __restrict__ lam_raw,
                           const float* __restrict__ dt_bias, T* __restrict__ dt, T* __restrict__ lam) {

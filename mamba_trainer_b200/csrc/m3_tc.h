@@ -14,7 +14,7 @@ namespace m3 {
 inline bool tc_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 inline bool tc_supported(const m3_scan_desc& s) {
   return s.dtype == M3_BF16 && s.head_dim == 64 && s.d_state == 128 && (s.rank == 1 || s.rank == 2 || s.rank == 4) &&
-         s.seq > 0 && tc_aligned(s.x) && tc_aligned(s.b) && tc_aligned(s.c) && tc_aligned(s.theta);
+         s.seq > 0 && tc_aligned(s.x) && tc_aligned(s.b) && tc_aligned(s.c) && tc_aligned(s.theta) && s.theta_stride % 8 == 0;
 }
 // Time steps per 128-row tile and tiles per stripe.
 inline int tc_tile_steps(int rank) { return 128 / rank; }
@@ -34,7 +34,8 @@ bool tc_make_tile_map(CUtensorMap* map, const void* base, int B, int T, int H, i
 // either end of the sequence arriving as zeros.  With `swizzle` the 16-byte chunks of a panel row are
 // XOR-swizzled by row & 7 (the 128-byte swizzle; the panel must then start on a 1024-byte boundary).
 // cols a multiple of 64; needs a 16-byte aligned base.
-bool tc_make_row_map(CUtensorMap* map, const void* base, int B, int T, int H, int cols, int steps, bool swizzle);
+// `tok_stride`: elements between consecutive tokens (0: dense, H * cols; else a multiple of 8 for a band of a wider row).
+bool tc_make_row_map(CUtensorMap* map, const void* base, int B, int T, int H, int cols, int steps, bool swizzle, int tok_stride = 0);
 
 struct TcFwdParams {
   alignas(64) CUtensorMap tm_b, tm_c, tm_x;   // tile maps of the direct form when use_tma, else row maps of b and c
@@ -51,6 +52,7 @@ struct TcFwdParams {
   int* err;           // device flag set when a bounded wait gave up
   int B, T, H, R, disc;
   int rev;            // the last `rev` heads walk time right to left
+  int ths;            // elements between consecutive tokens of theta
   uint32_t wait_limit; // iteration limit of the bounded waits (m3_ctx_set_wait_limit)
   // time segments of a stripe (role-split kernel; work distribution in m3_tc_roles.cuh): nseg == 1 hands nothing over
   int nseg, tps, grid;
@@ -86,6 +88,7 @@ struct TcBwdParams {
   int* err;
   int B, T, H, R, disc;
   int rev;            // the last `rev` heads walk time right to left
+  int ths;            // elements between consecutive tokens of theta and d theta
   uint32_t wait_limit;
   int nseg, tps, grid;   // as in TcFwdParams; the gradient of the state and the running sum of d phi are handed over
   float *seg_state, *seg_angle;

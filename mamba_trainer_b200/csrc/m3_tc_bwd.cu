@@ -712,11 +712,14 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
       if (ROT) {
         constexpr int LQ = LT / 4, NV = 4 / R;  // NV: (time step, 8-plane group) items per thread
         const int q = tid >> 6, m = tid & 63;
+        // theta and d theta of scan step t0 + l (they may be column bands of a wider row)
+        const ptrdiff_t th_step = rev ? -(ptrdiff_t)p.ths : (ptrdiff_t)p.ths;
+        const ptrdiff_t th0 = (ptrdiff_t)((size_t)b * T + (rev ? T - 1 - t0 : t0)) * p.ths + (ptrdiff_t)h * kNH;
         uint4 thq[NV];  // theta of this thread's items of the vector pass below, requested early
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
           const int iv = tid + 256 * i, l = iv >> 3, mg = iv & 7;
-          thq[i] = (t0 + l < T) ? __ldg(reinterpret_cast<const uint4*>(p.theta + (tok0 + (size_t)l * Hs) * kNH + mg * 8))
+          thq[i] = (t0 + l < T) ? __ldg(reinterpret_cast<const uint4*>(p.theta + th0 + l * th_step + mg * 8))
                                 : make_uint4(0u, 0u, 0u, 0u);
         }
         float run = 0.0f, loc[R == 2 ? 1 : LQ];  // (not rank 2:) the quarter's running sums wait in registers
@@ -760,7 +763,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
           if (t0 + l < T && p.dtheta) {
             uint4 qv;
             qv.x = pack_bf16(o[0], o[1]); qv.y = pack_bf16(o[2], o[3]); qv.z = pack_bf16(o[4], o[5]); qv.w = pack_bf16(o[6], o[7]);
-            *reinterpret_cast<uint4*>(p.dtheta + (tok0 + (size_t)l * Hs) * kNH + mg * 8) = qv;
+            *reinterpret_cast<uint4*>(p.dtheta + th0 + l * th_step + mg * 8) = qv;
           }
 #pragma unroll
           for (int o_ = 1; o_ < 8; o_ <<= 1) prod += __shfl_xor_sync(0xffffffffu, prod, o_);

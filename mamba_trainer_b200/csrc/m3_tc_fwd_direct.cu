@@ -359,7 +359,7 @@ bool tc_make_tile_map(CUtensorMap* map, const void* base, int B, int T, int H, i
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool tc_make_row_map(CUtensorMap* map, const void* base, int B, int T, int H, int cols, int steps, bool swizzle) {
+bool tc_make_row_map(CUtensorMap* map, const void* base, int B, int T, int H, int cols, int steps, bool swizzle, int tok_stride) {
   typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -371,7 +371,8 @@ bool tc_make_row_map(CUtensorMap* map, const void* base, int B, int T, int H, in
   }();
   if (!encode || cols % 64 || steps < 1 || steps > 256 || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
   const cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)H, (cuuint64_t)T, (cuuint64_t)B};
-  const cuuint64_t strides[3] = {(cuuint64_t)cols * 2, (cuuint64_t)H * cols * 2, (cuuint64_t)T * H * cols * 2};
+  const cuuint64_t tok = tok_stride ? (cuuint64_t)tok_stride * 2 : (cuuint64_t)H * cols * 2;
+  const cuuint64_t strides[3] = {(cuuint64_t)cols * 2, tok, (cuuint64_t)T * tok};
   const cuuint32_t box[4] = {64, 1, (cuuint32_t)steps, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,

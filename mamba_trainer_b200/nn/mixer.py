@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes as C
 from dataclasses import dataclass
+from functools import cached_property
 from typing import Optional
 
 import torch
@@ -21,12 +22,23 @@ import torch
 from .. import _ffi
 from ..error import ConfigError, ShapeError, UnsupportedError
 from ..ssm.config import Discretization
-from ..ssm.scan import Context, ScanInputs, SsmState, _DTYPES, _Saved, mamba3_scan, mamba3_step
+from ..ssm.scan import Context, SsmState, _DTYPES, _Saved
 
 
 def _p(t: Optional[torch.Tensor], offset: int = 0):
     """Device address of element `offset` of t (None -> NULL)."""
     return C.c_void_p(t.data_ptr() + offset * t.element_size()) if t is not None else None
+
+
+def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """t as a dense float32 tensor outside the tape; itself when it is one already."""
+    if t is None or (t.dtype is torch.float32 and t.is_contiguous()):
+        return t
+    return t.detach().to(torch.float32).contiguous()
+
+
+# The parameters in the order of m3_mixer_desc.
+_PARAMS = ("conv_w", "conv_b", "dt_bias", "a_log", "d_skip", "b_bias", "c_bias", "norm_w", "post_norm_w")
 
 
 @dataclass(frozen=True)
@@ -40,31 +52,31 @@ class MixerShape:
     learned_lambda: bool = True
     rotational: bool = True
 
-    @property
+    @cached_property
     def n_groups(self) -> int:
         return self.groups or self.heads
 
-    @property
+    @cached_property
     def d_inner(self) -> int:
         return self.heads * self.head_dim * self.rank
 
-    @property
+    @cached_property
     def bc_width(self) -> int:
         return self.n_groups * self.d_state * self.rank
 
-    @property
+    @cached_property
     def lambda_width(self) -> int:
         return self.heads if self.learned_lambda else 0
 
-    @property
+    @cached_property
     def theta_width(self) -> int:
         return self.heads * self.d_state // 2 if self.rotational else 0
 
-    @property
+    @cached_property
     def conv_channels(self) -> int:
         return self.d_inner + 2 * self.bc_width
 
-    @property
+    @cached_property
     def in_proj_width(self) -> int:
         return 2 * self.d_inner + 2 * self.bc_width + self.heads + self.lambda_width + self.theta_width
 
@@ -243,80 +255,72 @@ class MixerCore(torch.nn.Module):
         # RmsNormConfig::new(d_inner) (mamba3.rs:245-247): a gain of ones over the scan's flattened output
         self.post_gate_norm = post_gate_norm
         self.post_norm_w = par(torch.ones(shape.d_inner)) if post_gate_norm else None
+        for name in _PARAMS:   # absent parameters are named all the same
+            if name not in self._parameters:
+                delattr(self, name)
+                self.register_parameter(name, None)
 
     def empty_cache(self, batch: int, device, dtype=torch.float32) -> MixerCache:
         s = self.shape
         return MixerCache(torch.zeros((batch, self.conv_w.shape[0] - 1, s.conv_channels), device=device, dtype=dtype),
                           SsmState.zeros(batch, s.heads, s.head_dim, s.d_state, s.rotational, device))
 
-    @torch.no_grad()
+    def _call_desc(self, proj: torch.Tensor, path: int = _ffi.PATH_AUTO):
+        """The library's description of this mixer on `proj` (m3_mixer_desc) and the tensors it points into."""
+        s = self.shape
+        B, T, _ = proj.shape
+        p = self._parameters
+        par = [_f32(p[n]) for n in _PARAMS]
+        desc = _ffi.PACK_MIXER_DESC.pack(
+            B, T, s.heads, s.head_dim, s.d_state, s.rank, s.n_groups, self.chunk, _DTYPES[proj.dtype], self.disc,
+            s.rotational, p["conv_w"].shape[0], self.use_norm, self.post_gate_norm, path,
+            s.heads // 2 if self.bidirectional else 0, self.eps, 0,
+            proj.data_ptr(), *[0 if t is None else t.data_ptr() for t in par])
+        return desc, par
+
     def forward_cached(self, proj: torch.Tensor, cache: Optional[MixerCache] = None):
         """Inference with a carried state (Mamba3Mixer::apply_with_state, src/models/mamba3.rs:486-560):
         a prefill window or a single decoding step.  Returns (gated output, new MixerCache).  A window
-        of one position runs the decode kernel (mamba3_step), longer ones the scan."""
+        of one position runs the decode kernel, longer ones the scan; either way it is one call of the library."""
         s = self.shape
         if proj.dim() != 3 or proj.shape[2] != s.in_proj_width:
             raise ShapeError(f"expected [batch, seq, {s.in_proj_width}], got {tuple(proj.shape)}")
         if self.bidirectional:
             raise UnsupportedError("a bidirectional mixer has no causal state to carry")   # mamba3.rs:494-499
-        proj = proj.contiguous()
-        ctx = Context.for_device(proj.device)
-        lib, hd = ctx.lib, ctx.handle
-        B, T, W = proj.shape
-        el, code, dev = proj.dtype, _DTYPES[proj.dtype], proj.device
-        H, P, N, R, G = s.heads, s.head_dim, s.d_state, s.rank, s.n_groups
-        di, bc = s.d_inner, s.bc_width
-        off_dt = 2 * di + 2 * bc
-        off_lam, off_th = off_dt + H, off_dt + H + s.lambda_width
+        proj = proj.detach() if proj.is_contiguous() else proj.detach().contiguous()
+        dev, el = proj.device, proj.dtype
+        ctx = Context.for_device(dev)
+        B, T, _ = proj.shape
+        H, P, N = s.heads, s.head_dim, s.d_state
         if cache is None:
             cache = self.empty_cache(B, dev, el)
-        f = lambda t: None if t is None else t.detach().to(torch.float32).contiguous()
-        conv_w, conv_b, dt_bias = f(self.conv_w), f(self.conv_b), f(self.dt_bias)
-        b_bias, c_bias, norm_w = f(self.b_bias), f(self.c_bias), f(self.norm_w)
-        new = lambda *shape: torch.empty(shape, device=dev, dtype=el)
-        K = conv_w.shape[0]
-        hist = cache.conv.to(el).contiguous()
-        x, bcr, new_hist = new(B, T, H, P, R), new(B, T, 2 * bc), new(B, K - 1, di + 2 * bc)
-        cdesc = _ffi.ConvDesc(batch=B, seq=T, channels=di + 2 * bc, kernel_size=K, dtype=code, activation=1,
-                              x_stride=W, y_stride=di, x=_p(proj, di), history=_p(hist), weight=_p(conv_w),
-                              bias=_p(conv_b), split=di, y2_stride=2 * bc, y2=_p(bcr), dy2=None)
-        ctx.check(lib.m3_conv_forward(hd, C.byref(cdesc), _p(x), _p(new_hist)))
-        b, c = new(B, T, H, N, R), new(B, T, H, N, R)
-        bdesc = _ffi.BcDesc(batch=B, seq=T, heads=H, groups=G, d_state=N, rank=R, dtype=code,
-                            has_norm=1 if self.use_norm else 0, eps=float(self.eps), raw_stride=2 * bc,
-                            b_raw=_p(bcr), c_raw=_p(bcr, bc), b_bias=_p(b_bias), c_bias=_p(c_bias), norm_weight=_p(norm_w))
-        ctx.check(lib.m3_bc_forward(hd, C.byref(bdesc), _p(b), _p(c)))
-        dt = new(B, T, H)
-        lam = new(B, T, H) if s.learned_lambda else None
-        adesc = _ffi.ActDesc(batch=B, seq=T, heads=H, dtype=code, stride=W, dt_raw=_p(proj, off_dt),
-                             lambda_raw=_p(proj, off_lam) if s.learned_lambda else None, dt_bias=_p(dt_bias))
-        ctx.check(lib.m3_dt_lambda_forward(hd, C.byref(adesc), _p(dt), _p(lam)))
-        theta = proj[..., off_th:off_th + s.theta_width].reshape(B, T, H, N // 2).contiguous() if s.rotational else None
-        if T == 1:
-            y, ssm = mamba3_step(x[:, 0], b[:, 0], c[:, 0], dt[:, 0], lam[:, 0] if lam is not None else None,
-                                 self.a_log, theta[:, 0] if theta is not None else None, self.d_skip, cache.ssm,
-                                 self.disc)
-            y = y.unsqueeze(1)
-        else:
-            inp = ScanInputs.new(x, b, c, dt, self.a_log.detach(), lam).with_chunk_size(self.chunk)
-            inp = inp.with_discretization(self.disc).with_state(cache.ssm).with_state_output(True)
-            if theta is not None:
-                inp = inp.with_theta(theta)
-            if self.d_skip is not None:
-                inp = inp.with_skip(self.d_skip.detach())
-            res = mamba3_scan(inp)
-            y, ssm = res.y, res.state
-        y = y.contiguous()
-        out = new(B, T, di)
-        if self.post_gate_norm:
-            post_w = f(self.post_norm_w)
-            gdesc = _ffi.GateNormDesc(batch=B, seq=T, channels=di, dtype=code, z_stride=W, y=_p(y), z=_p(proj),
-                                      weight=_p(post_w), eps=float(self.eps))
-            ctx.check(lib.m3_gate_norm_forward(hd, C.byref(gdesc), _p(out)))
-        else:
-            gdesc = _ffi.GateDesc(batch=B, seq=T, channels=di, dtype=code, z_stride=W, y=_p(y), z=_p(proj))
-            ctx.check(lib.m3_gate_forward(hd, C.byref(gdesc), _p(out)))
-        return out, MixerCache(new_hist, ssm)
+        st = cache.ssm
+        conv = cache.conv
+        if conv.dtype is not el or not conv.is_contiguous():
+            conv = conv.to(el).contiguous()
+        h, lu = _f32(st.h), _f32(st.last_u)
+        ang = _f32(st.angle) if s.rotational else None
+        K = self._parameters["conv_w"].shape[0]
+        if conv.shape != (B, K - 1, s.conv_channels):
+            raise ShapeError(f"the cache's convolution history has shape {tuple(conv.shape)}, expected "
+                             f"{(B, K - 1, s.conv_channels)}")
+        if h.shape != (B, H, P, N) or lu.shape != (B, H, P, N) or (ang is not None and ang.shape != (B, H, N // 2)):
+            raise ShapeError(f"the cache's state does not match batch {B}, heads {H}, head_dim {P}, d_state {N}")
+        desc, keep = self._call_desc(proj)
+        out = torch.empty((B, T, s.d_inner), device=dev, dtype=el)
+        conv2 = torch.empty_like(conv)
+        h2, lu2 = torch.empty_like(h), torch.empty_like(lu)
+        ang2 = torch.empty((B, H, N // 2), device=dev, dtype=torch.float32) if s.rotational else None
+        io = _ffi.PACK_MIXER_WINDOW_IO.pack(
+            conv.data_ptr(), h.data_ptr(), lu.data_ptr(), 0 if ang is None else ang.data_ptr(), out.data_ptr(),
+            conv2.data_ptr(), h2.data_ptr(), lu2.data_ptr(), 0 if ang2 is None else ang2.data_ptr())
+        lib = ctx.lib
+        n = lib.m3_mixer_window_bytes(desc, io)
+        work = torch.empty(n, device=dev, dtype=torch.uint8) if n else None
+        rc = lib.m3_mixer_window(ctx.handle, desc, io, work.data_ptr() if n else None)
+        if rc:
+            ctx.check(rc)
+        return out, MixerCache(conv2, SsmState(h2, lu2, ang2))
 
     def forward(self, proj: torch.Tensor, path: int = _ffi.PATH_AUTO) -> torch.Tensor:
         """proj: the input projection's output [batch, seq, in_proj_width]; returns the gated scan

@@ -20,6 +20,10 @@ from .. import _ffi
 from ..error import ConfigError, NullError, RankError, ShapeError, UnsupportedError, from_status
 from .config import Discretization
 
+# The handle of torch's current stream, without building a Stream object (this is on every call's path).
+_current_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+
 _DTYPES = {torch.float32: _ffi.F32, torch.bfloat16: _ffi.BF16}
 
 
@@ -50,7 +54,7 @@ class Context:
         return ctx
 
     def bind_current_stream(self) -> None:
-        stream = torch.cuda.current_stream(self.device_index).cuda_stream
+        stream = _current_stream(self.device_index)
         if stream != self._stream:
             self.check(self.lib.m3_ctx_set_stream(self.handle, C.c_void_p(stream)))
             self._stream = stream
