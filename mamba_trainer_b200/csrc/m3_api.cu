@@ -7,6 +7,7 @@
 #include <new>
 
 #include "m3_internal.h"
+#include "m3_rows.cuh"
 #include "m3_tc.h"
 
 struct m3_saved {
@@ -16,6 +17,8 @@ struct m3_saved {
   char* ws_base = nullptr;
   size_t ws_bytes = 0;
   m3::GenericWs gws;
+  bool rows = false;               // the chunk-parallel family ran: its scratch is in rws
+  m3::rows::RowsWs rws;
   __nv_bfloat16* tc_ckpt_h = nullptr;  // tensor-core family: bf16 state entering each tile
   float* tc_ckpt_angle = nullptr;  // and the angle entering each tile
   bool tc_direct = false;          // the forward ran the direct form: so does the backward (same tile maps)
@@ -263,6 +266,34 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
   return M3_OK;
 }
 
+// Backward of a forward that ran the chunk-parallel family.  Its kernels move dy and the gradients four elements at a
+// time; a buffer that is not aligned to that goes through an aligned copy.
+cudaError_t rows_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3::rows::RowsBwdWs& rw, const m3::GenericBwdWs& bw,
+                               m3_scan_bwd_in in, uint32_t mask, m3_scan_grads g) {
+  const m3_scan_desc& s = saved->desc;
+  const size_t es = s.dtype == M3_F32 ? 4 : 2, tok = (size_t)s.batch * s.seq * s.heads * s.rank * es;
+  struct { const void* user; size_t bytes; void** slot; char* copy; } buf[] = {
+      {in.dy, tok * s.head_dim, const_cast<void**>(&in.dy), nullptr}, {g.dx, tok * s.head_dim, &g.dx, nullptr},
+      {g.db, tok * s.d_state, &g.db, nullptr}, {g.dc, tok * s.d_state, &g.dc, nullptr}};
+  cudaError_t e = cudaSuccess;
+  for (auto& b : buf) {
+    if (!(reinterpret_cast<uintptr_t>(b.user) & (4 * es - 1)) || e != cudaSuccess) continue;
+    e = m3::scratch_alloc(ctx, reinterpret_cast<void**>(&b.copy), b.bytes, ctx->stream);
+    if (e == cudaSuccess && b.slot == buf[0].slot)
+      e = cudaMemcpyAsync(b.copy, b.user, b.bytes, cudaMemcpyDeviceToDevice, ctx->stream);
+    *b.slot = b.copy;
+  }
+  if (e == cudaSuccess) e = m3::rows_backward(ctx->stream, saved->dims, s, saved->rws, rw, bw, in, mask, g, &ctx->launches);
+  const uint32_t bit[] = {0, M3_GRAD_X, M3_GRAD_B, M3_GRAD_C};
+  for (int i = 0; i < 4; ++i) {
+    if (!buf[i].copy) continue;
+    if (e == cudaSuccess && (mask & bit[i]))
+      e = cudaMemcpyAsync(const_cast<void*>(buf[i].user), buf[i].copy, buf[i].bytes, cudaMemcpyDeviceToDevice, ctx->stream);
+    cudaFreeAsync(buf[i].copy, ctx->stream);
+  }
+  return e;
+}
+
 }  // namespace
 
 extern "C" {
@@ -508,12 +539,22 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     }
     return M3_OK;
   }
-  const size_t bytes = m3::generic_ws_layout(d, nullptr, nullptr);
+  // Float32 arithmetic: the chunk-parallel family for the shapes models have, the generic one for everything else.
+  const bool rows = m3::rows_supported(*desc, out->y);
+  if (rows) d = m3::rows_dims(d);
+  const size_t bytes = rows ? m3::rows_ws_layout(d, nullptr, nullptr) : m3::generic_ws_layout(d, nullptr, nullptr);
   char* base = nullptr;
   M3_CUDA(ctx, m3::scratch_alloc(ctx, reinterpret_cast<void**>(&base), bytes, ctx->stream));
-  m3::GenericWs ws;
-  m3::generic_ws_layout(d, &ws, base);
-  cudaError_t e = m3::generic_forward(ctx->stream, d, *desc, *out, ws, &ctx->launches);
+  m3::GenericWs ws{};
+  m3::rows::RowsWs rws{};
+  cudaError_t e;
+  if (rows) {
+    m3::rows_ws_layout(d, &rws, base);
+    e = m3::rows_forward(ctx->stream, d, *desc, *out, rws, &ctx->launches);
+  } else {
+    m3::generic_ws_layout(d, &ws, base);
+    e = m3::generic_forward(ctx->stream, d, *desc, *out, ws, &ctx->launches);
+  }
   if (e != cudaSuccess) {
     cudaFreeAsync(base, ctx->stream);
     return cuda_fail(ctx, e, "generic forward");
@@ -530,6 +571,8 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     sv->ws_base = base;
     sv->ws_bytes = bytes;
     sv->gws = ws;
+    sv->rows = rows;
+    sv->rws = rws;
     sv->stream = ctx->stream;
     *saved = sv;
   } else {
@@ -550,13 +593,19 @@ int m3_scan_backward(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
   M3_CUDA(ctx, cudaSetDevice(ctx->device));
   if (saved->path == M3_PATH_TENSOR) return tc_backward_call(ctx, saved, in, grad_mask, grads);
   const m3::Dims& d = saved->dims;
-  const size_t bytes = m3::generic_bwd_ws_layout(d, nullptr, nullptr);
+  const size_t bytes = saved->rows ? m3::rows_bwd_ws_layout(d, nullptr, nullptr, nullptr) : m3::generic_bwd_ws_layout(d, nullptr, nullptr);
   char* base = nullptr;
   M3_CUDA(ctx, m3::scratch_alloc(ctx, reinterpret_cast<void**>(&base), bytes, ctx->stream));
   m3::GenericBwdWs bw;
-  m3::generic_bwd_ws_layout(d, &bw, base);
-  cudaError_t e = m3::generic_backward(ctx->stream, d, saved->desc, saved->gws, bw, *in, grad_mask, *grads,
-                                       &ctx->launches);
+  cudaError_t e;
+  if (saved->rows) {
+    m3::rows::RowsBwdWs rw;
+    m3::rows_bwd_ws_layout(d, &rw, &bw, base);
+    e = rows_backward_call(ctx, saved, rw, bw, *in, grad_mask, *grads);
+  } else {
+    m3::generic_bwd_ws_layout(d, &bw, base);
+    e = m3::generic_backward(ctx->stream, d, saved->desc, saved->gws, bw, *in, grad_mask, *grads, &ctx->launches);
+  }
   cudaError_t e2 = cudaFreeAsync(base, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "generic backward");
   if (e2 != cudaSuccess) return cuda_fail(ctx, e2, "cudaFreeAsync");

@@ -111,24 +111,28 @@ static cudaError_t backward_t(cudaStream_t st, const Dims& d, const m3_scan_desc
   return cudaGetLastError();
 }
 
-// The last two launches of any backward: per-token d dt / d lambda from (da, dg, dw, the
-// rotation term, the seed-state term) and the per-head reductions.  `d.Tp` and `d.C` give the
-// pitch of the per-token arrays and the number of partial sums per (batch, head).
-cudaError_t finalize_scalars(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const GenericBwdWs& bw,
-                             void* ddt, void* dlam, float* dalog, float* ddsk, uint64_t* launches) {
+// The last two launches of any backward: per-token d dt / d lambda from (da, dg, dw, the rotation term, the
+// seed-state term) - or, for the a / g / w form, da, dg, dw as they are - and the per-head reductions.  `d.Tp` and
+// `d.C` give the pitch of the per-token arrays and the number of partial sums per (batch, head).  `tokens` false: the
+// per-token part has been done.
+template <class T>
+static void final_tokens(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const GenericBwdWs& bw, void* ddt, void* dlam,
+                         const m3_scan_grads* raw) {
   const size_t total = (size_t)d.B * d.T * d.H;
-  const unsigned grid = (unsigned)((total + 255) / 256);
-  const int has_state = desc.h0 ? 1 : 0;
-  if (desc.dtype == M3_BF16) {
-    using T = __nv_bfloat16;
-    kb_final<T><<<grid, 256, 0, st>>>(d, static_cast<const T*>(desc.dt), static_cast<const T*>(desc.lambda), desc.a_log,
-                                      bw, has_state, static_cast<T*>(ddt), static_cast<T*>(dlam), nullptr, nullptr, nullptr);
-  } else {
-    kb_final<float><<<grid, 256, 0, st>>>(d, static_cast<const float*>(desc.dt), static_cast<const float*>(desc.lambda),
-                                          desc.a_log, bw, has_state, static_cast<float*>(ddt), static_cast<float*>(dlam),
-                                          nullptr, nullptr, nullptr);
+  kb_final<T><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
+      d, static_cast<const T*>(desc.dt), static_cast<const T*>(desc.lambda), desc.a_log, bw, (desc.h0 && !d.raw) ? 1 : 0,
+      static_cast<T*>(ddt), static_cast<T*>(dlam), raw ? static_cast<T*>(raw->da_raw) : nullptr,
+      raw ? static_cast<T*>(raw->dg_raw) : nullptr, raw ? static_cast<T*>(raw->dw_raw) : nullptr);
+}
+cudaError_t finalize_scalars(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const GenericBwdWs& bw,
+                             void* ddt, void* dlam, float* dalog, float* ddsk, uint64_t* launches, bool tokens,
+                             const m3_scan_grads* raw) {
+  uint64_t n = 0;
+  if (tokens) {
+    if (desc.dtype == M3_BF16) final_tokens<__nv_bfloat16>(st, d, desc, bw, ddt, dlam, raw);
+    else final_tokens<float>(st, d, desc, bw, ddt, dlam, raw);
+    n += 1;
   }
-  uint64_t n = 1;
   if (dalog || ddsk) {
     kb_reduce_heads<<<d.H, 256, 0, st>>>(d, desc.a_log, bw, dalog, ddsk);
     n += 1;

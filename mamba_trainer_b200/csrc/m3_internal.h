@@ -88,7 +88,8 @@ cudaError_t generic_backward(cudaStream_t st, const Dims& d, const m3_scan_desc&
                              const m3_scan_grads& grads, uint64_t* launches);
 
 cudaError_t finalize_scalars(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const GenericBwdWs& bw,
-                             void* ddt, void* dlam, float* dalog, float* ddsk, uint64_t* launches);
+                             void* ddt, void* dlam, float* dalog, float* ddsk, uint64_t* launches, bool tokens = true,
+                             const m3_scan_grads* raw = nullptr);
 
 // out[g][c] (+)= sum_{t < nterms} part[g * part_group_stride + t * stride + c] for c < ncols, g < groups;
 // fixed summation order (see m3_reduce.cu).

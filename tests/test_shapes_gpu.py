@@ -37,3 +37,58 @@ def test_decode_step_matches_the_parallel_pass(dtype, B, H, P, N, R, groups, K, 
         outs.append(o)
     got = torch.cat(outs, 1)
     assert ref_metric(got.float(), whole.float()) <= (2e-4 if dtype == torch.float32 else 3e-2)
+
+
+@pytest.mark.parametrize("dtype,B,T,H,N,R,rot,state,rev,disc", [
+    (torch.float32, 2, 64, 2, 128, 1, True, False, 0, 2),     # exactly one chunk
+    (torch.float32, 1, 1, 3, 64, 1, True, True, 0, 2),        # one token
+    (torch.float32, 1, 65, 2, 64, 1, False, True, 0, 2),      # one token past a chunk
+    (torch.float32, 2, 321, 2, 128, 2, True, True, 1, 2),     # ragged, a right-to-left head, carried state
+    (torch.float32, 1, 150, 2, 128, 4, True, False, 0, 1),
+    (torch.float32, 1, 77, 2, 64, 4, False, True, 2, 0),
+    (torch.bfloat16, 2, 200, 3, 64, 1, True, True, 0, 2),
+    (torch.bfloat16, 1, 333, 2, 64, 2, False, False, 1, 2),
+    (torch.bfloat16, 1, 90, 2, 64, 4, True, True, 0, 2),
+])
+def test_chunk_parallel_family_matches_the_oracle(dtype, B, T, H, N, R, rot, state, rev, disc):
+    """Outputs, states and every gradient against the float64 oracle: float32 as tight as the generic family's
+    tests, bf16 at 2e-2 (float32 arithmetic on bf16 inputs, so only inputs and outputs are rounded)."""
+    from test_scan_gpu import check_bf16, check_f32, compare_all, small_inputs
+    t, ds = small_inputs(B, T, H, 64, N, R, rot, state, seed=T + N + R)
+    d = Discretization(disc)
+    if d is not Discretization.LearnedTrapezoid:
+        t["lam"] = torch.full_like(t["lam"], d.fixed_lambda())
+    for k in ("b", "c"):
+        t[k] = t[k] / N ** 0.5
+    for k in ("x", "b", "c", "dt", "lam", "theta", "dy"):
+        if t[k] is not None:
+            t[k] = t[k].to(dtype)
+    compare_all(t, 64, check_f32 if dtype == torch.float32 else check_bf16, True, ds, discretization=d, reverse_heads=rev)
+
+
+def test_chunk_parallel_backward_takes_unaligned_gradients():
+    """dy and the gradient buffers of the C ABI may start anywhere; aligned ones give the same bits."""
+    import ctypes as C
+    from mamba_trainer_b200 import _ffi, synthetic
+    from mamba_trainer_b200.ssm import Context
+    w = synthetic.WORKLOADS[0].scaled(batch=1, heads=2, seq=100)
+    t = {k: v.cuda() if v is not None else None for k, v in synthetic.make_inputs(w, seed=3).items()}
+    ctx = Context.for_device(torch.device("cuda"))
+    p = lambda v: C.c_void_p(v.data_ptr()) if v is not None else None
+    desc = _ffi.ScanDesc(batch=1, seq=100, heads=2, head_dim=64, d_state=64, rank=1, chunk=64, dtype=_ffi.F32,
+                         discretization=2, x=p(t["x"]), b=p(t["b"]), c=p(t["c"]), dt=p(t["dt"]), lambda_=p(t["lam"]),
+                         a_log=p(t["a_log"]), d_skip=p(t["d_skip"]))
+    y, saved = torch.empty_like(t["x"]), C.c_void_p()
+    out = _ffi.ScanOut(y=p(y))
+    ctx.check(ctx.lib.m3_scan_forward(ctx.handle, C.byref(desc), C.byref(out), C.byref(saved)))
+    got = []
+    for off in (0, 1):
+        at = lambda v: torch.empty(v.numel() + 8, device="cuda")[off:off + v.numel()].view_as(v)
+        dy, dx, db, dc = at(t["dy"]), at(t["x"]), at(t["b"]), at(t["c"])
+        dy.copy_(t["dy"])
+        g = _ffi.ScanGrads(dx=p(dx), db=p(db), dc=p(dc))
+        ctx.check(ctx.lib.m3_scan_backward(ctx.handle, saved, C.byref(_ffi.ScanBwdIn(dy=p(dy))), _ffi.GRAD_ALL, C.byref(g)))
+        got.append((dx, db, dc))
+    ctx.check(ctx.lib.m3_saved_free(ctx.handle, saved))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
