@@ -338,6 +338,22 @@ pub struct m3_mixer_window_io {
     pub angle_out: *mut f32,
 }
 
+/// Gradients of a mixer pass: like the parameters, NULL where a parameter is absent.
+#[repr(C)]
+#[derive(Clone, Copy)]
+pub struct m3_mixer_grads {
+    pub dproj: *mut c_void,
+    pub dconv_weight: *mut f32,
+    pub dconv_bias: *mut f32,
+    pub ddt_bias: *mut f32,
+    pub da_log: *mut f32,
+    pub dd_skip: *mut f32,
+    pub db_bias: *mut f32,
+    pub dc_bias: *mut f32,
+    pub dnorm_weight: *mut f32,
+    pub dpost_weight: *mut f32,
+}
+
 extern "C" {
     pub fn m3_version() -> *const c_char;
 
@@ -403,4 +419,13 @@ extern "C" {
     pub fn m3_mixer_window_bytes(desc: *const m3_mixer_desc, io: *const m3_mixer_window_io) -> usize;
     pub fn m3_mixer_window(ctx: *mut m3_ctx, desc: *const m3_mixer_desc, io: *const m3_mixer_window_io,
                            workspace: *mut c_void) -> c_int;
+
+    /// Mamba3Mixer::project / finish around mamba3_scan: one training pass and its adjoint.
+    pub fn m3_mixer_activation_bytes(desc: *const m3_mixer_desc) -> usize;
+    pub fn m3_mixer_backward_bytes(desc: *const m3_mixer_desc) -> usize;
+    pub fn m3_mixer_forward(ctx: *mut m3_ctx, desc: *const m3_mixer_desc, out: *mut c_void, activations: *mut c_void,
+                            saved: *mut *mut m3_saved) -> c_int;
+    pub fn m3_mixer_backward(ctx: *mut m3_ctx, desc: *const m3_mixer_desc, saved: *const m3_saved,
+                             activations: *const c_void, dout: *const c_void, grads: *const m3_mixer_grads,
+                             workspace: *mut c_void) -> c_int;
 }

@@ -415,6 +415,21 @@ typedef struct {
 size_t m3_mixer_window_bytes(const m3_mixer_desc *desc, const m3_mixer_window_io *io);
 int m3_mixer_window(m3_ctx *ctx, const m3_mixer_desc *desc, const m3_mixer_window_io *io, void *workspace);
 
+/* One training pass of the mixer: forward_pass on its input projection's output, and its adjoint.  `activations`
+ * (m3_mixer_activation_bytes bytes of device memory, 256-byte aligned) receives what the backward pass needs besides
+ * proj and the parameters; keep all of them unchanged until then.  `saved` may be NULL (inference); otherwise it
+ * receives the scan's handle, freed with m3_saved_free.  The backward pass may run more than once; `workspace` holds
+ * m3_mixer_backward_bytes bytes for the span of the call. */
+typedef struct {
+  void *dproj;                /* like proj: every band of it is written */
+  float *dconv_weight, *dconv_bias, *ddt_bias, *da_log, *dd_skip, *db_bias, *dc_bias, *dnorm_weight, *dpost_weight;
+} m3_mixer_grads;             /* like the parameters; NULL where the parameter is absent */
+size_t m3_mixer_activation_bytes(const m3_mixer_desc *desc);
+size_t m3_mixer_backward_bytes(const m3_mixer_desc *desc);
+int m3_mixer_forward(m3_ctx *ctx, const m3_mixer_desc *desc, void *out, void *activations, m3_saved **saved);
+int m3_mixer_backward(m3_ctx *ctx, const m3_mixer_desc *desc, const m3_saved *saved, const void *activations,
+                      const void *dout, const m3_mixer_grads *grads, void *workspace);
+
 /* Bytes of device scratch a forward with this descriptor allocates (kept until
  * m3_saved_free when `saved` is requested). */
 size_t m3_scan_scratch_bytes(const m3_scan_desc *desc, int for_backward);

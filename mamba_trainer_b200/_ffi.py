@@ -98,10 +98,16 @@ class MixerWindowIo(C.Structure):
                                           "last_u_out", "angle_out")]
 
 
+class MixerGrads(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("dproj", "dconv_weight", "dconv_bias", "ddt_bias", "da_log", "dd_skip", "db_bias",
+                                          "dc_bias", "dnorm_weight", "dpost_weight")]
+
+
 # The mixer calls sit on latency-bound paths, where filling a ctypes structure field by field is a large part of
 # the call: these lay the same bytes out in one pack (0 for a NULL pointer).
 PACK_MIXER_DESC = struct.Struct("@16ifi10P")
 PACK_MIXER_WINDOW_IO = struct.Struct("@9P")
+PACK_MIXER_GRADS = struct.Struct("@10P")
 
 
 class HostIn(C.Structure):
@@ -145,6 +151,10 @@ SYMBOLS = {
     "m3_gate_norm_backward": (C.c_int, [C.c_void_p, C.POINTER(GateNormDesc), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "m3_mixer_window_bytes": (C.c_size_t, [C.c_char_p, C.c_char_p]),
     "m3_mixer_window": (C.c_int, [C.c_void_p, C.c_char_p, C.c_char_p, C.c_void_p]),
+    "m3_mixer_activation_bytes": (C.c_size_t, [C.c_char_p]),
+    "m3_mixer_backward_bytes": (C.c_size_t, [C.c_char_p]),
+    "m3_mixer_forward": (C.c_int, [C.c_void_p, C.c_char_p, C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p)]),
+    "m3_mixer_backward": (C.c_int, [C.c_void_p, C.c_char_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_char_p, C.c_void_p]),
     "m3_host_alloc": (C.c_int, [C.c_size_t, C.POINTER(C.c_void_p)]),
     "m3_host_free": (C.c_int, [C.c_void_p]),
     "m3_host_pipe_create": (C.c_int, [C.c_void_p, C.POINTER(ScanDesc), C.c_int, C.POINTER(C.c_void_p)]),

@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include "m3_internal.h"
+#include "m3_rows.cuh"
 #include "m3_tc.h"
 
 namespace {
@@ -63,7 +64,9 @@ extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, co
   }
   if (ctx->device < 0 || ctx->device >= kMaxDevices)
     return m3::fail(ctx, M3_ERR_UNSUPPORTED, "device ordinal %d outside the table of %d", ctx->device, kMaxDevices);
-  const size_t need = m3::generic_ws_layout(d, nullptr, nullptr);
+  const bool rows = m3::rows_supported(*desc, out->y);
+  if (rows) d = m3::rows_dims(d);
+  const size_t need = rows ? m3::rows_ws_layout(d, nullptr, nullptr) : m3::generic_ws_layout(d, nullptr, nullptr);
   if (need > (size_t)M3_NOALLOC_SCRATCH_BYTES)
     return m3::fail(ctx, M3_ERR_UNSUPPORTED,
                     "this scan needs %zu bytes of scratch; the built-in block holds %zu - use m3_scan_forward",
@@ -73,12 +76,18 @@ extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, co
   char* base = nullptr;
   e = scratch_address(ctx->device, &base);
   if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "cudaGetSymbolAddress");
-  m3::GenericWs ws;
-  m3::generic_ws_layout(d, &ws, base);
   // Every scratch region is written in full before it is read (padded rows are stored
   // as zeros, every chunk-state slot is produced by the chunk kernels), so nothing left
   // behind by the previous call needs clearing.
-  e = m3::generic_forward(ctx->stream, d, *desc, *out, ws, &ctx->launches);
+  if (rows) {
+    m3::rows::RowsWs ws;
+    m3::rows_ws_layout(d, &ws, base);
+    e = m3::rows_forward(ctx->stream, d, *desc, *out, ws, &ctx->launches);
+  } else {
+    m3::GenericWs ws;
+    m3::generic_ws_layout(d, &ws, base);
+    e = m3::generic_forward(ctx->stream, d, *desc, *out, ws, &ctx->launches);
+  }
   if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "forward on built-in scratch");
   return M3_OK;
 }

@@ -1,4 +1,4 @@
-"""The stretch of the Mamba-3 mixer between its input and output projections, as seven launches.
+"""The stretch of the Mamba-3 mixer between its input and output projections, as one call of the library each way.
 
 Mirrors Mamba3Mixer::project + mamba3_scan + finish of the reference (src/models/mamba3.rs:340-461,
 :475-484, :540-556; one direction or bidirectional, with or without post_gate_norm): the projection's output
@@ -8,7 +8,7 @@ column bands of it and the backward pass writes the bands of one gradient buffer
     convolution + SiLU over x|B|C  ->  B/C bias + RMS norm + layout  ->  softplus / sigmoid
     ->  scan  ->  y * silu(z)        (rms_norm(y) * gain * silu(z) with post_gate_norm)
 
-Every step runs in libm3scan; the node's backward calls the matching adjoints in reverse order.
+Every step runs in libm3scan (m3_mixer_forward, m3_mixer_backward, m3_mixer_window), which enqueues the whole stretch.
 """
 from __future__ import annotations
 
@@ -23,11 +23,6 @@ from .. import _ffi
 from ..error import ConfigError, ShapeError, UnsupportedError
 from ..ssm.config import Discretization
 from ..ssm.scan import Context, SsmState, _DTYPES, _Saved
-
-
-def _p(t: Optional[torch.Tensor], offset: int = 0):
-    """Device address of element `offset` of t (None -> NULL)."""
-    return C.c_void_p(t.data_ptr() + offset * t.element_size()) if t is not None else None
 
 
 def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -90,132 +85,44 @@ class MixerCache:
 
 
 class _MixerCore(torch.autograd.Function):
+    """The node: forward = m3_mixer_forward, backward rule = m3_mixer_backward.  `o` is the m3_mixer_desc of the call with
+    the gated output's width; the tensors it points into are the other arguments (float32, dense)."""
+
     @staticmethod
-    def forward(fctx, o, proj, conv_w, conv_b, dt_bias, a_log, d_skip, b_bias, c_bias, norm_w, post_w):
-        s: MixerShape = o["shape"]
+    def forward(fctx, o, proj, *par):
+        desc, width = o
         ctx = Context.for_device(proj.device)
-        lib, hd = ctx.lib, ctx.handle
-        B, T, W = proj.shape
-        el, dt_code = proj.dtype, _DTYPES[proj.dtype]
-        H, P, N, R, G = s.heads, s.head_dim, s.d_state, s.rank, s.n_groups
-        di, bc = s.d_inner, s.bc_width
-        off_x, off_dt = di, 2 * di + 2 * bc
-        off_lam, off_th = off_dt + H, off_dt + H + s.lambda_width
-        dev = proj.device
-        new = lambda *shape: torch.empty(shape, device=dev, dtype=el)
-        # 1. convolution + SiLU over x | B C, cut into two dense results
-        x, bcr = new(B, T, H, P, R), new(B, T, 2 * bc)
-        K = conv_w.shape[0]
-        cdesc = _ffi.ConvDesc(batch=B, seq=T, channels=di + 2 * bc, kernel_size=K, dtype=dt_code, activation=1,
-                              x_stride=W, y_stride=di, x=_p(proj, off_x), history=None, weight=_p(conv_w),
-                              bias=_p(conv_b), split=di, y2_stride=2 * bc, y2=_p(bcr), dy2=None)
-        if o["reverse_heads"]:
-            # direction-major bands (mamba3.rs:352-370): the second half of x, of B and of C belongs to
-            # the heads that walk right to left; their convolution runs right to left as well
-            cdesc.n_reversed = 3
-            for i, (lo, hi) in enumerate(((di // 2, di), (di + bc // 2, di + bc), (di + bc + bc // 2, di + 2 * bc))):
-                cdesc.reversed_lo[i], cdesc.reversed_hi[i] = lo, hi
-        ctx.check(lib.m3_conv_forward(hd, C.byref(cdesc), _p(x), None))
-        # 2. B / C: groups -> heads, bias, RMS norm, rank last
-        b, c = new(B, T, H, N, R), new(B, T, H, N, R)
-        bdesc = _ffi.BcDesc(batch=B, seq=T, heads=H, groups=G, d_state=N, rank=R, dtype=dt_code,
-                            has_norm=1 if o["norm"] else 0, eps=float(o["eps"]), raw_stride=2 * bc,
-                            b_raw=_p(bcr), c_raw=_p(bcr, bc), b_bias=_p(b_bias), c_bias=_p(c_bias),
-                            norm_weight=_p(norm_w))
-        ctx.check(lib.m3_bc_forward(hd, C.byref(bdesc), _p(b), _p(c)))
-        # 3. dt, lambda
-        dt = new(B, T, H)
-        lam = new(B, T, H) if s.learned_lambda else None
-        adesc = _ffi.ActDesc(batch=B, seq=T, heads=H, dtype=dt_code, stride=W, dt_raw=_p(proj, off_dt),
-                             lambda_raw=_p(proj, off_lam) if s.learned_lambda else None, dt_bias=_p(dt_bias))
-        ctx.check(lib.m3_dt_lambda_forward(hd, C.byref(adesc), _p(dt), _p(lam)))
-        # 4. scan (theta is read in place: a band of the projection is not dense, so it is copied once)
-        theta = proj[..., off_th:off_th + s.theta_width].reshape(B, T, H, N // 2).contiguous() if s.rotational else None
-        y = new(B, T, H, P, R)
-        sdesc = _ffi.ScanDesc(batch=B, seq=T, heads=H, head_dim=P, d_state=N, rank=R, chunk=int(o["chunk"]),
-                              dtype=dt_code, discretization=int(o["disc"]), dynamics=1 if s.rotational else 0,
-                              want_state=0, path=int(o["path"]), reverse_heads=int(o["reverse_heads"]),
-                              x=_p(x), b=_p(b), c=_p(c), dt=_p(dt), lambda_=_p(lam), theta=_p(theta),
-                              a_log=_p(a_log), d_skip=_p(d_skip))
-        sout = _ffi.ScanOut(y=_p(y))
+        lib = ctx.lib
+        B, T, _ = proj.shape
+        out = torch.empty((B, T, width), device=proj.device, dtype=proj.dtype)
+        act = torch.empty(lib.m3_mixer_activation_bytes(desc), device=proj.device, dtype=torch.uint8)
         track = any(fctx.needs_input_grad)
         saved = C.c_void_p()
-        ctx.check(lib.m3_scan_forward(hd, C.byref(sdesc), C.byref(sout), C.byref(saved) if track else None))
-        # 5. gate
-        out = new(B, T, di)
-        if o["post_norm"]:
-            gdesc = _ffi.GateNormDesc(batch=B, seq=T, channels=di, dtype=dt_code, z_stride=W, y=_p(y), z=_p(proj),
-                                      weight=_p(post_w), eps=float(o["eps"]))
-            ctx.check(lib.m3_gate_norm_forward(hd, C.byref(gdesc), _p(out)))
-        else:
-            gdesc = _ffi.GateDesc(batch=B, seq=T, channels=di, dtype=dt_code, z_stride=W, y=_p(y), z=_p(proj))
-            ctx.check(lib.m3_gate_forward(hd, C.byref(gdesc), _p(out)))
+        rc = lib.m3_mixer_forward(ctx.handle, desc, out.data_ptr(), act.data_ptr(), C.byref(saved) if track else None)
+        if rc:
+            ctx.check(rc)
         if track:
-            fctx.o, fctx.m3 = o, ctx
+            fctx.m3, fctx.desc = ctx, desc
             fctx.saved = _Saved(ctx, saved)
-            fctx.descs = (cdesc, bdesc, adesc, sdesc, gdesc)
-            fctx.keep = (proj, conv_w, conv_b, dt_bias, a_log, d_skip, b_bias, c_bias, norm_w, x, bcr, b, c, dt, lam, theta, y, post_w)
+            fctx.keep = (proj, act) + par
         return out
 
     @staticmethod
     def backward(fctx, dout):
-        o, ctx = fctx.o, fctx.m3
-        s: MixerShape = o["shape"]
-        lib, hd = ctx.lib, ctx.handle
+        ctx, desc = fctx.m3, fctx.desc
         ctx.bind_current_stream()
-        cdesc, bdesc, adesc, sdesc, gdesc = fctx.descs
-        proj, conv_w, conv_b, dt_bias, a_log, d_skip, b_bias, c_bias, norm_w, x, bcr, b, c, dt, lam, theta, y, post_w = fctx.keep
-        B, T, W = proj.shape
-        H, P, N, R = s.heads, s.head_dim, s.d_state, s.rank
-        di, bc = s.d_inner, s.bc_width
-        off_x, off_dt = di, 2 * di + 2 * bc
-        off_lam, off_th = off_dt + H, off_dt + H + s.lambda_width
-        dev, el = proj.device, proj.dtype
-        new = lambda *shape: torch.empty(shape, device=dev, dtype=el)
-        f32 = lambda *shape: torch.empty(shape, device=dev, dtype=torch.float32)
-        dproj = new(B, T, W)            # every band is written exactly once below
+        proj, act = fctx.keep[:2]
+        dev = proj.device
         dout = dout.contiguous()
-        # 5'. gate: dy (dense) and dz (band 0 of dproj)
-        dy = new(B, T, H, P, R)
-        dpost = None
-        if o["post_norm"]:
-            dpost = f32(di) if post_w is not None else None
-            ctx.check(lib.m3_gate_norm_backward(hd, C.byref(gdesc), _p(dout), _p(dy), _p(dproj), _p(dpost)))
-        else:
-            ctx.check(lib.m3_gate_backward(hd, C.byref(gdesc), _p(dout), _p(dy), _p(dproj)))
-        # 4'. scan
-        dx, db, dc, ddt = new(B, T, H, P, R), new(B, T, H, N, R), new(B, T, H, N, R), new(B, T, H)
-        dlam = new(B, T, H) if s.learned_lambda else None
-        dtheta = new(B, T, H, N // 2) if s.rotational else None
-        da_log, dd_skip = f32(H), (f32(H) if d_skip is not None else None)
-        grads = _ffi.ScanGrads(dx=_p(dx), db=_p(db), dc=_p(dc), ddt=_p(ddt), dlambda=_p(dlam), dtheta=_p(dtheta),
-                               da_log=_p(da_log), dd_skip=_p(dd_skip))
-        mask = _ffi.GRAD_X | _ffi.GRAD_B | _ffi.GRAD_C | _ffi.GRAD_DT | _ffi.GRAD_A_LOG
-        mask |= _ffi.GRAD_LAMBDA if s.learned_lambda else 0
-        mask |= _ffi.GRAD_THETA if s.rotational else 0
-        mask |= _ffi.GRAD_D_SKIP if d_skip is not None else 0
-        bin_ = _ffi.ScanBwdIn(dy=_p(dy))
-        ctx.check(lib.m3_scan_backward(hd, fctx.saved.handle, C.byref(bin_), mask, C.byref(grads)))
-        if s.rotational:
-            dproj[..., off_th:off_th + s.theta_width].copy_(dtheta.reshape(B, T, s.theta_width))
-        # 3'. dt, lambda -> their bands of dproj
-        ddt_bias = f32(H)
-        ctx.check(lib.m3_dt_lambda_backward(hd, C.byref(adesc), _p(ddt), _p(dlam), _p(dproj, off_dt),
-                                            _p(dproj, off_lam) if s.learned_lambda else None, _p(ddt_bias)))
-        # 2'. B / C -> gradient of the convolution's second result
-        dbcr = new(B, T, 2 * bc)
-        db_bias = f32(H, N) if b_bias is not None else None
-        dc_bias = f32(H, N) if c_bias is not None else None
-        dnorm = f32(N) if (norm_w is not None and o["norm"]) else None
-        ctx.check(lib.m3_bc_backward(hd, C.byref(bdesc), _p(db), _p(dc), _p(dbcr), _p(dbcr, bc), _p(db_bias),
-                                     _p(dc_bias), _p(dnorm)))
-        # 1'. convolution -> the x|B|C band of dproj
-        K = conv_w.shape[0]
-        dconv_w = f32(K, di + 2 * bc)
-        dconv_b = f32(di + 2 * bc) if conv_b is not None else None
-        cdesc.dy2 = _p(dbcr)
-        ctx.check(lib.m3_conv_backward(hd, C.byref(cdesc), _p(dx), _p(dproj, off_x), _p(dconv_w), _p(dconv_b), None))
-        return (None, dproj, dconv_w, dconv_b, ddt_bias, da_log, dd_skip, db_bias, dc_bias, dnorm, dpost)
+        dproj = torch.empty_like(proj)
+        grads = [None if t is None else torch.empty_like(t) for t in fctx.keep[2:]]
+        work = torch.empty(ctx.lib.m3_mixer_backward_bytes(desc), device=dev, dtype=torch.uint8)
+        rc = ctx.lib.m3_mixer_backward(
+            ctx.handle, desc, fctx.saved.handle, act.data_ptr(), dout.data_ptr(),
+            _ffi.PACK_MIXER_GRADS.pack(dproj.data_ptr(), *[0 if t is None else t.data_ptr() for t in grads]), work.data_ptr())
+        if rc:
+            ctx.check(rc)
+        return (None, dproj, *grads)
 
 
 class MixerCore(torch.nn.Module):
@@ -265,18 +172,15 @@ class MixerCore(torch.nn.Module):
         return MixerCache(torch.zeros((batch, self.conv_w.shape[0] - 1, s.conv_channels), device=device, dtype=dtype),
                           SsmState.zeros(batch, s.heads, s.head_dim, s.d_state, s.rotational, device))
 
-    def _call_desc(self, proj: torch.Tensor, path: int = _ffi.PATH_AUTO):
-        """The library's description of this mixer on `proj` (m3_mixer_desc) and the tensors it points into."""
+    def _pack_desc(self, proj: torch.Tensor, par, path: int = _ffi.PATH_AUTO) -> bytes:
+        """The library's description (m3_mixer_desc) of this mixer on `proj`, with parameters `par` (in _PARAMS' order)."""
         s = self.shape
         B, T, _ = proj.shape
-        p = self._parameters
-        par = [_f32(p[n]) for n in _PARAMS]
-        desc = _ffi.PACK_MIXER_DESC.pack(
+        return _ffi.PACK_MIXER_DESC.pack(
             B, T, s.heads, s.head_dim, s.d_state, s.rank, s.n_groups, self.chunk, _DTYPES[proj.dtype], self.disc,
-            s.rotational, p["conv_w"].shape[0], self.use_norm, self.post_gate_norm, path,
+            s.rotational, self._parameters["conv_w"].shape[0], self.use_norm, self.post_gate_norm, path,
             s.heads // 2 if self.bidirectional else 0, self.eps, 0,
             proj.data_ptr(), *[0 if t is None else t.data_ptr() for t in par])
-        return desc, par
 
     def forward_cached(self, proj: torch.Tensor, cache: Optional[MixerCache] = None):
         """Inference with a carried state (Mamba3Mixer::apply_with_state, src/models/mamba3.rs:486-560):
@@ -306,7 +210,8 @@ class MixerCore(torch.nn.Module):
                              f"{(B, K - 1, s.conv_channels)}")
         if h.shape != (B, H, P, N) or lu.shape != (B, H, P, N) or (ang is not None and ang.shape != (B, H, N // 2)):
             raise ShapeError(f"the cache's state does not match batch {B}, heads {H}, head_dim {P}, d_state {N}")
-        desc, keep = self._call_desc(proj)
+        par = [_f32(self._parameters[n]) for n in _PARAMS]
+        desc = self._pack_desc(proj, par)
         out = torch.empty((B, T, s.d_inner), device=dev, dtype=el)
         conv2 = torch.empty_like(conv)
         h2, lu2 = torch.empty_like(h), torch.empty_like(lu)
@@ -335,9 +240,8 @@ class MixerCore(torch.nn.Module):
         # reversed in memory.
         if proj.shape[1] == 0:                      # nothing to scan (scan.rs:134-144)
             return proj.new_zeros((proj.shape[0], 0, s.d_inner)) + 0.0 * proj.sum()
-        o = {"shape": s, "chunk": self.chunk, "eps": self.eps, "norm": self.use_norm, "disc": int(self.disc),
-             "path": path, "reverse_heads": s.heads // 2 if self.bidirectional else 0,
-             "post_norm": self.post_gate_norm}
-        f = lambda t: None if t is None else t.to(torch.float32).contiguous()
-        return _MixerCore.apply(o, proj.contiguous(), f(self.conv_w), f(self.conv_b), f(self.dt_bias), f(self.a_log),
-                                f(self.d_skip), f(self.b_bias), f(self.c_bias), f(self.norm_w), f(self.post_norm_w))
+        proj = proj.contiguous()
+        p = self._parameters
+        par = [t if t is None or (t.dtype is torch.float32 and t.is_contiguous()) else t.to(torch.float32).contiguous()
+               for t in (p[n] for n in _PARAMS)]
+        return _MixerCore.apply((self._pack_desc(proj, par, path), s.d_inner), proj, *par)

@@ -92,3 +92,36 @@ def test_chunk_parallel_backward_takes_unaligned_gradients():
     ctx.check(ctx.lib.m3_saved_free(ctx.handle, saved))
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,B,T,H,N,R,K,norm,learned,bidir", [
+    (torch.float32, 1, 1, 2, 128, 1, 4, True, True, False),      # one step, most of a block dead
+    (torch.float32, 2, 33, 3, 64, 1, 2, True, True, False),      # an odd number of 64-wide rows: half a warp dead
+    (torch.float32, 1, 131, 2, 64, 2, 3, False, False, False),   # no norm: the plain bias
+    (torch.float32, 2, 150, 4, 128, 2, 4, True, True, True),     # both directions
+    (torch.float32, 1, 70, 2, 64, 4, 1, True, True, False),
+    (torch.float32, 3, 600, 8, 128, 4, 4, True, True, False),    # long runs per warp
+])
+def test_mixer_front_matches_the_separate_steps(dtype, B, T, H, N, R, K, norm, learned, bidir):
+    """The fused launches in front of the scan against the convolution, B / C and activation steps of the C ABI run one
+    by one: a projection that starts off a 16-byte boundary takes those."""
+    from mamba_trainer_b200.nn import MixerCore, MixerShape
+    shape = MixerShape(H, 64, N, R, None, learned)
+    torch.manual_seed(T)
+    core = MixerCore(shape, conv_kernel=K, chunk=16, bc_norm=norm, norm_gain=norm, bidirectional=bidir, device="cuda")
+    with torch.no_grad():
+        for q in (core.b_bias, core.c_bias, core.conv_b, core.d_skip):
+            q.normal_(0, 0.3)
+    W = shape.in_proj_width
+    raw = torch.randn(B * T * W + 1, device="cuda")
+    dout = torch.randn(B, T, shape.d_inner, device="cuda")
+    res = []
+    for off in (0, 1):
+        buf = torch.empty(B * T * W + 8, device="cuda")
+        proj = buf[off:off + B * T * W].copy_(raw[:-1]).view(B, T, W).requires_grad_(True)
+        out = core(proj)
+        res.append((out,) + torch.autograd.grad(out, [proj] + list(core.parameters()), dout))
+    names = ["out", "proj"] + [n for n, _ in core.named_parameters()]
+    for n, a, e in zip(names, *res):
+        scale = max(1.0, float(e.abs().max()))
+        assert ((a - e).abs() <= 2e-5 * scale + 1e-4 * e.abs()).all(), (n, float((a - e).abs().max()), scale)
