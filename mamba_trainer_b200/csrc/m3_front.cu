@@ -21,7 +21,8 @@ namespace m3 {
 namespace {
 
 constexpr int KT = 4;    // taps the kernels are compiled for: a shorter convolution has leading zero taps
-constexpr int kWarps = 8;
+constexpr int kWarps = 8;    // of a block of the forward kernel
+constexpr int kBwdWarps = 4; // and of the backward one, whose threads need up to 170 registers: three blocks per SM
 
 template <class T>
 struct Four;   // four neighbouring elements
@@ -51,18 +52,72 @@ struct Four<__nv_bfloat16> {
   __device__ __forceinline__ void store(__nv_bfloat16* p) const { *reinterpret_cast<uint2*>(p) = v; }
 };
 
+// Two floats per instruction (packed fp32): these kernels are bound by instruction issue.
+__device__ __forceinline__ void mul4(const float (&a)[4], const float (&b)[4], float (&c)[4]) {
+  const float2 lo = __fmul2_rn(make_float2(a[0], a[1]), make_float2(b[0], b[1]));
+  const float2 hi = __fmul2_rn(make_float2(a[2], a[3]), make_float2(b[2], b[3]));
+  c[0] = lo.x; c[1] = lo.y; c[2] = hi.x; c[3] = hi.y;
+}
+__device__ __forceinline__ void add4(const float (&a)[4], const float (&b)[4], float (&c)[4]) {
+  const float2 lo = __fadd2_rn(make_float2(a[0], a[1]), make_float2(b[0], b[1]));
+  const float2 hi = __fadd2_rn(make_float2(a[2], a[3]), make_float2(b[2], b[3]));
+  c[0] = lo.x; c[1] = lo.y; c[2] = hi.x; c[3] = hi.y;
+}
+__device__ __forceinline__ float dot4(const float (&a)[4], const float (&b)[4]) {
+  const float2 s = __ffma2_rn(make_float2(a[2], a[3]), make_float2(b[2], b[3]),
+                              __fmul2_rn(make_float2(a[0], a[1]), make_float2(b[0], b[1])));
+  return s.x + s.y;
+}
+// sigmoid of four values by the special-function unit (2 ulp each step, denormals flushed: without that every
+// exponential and reciprocal carries three more instructions).
+__device__ __forceinline__ void sigmoid4(const float (&v)[4], float (&s)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float x, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(v[e] * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + x));
+    s[e] = r;
+  }
+}
+// Rounded to the element type, four at a time.
+__device__ __forceinline__ void round4(const float*, float (&)[4]) {}
+__device__ __forceinline__ void round4(const __nv_bfloat16*, float (&v)[4]) {
+  Four<__nv_bfloat16> q;
+  q.set(v);
+  q.get(v);
+}
+
 __device__ __forceinline__ void fma4(const float (&a)[4], const float (&b)[4], float (&c)[4]) {   // packed pairs
   const float2 lo = __ffma2_rn(make_float2(a[0], a[1]), make_float2(b[0], b[1]), make_float2(c[0], c[1]));
   const float2 hi = __ffma2_rn(make_float2(a[2], a[3]), make_float2(b[2], b[3]), make_float2(c[2], c[3]));
   c[0] = lo.x; c[1] = lo.y; c[2] = hi.x; c[3] = hi.y;
 }
 
-// Sum over the lanes of a row (N / 4 of them), on all of them.
-template <int N>
-__device__ __forceinline__ float row_sum(float v) {
+// Sums over the lanes of a row (N / 4 of them) of V = 2 or 4 values, on all of them: the halves of the row first split the
+// values between them, and the totals come back by V shuffles - 7 or 10 instead of 10 or 20.
+template <int N, int V>
+__device__ __forceinline__ void row_sums(float (&v)[V]) {
+  constexpr int L = N / 4;
+  const int lane = threadIdx.x & 31;
+  int nv = V;
 #pragma unroll
-  for (int o = N / 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int o = L / 2; o > 0; o >>= 1) {
+    if (nv > 1) {
+      nv >>= 1;
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i)
+        if (i < nv) {
+          const float send = up ? v[i] : v[i + nv], keep = up ? v[i + nv] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  const float mine = v[0];   // lane bits L/2 (and L/4): which value
+#pragma unroll
+  for (int i = 0; i < V; ++i) v[i] = __shfl_sync(0xffffffffu, mine, (lane & ~(L - 1)) | (i * (L / V)));
 }
 
 // The warp's place: 128 channels of the convolution from `c0 - 4 lane`, a run of time steps.
@@ -77,7 +132,7 @@ struct Place {
   bool rev;         // and runs right to left
   int tl, run, t0;  // the warp's place in time within the block, its steps, the first of them
 };
-template <int N, int R>
+template <int N, int R, int WARPS>
 __device__ __forceinline__ Place<N, R> place(const Front& f, int bx, int nx, int nb, int run) {
   using P = Place<N, R>;
   P p;
@@ -100,7 +155,7 @@ __device__ __forceinline__ Place<N, R> place(const Front& f, int bx, int nx, int
     p.rev = f.reverse && p.j >= f.bc / 2;
   }
   if (!p.live) { p.j = 0; p.c0 = p.bc ? f.di : 0; }
-  p.t0 = blockIdx.y * (kWarps * run) + p.tl * p.run;
+  p.t0 = blockIdx.y * (WARPS * run) + p.tl * p.run;
   return p;
 }
 
@@ -140,7 +195,7 @@ __device__ __forceinline__ void act_forward(const Front& f, const FrontOut& o, i
 }
 
 template <class T, int N, int R, int RUN>
-__global__ void __launch_bounds__(kWarps * 32) k_front_fwd(Front f, FrontOut o, int nx, int nb) {
+__global__ void __launch_bounds__(kWarps * 32, 3) k_front_fwd(Front f, FrontOut o, int nx, int nb) {
   using P = Place<N, R>;
   constexpr int kStage = R > 1 ? kWarps * 4 * 128 : 1;
   __shared__ __align__(16) T stage[kStage];   // ranks > 1: four steps of every warp's rows, [time lane][step][n * R + r]
@@ -149,7 +204,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_front_fwd(Front f, FrontOut o, 
     act_forward<T>(f, o, b, blockIdx.y * (kWarps * RUN), kWarps * RUN);
     return;
   }
-  const P p = place<N, R>(f, bx, nx, nb, RUN);
+  const P p = place<N, R, kWarps>(f, bx, nx, nb, RUN);
   float wt[KT][4], bs[4], bias[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gain[4] = {1.0f, 1.0f, 1.0f, 1.0f};
   load_taps(f, p.c0, wt, bs);
   const int g = p.j / (R * N), r = (p.j / N) % R, n = p.j % N;
@@ -159,91 +214,103 @@ __global__ void __launch_bounds__(kWarps * 32) k_front_fwd(Front f, FrontOut o, 
     if (bp) { q.load(bp + (size_t)g * N + n); q.get(bias); }
     if (f.has_norm && f.gain) { q.load(f.gain + n); q.get(gain); }
   }
-  Four<T> next[4];
-  float win[KT - 1 + 4][4];   // rows t - 3 .. t + 3 of the current four steps
-  {
-    Four<T> v;
+  // `inside`: every row this warp touches is one of the sequence's, so rows are reached by adding a stride
+  auto walk = [&](auto inside) {
+    constexpr bool IN = decltype(inside)::value;
+    const ptrdiff_t xs = p.rev ? -(ptrdiff_t)f.width : (ptrdiff_t)f.width;
+    const T* px = static_cast<const T*>(f.proj) + ((ptrdiff_t)b * f.T + (p.rev ? f.T - 1 - p.t0 : p.t0)) * f.width + f.di + p.c0;
+    auto row = [&](Four<T>& v, int s) {   // x of step t0 + s
+      if (IN) v.load(px + s * xs); else load_band<T>(v, f, b, p.t0 + s, p.c0, p.rev);
+    };
+    const size_t ow = p.bc ? f.bc : f.di;
+    T* out = p.bc ? static_cast<T*>(p.which ? o.c : o.b) : static_cast<T*>(o.x);
+    out += ((size_t)b * f.T + (p.rev ? f.T - 1 - p.t0 : p.t0)) * ow;
+    const ptrdiff_t os = p.rev ? -(ptrdiff_t)ow : (ptrdiff_t)ow;
+    Four<T> next[4];
+    float win[KT - 1 + 4][4];   // rows t - 3 .. t + 3 of the current four steps
+    {
+      Four<T> v;
 #pragma unroll
-    for (int k = 0; k < KT - 1; ++k) {
-      load_band<T>(v, f, b, p.t0 - (KT - 1) + k, p.c0, p.rev);
-      v.get(win[k]);
+      for (int k = 0; k < KT - 1; ++k) {
+        row(v, k - (KT - 1));
+        v.get(win[k]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) row(next[i], i);
     }
+#pragma unroll 1
+    for (int s = 0; s < p.run; s += 4) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) load_band<T>(next[i], f, b, p.t0 + i, p.c0, p.rev);
-  }
-  for (int s = 0; s < p.run; s += 4) {
+      for (int i = 0; i < 4; ++i) next[i].get(win[KT - 1 + i]);
+      if (s + 4 < p.run) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) next[i].get(win[KT - 1 + i]);
-    if (s + 4 < p.run) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) load_band<T>(next[i], f, b, p.t0 + s + 4 + i, p.c0, p.rev);
-    }
-    float y[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) y[i][e] = bs[e];
-#pragma unroll
-      for (int k = 0; k < KT; ++k) fma4(wt[k], win[i + k], y[i]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) y[i][e] = __fdividef(y[i][e], 1.0f + __expf(-y[i][e]));   // SiLU
-    }
-    if (p.bc) {
-      float ss[4];
+        for (int i = 0; i < 4; ++i) row(next[i], s + 4 + i);
+      }
+      float y[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        ss[i] = 0.0f;
+        float sg[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          y[i][e] = round_to(static_cast<const T*>(nullptr), y[i][e]) + bias[e];
-          ss[i] = fmaf(y[i][e], y[i][e], ss[i]);
-        }
+        for (int e = 0; e < 4; ++e) y[i][e] = bs[e];
+#pragma unroll
+        for (int k = 0; k < KT; ++k) fma4(wt[k], win[i + k], y[i]);
+        sigmoid4(y[i], sg);
+        mul4(y[i], sg, y[i]);   // SiLU
       }
-      if (f.has_norm) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) ss[i] = row_sum<N>(ss[i]);
+      if (p.bc) {
+        float ss[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float scale = rsqrtf(ss[i] * (1.0f / N) + f.eps);
+          round4(static_cast<const T*>(nullptr), y[i]);
+          add4(y[i], bias, y[i]);
+          ss[i] = dot4(y[i], y[i]);
+        }
+        if (f.has_norm) {
+          row_sums<N, 4>(ss);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) y[i][e] = y[i][e] * scale * gain[e];
+          for (int i = 0; i < 4; ++i) {
+            const float r_ = rsqrtf(ss[i] * (1.0f / N) + f.eps);
+            const float scale[4] = {r_, r_, r_, r_};
+            mul4(y[i], scale, y[i]);
+            mul4(y[i], gain, y[i]);
+          }
         }
       }
-    }
-    Four<T> q;
-    if (!p.bc || R == 1) {
+      Four<T> q;
+      if (!p.bc || R == 1) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = p.t0 + s + i;
-        if (!p.live || t >= f.T) continue;
-        const size_t tok = (size_t)b * f.T + (p.rev ? f.T - 1 - t : t);
-        T* dst = p.bc ? static_cast<T*>(p.which ? o.c : o.b) + tok * f.bc : static_cast<T*>(o.x) + tok * f.di;
-        q.set(y[i]);
-        q.store(dst + p.j);
+        for (int i = 0; i < 4; ++i) {
+          if (!IN && (!p.live || p.t0 + s + i >= f.T)) continue;
+          q.set(y[i]);
+          q.store(out + (s + i) * os + p.j);
+        }
+      } else {
+        T* st = stage + p.tl * (P::WR * 4 * 128);
+        __syncthreads();   // the previous four steps have left
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) stf(st, i * (P::WR * 128) + (n + e) * R + r, y[i][e]);
+        __syncthreads();
+        const int e0 = 4 * ((threadIdx.x >> 5) % P::WR * 32 + lane);   // this thread's four elements of every step
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (!IN && p.t0 + s + i >= f.T) continue;
+          q = *reinterpret_cast<const Four<T>*>(st + i * (P::WR * 128) + e0);
+          q.store(out + (s + i) * os + g * N * R + e0);
+        }
       }
-    } else {
-      T* st = stage + p.tl * (P::WR * 4 * 128);
-      __syncthreads();   // the previous four steps have left
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int k = 0; k < KT - 1; ++k)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) stf(st, i * (P::WR * 128) + (n + e) * R + r, y[i][e]);
-      __syncthreads();
-      const int e0 = 4 * ((threadIdx.x >> 5) % P::WR * 32 + lane);   // this thread's four elements of every step
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = p.t0 + s + i;
-        if (t >= f.T) continue;
-        const size_t tok = (size_t)b * f.T + (p.rev ? f.T - 1 - t : t);
-        q = *reinterpret_cast<const Four<T>*>(st + i * (P::WR * 128) + e0);
-        q.store(static_cast<T*>(p.which ? o.c : o.b) + (tok * f.H + g) * N * R + e0);
-      }
+        for (int e = 0; e < 4; ++e) win[k][e] = win[4 + k][e];
     }
-#pragma unroll
-    for (int k = 0; k < KT - 1; ++k)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) win[k][e] = win[4 + k][e];
-  }
+  };
+  // (the ranks of a group meet at block barriers in there: the choice is the block's)
+  const int blk = blockIdx.y * (kWarps * RUN);
+  const int ch = p.bc ? 128 * P::WR : 128, width = p.bc ? f.bc : f.di, base = p.j - p.j % ch;
+  if (blk >= KT - 1 && blk + kWarps * RUN <= f.T && base + ch <= width) walk(std::true_type{});
+  else walk(std::false_type{});
   // the K - 1 inputs the next window continues from, by the warp that has the last step
   if (o.hist && p.live && p.t0 < f.T && p.t0 + p.run >= f.T) {
     Four<T> v;
@@ -276,7 +343,7 @@ template <class T>
 __device__ __forceinline__ void act_backward(const Front& f, const FrontGrads& g, int b, int t0, int steps, float* part, float* red) {
   const T* proj = static_cast<const T*>(f.proj);
   T* dproj = static_cast<T*>(g.dproj);
-  constexpr int kThreads = kWarps * 32;
+  constexpr int kThreads = kBwdWarps * 32;
   for (int h0 = 0; h0 < f.H; h0 += kThreads) {
     const int nh = min(f.H - h0, kThreads), lanes = kThreads / nh, tl = threadIdx.x / nh, h = h0 + threadIdx.x % nh;
     float s = 0.0f;
@@ -307,18 +374,18 @@ __device__ __forceinline__ void act_backward(const Front& f, const FrontGrads& g
 }
 
 template <class T, int N, int R, int RUN>
-__global__ void __launch_bounds__(kWarps * 32, 2) k_front_bwd(Front f, FrontGrads gr, int nx, int nb) {
+__global__ void __launch_bounds__(kBwdWarps * 32, 3) k_front_bwd(Front f, FrontGrads gr, int nx, int nb) {
   using P = Place<N, R>;
-  __shared__ __align__(16) float ahead[kWarps][KT - 1][128];   // g of every warp's first three steps, for the warp before it
-  __shared__ __align__(16) float red[kWarps][128];
+  __shared__ __align__(16) float ahead[kBwdWarps][KT - 1][128];   // g of every warp's first three steps, for the warp before it
+  __shared__ __align__(16) float red[kBwdWarps][128];
   const int b = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, bx = blockIdx.x;
   const PartLayout pl = part_layout(f);
   float* part = gr.part + ((size_t)b * gridDim.y + blockIdx.y) * pl.total;
   if (bx == nx + 2 * nb) {
-    act_backward<T>(f, gr, b, blockIdx.y * (kWarps * RUN), kWarps * RUN, part + pl.act, &red[0][0]);
+    act_backward<T>(f, gr, b, blockIdx.y * (kBwdWarps * RUN), kBwdWarps * RUN, part + pl.act, &red[0][0]);
     return;
   }
-  const P p = place<N, R>(f, bx, nx, nb, RUN);
+  const P p = place<N, R, kBwdWarps>(f, bx, nx, nb, RUN);
   float wt[KT][4], bs[4], bias[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gain[4] = {1.0f, 1.0f, 1.0f, 1.0f};
   load_taps(f, p.c0, wt, bs);
   const int grp = p.j / (R * N), r = (p.j / N) % R, n = p.j % N;
@@ -328,35 +395,28 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_front_bwd(Front f, FrontGrad
     if (bp) { q.load(bp + (size_t)grp * N + n); q.get(bias); }
     if (f.has_norm && f.gain) { q.load(f.gain + n); q.get(gain); }
   }
-  const T* gin = static_cast<const T*>(!p.bc ? gr.dx : (p.which ? gr.dc : gr.db));
-  // the gradient of a step's four channels as the scan left it: x dense; B, C with the ranks interleaved
-  auto load_grad = [&](Four<T> (&v)[R], int t) {
-    if (t >= f.T) {
-#pragma unroll
-      for (int i = 0; i < R; ++i) v[i].clear();
-      return;
-    }
-    const size_t tok = (size_t)b * f.T + (p.rev ? f.T - 1 - t : t);
-    if (!p.bc) {
-      v[0].load(gin + tok * f.di + p.j);
-    } else {
-      const T* src = gin + (tok * f.H + grp) * N * R + (size_t)n * R;
-#pragma unroll
-      for (int i = 0; i < R; ++i) v[i].load(src + 4 * i);
-    }
-  };
+  const T* gin = static_cast<const T*>(!p.bc ? gr.dx : (p.which ? gr.dc : gr.db)) + (p.bc ? (grp * N + n) * R : p.j);
+  const size_t gwid = p.bc ? (size_t)f.bc : (size_t)f.di;
+  T* dband = static_cast<T*>(gr.dproj) + f.di + p.c0;
+  // this lane's rank of four neighbouring columns, out of the 4 R elements that the scan's layout interleaves
   auto pick = [&](const Four<T> (&v)[R], float (&o)[4]) {
     if (R == 1 || !p.bc) {
       v[0].get(o);
-    } else {
-      float all[R][4];
-#pragma unroll
-      for (int i = 0; i < R; ++i) v[i].get(all[i]);
+    } else if constexpr (sizeof(T) == 2) {
+      const uint32_t sel = (r & 1) ? 0x3244u : 0x1044u;   // the high or the low half of a word, as a float
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        o[e] = 0.0f;
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(v);
+        const uint32_t x = R == 2 ? w[e] : ((r & 2) ? w[(2 * e + 1) % (2 * R)] : w[(2 * e) % (2 * R)]);
+        o[e] = __uint_as_float(__byte_perm(x, 0u, sel));
+      }
+    } else {
+      const float* w = reinterpret_cast<const float*>(v);
 #pragma unroll
-        for (int rr = 0; rr < R; ++rr) o[e] = rr == r ? all[(e * R + rr) / 4][(e * R + rr) % 4] : o[e];
+      for (int e = 0; e < 4; ++e) {
+        o[e] = w[e * R];
+#pragma unroll
+        for (int rr = 1; rr < R; ++rr) o[e] = rr == r ? w[e * R + rr] : o[e];
       }
     }
   };
@@ -367,10 +427,11 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_front_bwd(Front f, FrontGrad
 #pragma unroll
     for (int k = 0; k < KT; ++k) pw[k][e] = 0.0f;
   }
-  // go = d pre of one step, from its taps' window and its gradient; own: the step feeds the parameter gradients
-  auto step = [&](const float (&w0)[4], const float (&w1)[4], const float (&w2)[4], const float (&w3)[4], const Four<T> (&gv)[R],
-                  bool own, float (&go)[4]) {
-    float pre[4], gy[4];
+  // go = d pre of one step, from its taps' window and its gradient; OWN: the step feeds the parameter gradients
+  auto step = [&](auto own, const float (&w0)[4], const float (&w1)[4], const float (&w2)[4], const float (&w3)[4],
+                  const Four<T> (&gv)[R], float (&go)[4]) {
+    constexpr bool OWN = decltype(own)::value;
+    float pre[4], gy[4], sg[4], ds[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) pre[e] = bs[e];
     fma4(wt[0], w0, pre);
@@ -378,104 +439,115 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_front_bwd(Front f, FrontGrad
     fma4(wt[2], w2, pre);
     fma4(wt[3], w3, pre);
     pick(gv, gy);
-    const float mine = own ? 1.0f : 0.0f;
-    float sg[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) sg[e] = __fdividef(1.0f, 1.0f + __expf(-pre[e]));
+    sigmoid4(pre, sg);
+    float v[4];
+    mul4(pre, sg, v);   // SiLU; its derivative is sg + v (1 - sg)
+    {
+      const float nv[4] = {-v[0], -v[1], -v[2], -v[3]};
+      add4(sg, v, ds);
+      fma4(nv, sg, ds);
+    }
     if (p.bc) {
-      float v[4], ss = 0.0f, dot = 0.0f;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        v[e] = round_to(static_cast<const T*>(nullptr), pre[e] * sg[e]) + bias[e];
-        ss = fmaf(v[e], v[e], ss);
-        dot = fmaf(gy[e] * gain[e], v[e], dot);
-      }
+      round4(static_cast<const T*>(nullptr), v);
+      add4(v, bias, v);
       if (f.has_norm) {
-#pragma unroll
-        for (int o = N / 8; o > 0; o >>= 1) {
-          ss += __shfl_xor_sync(0xffffffffu, ss, o);
-          dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        }
-        const float rstd = rsqrtf(ss * (1.0f / N) + f.eps), md = dot * rstd * (1.0f / N);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float xh = v[e] * rstd;
-          pgain[e] = fmaf(mine * gy[e], xh, pgain[e]);
-          gy[e] = rstd * (gy[e] * gain[e] - xh * md);
-        }
+        float dxh[4];
+        mul4(gy, gain, dxh);
+        float sums[2] = {dot4(v, v), dot4(dxh, v)};
+        row_sums<N, 2>(sums);
+        const float rstd = rsqrtf(sums[0] * (1.0f / N) + f.eps), md = -sums[1] * rstd * (1.0f / N);
+        const float rs4[4] = {rstd, rstd, rstd, rstd}, md4[4] = {md, md, md, md};
+        mul4(v, rs4, v);   // normalised
+        if (OWN) fma4(gy, v, pgain);
+        fma4(v, md4, dxh);
+        mul4(dxh, rs4, gy);
       }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) pbias[e] = fmaf(mine, gy[e], pbias[e]);
+      if (OWN) add4(pbias, gy, pbias);
     }
-    float og[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      go[e] = gy[e] * (sg[e] * (1.0f + pre[e] * (1.0f - sg[e])));   // gradients past T are zero, so go is too
-      og[e] = mine * go[e];
-      pb[e] += og[e];
+    mul4(gy, ds, go);   // gradients past T are zero, so go is too
+    if (OWN) {
+      add4(pb, go, pb);
+      fma4(go, w0, pw[0]);
+      fma4(go, w1, pw[1]);
+      fma4(go, w2, pw[2]);
+      fma4(go, w3, pw[3]);
     }
-    fma4(og, w0, pw[0]);
-    fma4(og, w1, pw[1]);
-    fma4(og, w2, pw[2]);
-    fma4(og, w3, pw[3]);
   };
-  T* dband = static_cast<T*>(gr.dproj) + f.di + p.c0;
-  // dx[t] = sum_delay w[K-1-delay] g[t + delay], from gw[j] = g[t + j]
-  auto emit = [&](int t, const float (&g0)[4], const float (&g1)[4], const float (&g2)[4], const float (&g3)[4]) {
-    if (!p.live || t < p.t0 || t >= f.T) return;
-    float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    fma4(wt[3], g0, o);
+  // dx[t] = sum_delay w[K-1-delay] g[t + delay], from gj = g[t + j]
+  const ptrdiff_t xs = p.rev ? -(ptrdiff_t)f.width : (ptrdiff_t)f.width;
+  T* const d0 = dband + ((ptrdiff_t)b * f.T + (p.rev ? f.T - 1 - p.t0 : p.t0)) * f.width;
+  auto emit = [&](int s, const float (&g0)[4], const float (&g1)[4], const float (&g2)[4], const float (&g3)[4]) {
+    if (!p.live || s < 0 || p.t0 + s >= f.T) return;
+    float o[4];
+    mul4(wt[3], g0, o);
     fma4(wt[2], g1, o);
     fma4(wt[1], g2, o);
     fma4(wt[0], g3, o);
     Four<T> q;
     q.set(o);
-    q.store(dband + ((size_t)b * f.T + (p.rev ? f.T - 1 - t : t)) * f.width);
+    q.store(d0 + s * xs);
   };
-  Four<T> nx_[2], ng[2][R];          // the rows of the next two steps
-  float win[KT][4], gw[KT - 1][4];   // x[t-3 .. t]; g[t-3 .. t-1]
-  {
-    Four<T> v;
+  const int last_tl = kBwdWarps / (p.bc ? P::WR : 1) - 1, stride = p.bc ? P::WR : 1;
+  float gw[4][4];   // g of the last four steps; step s in slot s & 3 (every loop over steps is unrolled by four)
+  auto walk = [&](auto inside) {
+    constexpr bool IN = decltype(inside)::value;
+    const T* px = static_cast<const T*>(f.proj) + ((ptrdiff_t)b * f.T + (p.rev ? f.T - 1 - p.t0 : p.t0)) * f.width + f.di + p.c0;
+    const ptrdiff_t gs = p.rev ? -(ptrdiff_t)gwid : (ptrdiff_t)gwid;
+    const T* pg = gin + ((ptrdiff_t)b * f.T + (p.rev ? f.T - 1 - p.t0 : p.t0)) * (ptrdiff_t)gwid;
+    auto row = [&](Four<T>& v, int s) {
+      if (IN) v.load(px + s * xs); else load_band<T>(v, f, b, p.t0 + s, p.c0, p.rev);
+    };
+    auto grad = [&](Four<T> (&v)[R], int s) {   // the gradient of a step as the scan left it
 #pragma unroll
-    for (int k = 0; k < KT - 1; ++k) {
-      load_band<T>(v, f, b, p.t0 - (KT - 1) + k, p.c0, p.rev);
-      v.get(win[k]);
+      for (int i = 0; i < R; ++i) {
+        if (!IN) v[i].clear();
+        if ((i == 0 || p.bc) && (IN || p.t0 + s < f.T)) v[i].load(pg + s * gs + 4 * i);
+      }
+    };
+    Four<T> nxt[2], ng[2][R];   // the rows of the next two steps
+    float win[4][4];            // x of the last four steps, in rotation like gw
+    {
+      Four<T> v;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) gw[k][e] = 0.0f;
-    }
+      for (int k = 1; k < KT; ++k) {
+        row(v, k - KT);
+        v.get(win[k]);
+      }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      load_band<T>(nx_[i], f, b, p.t0 + i, p.c0, p.rev);
-      load_grad(ng[i], p.t0 + i);
-    }
-  }
-  const int last_tl = kWarps / (p.bc ? P::WR : 1) - 1, stride = p.bc ? P::WR : 1;
-  // the run, then - to finish the last three rows - a few more steps by the warp that is last in time; the others take
-  // the three g they need from the warp behind them
-  const int total = p.tl == last_tl ? p.run + 4 : p.run;
-#pragma unroll 1
-  for (int s = 0; s < total; s += 2) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int t = p.t0 + s + i;
-      nx_[i].get(win[KT - 1]);
-      Four<T> gv[R];
-#pragma unroll
-      for (int j = 0; j < R; ++j) gv[j] = ng[i][j];
-      load_band<T>(nx_[i], f, b, t + 2, p.c0, p.rev);
-      load_grad(ng[i], t + 2);
-      float go[4];
-      step(win[0], win[1], win[2], win[3], gv, s < p.run, go);
-      if (s + i < KT - 1)   // for the warp before this one in time
-        *reinterpret_cast<float4*>(&ahead[warp][s + i][4 * lane]) = make_float4(go[0], go[1], go[2], go[3]);
-      if (t - 3 < p.t0 + p.run) emit(t - 3, gw[0], gw[1], gw[2], go);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        gw[0][e] = gw[1][e]; gw[1][e] = gw[2][e]; gw[2][e] = go[e];
-        win[0][e] = win[1][e]; win[1][e] = win[2][e]; win[2][e] = win[3][e];
+      for (int i = 0; i < 2; ++i) {
+        row(nxt[i], i);
+        grad(ng[i], i);
       }
     }
-  }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) gw[k][e] = 0.0f;
+    auto four = [&](auto own, int s0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int s = s0 + i;
+        nxt[i & 1].get(win[i]);
+        Four<T> gv[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) gv[j] = ng[i & 1][j];
+        row(nxt[i & 1], s + 2);
+        grad(ng[i & 1], s + 2);
+        step(own, win[(i + 1) & 3], win[(i + 2) & 3], win[(i + 3) & 3], win[i], gv, gw[i]);
+        if (s0 == 0 && i < KT - 1)   // for the warp before this one in time
+          *reinterpret_cast<float4*>(&ahead[warp][i][4 * lane]) = make_float4(gw[i][0], gw[i][1], gw[i][2], gw[i][3]);
+        if (s - 3 < p.run) emit(s - 3, gw[(i + 1) & 3], gw[(i + 2) & 3], gw[(i + 3) & 3], gw[i]);
+      }
+    };
+#pragma unroll 1
+    for (int s = 0; s < p.run; s += 4) four(std::true_type{}, s);
+    // the last three rows need three more g: the last warp in time works them out, the others take them from the warp
+    // behind them
+    if (p.tl == last_tl) four(std::false_type{}, p.run);
+  };
+  const int end = p.t0 + p.run + (p.tl == last_tl ? 6 : 2);   // rows are requested two steps ahead
+  if (p.t0 >= KT - 1 && end <= f.T) walk(std::true_type{});
+  else walk(std::false_type{});
   __syncthreads();
   if (p.tl != last_tl) {
     float h[KT - 1][4];
@@ -484,10 +556,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_front_bwd(Front f, FrontGrad
       const float4 q = *reinterpret_cast<const float4*>(&ahead[warp + stride][k][4 * lane]);
       h[k][0] = q.x; h[k][1] = q.y; h[k][2] = q.z; h[k][3] = q.w;
     }
-    const int t = p.t0 + p.run - 3;
-    emit(t, gw[0], gw[1], gw[2], h[0]);
-    emit(t + 1, gw[1], gw[2], h[0], h[1]);
-    emit(t + 2, gw[2], h[0], h[1], h[2]);
+    emit(p.run - 3, gw[1], gw[2], gw[3], h[0]);
+    emit(p.run - 2, gw[2], gw[3], h[0], h[1]);
+    emit(p.run - 1, gw[3], h[0], h[1], h[2]);
   }
   // the block's partial sums: its warps in time order, one quantity after the other (a fixed order)
   const int C = f.di + 2 * f.bc;
@@ -497,7 +568,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_front_bwd(Front f, FrontGrad
     __syncthreads();
     if (p.tl == 0 && p.live) {
       float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      for (int w = warp; w < kWarps; w += stride) {
+      for (int w = warp; w < kBwdWarps; w += stride) {
         const float4 q = *reinterpret_cast<const float4*>(&red[w][4 * lane]);
         s.x += q.x; s.y += q.y; s.z += q.z; s.w += q.w;
       }
@@ -513,46 +584,63 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_front_bwd(Front f, FrontGrad
   }
 }
 
-// out[c] = sum over blocks (for the B / C bias over the ranks too) of the partial sums, in a fixed order: block (32, 32)
-// owns 32 columns, thread row y every 32nd term, the 32 row sums are added in order.  blockIdx.y: which gradient; the
-// gain's columns are summed row by row of B and C here and over the rows by k_front_gain.
-__global__ void __launch_bounds__(1024) k_front_sums(Front f, FrontGrads g, int nblk) {
-  __shared__ float red[32][33];
-  const PartLayout pl = part_layout(f);
-  const int C = f.di + 2 * f.bc, c = blockIdx.x * 32 + threadIdx.x;
-  float* out = nullptr;
-  int ncols = 0, inner = 1, istride = 0;
-  size_t off = 0;
-  switch (blockIdx.y) {
-    case 0: out = g.dconv_w; ncols = f.K * C; off = pl.conv + (size_t)(KT - f.K) * C + c; break;
-    case 1: out = g.dconv_b; ncols = C; off = pl.conv + (size_t)KT * C + c; break;
-    case 2:
-    case 3:
-      out = blockIdx.y == 2 ? g.db_bias : g.dc_bias;
-      ncols = f.H * f.N; inner = f.R; istride = f.N;
-      off = pl.bias + (blockIdx.y == 3 ? f.bc : 0) + (size_t)(c / f.N) * f.R * f.N + c % f.N;
-      break;
-    case 4: out = g.dgain ? g.part + (size_t)nblk * pl.total : nullptr; ncols = 2 * f.bc; off = pl.gain + c; break;
-    default: out = g.ddt_bias; ncols = f.H; off = pl.act + c; break;
-  }
-  if (!out || blockIdx.x * 32 >= ncols) return;
+// out[c] = sum over blocks (for the B / C bias over the ranks too) of the partial sums, in a fixed order: block (32, 8)
+// owns 32 columns, thread row y every 8th term, the 8 row sums are added in order.  The blocks of the gradients follow one
+// another (a grid with a row per gradient is mostly blocks with nothing to do); the gain's columns are summed row by row of
+// B and C here and over the rows by k_front_gain.
+constexpr int kSumRows = 8;
+struct SumRange {
+  float* out;
+  size_t off;          // first column within a block's floats
+  int ncols, inner, istride, first_block;
+};
+struct SumPlan {
+  SumRange r[6];
+  int n, blocks;
+};
+__global__ void __launch_bounds__(32 * kSumRows) k_front_sums(SumPlan plan, const float* __restrict__ part, size_t pitch, int nblk,
+                                                             int N) {
+  __shared__ float red[kSumRows][33];
+  int i = 0;
+  while (i + 1 < plan.n && (int)blockIdx.x >= plan.r[i + 1].first_block) ++i;
+  const SumRange q = plan.r[i];
+  const int c = ((int)blockIdx.x - q.first_block) * 32 + threadIdx.x;
   float s = 0.0f;
-  if (c < ncols) {
-    const int n = nblk * inner;
-#pragma unroll 4
-    for (int t = threadIdx.y; t < n; t += 32) {
-      const int blk = inner == 1 ? t : t / inner;
-      s += g.part[(size_t)blk * pl.total + off + (size_t)(t - blk * inner) * istride];
+  if (c < q.ncols) {
+    // a bias column (head, n) is the sum over the head's ranks, N apart
+    const float* src = part + q.off + (q.inner > 1 ? (size_t)(c / N) * q.inner * N + c % N : c);
+    const int n = nblk * q.inner;
+#pragma unroll 8
+    for (int t = threadIdx.y; t < n; t += kSumRows) {
+      const int blk = q.inner == 1 ? t : t / q.inner;
+      s += src[(size_t)blk * pitch + (size_t)(t - blk * q.inner) * q.istride];
     }
   }
   red[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
-  if (threadIdx.y == 0 && c < ncols) {
+  if (threadIdx.y == 0 && c < q.ncols) {
     float tot = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) tot += red[i][threadIdx.x];
-    out[c] = tot;
+    for (int j = 0; j < kSumRows; ++j) tot += red[j][threadIdx.x];
+    q.out[c] = tot;
   }
+}
+SumPlan sum_plan(const Front& f, const FrontGrads& g, int nblk) {
+  const PartLayout pl = part_layout(f);
+  const int C = f.di + 2 * f.bc;
+  SumPlan p{};
+  auto add = [&](float* out, size_t off, int ncols, int inner, int istride) {
+    if (!out) return;
+    p.r[p.n++] = SumRange{out, off, ncols, inner, istride, p.blocks};
+    p.blocks += (ncols + 31) / 32;
+  };
+  add(g.dconv_w, pl.conv + (size_t)(KT - f.K) * C, f.K * C, 1, 0);
+  add(g.dconv_b, pl.conv + (size_t)KT * C, C, 1, 0);
+  add(g.db_bias, pl.bias, f.H * f.N, f.R, f.N);
+  add(g.dc_bias, pl.bias + f.bc, f.H * f.N, f.R, f.N);
+  add(g.dgain ? g.part + (size_t)nblk * pl.total : nullptr, pl.gain, 2 * f.bc, 1, 0);
+  add(g.ddt_bias, pl.act, f.H, 1, 0);
+  return p;
 }
 
 __global__ void __launch_bounds__(1024) k_front_gain(const float* __restrict__ rows, int nrows, int N, float* __restrict__ out) {
@@ -570,12 +658,10 @@ __global__ void __launch_bounds__(1024) k_front_gain(const float* __restrict__ r
   }
 }
 
-// Steps per warp: sixteen amortise the window's start and the warp's parameters; a grid of fewer than four blocks per SM
-// is cut finer so that every SM has work.
-int front_run(const Front& f, int tiles) {
-  const long long blocks = (long long)tiles * f.B * ((f.T + kWarps * 16 - 1) / (kWarps * 16));
-  return blocks >= 4 * 148 ? 16 : 4;
-}
+// Steps per warp: a block of 128 steps amortises the window's start and the warps' parameters; a grid of fewer than four
+// such blocks per SM is cut finer so that every SM has work.
+bool front_long(const Front& f, int tiles) { return (long long)tiles * f.B * ((f.T + 127) / 128) >= 4 * 148; }
+int bwd_steps(const Front& f, int tiles) { return kBwdWarps * (front_long(f, tiles) ? 32 : 8); }
 template <int N, int R>
 void front_tiles(const Front& f, int* nx, int* nb) {
   constexpr int kCh = 128 * Place<N, R>::WR;
@@ -587,7 +673,7 @@ template <class T, int N, int R>
 cudaError_t forward_t(cudaStream_t st, const Front& f, const FrontOut& o) {
   int nx, nb;
   front_tiles<N, R>(f, &nx, &nb);
-  const int run = front_run(f, nx + 2 * nb);
+  const int run = front_long(f, nx + 2 * nb) ? 16 : 4;
   const dim3 grid(nx + 2 * nb + 1, (f.T + kWarps * run - 1) / (kWarps * run), f.B);
   if (run == 16) k_front_fwd<T, N, R, 16><<<grid, kWarps * 32, 0, st>>>(f, o, nx, nb);
   else k_front_fwd<T, N, R, 4><<<grid, kWarps * 32, 0, st>>>(f, o, nx, nb);
@@ -597,11 +683,14 @@ template <class T, int N, int R>
 cudaError_t backward_t(cudaStream_t st, const Front& f, const FrontGrads& g) {
   int nx, nb;
   front_tiles<N, R>(f, &nx, &nb);
-  const int run = front_run(f, nx + 2 * nb), C = f.di + 2 * f.bc;
-  const dim3 grid(nx + 2 * nb + 1, (f.T + kWarps * run - 1) / (kWarps * run), f.B);
-  if (run == 16) k_front_bwd<T, N, R, 16><<<grid, kWarps * 32, 0, st>>>(f, g, nx, nb);
-  else k_front_bwd<T, N, R, 4><<<grid, kWarps * 32, 0, st>>>(f, g, nx, nb);
-  k_front_sums<<<dim3((f.K * C + 31) / 32, 6), dim3(32, 32), 0, st>>>(f, g, (int)(grid.y * grid.z));
+  const int steps = bwd_steps(f, nx + 2 * nb);
+  const dim3 grid(nx + 2 * nb + 1, (f.T + steps - 1) / steps, f.B);
+  if (steps == kBwdWarps * 32) k_front_bwd<T, N, R, 32><<<grid, kBwdWarps * 32, 0, st>>>(f, g, nx, nb);
+  else k_front_bwd<T, N, R, 8><<<grid, kBwdWarps * 32, 0, st>>>(f, g, nx, nb);
+  const int nblk = (int)(grid.y * grid.z);
+  const SumPlan plan = sum_plan(f, g, nblk);
+  if (plan.blocks)
+    k_front_sums<<<plan.blocks, dim3(32, kSumRows), 0, st>>>(plan, g.part, part_layout(f).total, nblk, N);
   if (g.dgain)
     k_front_gain<<<N / 32, dim3(32, 32), 0, st>>>(g.part + part_layout(f).total * grid.y * grid.z, 2 * f.H * R, N, g.dgain);
   return cudaGetLastError();
@@ -644,8 +733,8 @@ cudaError_t front_forward(cudaStream_t st, int dtype, const Front& f, const Fron
 size_t front_part_floats(const Front& f) {
   int nx, nb;
   dispatch(M3_F32, f, [&](auto, auto n, auto r) { front_tiles<n.value, r.value>(f, &nx, &nb); return 0; });
-  const int run = front_run(f, nx + 2 * nb);
-  return part_layout(f).total * f.B * ((f.T + kWarps * run - 1) / (kWarps * run)) + 2 * (size_t)f.bc;
+  const int steps = bwd_steps(f, nx + 2 * nb);
+  return part_layout(f).total * f.B * ((f.T + steps - 1) / steps) + 2 * (size_t)f.bc;
 }
 
 cudaError_t front_backward(cudaStream_t st, int dtype, const Front& f, const FrontGrads& g, uint64_t* launches) {
