@@ -217,7 +217,8 @@ int m3_step_forward(m3_ctx *ctx, const m3_step_desc *desc, const m3_step_out *ou
  * (m3_scan_scratch_bytes(desc, 0)) exceeds the block are refused with
  * M3_ERR_UNSUPPORTED.  Shapes the tensor-core family serves run there unless
  * desc->path says M3_PATH_GENERIC: with nothing kept for a backward pass that family
- * needs no scratch at all; everything else runs the generic family on the block.
+ * needs no scratch at all (few long stripes are cut into segments while what that takes fits the block);
+ * everything else runs the generic family on the block.
  * The first call on each device looks up the block's device address (with that
  * device current), and - CUDA loads a library's kernels and file-scope device arrays
  * when they are first touched - it is also the call during which the driver maps the

@@ -169,6 +169,7 @@ void split_chain_leave(m3_ctx* ctx) {
 template <class Params>
 cudaError_t plan_segments(m3_ctx* ctx, Params& p, int tiles, bool allow_split, char** scratch) {
   *scratch = nullptr;
+  p.ahead = 0;
   size_t bytes = 0;
   m3::tc_segment_plan(p.B * p.H, tiles, allow_split, &p.nseg, &p.tps, &p.grid, &bytes);
   if (p.nseg == 1) return cudaSuccess;
@@ -183,6 +184,33 @@ cudaError_t plan_segments(m3_ctx* ctx, Params& p, int tiles, bool allow_split, c
   return e;
 }
 
+// The same for segments that run side by side: their boundaries' states are enqueued ahead of the stripe kernel.
+// `nseg` and `tps` come from tc_ahead_plan; dy, dh as in tc_ahead.
+template <class Params>
+cudaError_t plan_ahead(m3_ctx* ctx, Params& p, const m3::Dims& d, const m3_scan_desc& desc, int nseg, int tps, const void* dy,
+                       const float* dh, const float* ckpt_angle, char** scratch) {
+  *scratch = nullptr;
+  const int BH = d.B * d.H, tiles = m3::tc_tiles(d.T, d.R);
+  m3::TcAhead a{};
+  a.nseg = nseg;
+  a.tps = tps;
+  const size_t bytes = m3::tc_ahead_bytes(BH, tiles, nseg, nullptr, nullptr);
+  cudaError_t e = cudaSuccess;
+  if (!ctx->no_scratch) e = m3::scratch_alloc(ctx, reinterpret_cast<void**>(scratch), bytes, ctx->stream);
+  if (e != cudaSuccess) return e;
+  m3::tc_ahead_bytes(BH, tiles, nseg, &a, ctx->no_scratch ? ctx->fixed_scratch : *scratch);
+  e = m3::tc_ahead(ctx->stream, d, desc, dy, dh, ckpt_angle, a);
+  ctx->launches += 2;
+  p.ahead = 1;
+  p.nseg = nseg;
+  p.tps = tps;
+  p.grid = BH * nseg < 148 ? BH * nseg : 148;
+  p.seg_state = a.seg_state;
+  p.seg_angle = a.seg_angle;
+  p.seg_flag = nullptr;
+  return e;
+}
+
 // Backward of a forward that ran the tensor-core family: one stripe kernel, then the shared
 // per-token / per-head finalisation.
 int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* in, uint32_t mask,
@@ -193,12 +221,17 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
   d.L = steps; d.C = tiles; d.Tp = tiles * steps; d.LR = 128;
   const size_t BH = (size_t)d.B * d.H;
   const size_t per_tok = BH * d.Tp, per_tile = BH * tiles;
-  const size_t nfloat = 4 * per_tok + 2 * per_tile + BH;
+  // few stripes: segments that run side by side; their sums of d phi are completed afterwards
+  int nseg = 1, tps = tiles;
+  const bool ahead = !saved->tc_direct && m3::tc_ahead_plan((int)BH, tiles, true, &nseg, &tps);
+  const size_t nphi = ahead && d.rot ? (per_tok + BH * nseg) * 64 : 0;
+  const size_t nfloat = 4 * per_tok + 2 * per_tile + BH + 4 + nphi;
   float* base = nullptr;
   M3_CUDA(ctx, m3::scratch_alloc(ctx, reinterpret_cast<void**>(&base), nfloat * sizeof(float), ctx->stream));
   m3::GenericBwdWs bw{};
   bw.da = base; bw.dg = base + per_tok; bw.dw = base + 2 * per_tok; bw.ddt_rot = base + 3 * per_tok;
   bw.partA = base + 4 * per_tok; bw.partD = bw.partA + per_tile; bw.ip0 = bw.partD + per_tile;
+  float* dphi = base + (4 * per_tok + 2 * per_tile + BH + 3) / 4 * 4;   // 16-byte aligned
   auto want = [&](uint32_t bit, const void* p) { return (mask & bit) && p; };
   using bf16 = __nv_bfloat16;
   m3::TcBwdParams p{};
@@ -246,10 +279,17 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
                   (!p.dc || m3::tc_make_row_map(&p.tm_dc, p.dc, d.B, d.T, d.H, 128 * d.R, steps, true))) ? 1 : 0;
   }
   char* seg = nullptr;
-  cudaError_t e = plan_segments(ctx, p, tiles, !p.use_tma, &seg);
+  cudaError_t e;
+  if (ahead) {
+    p.dphi = dphi;
+    p.dpsum = dphi + per_tok * 64;
+    e = plan_ahead(ctx, p, d, desc, nseg, tps, in->dy, in->dh, saved->tc_ckpt_angle, &seg);
+  } else {
+    e = plan_segments(ctx, p, tiles, !p.use_tma, &seg);
+  }
   if (e == cudaSuccess) e = m3::tc_backward(ctx->stream, p, d.rot != 0);
   if (seg) {
-    split_chain_leave(ctx);
+    if (!ahead) split_chain_leave(ctx);
     cudaFreeAsync(seg, ctx->stream);
   }
   if (e == cudaSuccess) {
@@ -258,7 +298,12 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
     void* dlam = (want(M3_GRAD_LAMBDA, g->dlambda) && d.disc == M3_LEARNED_TRAPEZOID) ? g->dlambda : nullptr;
     float* dalog = want(M3_GRAD_A_LOG, g->da_log) ? g->da_log : nullptr;
     float* ddsk = (want(M3_GRAD_D_SKIP, g->dd_skip) && desc.d_skip) ? g->dd_skip : nullptr;
-    e = m3::finalize_scalars(ctx->stream, d, desc, bw, ddt, dlam, dalog, ddsk, &ctx->launches);
+    if (ahead && d.rot) {
+      e = m3::rows_final(ctx->stream, d, desc, p.dphi, p.dpsum, tps, nseg, bw, ddt, dlam, p.dtheta, p.dangle0);
+      ctx->launches += 1;
+    }
+    if (e == cudaSuccess)
+      e = m3::finalize_scalars(ctx->stream, d, desc, bw, ddt, dlam, dalog, ddsk, &ctx->launches, !(ahead && d.rot));
   }
   cudaError_t e2 = cudaFreeAsync(base, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor-core backward");
@@ -485,9 +530,16 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     p.err = ctx->dev_err;
     p.B = d.B; p.T = d.T; p.H = d.H; p.R = d.R; p.disc = d.disc; p.rev = d.rev; p.ths = d.ths;
     p.wait_limit = ctx->wait_limit ? ctx->wait_limit : (1u << 18);
+    // Few stripes: segments of them run side by side (the role-split kernels only, which the forward pass also takes
+    // when it is the backward pass that will be cut; a caller that must not allocate has a fixed block for them).
+    const int ntiles = m3::tc_tiles(d.T, d.R);
+    int nseg = 1, tps = ntiles, bseg, btps;
+    const bool ahead = m3::tc_ahead_plan((int)BH, ntiles, false, &nseg, &tps) &&
+                       (!ctx->no_scratch || m3::tc_ahead_bytes((int)BH, ntiles, nseg, nullptr, nullptr) <= ctx->fixed_bytes);
+    const bool bwd_ahead = saved && m3::tc_ahead_plan((int)BH, ntiles, true, &bseg, &btps);
     // Rank 1 with real dynamics needs no conversion of its rows: bulk tensor copies land them in
     // operand layout (every head left to right, T a multiple of 8, 16-byte aligned tensors).
-    p.use_tma = (d.R == 1 && !d.rot && d.rev == 0 && d.T % 8 == 0 &&
+    p.use_tma = (!ahead && !bwd_ahead && d.R == 1 && !d.rot && d.rev == 0 && d.T % 8 == 0 &&
                  m3::tc_make_tile_map(&p.tm_b, p.b, d.B, d.T, d.H, 128) && m3::tc_make_tile_map(&p.tm_c, p.c, d.B, d.T, d.H, 128) &&
                  m3::tc_make_tile_map(&p.tm_x, p.x, d.B, d.T, d.H, 64)) ? 1 : 0;
     if (!p.use_tma) {
@@ -511,12 +563,13 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
       p.ckpt_h = reinterpret_cast<__nv_bfloat16*>(base);
       p.ckpt_angle = reinterpret_cast<float*>(base + nh * sizeof(__nv_bfloat16));
     }
-    // a caller that must not allocate gets whole stripes: cutting them needs hand-over scratch
+    // a caller that must not allocate gets whole stripes: cutting them needs scratch
     char* seg = nullptr;
-    cudaError_t te = plan_segments(ctx, p, m3::tc_tiles(d.T, d.R), !p.use_tma && !ctx->no_scratch, &seg);
+    cudaError_t te = ahead ? plan_ahead(ctx, p, d, *desc, nseg, tps, nullptr, nullptr, nullptr, &seg)
+                           : plan_segments(ctx, p, ntiles, !p.use_tma && !ctx->no_scratch, &seg);
     if (te == cudaSuccess) te = m3::tc_forward(ctx->stream, p, d.rot != 0);
     if (seg) {
-      split_chain_leave(ctx);
+      if (!ahead) split_chain_leave(ctx);
       cudaFreeAsync(seg, ctx->stream);
     }
     if (te != cudaSuccess) {

@@ -21,6 +21,8 @@ struct m3_ctx {
   uint32_t wait_limit = 0;          // iteration limit of the kernels' bounded waits; 0 = the default
   cudaMemPool_t pool = nullptr;     // this context's own scratch pool (freed memory is kept for reuse)
   bool no_scratch = false;          // set for the span of a call that must not allocate
+  char* fixed_scratch = nullptr;    // what such a call may use instead (m3_noalloc.cu)
+  size_t fixed_bytes = 0;
   char err[512] = {0};
 };
 

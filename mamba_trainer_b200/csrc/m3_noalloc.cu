@@ -54,16 +54,20 @@ extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, co
   if (rc != M3_OK) return rc;
   if (d.T == 0) return m3_scan_forward(ctx, desc, out, nullptr);  // that branch only copies the state
   if (!out->y) return m3::fail(ctx, M3_ERR_NULL, "y is required");
+  if (ctx->device < 0 || ctx->device >= kMaxDevices)
+    return m3::fail(ctx, M3_ERR_UNSUPPORTED, "device ordinal %d outside the table of %d", ctx->device, kMaxDevices);
   // Shapes the tensor-core family serves need no scratch at all when nothing is kept for a backward
-  // pass: that call allocates nothing either, and is the fast one.
+  // pass - or, for few long stripes, states at segment boundaries, which go to the block while they fit.
   if (m3::tc_supported(*desc) && !d.raw && desc->path != M3_PATH_GENERIC) {
-    ctx->no_scratch = true;  // whole stripes: no hand-over scratch between time segments
+    cudaError_t e = cudaSetDevice(ctx->device);
+    if (e == cudaSuccess) e = scratch_address(ctx->device, &ctx->fixed_scratch);
+    if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "cudaGetSymbolAddress");
+    ctx->fixed_bytes = M3_NOALLOC_SCRATCH_BYTES;
+    ctx->no_scratch = true;
     const int rc = m3_scan_forward(ctx, desc, out, nullptr);
     ctx->no_scratch = false;
     return rc;
   }
-  if (ctx->device < 0 || ctx->device >= kMaxDevices)
-    return m3::fail(ctx, M3_ERR_UNSUPPORTED, "device ordinal %d outside the table of %d", ctx->device, kMaxDevices);
   const bool rows = m3::rows_supported(*desc, out->y);
   if (rows) d = m3::rows_dims(d);
   const size_t need = rows ? m3::rows_ws_layout(d, nullptr, nullptr) : m3::generic_ws_layout(d, nullptr, nullptr);

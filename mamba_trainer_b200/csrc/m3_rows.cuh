@@ -285,7 +285,10 @@ __device__ __forceinline__ void load_rows(float* dst, const T* src, const Dims& 
 }
 
 // Rows of B or C (two tensors at once share the sines), rotated by -phi; `scale` (per step, or NULL) multiplies them.
-template <class T, int N, int R, int THREADS, int NTENS>
+// BF: the result is rounded to bf16 (exact in TF32: one product instead of three), as the tensor-core family's operands are.
+template <bool BF>
+__device__ __forceinline__ float operand(float v) { return BF ? __bfloat162float(__float2bfloat16_rn(v)) : v; }
+template <class T, int N, int R, int THREADS, int NTENS, bool BF = false>
 __device__ __forceinline__ void load_rotated(float* const (&dst)[NTENS], const T* const (&src)[NTENS], const float* phi,
                                              const float* scale, const Dims& d, const Chunk& c) {
   constexpr int LT = kRows / R, NH = N / 2, PER = NH * R / 4, NA = R == 1 ? 4 : (R == 2 ? 2 : 1);
@@ -316,8 +319,8 @@ __device__ __forceinline__ void load_rotated(float* const (&dst)[NTENS], const T
       float o1[4], o2[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        o1[j] = a[j] * cs[j / R] + b[j] * sn[j / R];
-        o2[j] = b[j] * cs[j / R] - a[j] * sn[j / R];
+        o1[j] = operand<BF>(a[j] * cs[j / R] + b[j] * sn[j / R]);
+        o2[j] = operand<BF>(b[j] * cs[j / R] - a[j] * sn[j / R]);
       }
       if (R == 1) {
         *reinterpret_cast<float4*>(dst[w] + at<N>(l, e)) = make_float4(o1[0], o1[1], o1[2], o1[3]);
@@ -334,7 +337,7 @@ __device__ __forceinline__ void load_rotated(float* const (&dst)[NTENS], const T
   }
 }
 // The same without a rotation.
-template <class T, int N, int R, int THREADS>
+template <class T, int N, int R, int THREADS, bool BF = false>
 __device__ __forceinline__ void load_scaled(float* dst, const T* src, const float* scale, const Dims& d, const Chunk& c) {
   constexpr int LT = kRows / R, PER = N * R / 4;
 #pragma unroll
@@ -343,7 +346,7 @@ __device__ __forceinline__ void load_scaled(float* dst, const T* src, const floa
     float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (t < d.T) v = load4(src + tok_index(d, c.b, t, c.h) * N * R + e);
     const float sc = scale[l];
-    const float f[4] = {v.x * sc, v.y * sc, v.z * sc, v.w * sc};
+    const float f[4] = {operand<BF>(v.x * sc), operand<BF>(v.y * sc), operand<BF>(v.z * sc), operand<BF>(v.w * sc)};
     if (R == 1) {
       *reinterpret_cast<float4*>(dst + at<N>(l, e)) = make_float4(f[0], f[1], f[2], f[3]);
     } else {
@@ -427,6 +430,10 @@ Dims rows_dims(Dims d);
 size_t rows_ws_layout(const Dims& d, rows::RowsWs* ws, char* base);
 cudaError_t rows_forward(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const m3_scan_out& out,
                          const rows::RowsWs& ws, uint64_t* launches);
+// The last pass over tokens for the tensor-core family's side-by-side segments (bf16, d_state 128, rotational): d.L steps
+// per tile, `per_seg` tiles per segment.
+cudaError_t rows_final(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const float* dphi, const float* dpsum, int per_seg,
+                       int nseg, const GenericBwdWs& bw, void* ddt, void* dlam, void* dtheta, float* dangle0);
 size_t rows_bwd_ws_layout(const Dims& d, rows::RowsBwdWs* rw, GenericBwdWs* bw, char* base);
 cudaError_t rows_backward(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const rows::RowsWs& ws,
                           const rows::RowsBwdWs& rw, const GenericBwdWs& bw, const m3_scan_bwd_in& in, uint32_t mask,

@@ -433,13 +433,14 @@ __global__ void __launch_bounds__(kAdj, 1) k_rows_adjoint(Dims d, m3_scan_desc i
 }
 
 // ---- rotational dynamics: the later chunks' d phi on top, then per token d theta, d dt and d lambda (the arithmetic of
-// kb_final).  A warp per step, lanes over planes.
+// kb_final).  A warp per step, lanes over planes; a block per d.L steps, `per_seg` blocks to a segment whose sums of d phi
+// are complete within it, `nseg` of those (here the chunks; the tensor-core family's segments are longer).
 template <class T, int N>
 __global__ void __launch_bounds__(256) k_rows_final(Dims d, m3_scan_desc in, RowsBwdWs rw, GenericBwdWs bw, int has_state,
                                                     T* __restrict__ ddt, T* __restrict__ dlam, T* __restrict__ dtheta,
-                                                    float* __restrict__ dangle0) {
+                                                    float* __restrict__ dangle0, int per_seg, int nseg) {
   constexpr int NH = N / 2, NQ = 256 / NH, PL = NH / 32;
-  __shared__ float s_off[NQ][NH], s_rot[kRows];
+  __shared__ float s_off[NQ][NH], s_rot[128];
   const Chunk c = this_chunk(d);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const T* dt = static_cast<const T*>(in.dt);
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(256) k_rows_final(Dims d, m3_scan_desc in, Row
     const int q = tid / NH, m = tid % NH;
     float s = 0.0f;
 #pragma unroll 4
-    for (int k = c.k + 1 + q; k < d.C; k += NQ) s += rw.dpsum[((size_t)c.bh * d.C + k) * NH + m];
+    for (int k = c.k / per_seg + 1 + q; k < nseg; k += NQ) s += rw.dpsum[((size_t)c.bh * nseg + k) * NH + m];
     s_off[q][m] = s;
   }
   __syncthreads();
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(256) k_rows_final(Dims d, m3_scan_desc in, Row
 #pragma unroll
     for (int q = 0; q < NQ; ++q) off[i] += s_off[q][lane + 32 * i];
     if (c.k == 0 && warp == 0 && dangle0)
-      dangle0[(size_t)c.bh * NH + lane + 32 * i] = off[i] + rw.dpsum[(size_t)c.bh * d.C * NH + lane + 32 * i];
+      dangle0[(size_t)c.bh * NH + lane + 32 * i] = off[i] + rw.dpsum[(size_t)c.bh * nseg * NH + lane + 32 * i];
   }
 #pragma unroll 4
   for (int l = warp; l < d.L; l += 8) {
@@ -524,7 +525,7 @@ cudaError_t backward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, c
   if (ROT) {
     k_rows_final<T, N><<<grid, 256, 0, st>>>(d, in, rw, bw, has_state ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam),
                                              static_cast<T*>(want(M3_GRAD_THETA, g.dtheta)),
-                                             in.angle0 ? static_cast<float*>(want(M3_GRAD_ANGLE0, g.dangle0)) : nullptr);
+                                             in.angle0 ? static_cast<float*>(want(M3_GRAD_ANGLE0, g.dangle0)) : nullptr, 1, d.C);
     n += 1;
   }
   if (launches) *launches += n;
@@ -537,6 +538,15 @@ cudaError_t backward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, c
 
 }  // namespace
 }  // namespace rows
+
+cudaError_t rows_final(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const float* dphi, const float* dpsum, int per_seg,
+                       int nseg, const GenericBwdWs& bw, void* ddt, void* dlam, void* dtheta, float* dangle0) {
+  using T = __nv_bfloat16;
+  const rows::RowsBwdWs rw{nullptr, const_cast<float*>(dphi), const_cast<float*>(dpsum)};
+  rows::k_rows_final<T, 128><<<dim3((d.T + d.L - 1) / d.L, d.B * d.H), 256, 0, st>>>(
+      d, in, rw, bw, in.h0 ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam), static_cast<T*>(dtheta), dangle0, per_seg, nseg);
+  return cudaGetLastError();
+}
 
 size_t rows_bwd_ws_layout(const Dims& d, rows::RowsBwdWs* rw, GenericBwdWs* bw, char* base) {
   size_t off = 0;

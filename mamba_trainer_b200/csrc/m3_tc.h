@@ -56,6 +56,7 @@ struct TcFwdParams {
   uint32_t wait_limit; // iteration limit of the bounded waits (m3_ctx_set_wait_limit)
   // time segments of a stripe (role-split kernel; work distribution in m3_tc_roles.cuh): nseg == 1 hands nothing over
   int nseg, tps, grid;
+  int ahead;          // 1: seg_state and seg_angle hold every boundary's state before the launch (m3_tc_ahead.cu)
   float *seg_state, *seg_angle;
   int* seg_flag;
 };
@@ -64,6 +65,20 @@ struct TcFwdParams {
 // the end (about six per SM), segments of at least four tiles.  Returns segments per stripe, tiles per
 // segment and the grid; bytes of hand-over scratch (state, angle, flags) through *scratch_bytes.
 void tc_segment_plan(int BH, int tiles, bool allow_split, int* nseg, int* tps, int* grid, size_t* scratch_bytes);
+
+// Segments that run side by side (m3_tc_ahead.cu): the state and angle at every boundary are worked out first, in the
+// seg_state / seg_angle the stripe kernels read, and nothing is handed over.
+struct Dims;
+struct TcAhead {
+  int nseg, tps;
+  float *hs, *asum, *cd;          // per tile
+  float *seg_state, *seg_angle;   // per segment
+};
+bool tc_ahead_plan(int BH, int tiles, bool backward, int* nseg, int* tps);
+size_t tc_ahead_bytes(int BH, int tiles, int nseg, TcAhead* a, char* base);
+// dy NULL: forward; else the gradient of the state (dh: the one reaching the returned state, or NULL).
+cudaError_t tc_ahead(cudaStream_t st, Dims d, const m3_scan_desc& in, const void* dy, const float* dh, const float* ckpt_angle,
+                     const TcAhead& a);
 
 cudaError_t tc_forward(cudaStream_t st, const TcFwdParams& p, bool rotational);
 // The direct form (rank 1, real dynamics, use_tma): m3_tc_fwd_direct.cu.
@@ -91,6 +106,8 @@ struct TcBwdParams {
   int ths;            // elements between consecutive tokens of theta and d theta
   uint32_t wait_limit;
   int nseg, tps, grid;   // as in TcFwdParams; the gradient of the state and the running sum of d phi are handed over
+  int ahead;             // with it, the sums of d phi stay within a segment: dphi [BH, tiles * steps, 64] receives them and
+  float *dphi, *dpsum;   // dpsum [BH, nseg, 64] the segments' totals, for k_rows_final to finish
   float *seg_state, *seg_angle;
   int* seg_flag;
 };

@@ -40,8 +40,10 @@ constexpr uint32_t TM_G = 0, TM_DM = 128, TM_T1 = 256, TM_DH = 384, TM_TAB = 448
 // phase B reuse: dB^ accumulates over G's columns, dX~ and U over dM's.
 constexpr uint32_t TM_DB = 0, TM_DX = 128, TM_U = 192;
 
-template <int R, bool ROT, bool SPLIT>
+// MODE as in m3_tc_fwd.cu.
+template <int R, bool ROT, int MODE>
 __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_constant__ TcBwdParams p) {
+  constexpr bool SPLIT = MODE != 0, AHEAD = MODE == 2;
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int LT = kRows / R;
   using RT = RawTile<R>;
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
         // dH^T <- gradient reaching the returned h (or zero) for the stripe's last segment, else what the
         // segment after this one handed over (bounded wait for its flag); likewise the running sum of d phi
         const bool seeded = seg + 1 < nseg;
-        if (seeded) {
+        if (!AHEAD && seeded) {
           if (tid == 0) *s_ok = wait_flag(p.seg_flag + (size_t)bh * nseg + seg + 1, wait_limit << 4) ? 1 : 0;
           epi_sync();
           if (!*s_ok) dead = true;
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
           tmem_st16(tmem_addr(tm, quad * 32, TM_DH + p0), v);
         }
         tmem_wait_st();
-        if (tid < kNH) s_dcar[tid] = seeded ? __ldcg(p.seg_angle + ((size_t)bh * nseg + seg + 1) * kNH + tid) : 0.0f;
+        if (tid < kNH) s_dcar[tid] = !AHEAD && seeded ? __ldcg(p.seg_angle + ((size_t)bh * nseg + seg + 1) * kNH + tid) : 0.0f;
         epi_sync();
       }
       for (int k = k_hi - 1; k >= k_lo; --k, ++it) {
@@ -742,7 +744,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
         epi_sync();
         if (q == 0) {
           s_dcar[m] = total;
-          if (k == 0 && p.dangle0) p.dangle0[(size_t)bh * kNH + m] = total;
+          if (!AHEAD && k == 0 && p.dangle0) p.dangle0[(size_t)bh * kNH + m] = total;
         }
         // vector pass: d theta = d step * dt (16-byte stores) and the rotation's share of d dt
 #pragma unroll
@@ -750,6 +752,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
           const int iv = tid + 256 * i, l = iv >> 3, mg = iv & 7;
           const float4 d0 = *reinterpret_cast<const float4*>(&sDphi[phi_idx(l, mg * 8)]);
           const float4 d1 = *reinterpret_cast<const float4*>(&sDphi[phi_idx(l, mg * 8 + 4)]);
+          if constexpr (AHEAD) {   // later segments' share is not known yet
+            float4* dst = reinterpret_cast<float4*>(p.dphi + ((size_t)bh * Tp + t0 + l) * kNH + mg * 8);
+            dst[0] = d0;
+            dst[1] = d1;
+            continue;
+          }
           const float ds[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
           const uint32_t tw[4] = {thq[i].x, thq[i].y, thq[i].z, thq[i].w};
           const float dtl = ts.dt[l];
@@ -794,7 +802,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
         const size_t o = (size_t)bh * Tp + t0 + l;
         p.dw[o] = col + sg * q;
         p.dg[o] = dgv;
-        if (ROT) p.ddt_rot[o] = part_rot[l];
+        if (ROT && !AHEAD) p.ddt_rot[o] = part_rot[l];
       }
       epi_sync();
       if (warp == 0) {  // reverse inclusive scan of d acum (+ the chunk-decay terms on the last step)
@@ -838,9 +846,10 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
       {
         // ---- the item's first tile is done: the gradient of the seed state, or the hand-over to the
         //      segment before this one ------------------------------------------------------------------
-        const bool hand_over = seg > 0;
+        const bool hand_over = !AHEAD && seg > 0, seed = seg == 0;
+        if (AHEAD && ROT && tid < kNH) p.dpsum[((size_t)bh * nseg + seg) * kNH + tid] = s_dcar[tid];
         float first = 0.0f;
-        if (!hand_over && p.h0) {
+        if (seed && p.h0) {
           const size_t i0 = tok_at(0);
           const float l0 = p.disc == 0 ? 1.0f : (p.disc == 1 ? 0.5f : bf(p.lam, i0));
           first = (1.0f - l0) * bf(p.dt, i0);
@@ -857,7 +866,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
               float* dst = p.seg_state + ((size_t)bh * nseg + seg) * kP * kN;
 #pragma unroll
               for (int j = 0; j < 16; ++j) __stcg(dst + (size_t)(p0 + j) * kN + row, v[j]);
-            } else {
+            } else if (seed) {
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
                 const size_t o = ((size_t)bh * kP + p0 + j) * kN + row;
@@ -876,7 +885,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
           if (tid == 0) raise_handover(p.seg_flag + (size_t)bh * nseg + seg);
         } else {
           const float tot = epi_sum(ip, s_red);
-          if (tid == 0) p.ip0[bh] = tot;
+          if (tid == 0 && seed) p.ip0[bh] = tot;
         }
       }
     }
@@ -889,7 +898,9 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
 
 template <int R>
 cudaError_t launch_r(cudaStream_t st, const TcBwdParams& p, bool rot) {
-  auto kern = p.nseg > 1 ? (rot ? tc_bwd_kernel<R, true, true> : tc_bwd_kernel<R, false, true>) : (rot ? tc_bwd_kernel<R, true, false> : tc_bwd_kernel<R, false, false>);
+  auto kern = p.nseg == 1 ? (rot ? tc_bwd_kernel<R, true, 0> : tc_bwd_kernel<R, false, 0>)
+              : p.ahead   ? (rot ? tc_bwd_kernel<R, true, 2> : tc_bwd_kernel<R, false, 2>)
+                          : (rot ? tc_bwd_kernel<R, true, 1> : tc_bwd_kernel<R, false, 1>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
   if (e != cudaSuccess) return e;
   kern<<<p.grid, kCtaThreads, kSmemBytes, st>>>(p);

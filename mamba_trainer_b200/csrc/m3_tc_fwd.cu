@@ -41,8 +41,11 @@ struct FwdSmem {
 };
 constexpr uint32_t TM_G = 0, TM_Y = 128, TM_H = 192, TM_COLS = 256;
 
-template <int R, bool ROT, bool SPLIT>
+// MODE 0: whole stripes; 1: stripes cut into segments that hand over to one another; 2: segments whose entering states
+// are known before the launch (m3_tc_ahead.cu).
+template <int R, bool ROT, int MODE>
 __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_constant__ TcFwdParams p) {
+  constexpr bool SPLIT = MODE != 0, AHEAD = MODE == 2;
   extern __shared__ __align__(1024) uint8_t smem[];
   using SM = FwdSmem<R>;
   constexpr int LT = kRows / R;  // time steps per tile
@@ -238,13 +241,13 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_con
       const size_t tok_base = ((size_t)b * T + (rev ? T - 1 : 0)) * H + h;
       auto tok_at = [&](int s) { return tok_base + (size_t)((ptrdiff_t)s * Hs); };
       const float dsk = p.d_skip ? p.d_skip[h] : 0.0f;
-      const bool hand_over = seg + 1 < nseg;
+      const bool hand_over = !AHEAD && seg + 1 < nseg;
       // ---- the item's first tile: the state and the running angle start from the caller's (first segment)
       //      or from what the previous segment handed over (bounded wait for its flag); the tile's angle
       //      table, which every later tile has ready from its predecessor's step 3 ----------------------------
       {
         issue_px<R>(raw_x, p.x, tok_at(k_lo * LT), Hs, T, k_lo * LT);
-        if (seg > 0) {
+        if (!AHEAD && seg > 0) {
           if (tid == 0) *s_ok = wait_flag(p.seg_flag + (size_t)bh * nseg + seg - 1, wait_limit << 4) ? 1 : 0;
           epi_sync();
           if (!*s_ok) dead = true;
@@ -481,7 +484,9 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_con
 
 template <int R>
 cudaError_t launch_r(cudaStream_t st, const TcFwdParams& p, bool rot) {
-  auto kern = p.nseg > 1 ? (rot ? tc_fwd_kernel<R, true, true> : tc_fwd_kernel<R, false, true>) : (rot ? tc_fwd_kernel<R, true, false> : tc_fwd_kernel<R, false, false>);
+  auto kern = p.nseg == 1 ? (rot ? tc_fwd_kernel<R, true, 0> : tc_fwd_kernel<R, false, 0>)
+              : p.ahead   ? (rot ? tc_fwd_kernel<R, true, 2> : tc_fwd_kernel<R, false, 2>)
+                          : (rot ? tc_fwd_kernel<R, true, 1> : tc_fwd_kernel<R, false, 1>);
   constexpr uint32_t bytes = FwdSmem<R>::bytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e != cudaSuccess) return e;

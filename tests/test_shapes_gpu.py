@@ -125,3 +125,32 @@ def test_mixer_front_matches_the_separate_steps(dtype, B, T, H, N, R, K, norm, l
     for n, a, e in zip(names, *res):
         scale = max(1.0, float(e.abs().max()))
         assert ((a - e).abs() <= 2e-5 * scale + 1e-4 * e.abs()).all(), (n, float((a - e).abs().max()), scale)
+
+
+@pytest.mark.parametrize("R,rot,T,state,rev", [
+    (1, True, 385, True, 0),      # four tiles, the last one a single step
+    (1, False, 1000, True, 0),    # real dynamics: the role-split kernels instead of the direct ones
+    (2, True, 1000, True, 1),     # a right-to-left head, carried state and angle
+    (2, True, 449, False, 0),     # the second half of the last tile is padding
+    (4, True, 321, True, 0),
+    (4, False, 96, False, 1),     # three tiles: the fewest that are cut
+])
+def test_side_by_side_segments_match_the_oracle(R, rot, T, state, rev):
+    """Few stripes of the tensor-core family: segments of a stripe run at once from states worked out ahead of them."""
+    from test_scan_gpu import check_bf16, compare_all, small_inputs
+    t, ds = small_inputs(2, T, 2, 64, 128, R, rot, state, seed=T + R)
+    for k in ("b", "c"):
+        t[k] = t[k] / 128 ** 0.5
+    t["dt"] = t["dt"] * 0.2
+    if rot:
+        t["theta"] = t["theta"] * 0.3
+    for k in ("x", "b", "c", "dt", "lam", "theta", "dy"):
+        if t[k] is not None:
+            t[k] = t[k].to(torch.bfloat16)
+
+    def check(name, a, e):   # d theta: as in the tests of the stripe kernels, amplified by cancellation
+        if name == "dtheta":
+            assert float((a.double().cpu() - e).norm() / e.norm()) <= 3e-2, name
+        else:
+            check_bf16(name, a, e)
+    compare_all(t, 64, check, True, ds, path=2, reverse_heads=rev)
