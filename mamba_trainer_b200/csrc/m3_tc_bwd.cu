@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
       const float A = -expf(p.a_log[h]);
       lookahead_load<R>(ld, p.dt, p.lam, p.disc, b, h, H, T, (im.k_hi - 1) * LT, rev);
       for (int k = im.k_hi - 1; k >= im.k_lo; --k, ++it) {
-        if (it > 0) bar_sync(BAR_FREE, kPairCount);
+        if (it > 0) bar_sync(bar_free(it), kPairCount);
         lookahead_scalars<R>(scal_set(it & 1), ld, A, T, k * LT);
         bar_arrive(bar_ahead(it), kPairCount);
         if (k > im.k_lo) lookahead_load<R>(ld, p.dt, p.lam, p.disc, b, h, H, T, (k - 1) * LT, rev);
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
       const int l_end = T - 1 - t0;  // row of the final token when last_tile
       const TileScalars ts = scal_set(it & 1);
       bar_sync(bar_ahead(it), kPairCount);  // the tile's scalars
-      if (it == 0 && total > 1) epi_signal(BAR_FREE, kPairCount, dead);  // the other set has never been used
+      if (it == 0 && total > 1) epi_signal(bar_free(1), kPairCount, dead);  // the other set has never been used
       // ---- 1. the tile's rows have been landing since the previous tile let go of the buffers --------
       if (!dead) dead = !warp_all(mbar_wait(&bars[2], it & 1, wait_limit));
       if (ROT) {
@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
         if (lane == 0) p.partA[(size_t)bh * ntiles + k] = pa;
       }
       // this tile's scalars are spent: the look-ahead warp may overwrite their set
-      if (it + 2 < total) epi_signal(BAR_FREE, kPairCount, dead);
+      if (it + 2 < total) epi_signal(bar_free(it), kPairCount, dead);
       epi_sync();
       }
       {

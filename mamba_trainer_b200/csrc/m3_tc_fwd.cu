@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_con
       const float A = -expf(p.a_log[h]);
       lookahead_load<R>(ld, p.dt, p.lam, p.disc, b, h, H, T, it.k_lo * LT, rev);
       for (int k = it.k_lo; k < it.k_hi; ++k, ++g) {
-        if (g > 0) bar_sync(BAR_FREE, kPairCount);
+        if (g > 0) bar_sync(bar_free(g), kPairCount);
         lookahead_scalars<R>(scal_set(g & 1), ld, A, T, k * LT);
         bar_arrive(bar_ahead(g), kPairCount);
         if (k + 1 < it.k_hi) lookahead_load<R>(ld, p.dt, p.lam, p.disc, b, h, H, T, (k + 1) * LT, rev);
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_con
                                  : (p.angle0 ? p.angle0[(size_t)bh * kNH + tid] : 0.0f);
         epi_sync();
         angle_table(g, bh, k_lo, rev);
-        if (g == 0 && total > 1) epi_signal(BAR_FREE, kPairCount, dead);  // set 1 has never been used
+        if (g == 0 && total > 1) epi_signal(bar_free(1), kPairCount, dead);  // set 1 has never been used
         epi_sync();
         const float* src = seg > 0 ? p.seg_state + ((size_t)bh * nseg + seg - 1) * kP * kN
                                    : (p.h0 ? p.h0 + (size_t)bh * kP * kN : nullptr);
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_con
       epi_signal(BAR_MID, kPairCount, dead);
       // this tile's scalars are spent with the band: the look-ahead warp, whose code runs cold and slowly, may
       // overwrite their set with those of the tile after next from here on
-      if (g + 2 < total) epi_signal(BAR_FREE, kPairCount, dead);
+      if (g + 2 < total) epi_signal(bar_free(g), kPairCount, dead);
       // ---- 3. the next tile's angle table, while the second group of products runs (a tile that opens an
       //         item builds its own: its predecessor, which may be this very item, must have handed over) ---
       if (k + 1 < k_hi) angle_table(g + 1, bh, k + 1, rev);

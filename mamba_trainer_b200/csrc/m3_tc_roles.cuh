@@ -36,7 +36,10 @@ enum : int {
   BAR_AHEAD = 4,  // 288: scalars of a tile are ready (look-ahead warp arrives; epilogue warps sync); even tiles
   BAR_AHEAD_ODD = 7,  // the same for odd tiles: the look-ahead warp may finish a tile before its predecessor's
                       // scalars have been picked up, and a barrier holds one pending phase only
-  BAR_FREE = 5,   // 288: a set of scalars is free again (epilogue warps arrive; look-ahead warp syncs)
+  BAR_FREE = 5,   // 288: the set of scalars of an even tile is free for it (epilogue warps arrive; look-ahead warp syncs)
+  BAR_FREE_ODD = 10,  // the same for odd tiles.  One barrier for both would hold two pending phases whenever the look-ahead
+                      // warp, held up by its loads, has not joined the first yet; with two, the epilogue warps have
+                      // synced on the scalars of tile n - which follow its FREE phase - before they signal n + 2's
   BAR_TAIL = 6,   // 288: a tile's gradients are staged, its operands spent (epilogue warps arrive; copy warp syncs)
   BAR_TABLE = 8,  // 256: (backward) every epilogue warp has copied its angle-table words out of the buffer M takes over
   BAR_OPS0 = 9,   // 288: the x / dy operands of a tile are staged, ahead of B and C (epilogue warps arrive; issuer syncs)
@@ -49,6 +52,7 @@ __device__ __forceinline__ void bar_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 __device__ __forceinline__ void epi_sync() { bar_sync(BAR_EPI, kEpiThreads); }
+__device__ __forceinline__ int bar_free(int tile_index) { return (tile_index & 1) ? BAR_FREE_ODD : BAR_FREE; }
 __device__ __forceinline__ int bar_ahead(int tile_index) { return (tile_index & 1) ? BAR_AHEAD_ODD : BAR_AHEAD; }
 // An epilogue warp's side of a barrier a helper warp syncs on: arrive and go on - unless the warp has
 // given up a bounded wait and only keeps the protocol alive: then it waits for the helper like everyone,
