@@ -6,7 +6,6 @@ library has not been built: there is no CPU or eager fallback behind this module
 from __future__ import annotations
 
 import ctypes as C
-import struct
 from pathlib import Path
 
 _LIB_PATH = Path(__file__).resolve().parent / "libm3scan.so"
@@ -103,13 +102,6 @@ class MixerGrads(C.Structure):
                                           "dc_bias", "dnorm_weight", "dpost_weight")]
 
 
-# The mixer calls sit on latency-bound paths, where filling a ctypes structure field by field is a large part of
-# the call: these lay the same bytes out in one pack (0 for a NULL pointer).
-PACK_MIXER_DESC = struct.Struct("@16ifi10P")
-PACK_MIXER_WINDOW_IO = struct.Struct("@9P")
-PACK_MIXER_GRADS = struct.Struct("@10P")
-
-
 class HostIn(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("x", "b", "c", "dt", "lambda_", "theta", "dy")]
 
@@ -149,12 +141,13 @@ SYMBOLS = {
     "m3_gate_backward": (C.c_int, [C.c_void_p, C.POINTER(GateDesc), C.c_void_p, C.c_void_p, C.c_void_p]),
     "m3_gate_norm_forward": (C.c_int, [C.c_void_p, C.POINTER(GateNormDesc), C.c_void_p]),
     "m3_gate_norm_backward": (C.c_int, [C.c_void_p, C.POINTER(GateNormDesc), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
-    "m3_mixer_window_bytes": (C.c_size_t, [C.c_char_p, C.c_char_p]),
-    "m3_mixer_window": (C.c_int, [C.c_void_p, C.c_char_p, C.c_char_p, C.c_void_p]),
-    "m3_mixer_activation_bytes": (C.c_size_t, [C.c_char_p]),
-    "m3_mixer_backward_bytes": (C.c_size_t, [C.c_char_p]),
-    "m3_mixer_forward": (C.c_int, [C.c_void_p, C.c_char_p, C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p)]),
-    "m3_mixer_backward": (C.c_int, [C.c_void_p, C.c_char_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_char_p, C.c_void_p]),
+    "m3_mixer_window_bytes": (C.c_size_t, [C.POINTER(MixerDesc), C.POINTER(MixerWindowIo)]),
+    "m3_mixer_window": (C.c_int, [C.c_void_p, C.POINTER(MixerDesc), C.POINTER(MixerWindowIo), C.c_void_p]),
+    "m3_mixer_activation_bytes": (C.c_size_t, [C.POINTER(MixerDesc)]),
+    "m3_mixer_backward_bytes": (C.c_size_t, [C.POINTER(MixerDesc)]),
+    "m3_mixer_forward": (C.c_int, [C.c_void_p, C.POINTER(MixerDesc), C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p)]),
+    "m3_mixer_backward": (C.c_int, [C.c_void_p, C.POINTER(MixerDesc), C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(MixerGrads),
+                                    C.c_void_p]),
     "m3_host_alloc": (C.c_int, [C.c_size_t, C.POINTER(C.c_void_p)]),
     "m3_host_free": (C.c_int, [C.c_void_p]),
     "m3_host_pipe_create": (C.c_int, [C.c_void_p, C.POINTER(ScanDesc), C.c_int, C.POINTER(C.c_void_p)]),
@@ -164,6 +157,7 @@ SYMBOLS = {
 }
 
 _lib = None
+_ext = None
 
 
 def lib_path() -> Path:
@@ -186,3 +180,24 @@ def load():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def extension():
+    """The torch extension over the library (csrc/m3_torch.cpp): the scan's and the mixer's autograd nodes."""
+    global _ext
+    if _ext is None:
+        load()
+        import torch  # noqa: F401  (its libraries are what the extension links to)
+
+        from .error import from_status
+        path = _LIB_PATH.parent / "_m3torch.so"
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: build it with `python -m mamba_trainer_b200.build` "
+                               "(there is no fallback implementation)")
+        import importlib.util
+        spec = importlib.util.spec_from_file_location("mamba_trainer_b200._m3torch", str(path))
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_from_status(from_status)
+        _ext = mod
+    return _ext

@@ -404,6 +404,7 @@ int m3_ctx_destroy(m3_ctx* ctx) {
 
 int m3_ctx_set_stream(m3_ctx* ctx, void* cuda_stream) {
   if (!ctx) return M3_ERR_NULL;
+  if (!ctx->own_stream && ctx->stream == cuda_stream) return M3_OK;
   if (ctx->own_stream && ctx->stream) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);

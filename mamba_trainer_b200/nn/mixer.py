@@ -12,7 +12,6 @@ Every step runs in libm3scan (m3_mixer_forward, m3_mixer_backward, m3_mixer_wind
 """
 from __future__ import annotations
 
-import ctypes as C
 from dataclasses import dataclass
 from functools import cached_property
 from typing import Optional
@@ -22,14 +21,7 @@ import torch
 from .. import _ffi
 from ..error import ConfigError, ShapeError, UnsupportedError
 from ..ssm.config import Discretization
-from ..ssm.scan import Context, SsmState, _DTYPES, _Saved
-
-
-def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    """t as a dense float32 tensor outside the tape; itself when it is one already."""
-    if t is None or (t.dtype is torch.float32 and t.is_contiguous()):
-        return t
-    return t.detach().to(torch.float32).contiguous()
+from ..ssm.scan import Context, SsmState, _DTYPES
 
 
 # The parameters in the order of m3_mixer_desc.
@@ -84,47 +76,6 @@ class MixerCache:
     ssm: SsmState
 
 
-class _MixerCore(torch.autograd.Function):
-    """The node: forward = m3_mixer_forward, backward rule = m3_mixer_backward.  `o` is the m3_mixer_desc of the call with
-    the gated output's width; the tensors it points into are the other arguments (float32, dense)."""
-
-    @staticmethod
-    def forward(fctx, o, proj, *par):
-        desc, width = o
-        ctx = Context.for_device(proj.device)
-        lib = ctx.lib
-        B, T, _ = proj.shape
-        out = torch.empty((B, T, width), device=proj.device, dtype=proj.dtype)
-        act = torch.empty(lib.m3_mixer_activation_bytes(desc), device=proj.device, dtype=torch.uint8)
-        track = any(fctx.needs_input_grad)
-        saved = C.c_void_p()
-        rc = lib.m3_mixer_forward(ctx.handle, desc, out.data_ptr(), act.data_ptr(), C.byref(saved) if track else None)
-        if rc:
-            ctx.check(rc)
-        if track:
-            fctx.m3, fctx.desc = ctx, desc
-            fctx.saved = _Saved(ctx, saved)
-            fctx.keep = (proj, act) + par
-        return out
-
-    @staticmethod
-    def backward(fctx, dout):
-        ctx, desc = fctx.m3, fctx.desc
-        ctx.bind_current_stream()
-        proj, act = fctx.keep[:2]
-        dev = proj.device
-        dout = dout.contiguous()
-        dproj = torch.empty_like(proj)
-        grads = [None if t is None else torch.empty_like(t) for t in fctx.keep[2:]]
-        work = torch.empty(ctx.lib.m3_mixer_backward_bytes(desc), device=dev, dtype=torch.uint8)
-        rc = ctx.lib.m3_mixer_backward(
-            ctx.handle, desc, fctx.saved.handle, act.data_ptr(), dout.data_ptr(),
-            _ffi.PACK_MIXER_GRADS.pack(dproj.data_ptr(), *[0 if t is None else t.data_ptr() for t in grads]), work.data_ptr())
-        if rc:
-            ctx.check(rc)
-        return (None, dproj, *grads)
-
-
 class MixerCore(torch.nn.Module):
     """Parameters and forward of the mixer between its projections (src/models/mamba3.rs:140-270 for
     the parameters; float32 masters, activations float32 or bfloat16)."""
@@ -172,15 +123,12 @@ class MixerCore(torch.nn.Module):
         return MixerCache(torch.zeros((batch, self.conv_w.shape[0] - 1, s.conv_channels), device=device, dtype=dtype),
                           SsmState.zeros(batch, s.heads, s.head_dim, s.d_state, s.rotational, device))
 
-    def _pack_desc(self, proj: torch.Tensor, par, path: int = _ffi.PATH_AUTO) -> bytes:
-        """The library's description (m3_mixer_desc) of this mixer on `proj`, with parameters `par` (in _PARAMS' order)."""
-        s = self.shape
-        B, T, _ = proj.shape
-        return _ffi.PACK_MIXER_DESC.pack(
-            B, T, s.heads, s.head_dim, s.d_state, s.rank, s.n_groups, self.chunk, _DTYPES[proj.dtype], self.disc,
-            s.rotational, self._parameters["conv_w"].shape[0], self.use_norm, self.post_gate_norm, path,
-            s.heads // 2 if self.bidirectional else 0, self.eps, 0,
-            proj.data_ptr(), *[0 if t is None else t.data_ptr() for t in par])
+    def _spec(self, path: int = _ffi.PATH_AUTO):
+        """The parameters in _PARAMS' order, the integers of m3_mixer_desc, eps and d_inner: what the native node takes."""
+        s, p = self.shape, self._parameters
+        return ([p[n] for n in _PARAMS],
+                (s.heads, s.head_dim, s.d_state, s.rank, s.n_groups, self.chunk, self.disc, s.rotational, self.use_norm,
+                 self.post_gate_norm, path, s.heads // 2 if self.bidirectional else 0), self.eps, s.d_inner)
 
     def forward_cached(self, proj: torch.Tensor, cache: Optional[MixerCache] = None):
         """Inference with a carried state (Mamba3Mixer::apply_with_state, src/models/mamba3.rs:486-560):
@@ -191,41 +139,23 @@ class MixerCore(torch.nn.Module):
             raise ShapeError(f"expected [batch, seq, {s.in_proj_width}], got {tuple(proj.shape)}")
         if self.bidirectional:
             raise UnsupportedError("a bidirectional mixer has no causal state to carry")   # mamba3.rs:494-499
-        proj = proj.detach() if proj.is_contiguous() else proj.detach().contiguous()
-        dev, el = proj.device, proj.dtype
-        ctx = Context.for_device(dev)
-        B, T, _ = proj.shape
+        if proj.dtype not in _DTYPES:
+            raise UnsupportedError(f"element type {proj.dtype}: float32 and bfloat16 are served")
+        B = proj.shape[0]
         H, P, N = s.heads, s.head_dim, s.d_state
         if cache is None:
-            cache = self.empty_cache(B, dev, el)
+            cache = self.empty_cache(B, proj.device, proj.dtype)
         st = cache.ssm
-        conv = cache.conv
-        if conv.dtype is not el or not conv.is_contiguous():
-            conv = conv.to(el).contiguous()
-        h, lu = _f32(st.h), _f32(st.last_u)
-        ang = _f32(st.angle) if s.rotational else None
         K = self._parameters["conv_w"].shape[0]
-        if conv.shape != (B, K - 1, s.conv_channels):
-            raise ShapeError(f"the cache's convolution history has shape {tuple(conv.shape)}, expected "
+        if cache.conv.shape != (B, K - 1, s.conv_channels):
+            raise ShapeError(f"the cache's convolution history has shape {tuple(cache.conv.shape)}, expected "
                              f"{(B, K - 1, s.conv_channels)}")
-        if h.shape != (B, H, P, N) or lu.shape != (B, H, P, N) or (ang is not None and ang.shape != (B, H, N // 2)):
+        if st.h.shape != (B, H, P, N) or st.last_u.shape != (B, H, P, N) or (
+                s.rotational and st.angle is not None and st.angle.shape != (B, H, N // 2)):
             raise ShapeError(f"the cache's state does not match batch {B}, heads {H}, head_dim {P}, d_state {N}")
-        par = [_f32(self._parameters[n]) for n in _PARAMS]
-        desc = self._pack_desc(proj, par)
-        out = torch.empty((B, T, s.d_inner), device=dev, dtype=el)
-        conv2 = torch.empty_like(conv)
-        h2, lu2 = torch.empty_like(h), torch.empty_like(lu)
-        ang2 = torch.empty((B, H, N // 2), device=dev, dtype=torch.float32) if s.rotational else None
-        io = _ffi.PACK_MIXER_WINDOW_IO.pack(
-            conv.data_ptr(), h.data_ptr(), lu.data_ptr(), 0 if ang is None else ang.data_ptr(), out.data_ptr(),
-            conv2.data_ptr(), h2.data_ptr(), lu2.data_ptr(), 0 if ang2 is None else ang2.data_ptr())
-        lib = ctx.lib
-        n = lib.m3_mixer_window_bytes(desc, io)
-        work = torch.empty(n, device=dev, dtype=torch.uint8) if n else None
-        rc = lib.m3_mixer_window(ctx.handle, desc, io, work.data_ptr() if n else None)
-        if rc:
-            ctx.check(rc)
-        return out, MixerCache(conv2, SsmState(h2, lu2, ang2))
+        out, conv, h, last_u, angle = _ffi.extension().window(
+            Context.of(proj.device).handle.value, proj, *self._spec(), cache.conv, st.h, st.last_u, st.angle)
+        return out, MixerCache(conv, SsmState(h, last_u, angle))
 
     def forward(self, proj: torch.Tensor, path: int = _ffi.PATH_AUTO) -> torch.Tensor:
         """proj: the input projection's output [batch, seq, in_proj_width]; returns the gated scan
@@ -240,8 +170,4 @@ class MixerCore(torch.nn.Module):
         # reversed in memory.
         if proj.shape[1] == 0:                      # nothing to scan (scan.rs:134-144)
             return proj.new_zeros((proj.shape[0], 0, s.d_inner)) + 0.0 * proj.sum()
-        proj = proj.contiguous()
-        p = self._parameters
-        par = [t if t is None or (t.dtype is torch.float32 and t.is_contiguous()) else t.to(torch.float32).contiguous()
-               for t in (p[n] for n in _PARAMS)]
-        return _MixerCore.apply((self._pack_desc(proj, par, path), s.d_inner), proj, *par)
+        return _ffi.extension().mixer(Context.of(proj.device).handle.value, proj, *self._spec(path))

@@ -3,7 +3,7 @@
 `ScanInputs`, `ScanOutput`, `SsmState` and `mamba3_scan` keep the names, argument
 meaning and error behaviour of src/ssm/scan.rs (:294-358, :361-443, :446-452,
 :458-618).  Where the reference composes ~25 differentiable primitives and lets its
-tape derive the backward pass, this module registers ONE node whose backward rule is
+tape derive the backward pass, this module registers ONE node (csrc/m3_torch.cpp) whose backward rule is
 the library's hand-written adjoint - the arrangement `Var::record_with_mask`
 (src/autograd/var.rs:169-204) gives a fused op in the reference.  PyTorch supplies
 device memory, streams and the tape; all arithmetic happens in libm3scan.so.
@@ -40,24 +40,28 @@ class Context:
         if rc != _ffi.OK:
             raise from_status(rc, f"m3_ctx_create({device_index}) failed")
         self.handle = handle
-        self._stream = None
 
     @classmethod
     def for_device(cls, device: torch.device) -> "Context":
+        """The device's context, bound to torch's current stream."""
+        ctx = cls.of(device)
+        ctx.bind_current_stream()
+        return ctx
+
+    @classmethod
+    def of(cls, device: torch.device) -> "Context":
+        """The device's context, for the native nodes, which bind the stream themselves."""
         if device.type != "cuda":
             raise UnsupportedError(f"the fused scan runs on CUDA devices only, got {device}")
         idx = device.index if device.index is not None else torch.cuda.current_device()
         ctx = cls._by_device.get(idx)
         if ctx is None:
             ctx = cls._by_device[idx] = Context(idx)
-        ctx.bind_current_stream()
         return ctx
 
     def bind_current_stream(self) -> None:
-        stream = _current_stream(self.device_index)
-        if stream != self._stream:
-            self.check(self.lib.m3_ctx_set_stream(self.handle, C.c_void_p(stream)))
-            self._stream = stream
+        # (every time: the native nodes bind the stream of their own calls)
+        self.check(self.lib.m3_ctx_set_stream(self.handle, _current_stream(self.device_index)))
 
     def check(self, rc: int) -> None:
         if rc != _ffi.OK:
@@ -187,79 +191,6 @@ class ScanOutput:
 
 def _ptr(t: Optional[torch.Tensor]):
     return C.c_void_p(t.data_ptr()) if t is not None else None
-
-
-class _FusedScan(torch.autograd.Function):
-    """The fused node: forward = m3_scan_forward, backward rule = m3_scan_backward."""
-
-    @staticmethod
-    def forward(fctx, opts, x, b, c, dt, a_log, lam, theta, d_skip, h0, last_u0, angle0):
-        ctx = Context.for_device(x.device)
-        B, T, H, P, R = x.shape
-        N = b.shape[3]
-        desc = _ffi.ScanDesc(
-            batch=B, seq=T, heads=H, head_dim=P, d_state=N, rank=R, chunk=int(opts["chunk"]),
-            dtype=_DTYPES[x.dtype], discretization=int(opts["disc"]),
-            dynamics=1 if theta is not None else 0, want_state=1 if opts["want_state"] else 0,
-            path=int(opts["path"]), reverse_heads=int(opts.get("rev", 0)),
-            x=_ptr(x), b=_ptr(b), c=_ptr(c), dt=_ptr(dt), lambda_=_ptr(lam), theta=_ptr(theta),
-            a_log=_ptr(a_log), d_skip=_ptr(d_skip), h0=_ptr(h0), last_u0=_ptr(last_u0), angle0=_ptr(angle0))
-        y = torch.empty_like(x)
-        h = lu = ang = None
-        if opts["want_state"]:
-            h = torch.empty((B, H, P, N), device=x.device, dtype=torch.float32)
-            lu = torch.empty((B, H, P, N), device=x.device, dtype=torch.float32)
-            if theta is not None:
-                ang = torch.empty((B, H, N // 2), device=x.device, dtype=torch.float32)
-        out = _ffi.ScanOut(y=_ptr(y), h=_ptr(h), last_u=_ptr(lu), angle=_ptr(ang))
-        tensors = (x, b, c, dt, a_log, lam, theta, d_skip, h0, last_u0, angle0)
-        # forward runs with grad mode off, so ask the node which parents are tracked
-        # (the `wanted` mask of Var::record_with_mask); none => inference, no rule built.
-        track = any(fctx.needs_input_grad)
-        saved = C.c_void_p()
-        ctx.check(ctx.lib.m3_scan_forward(ctx.handle, C.byref(desc), C.byref(out),
-                                          C.byref(saved) if track else None))
-        if track:
-            fctx.m3 = ctx
-            fctx.saved = _Saved(ctx, saved)
-            fctx.save_for_backward(*[t for t in tensors if t is not None])
-            fctx.present = [t is not None for t in tensors]
-            fctx.set_materialize_grads(False)
-        outs = [y] + [t for t in (h, lu, ang) if t is not None]
-        fctx.n_state_out = len(outs) - 1
-        fctx.has_angle = ang is not None
-        return tuple(outs)
-
-    @staticmethod
-    def backward(fctx, dy, *dstate):
-        ctx = fctx.m3
-        ctx.bind_current_stream()
-        it = iter(fctx.saved_tensors)
-        x, b, c, dt, a_log, lam, theta, d_skip, h0, lu0, ang0 = (
-            next(it) if p else None for p in fctx.present)
-        dstate = list(dstate) + [None] * (3 - len(dstate))
-        dh, dlu, dang = dstate[0], dstate[1], dstate[2] if fctx.has_angle else None
-        if dy is None:
-            dy = torch.zeros_like(x)
-        need = fctx.needs_input_grad[1:]
-        names = ("x", "b", "c", "dt", "a_log", "lam", "theta", "d_skip", "h0", "lu0", "ang0")
-        inputs = dict(zip(names, (x, b, c, dt, a_log, lam, theta, d_skip, h0, lu0, ang0)))
-        grads, mask = {}, 0
-        for i, name in enumerate(names):
-            t = inputs[name]
-            if t is not None and need[i]:
-                grads[name] = torch.empty_like(t)
-                mask |= 1 << i
-        cont = lambda t: t.contiguous() if t is not None else None
-        dy, dh, dlu, dang = cont(dy), cont(dh), cont(dlu), cont(dang)
-        bin_ = _ffi.ScanBwdIn(dy=_ptr(dy), dh=_ptr(dh), dlast_u=_ptr(dlu), dangle=_ptr(dang))
-        g = lambda n: _ptr(grads.get(n))
-        gout = _ffi.ScanGrads(dx=g("x"), db=g("b"), dc=g("c"), ddt=g("dt"), dlambda=g("lam"),
-                              dtheta=g("theta"), da_log=g("a_log"), dd_skip=g("d_skip"),
-                              dh0=g("h0"), dlast_u0=g("lu0"), dangle0=g("ang0"))
-        ctx.check(ctx.lib.m3_scan_backward(ctx.handle, fctx.saved.handle, C.byref(bin_),
-                                           C.c_uint32(mask), C.byref(gout)))
-        return (None,) + tuple(grads.get(n) for n in names)
 
 
 class _FusedSsd(torch.autograd.Function):
@@ -447,15 +378,11 @@ def mamba3_scan(inputs: ScanInputs) -> ScanOutput:
             state = st.clone() if st is not None else SsmState.zeros(B, H, P, N, theta is not None, x.device)
         return ScanOutput(x, state)
 
-    el = x.dtype
-    big = lambda t: None if t is None else t.to(el).contiguous()
-    f32 = lambda t: None if t is None else t.to(torch.float32).contiguous()
-    opts = {"chunk": inputs.chunk_size, "disc": int(disc), "want_state": bool(inputs.want_state),
-            "path": inputs.path, "rev": inputs.reverse_heads}
-    outs = _FusedScan.apply(
-        opts, x.contiguous(), big(b), big(c), big(inputs.dt), f32(inputs.a_log), big(lam), big(theta),
-        f32(inputs.d_skip), f32(st.h) if st else None, f32(st.last_u) if st else None,
-        f32(st.angle) if (st and theta is not None and st.angle is not None) else None)
+    # the node is native (csrc/m3_torch.cpp): it brings the inputs to x's element type, parameters and states to float32
+    outs = _ffi.extension().scan(
+        Context.of(x.device).handle.value, x, b, c, inputs.dt, inputs.a_log, lam, theta, inputs.d_skip, st.h if st else None,
+        st.last_u if st else None, st.angle if (st and theta is not None) else None, inputs.chunk_size, int(disc),
+        bool(inputs.want_state), inputs.path, inputs.reverse_heads)
     y = outs[0]
     state = None
     if inputs.want_state:
