@@ -4,9 +4,12 @@
 // A CTA works on one chunk of 64 rows rho = (t, r) (64 / R time steps) of one (batch, head); all chunks of all stripes
 // run at once and only the pass over chunk states is sequential (m3_rows_fwd.cu says which kernels there are).
 //
-// Contractions run on the tensor cores in split TF32: an operand x is hi + lo, hi = x rounded to TF32's 11 significant
-// bits, lo = the rest, and a product is lo hi + hi lo + hi hi with float32 accumulation, which keeps 23 of the 24 bits
-// of every product (what is dropped, lo lo and the last bit of lo, is below 2^-22).  mma.sync m16n8k8 runs 278 TFLOP/s
+// Contractions run on the tensor cores in split TF32: an operand x is hi + lo, hi = x cut to TF32's 11 significant
+// bits, lo = the rest rounded to as many, and a product is lo hi + hi lo + hi hi with float32 accumulation: what is
+// dropped (lo lo, and the rounding of lo) is below 2^-20 of a product and unbiased, as a float32 sum's own rounding is.
+// Fragments come four words at a time by ldmatrix where the operand is stored along the contraction (a word at a time,
+// with four operations for the split, the kernels were bound by issue: float32, 8 x 1024 x 16 heads, d_state 128: the
+// adjoint 478 -> 472 us, the outputs 166 -> 159 us; what bounds them now is the phases between block barriers).  mma.sync m16n8k8 runs 278 TFLOP/s
 // on a B200, so 93 after the threefold product, against 51 measured for float32 FMAs from registers (and half of that
 // in the 64 x 64 block products of the generic family).  tcgen05's kind::tf32 would be faster still, but wants every
 // operand K-major in shared memory: half of the operands here are contracted along their rows.  An operand whose values
@@ -29,9 +32,18 @@ __host__ __device__ __forceinline__ constexpr int fsw(int row) { return ((row & 
 template <int LD>
 __device__ __forceinline__ int at(int row, int col) { return row * LD + (col ^ fsw(row)); }
 
+// The tensor core reads the upper 19 bits of a TF32 operand, so x as it stands is its own hi part (truncated); lo is what
+// truncation leaves, rounded to the bits that will be read (half of the last one added): three operations.
 __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;   // round to nearest (ties away), 13 bits dropped
-  lo = __float_as_uint(x - __uint_as_float(hi)) & 0xffffe000u;
+  hi = __float_as_uint(x);
+  lo = __float_as_uint(x - __uint_as_float(hi & 0xffffe000u)) + 0x1000u;
+}
+// Four 8-row x 4-column pieces of float32 by one instruction: word q of row g of each is this lane's.
+__device__ __forceinline__ void ldm4f(uint32_t (&r)[4], const float* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p))
+               : "memory");
 }
 __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
   asm volatile(
@@ -47,45 +59,53 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
 template <int MT, int NT, bool AKC, bool BKC, bool AEX, bool BEX, int LDA, int LDB>
 __device__ __forceinline__ void warp_mma(float (&acc)[MT][NT][4], const float* sA, int m0, const float* sB, int n0, int k0,
                                          int k1) {
+  static_assert(!BKC || NT % 2 == 0, "a load brings two column tiles");
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  const int fg = fsw(g), fq = fsw(q), fq4 = fq ^ 4;
+  const int fq = fsw(q), fq4 = fq ^ 4, f7 = fsw(lane & 7);
+  // this lane's row and column group in a load of four pieces (operands stored along k)
+  const float* pa = sA + (m0 + (lane & 15)) * LDA;
+  const float* pb = sB + (n0 + (lane & 7) + ((lane >> 4) << 3)) * LDB;
+  const int ka = (lane >> 4) << 2, kb = ((lane >> 3) & 1) << 2;
 #pragma unroll 2
   for (int k = k0; k < k1; k += 8) {
     uint32_t ah[MT][4], al[MT][4], bh[NT][2], bl[NT][2];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
-      const int m = m0 + 16 * mt + g;
-      float v[4];
       if (AKC) {
-        const float* r0 = sA + m * LDA;
-        const float* r1 = r0 + 8 * LDA;
-        const int c0 = (k + q) ^ fg, c1 = (k + q + 4) ^ fg;
-        v[0] = r0[c0]; v[1] = r1[c0]; v[2] = r0[c1]; v[3] = r1[c1];
+        ldm4f(ah[mt], pa + 16 * mt * LDA + ((k + ka) ^ f7));
       } else {
+        const int m = m0 + 16 * mt + g;
         const float* r0 = sA + (k + q) * LDA;
         const float* r1 = r0 + 4 * LDA;
-        v[0] = r0[m ^ fq]; v[1] = r0[(m + 8) ^ fq]; v[2] = r1[m ^ fq4]; v[3] = r1[(m + 8) ^ fq4];
+        ah[mt][0] = __float_as_uint(r0[m ^ fq]); ah[mt][1] = __float_as_uint(r0[(m + 8) ^ fq]);
+        ah[mt][2] = __float_as_uint(r1[m ^ fq4]); ah[mt][3] = __float_as_uint(r1[(m + 8) ^ fq4]);
       }
+      if (!AEX) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (AEX) ah[mt][i] = __float_as_uint(v[i]); else split_tf32(v[i], ah[mt][i], al[mt][i]);
+        for (int i = 0; i < 4; ++i) split_tf32(__uint_as_float(ah[mt][i]), ah[mt][i], al[mt][i]);
       }
     }
+    if (BKC) {
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const int n = n0 + 8 * nt + g;
-      float v[2];
-      if (BKC) {
-        const float* r0 = sB + n * LDB;
-        v[0] = r0[(k + q) ^ fg]; v[1] = r0[(k + q + 4) ^ fg];
-      } else {
+      for (int np = 0; np < NT / 2; ++np) {
+        uint32_t r[4];
+        ldm4f(r, pb + 16 * np * LDB + ((k + kb) ^ f7));
+        bh[2 * np][0] = r[0]; bh[2 * np][1] = r[1];
+        bh[(2 * np + 1) % NT][0] = r[2]; bh[(2 * np + 1) % NT][1] = r[3];
+      }
+    } else {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int n = n0 + 8 * nt + g;
         const float* r0 = sB + (k + q) * LDB;
-        v[0] = r0[n ^ fq]; v[1] = r0[4 * LDB + (n ^ fq4)];
+        bh[nt][0] = __float_as_uint(r0[n ^ fq]); bh[nt][1] = __float_as_uint(r0[4 * LDB + (n ^ fq4)]);
       }
+    }
+    if (!BEX) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        if (BEX) bh[nt][i] = __float_as_uint(v[i]); else split_tf32(v[i], bh[nt][i], bl[nt][i]);
-      }
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) split_tf32(__uint_as_float(bh[nt][i]), bh[nt][i], bl[nt][i]);
     }
     if (!AEX) {
 #pragma unroll
