@@ -79,14 +79,19 @@ __global__ void __launch_bounds__(256) k_rows_seed(Dims d, m3_scan_desc in, Rows
   if (threadIdx.x == 0) ip0[bh] = s;
 }
 
-constexpr int kAdj = 512;   // threads of k_rows_adjoint: 16 warps, one CTA per SM (177 KB of shared memory at d_state 128)
+// Threads of k_rows_adjoint.  d_state 128: 16 warps, one CTA per SM (177 KB of shared memory).  d_state 64: 8 warps with
+// tiles twice as wide, so that two CTAs share an SM and one's products run beside the other's loads and epilogues
+// (bf16, 4 x 1500 tokens x 8 heads: 120 -> 93 us).
+template <int N>
+constexpr int kAdjThreads = N == 64 ? 256 : 512;
 template <int N, int R>
 struct AdjSmem {
+  static constexpr int kThreads = kAdjThreads<N>, WC = kThreads / 128, WN = kThreads / 64;   // warp columns: see the kernel
   float c[kRows * N], b[kRows * N], x[kRows * kP], dy[kRows * kP];
   float hs[2 * kRows * N];   // H_k and dS_k; then M and dG; then dB and dC on their way out
   float phi[(kRows / R) * (N / 2)];
-  float row[4][kRows], col[4][kRows], dw[4][kRows], dg[4][kRows], q[4][kRows], t1[8][kRows];   // partial sums per warp column / row
-  float sq[kAdj], red[16], dac[kRows / R], dast[kRows / R];
+  float row[WC][kRows], col[4][kRows], dw[4][kRows], dg[WC][kRows], q[WC][kRows], t1[WN][kRows];   // partial sums per warp column / row
+  float sq[kThreads], red[16], dac[kRows / R], dast[kRows / R];
   Scal<R> s;
 };
 
@@ -95,6 +100,7 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 
 // Sum over the block; complete for every thread.
+template <int kAdj>
 __device__ __forceinline__ float adj_sum(float v, float* red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -107,6 +113,8 @@ __device__ __forceinline__ float adj_sum(float v, float* red) {
   return s;
 }
 
+static_assert(sizeof(AdjSmem<64, 1>) <= 115712, "two CTAs share an SM");
+
 template <class T>
 struct AdjOut {
   T *dx, *db, *dc;                  // NULL skips the store
@@ -116,11 +124,11 @@ struct AdjOut {
 };
 
 template <class T, int N, int R, bool ROT>
-__global__ void __launch_bounds__(kAdj, 1) k_rows_adjoint(Dims d, m3_scan_desc in, const T* __restrict__ dy, RowsWs ws,
+__global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoint(Dims d, m3_scan_desc in, const T* __restrict__ dy, RowsWs ws,
                                                           RowsBwdWs rw, AdjOut<T> out) {
   extern __shared__ __align__(16) unsigned char smem[];
   AdjSmem<N, R>& sm = *reinterpret_cast<AdjSmem<N, R>*>(smem);
-  constexpr int NH = N / 2, PN = kP * N, LT = kRows / R;
+  constexpr int NH = N / 2, PN = kP * N, LT = kRows / R, kAdj = kAdjThreads<N>;
   constexpr bool EX = sizeof(T) == 2;   // x and dy of a bf16 tensor are exact in TF32
   const Chunk c = this_chunk(d);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q4 = lane & 3;
@@ -152,16 +160,18 @@ __global__ void __launch_bounds__(kAdj, 1) k_rows_adjoint(Dims d, m3_scan_desc i
   __syncthreads();
   const Scal<R>& ts = sm.s;
   // ---- products that need the states ------------------------------------------------------------------------
-  constexpr int NT = N / 64;   // [64 x N] results: warps 2 (32 rows) x 8 (N / 8 columns)
+  constexpr int WC = AdjSmem<N, R>::WC, WN = AdjSmem<N, R>::WN;
+  constexpr int NT = N / (8 * WN);   // [64 x N] results: warps 2 (32 rows) x WN
   const int wm = warp & 1, wn = warp >> 1, M0 = 32 * wm, N0 = 8 * NT * wn;
-  const int m0 = 16 * (warp & 3), n0 = 16 * (warp >> 2);   // [64 x 64] results: warps 4 x 4
-  float dc[2][NT][4], db[2][NT][4], dx[1][2][4];
+  constexpr int NX = 8 / WC;         // [64 x 64] results: warps 4 (16 rows) x WC
+  const int m0 = 16 * (warp & 3), n0 = 8 * NX * (warp >> 2);
+  float dc[2][NT][4], db[2][NT][4], dx[1][NX][4];
   zero(dc);
   zero(db);
   zero(dx);
   warp_mma<2, NT, true, false, EX, false, kP, N>(dc, sm.dy, M0, sH, N0, 0, kP);   // T1 = dY~ H_k
   warp_mma<2, NT, true, false, EX, false, kP, N>(db, sm.x, M0, sS, N0, 0, kP);    // X~ dS_k
-  warp_mma<1, 2, true, true, false, false, N, N>(dx, sm.b, m0, sS, n0, 0, N);     // U = B^ dS_k^T
+  warp_mma<1, NX, true, true, false, false, N, N>(dx, sm.b, m0, sS, n0, 0, N);     // U = B^ dS_k^T
   {
     float t1[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};   // <T1, C^> of the rows
     for_acc(dc, M0, N0, [&](int row, int col, float& a, float& b) {
@@ -210,21 +220,23 @@ __global__ void __launch_bounds__(kAdj, 1) k_rows_adjoint(Dims d, m3_scan_desc i
     }
   }
   // ---- the band: G = C^ B^^T, dM = dY~ X~^T below the diagonal ------------------------------------------------
-  float gm[1][2][4], dm[1][2][4];
+  float gm[1][NX][4], dm[1][NX][4];
   zero(gm);
   zero(dm);
   const bool below = n0 < m0 + 16;
   if (below) {
-    warp_mma<1, 2, true, true, false, false, N, N>(gm, sm.c, m0, sm.b, n0, 0, N);
-    warp_mma<1, 2, true, true, EX, EX, kP, kP>(dm, sm.dy, m0, sm.x, n0, 0, kP);
+    warp_mma<1, NX, true, true, false, false, N, N>(gm, sm.c, m0, sm.b, n0, 0, N);
+    warp_mma<1, NX, true, true, EX, EX, kP, kP>(dm, sm.dy, m0, sm.x, n0, 0, kP);
   }
-  dcd = adj_sum(dcd, sm.red);   // the states have been read by everyone: M and dG take their place
-  dD = adj_sum(dD, sm.red);
+  dcd = adj_sum<kAdj>(dcd, sm.red);   // the states have been read by everyone: M and dG take their place
+  dD = adj_sum<kAdj>(dD, sm.red);
   {
     float rowE[2] = {0.0f, 0.0f}, dgp[2] = {0.0f, 0.0f};
-    float colE[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}}, dwE[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+    float colE[NX][2], dwE[NX][2];
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+    for (int nt = 0; nt < NX; ++nt) colE[nt][0] = colE[nt][1] = dwE[nt][0] = dwE[nt][1] = 0.0f;
+#pragma unroll
+    for (int nt = 0; nt < NX; ++nt)
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         const int row = m0 + 8 * hh + g, l = row / R;
@@ -261,7 +273,7 @@ __global__ void __launch_bounds__(kAdj, 1) k_rows_adjoint(Dims d, m3_scan_desc i
       }
     }
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+    for (int nt = 0; nt < NX; ++nt)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const float a = group_sum(colE[nt][j]), b = group_sum(dwE[nt][j]);
@@ -273,7 +285,7 @@ __global__ void __launch_bounds__(kAdj, 1) k_rows_adjoint(Dims d, m3_scan_desc i
   }
   __syncthreads();
   // ---- dX~ += M^T dY~, dB^ += dG^T C^, dC^ += dG B^ (only the triangle's half of each sum) ---------------------
-  warp_mma<1, 2, false, false, false, EX, kRows, kP>(dx, sM, m0, sm.dy, n0, m0, kRows);
+  warp_mma<1, NX, false, false, false, EX, kRows, kP>(dx, sM, m0, sm.dy, n0, m0, kRows);
   warp_mma<2, NT, false, false, false, false, kRows, N>(db, sG, M0, sm.c, N0, M0, kRows);
   warp_mma<2, NT, true, false, false, false, kRows, N>(dc, sG, M0, sm.b, N0, 0, M0 + 32);
   __syncthreads();   // M, dG and dY~ are spent
@@ -374,15 +386,18 @@ __global__ void __launch_bounds__(kAdj, 1) k_rows_adjoint(Dims d, m3_scan_desc i
     for (int r = 0; r < R; ++r) {
       const int ro = l * R + r;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < WC; ++i) {
         rows_ += sm.row[i][ro];
         dgv += sm.dg[i][ro];
         q += sm.q[i][ro];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
         col += sm.col[i][ro];
         dwv += sm.dw[i][ro];
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) t1 += sm.t1[i][ro];
+      for (int i = 0; i < WN; ++i) t1 += sm.t1[i][ro];
     }
     const float ac = ts.ac[l], raw = cd - ac, sg = exp_decay(raw);
     const float dast = sg * ts.w[l] * q * clamp_inside(raw);
@@ -514,7 +529,7 @@ cudaError_t backward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, c
   const AdjOut<T> out{static_cast<T*>(want(M3_GRAD_X, g.dx)), static_cast<T*>(want(M3_GRAD_B, g.db)),
                       static_cast<T*>(want(M3_GRAD_C, g.dc)), bw.da, bw.dg, bw.dw, bw.partA, bw.partD,
                       d.raw ? nullptr : up.dlast_u, up.dangle};
-  k_rows_adjoint<T, N, R, ROT><<<grid, kAdj, sizeof(AdjSmem<N, R>), st>>>(d, in, static_cast<const T*>(up.dy), ws, rw, out);
+  k_rows_adjoint<T, N, R, ROT><<<grid, kAdjThreads<N>, sizeof(AdjSmem<N, R>), st>>>(d, in, static_cast<const T*>(up.dy), ws, rw, out);
   if (has_state) {
     k_rows_seed<T, N><<<d.B * d.H, 256, 0, st>>>(d, in, rw, bw.ip0, static_cast<float*>(want(M3_GRAD_H0, g.dh0)),
                                                  d.raw ? nullptr : static_cast<float*>(want(M3_GRAD_LAST_U0, g.dlast_u0)));

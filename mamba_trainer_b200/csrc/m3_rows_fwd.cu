@@ -130,7 +130,7 @@ struct OutSmem {
   Scal<R> s;
 };
 template <class T, int N, int R, bool ROT>
-__global__ void __launch_bounds__(256, 2) k_rows_out(Dims d, m3_scan_desc in, RowsWs ws, T* __restrict__ y,
+__global__ void __launch_bounds__(256, N == 64 ? 3 : 2) k_rows_out(Dims d, m3_scan_desc in, RowsWs ws, T* __restrict__ y,
                                                      float* __restrict__ last_u) {
   extern __shared__ __align__(16) unsigned char smem[];
   OutSmem<N, R>& sm = *reinterpret_cast<OutSmem<N, R>*>(smem);
