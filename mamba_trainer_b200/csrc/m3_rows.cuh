@@ -329,7 +329,9 @@ __device__ __forceinline__ void load_rotated(float* const (&dst)[NTENS], const T
     const float sc = scale ? scale[l] : 1.0f;
 #pragma unroll
     for (int j = 0; j < NA; ++j) {
-      sincosf(phi[l * NH + e / R + j], &sn[j], &cs[j]);
+      // (the angle is wrapped: the special-function unit's sine is good to 2^-21 there, far below a bf16 operand)
+      if (BF) __sincosf(phi[l * NH + e / R + j], &sn[j], &cs[j]);
+      else sincosf(phi[l * NH + e / R + j], &sn[j], &cs[j]);
       cs[j] *= sc;
       sn[j] *= sc;
     }

@@ -2,13 +2,14 @@
 // side.  The stripe kernels keep the state in TMEM and walk a stripe tile by tile, so a launch of fewer stripes than SMs
 // leaves SMs idle however long the sequence is (16 stripes of 14 tiles: 94 us on 16 of 148 SMs).  Two short launches
 // come first here:
-//   k_tile_state  per 128-row tile, all tiles of all stripes at once: the tile's own contribution to the state,
+//   k_tile_state  per half tile (64 rows), all of all stripes at once: its own contribution to the state,
 //                 X~^T diag(sw) B^ (backward, to its gradient: (exp(acum) dY~)^T C^), its decay and its angle
-//   k_tile_pass   sequential over tiles, parallel over state elements: the state (and the angle) at every segment
+//   k_tile_pass   sequential over half tiles, parallel over state elements: the state (and the angle) at every segment
 //                 boundary, in the place where the stripe kernels expect what the segment before handed over
 // after which the segments are independent.  The contraction is mma.sync on operands rounded to bf16, like the stripe
 // kernels' own; accumulation and states are float32.  The price is one more reading of B and x (C and dy) and a state per
-// tile; tc_ahead_plan weighs it.
+// half tile; tc_ahead_plan weighs it.  (Whole tiles, two halves one after the other in a block, took 31 us for 224 tiles of
+// rank 1 where half tiles take 25: there are few blocks, so what counts is the chain inside one.)
 #include "m3_rows.cuh"
 #include "m3_tc.h"
 
@@ -20,66 +21,100 @@ constexpr int kN = 128, kNH = 64, kPN = kP * kN;
 
 template <int R>
 struct TileSmem {
-  float b[kRows * kN], x[kRows * kP], phi[(kRows / R) * kNH], q[256], base[kNH];
-  Scal<R> s[2];
+  float b[kRows * kN];
+  union {   // the angles are spent when x (from registers) takes their place: four blocks share an SM
+    float x[kRows * kP];
+    float phi[(kRows / R) * kNH];
+  };
+  float q[256], base[kNH];
+  Scal<R> s;
 };
 
-// A tile is two chunks of 64 rows.  Forward: rows rotated by the angle since the tile's start.  Backward: by the absolute
-// angle (the forward pass left the one entering every tile).
+// This thread's words of a half tile's rows of x or dy, and what load_rows makes of them.
+template <int R>
+struct RawRows {
+  static constexpr int PER = kP * R / 4, NI = (kRows / R) * PER / 256;
+  uint2 w[NI];
+  __device__ __forceinline__ void load(const __nv_bfloat16* src, const Dims& d, const Chunk& c) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int it = threadIdx.x + i * 256, l = it / PER, e = 4 * (it - l * PER), t = c.t0 + l;
+      w[i] = make_uint2(0u, 0u);
+      if (t < d.T) w[i] = __ldg(reinterpret_cast<const uint2*>(src + tok_index(d, c.b, t, c.h) * kP * R + e));
+    }
+  }
+  __device__ __forceinline__ void store(float* dst) const {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int it = threadIdx.x + i * 256, l = it / PER, e = 4 * (it - l * PER);
+      const float f[4] = {__uint_as_float(w[i].x << 16), __uint_as_float(w[i].x & 0xffff0000u), __uint_as_float(w[i].y << 16),
+                          __uint_as_float(w[i].y & 0xffff0000u)};
+      if (R == 1) {
+        *reinterpret_cast<float4*>(dst + at<kP>(l, e)) = make_float4(f[0], f[1], f[2], f[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dst[at<kP>(l * R + (e + j) % R, (e + j) / R)] = f[j];
+      }
+    }
+  }
+};
+
+// Forward: rows rotated by the angle since the half tile's start.  Backward: by the absolute angle; the forward pass left
+// the one entering every whole tile, so the second half adds up the first one's.
 template <int R, bool ROT, bool BWD>
-__global__ void __launch_bounds__(256, 3) k_tile_state(Dims d, m3_scan_desc in, const __nv_bfloat16* __restrict__ dy,
+__global__ void __launch_bounds__(256, 4) k_tile_state(Dims d, m3_scan_desc in, const __nv_bfloat16* __restrict__ dy,
                                                        const float* __restrict__ ckpt_angle, float* __restrict__ hs,
                                                        float* __restrict__ asum, float* __restrict__ cd_out) {
   using T = __nv_bfloat16;
   extern __shared__ __align__(16) unsigned char smem[];
   TileSmem<R>& sm = *reinterpret_cast<TileSmem<R>*>(smem);
   constexpr int LT = kRows / R;
-  Chunk c = this_chunk(d);
-  const int tile = c.k;
-  const size_t slot = (size_t)c.bh * d.C + tile;
-  c.t0 = tile * 2 * LT;
-  chunk_scalars<T, R>(sm.s[0], d, c, in);
-  c.t0 += LT;
-  chunk_scalars<T, R>(sm.s[1], d, c, in);
-  const float cd0 = sm.s[0].ac[LT - 1], cd1 = sm.s[1].ac[LT - 1];
-  if (threadIdx.x == 0) cd_out[slot] = cd0 + cd1;
-  if (threadIdx.x < LT) {   // the half farther from the end the state leaves by decays over the other half too
-    if (BWD) sm.s[1].eac[threadIdx.x] *= exp_decay(cd0);
-    else sm.s[0].sw[threadIdx.x] *= exp_decay(cd1);
+  const Chunk c = this_chunk(d);
+  const size_t slot = (size_t)c.bh * d.C + c.k;
+  const int tid = threadIdx.x;
+  RawRows<R> raw;
+  raw.load(BWD ? dy : static_cast<const T*>(in.x), d, c);
+  if (ROT && BWD) {
+    const int q = tid >> 6, m = tid & 63;
+    float s = q == 0 ? ckpt_angle[((size_t)c.bh * ((d.C + 1) / 2) + c.k / 2) * kNH + m] : 0.0f;
+    if (c.k & 1) {
+#pragma unroll
+      for (int i = 0; i < LT / 4; ++i) {
+        const int t = c.t0 - LT + q * (LT / 4) + i;   // the half before this one is whole
+        s += ldf(static_cast<const T*>(in.dt), tok_index(d, c.b, t, c.h)) *
+             ldf(static_cast<const T*>(in.theta), theta_index(d, c.b, t, c.h) + m);
+      }
+    }
+    sm.q[tid] = s;
   }
-  if (ROT && threadIdx.x < kNH) sm.base[threadIdx.x] = BWD ? ckpt_angle[slot * kNH + threadIdx.x] : 0.0f;
+  chunk_scalars<T, R>(sm.s, d, c, in);   // (its barriers also complete q)
+  if (tid == 0) cd_out[slot] = sm.s.ac[LT - 1];
+  const float* scale = BWD ? sm.s.eac : sm.s.sw;
+  const T* rows_in = static_cast<const T*>(BWD ? in.c : in.b);
+  if constexpr (ROT) {
+    if (tid < kNH) sm.base[tid] = BWD ? wrap_angle(sm.q[tid] + sm.q[tid + 64] + sm.q[tid + 128] + sm.q[tid + 192]) : 0.0f;
+    __syncthreads();
+    chunk_angles<T, kN, R, 256>(sm.phi, sm.q, sm.s, d, c, static_cast<const T*>(in.theta), sm.base,
+                                [&](int m, float sum) { if (!BWD) asum[slot * kNH + m] = sum; });
+    __syncthreads();
+    float* const to[1] = {sm.b};
+    const T* const from[1] = {rows_in};
+    load_rotated<T, kN, R, 256, 1, true>(to, from, sm.phi, scale, d, c);
+    __syncthreads();
+  } else {
+    load_scaled<T, kN, R, 256, true>(sm.b, rows_in, scale, d, c);
+  }
+  raw.store(sm.x);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, m0 = 32 * (warp & 1), n0 = 32 * (warp >> 1);
+  const int warp = tid >> 5, m0 = 32 * (warp & 1), n0 = 32 * (warp >> 1);
   float acc[2][4][4];
   zero(acc);
-#pragma unroll 1
-  for (int half = 0; half < 2; ++half) {
-    c.t0 = (tile * 2 + half) * LT;
-    if (c.t0 >= d.T && half) break;   // nothing but padding
-    const Scal<R>& s = sm.s[half];
-    const float* scale = BWD ? s.eac : s.sw;
-    load_rows<T, R, kP, 256>(sm.x, BWD ? dy : static_cast<const T*>(in.x), d, c);
-    const T* rows_in = static_cast<const T*>(BWD ? in.c : in.b);
-    if constexpr (ROT) {
-      chunk_angles<T, kN, R, 256>(sm.phi, sm.q, s, d, c, static_cast<const T*>(in.theta), sm.base, [](int, float) {});
-      __syncthreads();
-      if (threadIdx.x < kNH) sm.base[threadIdx.x] = sm.phi[(LT - 1) * kNH + threadIdx.x];   // wrapped
-      float* const to[1] = {sm.b};
-      const T* const from[1] = {rows_in};
-      load_rotated<T, kN, R, 256, 1, true>(to, from, sm.phi, scale, d, c);
-    } else {
-      load_scaled<T, kN, R, 256, true>(sm.b, rows_in, scale, d, c);
-    }
-    __syncthreads();
-    warp_mma<2, 4, false, false, true, true, kP, kN>(acc, sm.x, m0, sm.b, n0, 0, kRows);
-    __syncthreads();
-  }
+  warp_mma<2, 4, false, false, true, true, kP, kN>(acc, sm.x, m0, sm.b, n0, 0, kRows);
   store_acc<kN>(acc, m0, n0, hs + slot * kPN);
-  if (ROT && !BWD && threadIdx.x < kNH) asum[slot * kNH + threadIdx.x] = sm.base[threadIdx.x];
 }
 
-// A thread owns planes (m, m + 64) of rows p, p + 32 and walks the tiles in time (backward: against it); U tiles are
-// requested before the first is used.  seg_state / seg_angle of segment s: what leaves it towards the next one walked.
+// A thread owns planes (m, m + 64) of rows p, p + 32 and walks the half tiles in time (backward: against it); U of them
+// are requested before the first is used; tps is in half tiles here.  seg_state / seg_angle of segment s: what leaves it towards the next one walked.
 template <bool ROT, bool BWD>
 __global__ void __launch_bounds__(256) k_tile_pass(Dims d, m3_scan_desc in, const float* __restrict__ dh,
                                                    const float* __restrict__ hs, const float* __restrict__ asum,
@@ -154,7 +189,7 @@ cudaError_t ahead_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, cons
   if (e != cudaSuccess) return e;
   kern<<<dim3(d.C, d.B * d.H), 256, sizeof(TileSmem<R>), st>>>(d, in, static_cast<const __nv_bfloat16*>(dy), ckpt_angle, a.hs,
                                                               a.asum, a.cd);
-  k_tile_pass<ROT, BWD><<<dim3(32 * kNH / 256, d.B * d.H), 256, 0, st>>>(d, in, dh, a.hs, a.asum, a.cd, a.tps, a.nseg, a.seg_state,
+  k_tile_pass<ROT, BWD><<<dim3(32 * kNH / 256, d.B * d.H), 256, 0, st>>>(d, in, dh, a.hs, a.asum, a.cd, 2 * a.tps, a.nseg, a.seg_state,
                                                                         a.seg_angle);
   return cudaGetLastError();
 }
@@ -168,7 +203,7 @@ cudaError_t ahead_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, cons
 // third of the SMs too little is idle to pay for it.
 bool tc_ahead_plan(int BH, int tiles, bool backward, int* nseg, int* tps) {
   constexpr int kSms = 148;
-  if (BH > kSms / 3 || tiles < 3 || (size_t)BH * tiles > (1u << 15)) return false;   // at most 1 GB of tile states
+  if (BH > kSms / 3 || tiles < 3 || (size_t)BH * tiles > (1u << 14)) return false;   // at most 1 GB of states
   const float c = backward ? 15.0f : 5.5f;
   const float pre = 10.0f + 1.3f * (float)((BH * (long long)tiles + kSms - 1) / kSms) + 0.15f * tiles;
   float best = 0.9f * tiles * c;
@@ -195,9 +230,9 @@ size_t tc_ahead_bytes(int BH, int tiles, int nseg, TcAhead* a, char* base) {
     return p;
   };
   TcAhead t{};
-  t.hs = take((size_t)BH * tiles * rows::kPN);
-  t.asum = take((size_t)BH * tiles * rows::kNH);
-  t.cd = take((size_t)BH * tiles);
+  t.hs = take((size_t)BH * 2 * tiles * rows::kPN);
+  t.asum = take((size_t)BH * 2 * tiles * rows::kNH);
+  t.cd = take((size_t)BH * 2 * tiles);
   t.seg_state = take((size_t)BH * nseg * rows::kPN);
   t.seg_angle = take((size_t)BH * nseg * rows::kNH);
   if (a) {
@@ -210,8 +245,8 @@ size_t tc_ahead_bytes(int BH, int tiles, int nseg, TcAhead* a, char* base) {
 
 cudaError_t tc_ahead(cudaStream_t st, Dims d, const m3_scan_desc& in, const void* dy, const float* dh, const float* ckpt_angle,
                      const TcAhead& a) {
-  d.L = tc_tile_steps(d.R);
-  d.C = tc_tiles(d.T, d.R);
+  d.L = tc_tile_steps(d.R) / 2;
+  d.C = (d.T + d.L - 1) / d.L;   // (an odd number when the last tile has one half only)
   auto go = [&](auto r, auto rot) {
     return dy ? rows::ahead_t<r.value, rot.value, true>(st, d, in, dy, dh, ckpt_angle, a)
               : rows::ahead_t<r.value, rot.value, false>(st, d, in, nullptr, nullptr, nullptr, a);
