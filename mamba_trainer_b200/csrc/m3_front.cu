@@ -321,6 +321,9 @@ __global__ void __launch_bounds__(kWarps * 32, 3) k_front_fwd(Front f, FrontOut 
   }
 }
 
+constexpr int kAhead = 8;   // steps by which the backward walk's rows are brought into L2 before they are loaded
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // ---- backward ----------------------------------------------------------------------------------------------------
 // Partial sums of a block (blockIdx.y, blockIdx.z): taps and bias of its channels, [K + 1][di + 2 bc]; for its B / C
 // channels the gradients of the bias [bc-channel] (summed over ranks afterwards) and of the gain; dt's bias [H].
@@ -533,6 +536,10 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 3) k_front_bwd(Front f, FrontG
         for (int j = 0; j < R; ++j) gv[j] = ng[i & 1][j];
         row(nxt[i & 1], s + 2);
         grad(ng[i & 1], s + 2);
+        if (IN && s + kAhead < p.run) {
+          prefetch_l2(px + (s + kAhead) * xs);
+          prefetch_l2(pg + (s + kAhead) * gs);
+        }
         step(own, win[(i + 1) & 3], win[(i + 2) & 3], win[(i + 3) & 3], win[i], gv, gw[i]);
         if (s0 == 0 && i < KT - 1)   // for the warp before this one in time
           *reinterpret_cast<float4*>(&ahead[warp][i][4 * lane]) = make_float4(gw[i][0], gw[i][1], gw[i][2], gw[i][3]);
