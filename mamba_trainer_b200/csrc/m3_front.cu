@@ -430,50 +430,73 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 3) k_front_bwd(Front f, FrontG
 #pragma unroll
     for (int k = 0; k < KT; ++k) pw[k][e] = 0.0f;
   }
-  // go = d pre of one step, from its taps' window and its gradient; OWN: the step feeds the parameter gradients
-  auto step = [&](auto own, const float (&w0)[4], const float (&w1)[4], const float (&w2)[4], const float (&w3)[4],
-                  const Four<T> (&gv)[R], float (&go)[4]) {
+  // go[u] = d pre of two consecutive steps, from the five rows of their taps' windows and their gradients; OWN: the steps
+  // feed the parameter gradients.  Two at a time: a step is one chain (exponential, reciprocal, row sums by shuffles,
+  // reciprocal root), twelve warps do not cover it, and four row sums share their shuffles.
+  auto two_steps = [&](auto own, const float (&r0)[4], const float (&r1)[4], const float (&r2)[4], const float (&r3)[4],
+                       const float (&r4)[4], const Four<T> (&g0)[R], const Four<T> (&g1)[R], float (&go)[2][4]) {
     constexpr bool OWN = decltype(own)::value;
-    float pre[4], gy[4], sg[4], ds[4];
+    float v[2][4], ds[2][4], gy[2][4];
+    pick(g0, gy[0]);
+    pick(g1, gy[1]);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) pre[e] = bs[e];
-    fma4(wt[0], w0, pre);
-    fma4(wt[1], w1, pre);
-    fma4(wt[2], w2, pre);
-    fma4(wt[3], w3, pre);
-    pick(gv, gy);
-    sigmoid4(pre, sg);
-    float v[4];
-    mul4(pre, sg, v);   // SiLU; its derivative is sg + v (1 - sg)
-    {
-      const float nv[4] = {-v[0], -v[1], -v[2], -v[3]};
-      add4(sg, v, ds);
-      fma4(nv, sg, ds);
+    for (int u = 0; u < 2; ++u) {
+      float pre[4], sg[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) pre[e] = bs[e];
+      fma4(wt[0], u ? r1 : r0, pre);
+      fma4(wt[1], u ? r2 : r1, pre);
+      fma4(wt[2], u ? r3 : r2, pre);
+      fma4(wt[3], u ? r4 : r3, pre);
+      sigmoid4(pre, sg);
+      mul4(pre, sg, v[u]);   // SiLU; its derivative is sg + v (1 - sg)
+      const float nv[4] = {-v[u][0], -v[u][1], -v[u][2], -v[u][3]};
+      add4(sg, v[u], ds[u]);
+      fma4(nv, sg, ds[u]);
     }
     if (p.bc) {
-      round4(static_cast<const T*>(nullptr), v);
-      add4(v, bias, v);
-      if (f.has_norm) {
-        float dxh[4];
-        mul4(gy, gain, dxh);
-        float sums[2] = {dot4(v, v), dot4(dxh, v)};
-        row_sums<N, 2>(sums);
-        const float rstd = rsqrtf(sums[0] * (1.0f / N) + f.eps), md = -sums[1] * rstd * (1.0f / N);
-        const float rs4[4] = {rstd, rstd, rstd, rstd}, md4[4] = {md, md, md, md};
-        mul4(v, rs4, v);   // normalised
-        if (OWN) fma4(gy, v, pgain);
-        fma4(v, md4, dxh);
-        mul4(dxh, rs4, gy);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        round4(static_cast<const T*>(nullptr), v[u]);
+        add4(v[u], bias, v[u]);
       }
-      if (OWN) add4(pbias, gy, pbias);
+      if (f.has_norm) {
+        float sums[4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          float dxh[4];
+          mul4(gy[u], gain, dxh);
+          sums[2 * u] = dot4(v[u], v[u]);
+          sums[2 * u + 1] = dot4(dxh, v[u]);
+        }
+        row_sums<N, 4>(sums);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const float rstd = rsqrtf(sums[2 * u] * (1.0f / N) + f.eps), md = -sums[2 * u + 1] * rstd * (1.0f / N);
+          const float rs4[4] = {rstd, rstd, rstd, rstd}, md4[4] = {md, md, md, md};
+          float dxh[4];
+          mul4(gy[u], gain, dxh);
+          mul4(v[u], rs4, v[u]);   // normalised
+          if (OWN) fma4(gy[u], v[u], pgain);
+          fma4(v[u], md4, dxh);
+          mul4(dxh, rs4, gy[u]);
+        }
+      }
+      if (OWN) {
+        add4(pbias, gy[0], pbias);
+        add4(pbias, gy[1], pbias);
+      }
     }
-    mul4(gy, ds, go);   // gradients past T are zero, so go is too
-    if (OWN) {
-      add4(pb, go, pb);
-      fma4(go, w0, pw[0]);
-      fma4(go, w1, pw[1]);
-      fma4(go, w2, pw[2]);
-      fma4(go, w3, pw[3]);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      mul4(gy[u], ds[u], go[u]);   // gradients past T are zero, so go is too
+      if (OWN) {
+        add4(pb, go[u], pb);
+        fma4(go[u], u ? r1 : r0, pw[0]);
+        fma4(go[u], u ? r2 : r1, pw[1]);
+        fma4(go[u], u ? r3 : r2, pw[2]);
+        fma4(go[u], u ? r4 : r3, pw[3]);
+      }
     }
   };
   // dx[t] = sum_delay w[K-1-delay] g[t + delay], from gj = g[t + j]
@@ -528,22 +551,36 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 3) k_front_bwd(Front f, FrontG
       for (int e = 0; e < 4; ++e) gw[k][e] = 0.0f;
     auto four = [&](auto own, int s0) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 4; i += 2) {
         const int s = s0 + i;
-        nxt[i & 1].get(win[i]);
-        Four<T> gv[R];
+        float x3[4], x4[4], go[2][4];
+        nxt[0].get(x3);
+        nxt[1].get(x4);
+        Four<T> g0[R], g1[R];
 #pragma unroll
-        for (int j = 0; j < R; ++j) gv[j] = ng[i & 1][j];
-        row(nxt[i & 1], s + 2);
-        grad(ng[i & 1], s + 2);
-        if (IN && s + kAhead < p.run) {
-          prefetch_l2(px + (s + kAhead) * xs);
-          prefetch_l2(pg + (s + kAhead) * gs);
+        for (int j = 0; j < R; ++j) { g0[j] = ng[0][j]; g1[j] = ng[1][j]; }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          row(nxt[u], s + 2 + u);
+          grad(ng[u], s + 2 + u);
+          if (IN && s + u + kAhead < p.run) {
+            prefetch_l2(px + (s + u + kAhead) * xs);
+            prefetch_l2(pg + (s + u + kAhead) * gs);
+          }
         }
-        step(own, win[(i + 1) & 3], win[(i + 2) & 3], win[(i + 3) & 3], win[i], gv, gw[i]);
-        if (s0 == 0 && i < KT - 1)   // for the warp before this one in time
-          *reinterpret_cast<float4*>(&ahead[warp][i][4 * lane]) = make_float4(gw[i][0], gw[i][1], gw[i][2], gw[i][3]);
-        if (s - 3 < p.run) emit(s - 3, gw[(i + 1) & 3], gw[(i + 2) & 3], gw[(i + 3) & 3], gw[i]);
+        two_steps(own, win[(i + 1) & 3], win[(i + 2) & 3], win[(i + 3) & 3], x3, x4, g0, g1, go);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int c = i + u;
+          if (s0 == 0 && c < KT - 1)   // for the warp before this one in time
+            *reinterpret_cast<float4*>(&ahead[warp][c][4 * lane]) = make_float4(go[u][0], go[u][1], go[u][2], go[u][3]);
+          if (s + u - 3 < p.run) emit(s + u - 3, gw[(c + 1) & 3], gw[(c + 2) & 3], gw[(c + 3) & 3], go[u]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            gw[c][e] = go[u][e];
+            win[c][e] = u ? x4[e] : x3[e];
+          }
+        }
       }
     };
 #pragma unroll 1
