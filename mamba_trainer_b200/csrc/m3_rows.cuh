@@ -304,6 +304,10 @@ __device__ __forceinline__ void load_rows(float* dst, const T* src, const Dims& 
   }
 }
 
+// sin and cos of an angle in [-pi, pi], by the function that takes it in units of pi: no branch for large arguments, whose
+// code and stack sincosf carries; the scaling moves the angle by less than its own last bit.
+__device__ __forceinline__ void sincos_wrapped(float phi, float* sn, float* cs) { sincospif(phi * 0.31830988618379067f, sn, cs); }
+
 // Rows of B or C (two tensors at once share the sines), rotated by -phi; `scale` (per step, or NULL) multiplies them.
 // BF: the result is rounded to bf16 (exact in TF32: one product instead of three), as the tensor-core family's operands are.
 template <bool BF>
@@ -331,7 +335,7 @@ __device__ __forceinline__ void load_rotated(float* const (&dst)[NTENS], const T
     for (int j = 0; j < NA; ++j) {
       // (the angle is wrapped: the special-function unit's sine is good to 2^-21 there, far below a bf16 operand)
       if (BF) __sincosf(phi[l * NH + e / R + j], &sn[j], &cs[j]);
-      else sincosf(phi[l * NH + e / R + j], &sn[j], &cs[j]);
+      else sincos_wrapped(phi[l * NH + e / R + j], &sn[j], &cs[j]);
       cs[j] *= sc;
       sn[j] *= sc;
     }

@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoin
       float cs[NA], sn[NA], dp[NA];
 #pragma unroll
       for (int j = 0; j < NA; ++j) {
-        sincosf(sm.phi[l * NH + e / R + j], &sn[j], &cs[j]);
+        sincos_wrapped(sm.phi[l * NH + e / R + j], &sn[j], &cs[j]);
         dp[j] = 0.0f;
       }
 #pragma unroll

@@ -22,7 +22,7 @@ struct StateSmem {
   Scal<R> s;
 };
 template <class T, int N, int R, bool ROT, bool BWD>
-__global__ void __launch_bounds__(256) k_rows_state(Dims d, m3_scan_desc in, const T* __restrict__ dy, RowsWs ws,
+__global__ void __launch_bounds__(256, N == 64 ? 4 : 3) k_rows_state(Dims d, m3_scan_desc in, const T* __restrict__ dy, RowsWs ws,
                                                     float* __restrict__ dst) {
   extern __shared__ __align__(16) unsigned char smem[];
   StateSmem<N, R>& sm = *reinterpret_cast<StateSmem<N, R>*>(smem);
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) k_rows_pass(Dims d, m3_scan_desc in, Rows
       if (in.last_u0 && !d.raw) carry[i] += first * in.last_u0[(size_t)bh * PN + plain[i]];
     }
   }
-  float ang = ROT && in.angle0 ? in.angle0[(size_t)bh * NH + m] : 0.0f;
+  float ang = ROT && in.angle0 ? wrap_angle(in.angle0[(size_t)bh * NH + m]) : 0.0f;
   float* hs = ws.hs + (size_t)bh * d.C * PN;
   for (int k0 = 0; k0 < d.C; k0 += U) {
     float s[U][4], ecd[U], da[U];
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256) k_rows_pass(Dims d, m3_scan_desc in, Rows
       const size_t k = k0 + u;
       float sn = 0.0f, cs = 1.0f;
       if (ROT) {
-        sincosf(ang, &sn, &cs);
+        sincos_wrapped(ang, &sn, &cs);
         if (p == 0) ws.abase[((size_t)bh * d.C + k) * NH + m] = ang;
         ang = wrap_angle(ang + da[u]);
       }
