@@ -190,15 +190,15 @@ template <class Params>
 cudaError_t plan_ahead(m3_ctx* ctx, Params& p, const m3::Dims& d, const m3_scan_desc& desc, int nseg, int tps, const void* dy,
                        const float* dh, const float* ckpt_angle, char** scratch) {
   *scratch = nullptr;
-  const int BH = d.B * d.H, tiles = m3::tc_tiles(d.T, d.R);
+  const int BH = d.B * d.H;
   m3::TcAhead a{};
   a.nseg = nseg;
   a.tps = tps;
-  const size_t bytes = m3::tc_ahead_bytes(BH, tiles, nseg, nullptr, nullptr);
+  const size_t bytes = m3::tc_ahead_bytes(BH, &a, nullptr);
   cudaError_t e = cudaSuccess;
   if (!ctx->no_scratch) e = m3::scratch_alloc(ctx, reinterpret_cast<void**>(scratch), bytes, ctx->stream);
   if (e != cudaSuccess) return e;
-  m3::tc_ahead_bytes(BH, tiles, nseg, &a, ctx->no_scratch ? ctx->fixed_scratch : *scratch);
+  m3::tc_ahead_bytes(BH, &a, ctx->no_scratch ? ctx->fixed_scratch : *scratch);
   e = m3::tc_ahead(ctx->stream, d, desc, dy, dh, ckpt_angle, a);
   ctx->launches += 2;
   p.ahead = 1;
@@ -223,7 +223,7 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
   const size_t per_tok = BH * d.Tp, per_tile = BH * tiles;
   // few stripes: segments that run side by side; their sums of d phi are completed afterwards
   int nseg = 1, tps = tiles;
-  const bool ahead = !saved->tc_direct && m3::tc_ahead_plan((int)BH, tiles, true, &nseg, &tps);
+  const bool ahead = !saved->tc_direct && m3::tc_ahead_plan((int)BH, tiles, true, false, &nseg, &tps);
   const size_t nphi = ahead && d.rot ? (per_tok + BH * nseg) * 64 : 0;
   const size_t nfloat = 4 * per_tok + 2 * per_tile + BH + 4 + nphi;
   float* base = nullptr;
@@ -535,12 +535,18 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     // when it is the backward pass that will be cut; a caller that must not allocate has a fixed block for them).
     const int ntiles = m3::tc_tiles(d.T, d.R);
     int nseg = 1, tps = ntiles, bseg, btps;
-    const bool ahead = m3::tc_ahead_plan((int)BH, ntiles, false, &nseg, &tps) &&
-                       (!ctx->no_scratch || m3::tc_ahead_bytes((int)BH, ntiles, nseg, nullptr, nullptr) <= ctx->fixed_bytes);
-    const bool bwd_ahead = saved && m3::tc_ahead_plan((int)BH, ntiles, true, &bseg, &btps);
+    const bool direct = d.R == 1 && !d.rot && d.rev == 0 && d.T % 8 == 0;
+    bool ahead = m3::tc_ahead_plan((int)BH, ntiles, false, direct, &nseg, &tps);
+    if (ahead && ctx->no_scratch) {
+      m3::TcAhead a{};
+      a.nseg = nseg;
+      a.tps = tps;
+      ahead = m3::tc_ahead_bytes((int)BH, &a, nullptr) <= ctx->fixed_bytes;
+    }
+    const bool bwd_ahead = saved && m3::tc_ahead_plan((int)BH, ntiles, true, direct, &bseg, &btps);
     // Rank 1 with real dynamics needs no conversion of its rows: bulk tensor copies land them in
     // operand layout (every head left to right, T a multiple of 8, 16-byte aligned tensors).
-    p.use_tma = (!ahead && !bwd_ahead && d.R == 1 && !d.rot && d.rev == 0 && d.T % 8 == 0 &&
+    p.use_tma = (!ahead && !bwd_ahead && direct &&
                  m3::tc_make_tile_map(&p.tm_b, p.b, d.B, d.T, d.H, 128) && m3::tc_make_tile_map(&p.tm_c, p.c, d.B, d.T, d.H, 128) &&
                  m3::tc_make_tile_map(&p.tm_x, p.x, d.B, d.T, d.H, 64)) ? 1 : 0;
     if (!p.use_tma) {

@@ -70,15 +70,18 @@ void tc_segment_plan(int BH, int tiles, bool allow_split, int* nseg, int* tps, i
 // seg_state / seg_angle the stripe kernels read, and nothing is handed over.
 struct Dims;
 struct TcAhead {
-  int nseg, tps;
-  float *hs, *asum, *cd;          // per tile
+  int nseg, tps;                  // segments of a stripe, tiles of a segment
+  int gps, gt;                    // groups of a segment, tiles of a group
+  float *hs, *asum, *cd;          // per group
   float *seg_state, *seg_angle;   // per segment
 };
-bool tc_ahead_plan(int BH, int tiles, bool backward, int* nseg, int* tps);
-size_t tc_ahead_bytes(int BH, int tiles, int nseg, TcAhead* a, char* base);
+// `direct`: whole stripes would run the direct form.
+bool tc_ahead_plan(int BH, int tiles, bool backward, bool direct, int* nseg, int* tps);
+// nseg and tps given: fills in the rest; bytes of scratch.
+size_t tc_ahead_bytes(int BH, TcAhead* a, char* base);
 // dy NULL: forward; else the gradient of the state (dh: the one reaching the returned state, or NULL).
-cudaError_t tc_ahead(cudaStream_t st, Dims d, const m3_scan_desc& in, const void* dy, const float* dh, const float* ckpt_angle,
-                     const TcAhead& a);
+cudaError_t tc_ahead(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const void* dy, const float* dh,
+                     const float* ckpt_angle, const TcAhead& a);
 
 cudaError_t tc_forward(cudaStream_t st, const TcFwdParams& p, bool rotational);
 // The direct form (rank 1, real dynamics, use_tma): m3_tc_fwd_direct.cu.
