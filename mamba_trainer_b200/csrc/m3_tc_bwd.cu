@@ -591,72 +591,72 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
       if (!dead) dead = !warp_all(mbar_wait(&bars[4], it & 1, wait_limit));  // the other four products
       if (!dead) {
         tc_fence_after();
-        {  // dB^ (TM_DB, operand sB, out db) then dC^ (TM_T1, operand sC, out dc)
-          float gq[4][16], tabv[2][16];
+        // dB^ (TM_DB, operand sB, out db), then dC^ (TM_T1, operand sC, out dc).  As two copies of this body rank 4 spilled
+        // some 300 bytes a thread; as a loop 12, and its second pass finds its code in the instruction caches (cfg3 forward
+        // + backward 9.32 -> 8.95 ms).  The lower ranks, which spill less, lose 1 to 3 % as a loop.
+        float tabv[2][16];
+        if (ROT) {
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) tmem_ld16_issue(tmem_addr(tm, quad * 32, TM_DB + gcol(q4)), gq[q4]);
+          for (int mc = 0; mc < 2; ++mc) tmem_ld16_issue(tmem_addr(tm, quad * 32, TM_TAB + 32 * ch + 16 * mc), tabv[mc]);
+        }
+#pragma unroll(R == 4 ? 1 : 2)
+        for (int pass = 0; pass < 2; ++pass) {
+          const bool is_b = pass == 0;
+          const uint32_t from = is_b ? TM_DB : TM_T1;
+          const uint8_t* sop = is_b ? sB : sC;
+          uint8_t* stg = is_b ? sXw : sDG;   // sigma_w X~ and exp(acum) dY~ are spent: 32 KB to stage dB; so is dG: dC
+          float g[4][16];
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) tmem_ld16_issue(tmem_addr(tm, quad * 32, from + gcol(q4)), g[q4]);
+          tmem_wait_ld();
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) tmem_ld_fence(g[q4]);
+          if (ROT) { tmem_ld_fence(tabv[0]); tmem_ld_fence(tabv[1]); }
+          if (is_b && at_end && p.dlu) {  // d last_u reaches B^ of the final token: += dlu^T x
+#pragma unroll 1
+            for (int q4 = 0; q4 < 4; ++q4)
+#pragma unroll 1
+              for (int j = 0; j < 16; ++j) {
+                const int n = gcol(q4) + j;
+                float s_ = 0.0f;
+                for (int pp = 0; pp < kP; ++pp)
+                  s_ += p.dlu[((size_t)bh * kP + pp) * kN + n] *
+                        __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sX + tile_off(row, pp, kP)));
+#pragma unroll
+                for (int a4 = 0; a4 < 4; ++a4)
+#pragma unroll
+                  for (int jj = 0; jj < 16; ++jj) g[a4][jj] += (a4 == q4 && jj == j) ? s_ : 0.0f;
+              }
+          }
           if (ROT) {
 #pragma unroll
-            for (int mc = 0; mc < 2; ++mc) tmem_ld16_issue(tmem_addr(tm, quad * 32, TM_TAB + 32 * ch + 16 * mc), tabv[mc]);
-          }
-          tmem_wait_ld();
+            for (int mc = 0; mc < 2; ++mc) {
+              const int m0 = 32 * ch + 16 * mc;
+              float (&g1)[16] = g[mc];
+              float (&g2)[16] = g[2 + mc];
+              float o1[16], o2[16];
+              load_chunk(sop, tile_off(row, m0, kN), *reinterpret_cast<float(*)[8]>(&o1[0]));
+              load_chunk(sop, tile_off(row, m0 + 8, kN), *reinterpret_cast<float(*)[8]>(&o1[8]));
+              load_chunk(sop, tile_off(row, kNH + m0, kN), *reinterpret_cast<float(*)[8]>(&o2[0]));
+              load_chunk(sop, tile_off(row, kNH + m0 + 8, kN), *reinterpret_cast<float(*)[8]>(&o2[8]));
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) tmem_ld_fence(gq[q4]);
-          if (ROT) { tmem_ld_fence(tabv[0]); tmem_ld_fence(tabv[1]); }
-          auto finish = [&](float (&g)[4][16], const uint8_t* sop, uint8_t* stg, bool is_b) {
-            if (is_b && at_end && p.dlu) {  // d last_u reaches B^ of the final token: += dlu^T x
-#pragma unroll 1
-              for (int q4 = 0; q4 < 4; ++q4)
-#pragma unroll 1
-                for (int j = 0; j < 16; ++j) {
-                  const int n = gcol(q4) + j;
-                  float s_ = 0.0f;
-                  for (int pp = 0; pp < kP; ++pp)
-                    s_ += p.dlu[((size_t)bh * kP + pp) * kN + n] *
-                          __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sX + tile_off(row, pp, kP)));
-#pragma unroll
-                  for (int a4 = 0; a4 < 4; ++a4)
-#pragma unroll
-                    for (int jj = 0; jj < 16; ++jj) g[a4][jj] += (a4 == q4 && jj == j) ? s_ : 0.0f;
-                }
-            }
-            if (ROT) {
-#pragma unroll
-              for (int mc = 0; mc < 2; ++mc) {
-                const int m0 = 32 * ch + 16 * mc;
-                float (&g1)[16] = g[mc];
-                float (&g2)[16] = g[2 + mc];
-                float o1[16], o2[16];
-                load_chunk(sop, tile_off(row, m0, kN), *reinterpret_cast<float(*)[8]>(&o1[0]));
-                load_chunk(sop, tile_off(row, m0 + 8, kN), *reinterpret_cast<float(*)[8]>(&o1[8]));
-                load_chunk(sop, tile_off(row, kNH + m0, kN), *reinterpret_cast<float(*)[8]>(&o2[0]));
-                load_chunk(sop, tile_off(row, kNH + m0 + 8, kN), *reinterpret_cast<float(*)[8]>(&o2[8]));
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  dphi[16 * mc + j] += g1[j] * o2[j] - g2[j] * o1[j];
-                  const uint32_t cw = __float_as_uint(tabv[mc][j]);
-                  const float2 csn = __half22float2(*reinterpret_cast<const __half2*>(&cw));
-                  const float cs = csn.x, sn = csn.y;
-                  const float u1 = g1[j] * cs - g2[j] * sn, u2 = g1[j] * sn + g2[j] * cs;
-                  g1[j] = u1; g2[j] = u2;
-                }
+              for (int j = 0; j < 16; ++j) {
+                dphi[16 * mc + j] += g1[j] * o2[j] - g2[j] * o1[j];
+                const uint32_t cw = __float_as_uint(tabv[mc][j]);
+                const float2 csn = __half22float2(*reinterpret_cast<const __half2*>(&cw));
+                const float cs = csn.x, sn = csn.y;
+                const float u1 = g1[j] * cs - g2[j] * sn, u2 = g1[j] * sn + g2[j] * cs;
+                g1[j] = u1; g2[j] = u2;
               }
             }
-            if constexpr (R == 2) {
+          }
+          if constexpr (R == 2) {
 #pragma unroll
-              for (int q4 = 0; q4 < 4; q4 += 2) stage_out32<R>(stg, row, gcol(q4), g[q4], g[q4 + 1], rev);
-            } else {
+            for (int q4 = 0; q4 < 4; q4 += 2) stage_out32<R>(stg, row, gcol(q4), g[q4], g[q4 + 1], rev);
+          } else {
 #pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4) stage_out16<R>(stg, row, gcol(q4), g[q4], rev);
-            }
-          };
-          finish(gq, sB, sXw, true);     // sigma_w X~ and exp(acum) dY~ are spent: 32 KB to stage dB
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) tmem_ld16_issue(tmem_addr(tm, quad * 32, TM_T1 + gcol(q4)), gq[q4]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) tmem_ld_fence(gq[q4]);
-          finish(gq, sC, sDG, false);    // dG is spent: its buffer stages dC
+            for (int q4 = 0; q4 < 4; ++q4) stage_out16<R>(stg, row, gcol(q4), g[q4], rev);
+          }
         }
       }
       fence_async_smem();  // the staged gradients, for the stores that read them
