@@ -127,18 +127,19 @@ def test_mixer_front_matches_the_separate_steps(dtype, B, T, H, N, R, K, norm, l
         assert ((a - e).abs() <= 2e-5 * scale + 1e-4 * e.abs()).all(), (n, float((a - e).abs().max()), scale)
 
 
-@pytest.mark.parametrize("R,rot,T,state,rev", [
-    (1, True, 385, True, 0),      # four tiles, the last one a single step
-    (1, False, 1000, True, 0),    # real dynamics: the role-split kernels instead of the direct ones
-    (2, True, 1000, True, 1),     # a right-to-left head, carried state and angle
-    (2, True, 449, False, 0),     # the second half of the last tile is padding
-    (4, True, 321, True, 0),
-    (4, False, 96, False, 1),     # three tiles: the fewest that are cut
+@pytest.mark.parametrize("B,H,R,rot,T,state,rev", [
+    (2, 2, 1, True, 385, True, 0),      # four tiles, the last one a single step
+    (2, 2, 1, False, 1000, True, 0),    # real dynamics: the role-split kernels instead of the direct ones
+    (2, 2, 2, True, 1000, True, 1),     # a right-to-left head, carried state and angle
+    (2, 2, 2, True, 449, False, 0),     # the second half of the last tile is padding
+    (2, 2, 4, True, 321, True, 0),
+    (2, 2, 4, False, 96, False, 1),     # three tiles: the fewest that are cut
+    (5, 8, 4, True, 999, True, 0),       # 32 tiles of 40 stripes: states of groups of several tiles, the last one shorter
 ])
-def test_side_by_side_segments_match_the_oracle(R, rot, T, state, rev):
+def test_side_by_side_segments_match_the_oracle(B, H, R, rot, T, state, rev):
     """Few stripes of the tensor-core family: segments of a stripe run at once from states worked out ahead of them."""
     from test_scan_gpu import check_bf16, compare_all, small_inputs
-    t, ds = small_inputs(2, T, 2, 64, 128, R, rot, state, seed=T + R)
+    t, ds = small_inputs(B, T, H, 64, 128, R, rot, state, seed=T + R)
     for k in ("b", "c"):
         t[k] = t[k] / 128 ** 0.5
     t["dt"] = t["dt"] * 0.2
