@@ -126,9 +126,10 @@ struct Place {
   static constexpr int WR = R * N > 128 ? R * N / 128 : 1;   // warps that hold one group's ranks
   bool bc;          // B or C (else x)
   int which;        // 0: B, 1: C
+  int base;         // the block's first channel of its band (x, B or C)
   int c0;           // this lane's first channel of the convolution
-  int j;            // and of its band (x, B or C)
-  bool live;        // the channel exists
+  int j;            // and of its band
+  bool live;        // the channel exists (a lane past the band's end reads the band's first channels and stores nothing)
   bool rev;         // and runs right to left
   int tl, run, t0;  // the warp's place in time within the block, its steps, the first of them
 };
@@ -141,20 +142,20 @@ __device__ __forceinline__ Place<N, R> place(const Front& f, int bx, int nx, int
   if (!p.bc) {
     p.which = 0;
     p.tl = w; p.run = run;
-    p.j = bx * 128 + 4 * lane;
-    p.live = p.j < f.di;
-    p.c0 = p.j;
-    p.rev = f.reverse && p.j >= f.di / 2;
+    p.base = bx * 128;
+    p.j = p.base + 4 * lane;
   } else {
     const int i = bx - nx;
     p.which = i / nb;
     p.tl = w / P::WR; p.run = run * P::WR;
-    p.j = ((i - p.which * nb) * P::WR + w % P::WR) * 128 + 4 * lane;
-    p.live = p.j < f.bc;
-    p.c0 = f.di + p.which * f.bc + p.j;
-    p.rev = f.reverse && p.j >= f.bc / 2;
+    p.base = (i - p.which * nb) * P::WR * 128;
+    p.j = p.base + w % P::WR * 128 + 4 * lane;
   }
-  if (!p.live) { p.j = 0; p.c0 = p.bc ? f.di : 0; }
+  const int width = p.bc ? f.bc : f.di;
+  p.live = p.j < width;
+  if (!p.live) p.j = 0;
+  p.c0 = (p.bc ? f.di + p.which * f.bc : 0) + p.j;
+  p.rev = f.reverse && p.j >= width / 2;
   p.t0 = blockIdx.y * (WARPS * run) + p.tl * p.run;
   return p;
 }
@@ -306,10 +307,10 @@ __global__ void __launch_bounds__(kWarps * 32, 3) k_front_fwd(Front f, FrontOut 
         for (int e = 0; e < 4; ++e) win[k][e] = win[4 + k][e];
     }
   };
-  // (the ranks of a group meet at block barriers in there: the choice is the block's)
-  const int blk = blockIdx.y * (kWarps * RUN);
-  const int ch = p.bc ? 128 * P::WR : 128, width = p.bc ? f.bc : f.di, base = p.j - p.j % ch;
-  if (blk >= KT - 1 && blk + kWarps * RUN <= f.T && base + ch <= width) walk(std::true_type{});
+  // (the ranks of a group meet at block barriers in there, and the walk of inside blocks stores without asking for `live`:
+  // the choice is the block's)
+  const int blk = blockIdx.y * (kWarps * RUN), ch = p.bc ? 128 * P::WR : 128;
+  if (blk >= KT - 1 && blk + kWarps * RUN <= f.T && p.base + ch <= (p.bc ? f.bc : f.di)) walk(std::true_type{});
   else walk(std::false_type{});
   // the K - 1 inputs the next window continues from, by the warp that has the last step
   if (o.hist && p.live && p.t0 < f.T && p.t0 + p.run >= f.T) {

@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from _util import ref_metric
+from _util import norm_rel, ref_metric
 from mamba_trainer_b200.ssm import Discretization
 
 pytestmark = pytest.mark.gpu
@@ -96,7 +96,7 @@ def test_chunk_parallel_backward_takes_unaligned_gradients():
 
 @pytest.mark.parametrize("dtype,B,T,H,N,R,K,norm,learned,bidir", [
     (torch.float32, 1, 1, 2, 128, 1, 4, True, True, False),      # one step, most of a block dead
-    (torch.float32, 2, 33, 3, 64, 1, 2, True, True, False),      # an odd number of 64-wide rows: half a warp dead
+    (torch.float32, 2, 33, 3, 64, 1, 2, True, True, False),      # odd heads: no row of four, the separate steps both times
     (torch.float32, 1, 131, 2, 64, 2, 3, False, False, False),   # no norm: the plain bias
     (torch.float32, 2, 150, 4, 128, 2, 4, True, True, True),     # both directions
     (torch.float32, 1, 70, 2, 64, 4, 1, True, True, False),
@@ -125,6 +125,50 @@ def test_mixer_front_matches_the_separate_steps(dtype, B, T, H, N, R, K, norm, l
     for n, a, e in zip(names, *res):
         scale = max(1.0, float(e.abs().max()))
         assert ((a - e).abs() <= 2e-5 * scale + 1e-4 * e.abs()).all(), (n, float((a - e).abs().max()), scale)
+
+
+@pytest.mark.parametrize("dtype,B,T,H,P,N,R,bidir", [
+    (torch.float32, 2, 64, 6, 32, 128, 1, True),      # d_inner 192: the second tile of x is half dead, no block inside
+    (torch.float32, 1, 131, 6, 32, 64, 1, True),      # the same with blocks whose every step is inside the sequence
+    (torch.float32, 2, 131, 2, 32, 64, 1, False),     # one direction, d_inner 64
+    (torch.float32, 12, 1290, 6, 32, 64, 1, True),    # blocks of 128 steps
+    (torch.bfloat16, 1, 131, 6, 32, 64, 1, True),
+    (torch.bfloat16, 2, 99, 6, 32, 128, 2, True),
+    (torch.bfloat16, 1, 200, 6, 16, 64, 4, True),     # d_inner 384: whole tiles, a direction change inside one
+    (torch.bfloat16, 1, 70, 4, 24, 64, 1, False),     # d_inner 96
+])
+def test_mixer_front_tiles_past_the_bands_end(dtype, B, T, H, P, N, R, bidir):
+    """Bands that do not fill the front's 128-channel tiles: no lane past a band's end writes anything, whichever way its
+    blocks run.  Against the separate steps, and the launch counts say that one run took each form."""
+    from mamba_trainer_b200.nn import MixerCore, MixerShape
+    from mamba_trainer_b200.ssm import Context
+    shape = MixerShape(H, P, N, R, None, True)
+    torch.manual_seed(T)
+    core = MixerCore(shape, chunk=64, bidirectional=bidir, device="cuda")
+    with torch.no_grad():
+        for q in (core.b_bias, core.c_bias, core.conv_b, core.d_skip):
+            q.normal_(0, 0.3)
+    W = shape.in_proj_width
+    raw = torch.randn(B * T * W, device="cuda").to(dtype)
+    dout = torch.randn(B, T, shape.d_inner, device="cuda").to(dtype)
+    ctx = Context.for_device(torch.device("cuda"))
+    res, launches = [], []
+    for off in (0, 1):
+        buf = torch.empty(B * T * W + 8, device="cuda", dtype=dtype)
+        proj = buf[off:off + B * T * W].copy_(raw).view(B, T, W).requires_grad_(True)
+        before = ctx.lib.m3_launch_count(ctx.handle)
+        out = core(proj)
+        res.append((out,) + torch.autograd.grad(out, [proj] + list(core.parameters()), dout))
+        launches.append(ctx.lib.m3_launch_count(ctx.handle) - before)
+    assert launches[0] < launches[1], launches
+    names = ["out", "proj"] + [n for n, _ in core.named_parameters()]
+    for n, a, e in zip(names, *res):
+        a, e = a.float(), e.float()
+        scale = max(1.0, float(e.abs().max()))
+        if dtype == torch.float32:
+            assert ((a - e).abs() <= 2e-5 * scale + 1e-4 * e.abs()).all(), (n, float((a - e).abs().max()), scale)
+        else:   # a flipped rounding of x, B or C is 2^-8 of the value and travels on: the bound of the other bf16 tests
+            assert norm_rel(a, e) <= 2e-2 and ref_metric(a, e) <= 2e-2 * scale, (n, norm_rel(a, e), ref_metric(a, e), scale)
 
 
 @pytest.mark.parametrize("B,H,R,rot,T,state,rev", [
