@@ -380,6 +380,9 @@ extern "C" {
     /// The node's backward rule; may run more than once per saved handle (backward_retain).
     pub fn m3_scan_backward(ctx: *mut m3_ctx, saved: *const m3_saved, input: *const m3_scan_bwd_in, grad_mask: u32,
                             grads: *const m3_scan_grads) -> c_int;
+    /// The same with the forward's inputs at new addresses (brought back or computed again since).
+    pub fn m3_scan_backward_moved(ctx: *mut m3_ctx, saved: *const m3_saved, inputs: *const m3_scan_desc,
+                                  input: *const m3_scan_bwd_in, grad_mask: u32, grads: *const m3_scan_grads) -> c_int;
     pub fn m3_saved_free(ctx: *mut m3_ctx, saved: *mut m3_saved) -> c_int;
     pub fn m3_scan_scratch_bytes(desc: *const m3_scan_desc, for_backward: c_int) -> usize;
 

@@ -185,6 +185,12 @@ int m3_scan_forward(m3_ctx *ctx, const m3_scan_desc *desc, const m3_scan_out *ou
  * consume `saved`, so it may run again (backward_retain, var.rs:218-221). */
 int m3_scan_backward(m3_ctx *ctx, const m3_saved *saved, const m3_scan_bwd_in *in,
                      uint32_t grad_mask, const m3_scan_grads *grads);
+/* The same, reading the forward's inputs where `inputs` has them: their memory need not outlive the forward pass
+ * when the caller brings the values back first (from host memory, or computed again under activation
+ * checkpointing).  `inputs` is the forward's descriptor but for the addresses, each of which has the alignment
+ * (modulo 16 bytes) that it had then. */
+int m3_scan_backward_moved(m3_ctx *ctx, const m3_saved *saved, const m3_scan_desc *inputs, const m3_scan_bwd_in *in,
+                           uint32_t grad_mask, const m3_scan_grads *grads);
 
 int m3_saved_free(m3_ctx *ctx, m3_saved *saved);
 
@@ -418,8 +424,9 @@ int m3_mixer_window(m3_ctx *ctx, const m3_mixer_desc *desc, const m3_mixer_windo
 
 /* One training pass of the mixer: forward_pass on its input projection's output, and its adjoint.  `activations`
  * (m3_mixer_activation_bytes bytes of device memory, 256-byte aligned) receives what the backward pass needs besides
- * proj and the parameters; keep all of them unchanged until then.  `saved` may be NULL (inference); otherwise it
- * receives the scan's handle, freed with m3_saved_free.  The backward pass may run more than once; `workspace` holds
+ * proj and the parameters; keep all of them unchanged until then (they may move: the backward pass reads them where
+ * its own descriptor has them, at the alignment modulo 16 bytes that they had).  `saved` may be NULL (inference);
+ * otherwise it receives the scan's handle, freed with m3_saved_free.  The backward pass may run more than once; `workspace` holds
  * m3_mixer_backward_bytes bytes for the span of the call. */
 typedef struct {
   void *dproj;                /* like proj: every band of it is written */

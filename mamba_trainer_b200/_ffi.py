@@ -126,6 +126,8 @@ SYMBOLS = {
     "m3_download": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t]),
     "m3_scan_forward": (C.c_int, [C.c_void_p, C.POINTER(ScanDesc), C.POINTER(ScanOut), C.POINTER(C.c_void_p)]),
     "m3_scan_backward": (C.c_int, [C.c_void_p, C.c_void_p, C.POINTER(ScanBwdIn), C.c_uint32, C.POINTER(ScanGrads)]),
+    "m3_scan_backward_moved": (C.c_int, [C.c_void_p, C.c_void_p, C.POINTER(ScanDesc), C.POINTER(ScanBwdIn), C.c_uint32,
+                                         C.POINTER(ScanGrads)]),
     "m3_saved_free": (C.c_int, [C.c_void_p, C.c_void_p]),
     "m3_scan_scratch_bytes": (C.c_size_t, [C.POINTER(ScanDesc), C.c_int]),
     "m3_step_forward": (C.c_int, [C.c_void_p, C.POINTER(StepDesc), C.POINTER(StepOut)]),

@@ -1,6 +1,7 @@
 // C ABI of libm3scan: contexts, device buffers, and the forward / backward entry
 // points that validate a descriptor, lay out scratch and enqueue a kernel family.
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -643,6 +644,29 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     M3_CUDA(ctx, cudaFreeAsync(base, ctx->stream));
   }
   return M3_OK;
+}
+
+int m3_scan_backward_moved(m3_ctx* ctx, const m3_saved* saved, const m3_scan_desc* inputs, const m3_scan_bwd_in* in,
+                           uint32_t grad_mask, const m3_scan_grads* grads) {
+  if (!ctx) return M3_ERR_NULL;
+  if (!saved || !inputs) return fail(ctx, M3_ERR_NULL, "saved context and inputs are required");
+  const m3_scan_desc &was = saved->desc, &now = *inputs;
+  // the extents and options are the int32 fields in front of the pointers
+  if (memcmp(&was, &now, offsetof(m3_scan_desc, x)) != 0)
+    return fail(ctx, M3_ERR_CONFIG, "the inputs' descriptor differs from the forward pass's in more than addresses");
+  const void* const a[] = {was.x, was.b, was.c, was.dt, was.lambda, was.theta, was.a_log, was.d_skip, was.h0, was.last_u0,
+                           was.angle0, was.a_raw, was.g_raw, was.w_raw};
+  const void* const b[] = {now.x, now.b, now.c, now.dt, now.lambda, now.theta, now.a_log, now.d_skip, now.h0, now.last_u0,
+                           now.angle0, now.a_raw, now.g_raw, now.w_raw};
+  for (size_t i = 0; i < sizeof(a) / sizeof(a[0]); ++i) {
+    if (!a[i] != !b[i]) return fail(ctx, M3_ERR_NULL, "the inputs present differ from the forward pass's");
+    // what the forward pass chose by the addresses (family, tile maps) has to fit the new ones
+    if ((reinterpret_cast<uintptr_t>(a[i]) ^ reinterpret_cast<uintptr_t>(b[i])) & 15)
+      return fail(ctx, M3_ERR_UNSUPPORTED, "an input moved to another alignment (modulo 16 bytes)");
+  }
+  m3_saved moved = *saved;   // no owner: the scratch stays the handle's
+  moved.desc = now;
+  return m3_scan_backward(ctx, &moved, in, grad_mask, grads);
 }
 
 int m3_scan_backward(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* in, uint32_t grad_mask,

@@ -343,7 +343,7 @@ int m3_mixer_backward(m3_ctx* ctx, const m3_mixer_desc* s, const m3_saved* saved
   sg.dx = b.dx; sg.db = b.db; sg.dc = b.dc; sg.ddt = b.ddt; sg.dlambda = b.dlam;
   sg.dtheta = b.dtheta ? b.dtheta : (m.rot ? band(m.off_th) : nullptr);
   sg.da_log = g->da_log; sg.dd_skip = g->dd_skip;
-  M3_TRY(m3_scan_backward(ctx, saved, &in, M3_GRAD_ALL, &sg));
+  M3_TRY(m3_scan_backward_moved(ctx, saved, &t.scan, &in, M3_GRAD_ALL, &sg));
   if (b.dtheta) {
     const cudaError_t e = copy_theta(ctx, s, m, band(m.off_th), (size_t)m.width * m.es, b.dtheta,
                                      (size_t)s->heads * (s->d_state / 2) * m.es);

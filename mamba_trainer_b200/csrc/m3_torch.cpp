@@ -60,15 +60,54 @@ Tensor as(const Tensor& t, at::ScalarType el) {
   return t.scalar_type() == el && t.is_contiguous() ? t : t.to(el).contiguous();
 }
 Tensor as(const OptTensor& t, at::ScalarType el) { return t.has_value() ? as(*t, el) : Tensor(); }
+
+// A tensor of the forward pass for the backward pass: saved the way autograd saves one, so saved-tensor hooks (activation
+// checkpointing, offloading) may drop it and give back another.  Backward passes take every address from what unpack()
+// returns, which has the forward's element type, density and alignment modulo 16 bytes (the library chose kernels and
+// layouts by them).
+struct Saved {
+  torch::autograd::SavedVariable var;
+  at::ScalarType el{};
+  c10::Device device{c10::kCPU};
+  int64_t numel = 0, align = 0;
+  bool present = false;
+
+  void set(const Tensor& t) {
+    if (!t.defined()) return;
+    var = torch::autograd::SavedVariable(t, false);
+    el = t.scalar_type(); device = t.device(); numel = t.numel();
+    align = reinterpret_cast<uintptr_t>(t.data_ptr()) % 16;
+    present = true;
+  }
+  Tensor unpack(std::shared_ptr<torch::autograd::Node> node) const {   // refuses a second pass unless the graph is retained
+    if (!present) return Tensor();
+    const Tensor v = var.unpack(std::move(node));
+    TORCH_CHECK(v.numel() == numel, "a saved tensor came back with ", v.numel(), " elements instead of ", numel);
+    if (fits(v)) return v;
+    at::NoGradGuard no_grad;
+    const Tensor t = as(v.to(device), el);
+    if (fits(t)) return t;
+    const int64_t es = t.element_size();   // (an allocation starts on 16 bytes)
+    return at::empty({numel + 16 / es}, t.options()).narrow(0, align / es, numel).view(t.sizes()).copy_(t);
+  }
+  bool fits(const Tensor& t) const {
+    return t.scalar_type() == el && t.device() == device && t.is_contiguous() &&
+           static_cast<int64_t>(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16) == align;
+  }
+};
 int dtype_code(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? M3_BF16 : M3_F32; }
 
 // ---- the scan -----------------------------------------------------------------------------------------------------
 constexpr int kScanInputs = 11;   // x, b, c, dt, a_log, lambda, theta, d_skip, h0, last_u0, angle0: the bits of grad_mask
+void scan_inputs(m3_scan_desc& d, const Tensor (&t)[kScanInputs]) {
+  d.x = ptr(t[0]); d.b = ptr(t[1]); d.c = ptr(t[2]); d.dt = ptr(t[3]); d.a_log = fptr(t[4]); d.lambda = ptr(t[5]);
+  d.theta = ptr(t[6]); d.d_skip = fptr(t[7]); d.h0 = fptr(t[8]); d.last_u0 = fptr(t[9]); d.angle0 = fptr(t[10]);
+}
 struct ScanNode : public torch::autograd::Node {
   m3_ctx* ctx = nullptr;
   m3_saved* handle = nullptr;
-  torch::autograd::SavedVariable in[kScanInputs];
-  bool present[kScanInputs] = {};
+  m3_scan_desc desc{};   // extents and options
+  Saved in[kScanInputs];
   bool has_state = false, has_angle = false;
 
   ~ScanNode() override { free_handle(); }
@@ -79,18 +118,19 @@ struct ScanNode : public torch::autograd::Node {
     handle = nullptr;
   }
   void release_variables() override {
-    for (auto& v : in) v.reset_data();
+    for (auto& v : in) v.var.reset_data();
     free_handle();
   }
   std::string name() const override { return "Mamba3ScanBackward"; }
 
   variable_list apply(variable_list&& up) override {
     Tensor t[kScanInputs], g[kScanInputs];
-    for (int i = 0; i < kScanInputs; ++i)
-      if (present[i]) t[i] = in[i].unpack(shared_from_this());   // refuses a second pass unless the graph is retained
+    for (int i = 0; i < kScanInputs; ++i) t[i] = in[i].unpack(shared_from_this());
+    m3_scan_desc d = desc;
+    scan_inputs(d, t);
     uint32_t mask = 0;
     for (int i = 0; i < kScanInputs; ++i)
-      if (present[i] && task_should_compute_output(i)) {
+      if (in[i].present && task_should_compute_output(i)) {
         g[i] = at::empty_like(t[i], at::MemoryFormat::Contiguous);
         mask |= 1u << i;
       }
@@ -107,7 +147,7 @@ struct ScanNode : public torch::autograd::Node {
     {
       std::lock_guard<std::mutex> lock(lock_of(ctx));
       bind(ctx, t[0]);
-      rc = m3_scan_backward(ctx, handle, &bin, mask, &out);
+      rc = m3_scan_backward_moved(ctx, handle, &d, &bin, mask, &out);
     }
     if (rc != M3_OK) raise_status(ctx, rc);
     return variable_list(g, g + kScanInputs);
@@ -130,8 +170,7 @@ std::vector<OptTensor> scan(uintptr_t handle, const Tensor& x0, const Tensor& b0
   d.batch = B; d.seq = T; d.heads = H; d.head_dim = P; d.d_state = N; d.rank = R; d.chunk = chunk; d.dtype = dtype_code(x);
   d.discretization = disc; d.dynamics = t[6].defined() ? M3_ROTATIONAL : M3_REAL; d.want_state = want_state; d.path = path;
   d.reverse_heads = rev;
-  d.x = ptr(x); d.b = ptr(t[1]); d.c = ptr(t[2]); d.dt = ptr(t[3]); d.a_log = fptr(t[4]); d.lambda = ptr(t[5]);
-  d.theta = ptr(t[6]); d.d_skip = fptr(t[7]); d.h0 = fptr(t[8]); d.last_u0 = fptr(t[9]); d.angle0 = fptr(t[10]);
+  scan_inputs(d, t);
   const auto f32 = x.options().dtype(at::kFloat).requires_grad(false);
   Tensor y = at::empty(x.sizes(), x.options().requires_grad(false)), h, lu, ang;
   if (want_state) {
@@ -156,12 +195,9 @@ std::vector<OptTensor> scan(uintptr_t handle, const Tensor& x0, const Tensor& b0
     std::shared_ptr<ScanNode> node(new ScanNode(), torch::autograd::deleteNode);
     node->ctx = ctx;
     node->handle = saved;
+    node->desc = d;
     node->set_next_edges(torch::autograd::collect_next_edges(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10]));
-    for (int i = 0; i < kScanInputs; ++i)
-      if (t[i].defined()) {
-        node->in[i] = torch::autograd::SavedVariable(t[i], false);
-        node->present[i] = true;
-      }
+    for (int i = 0; i < kScanInputs; ++i) node->in[i].set(t[i]);
     node->has_state = want_state;
     node->has_angle = ang.defined();
     variable_list outs{y};
@@ -178,6 +214,11 @@ constexpr int kMixerParams = 9;   // in the order of m3_mixer_desc
 struct Spec {   // the integers of m3_mixer_desc between its extents and its pointers
   int heads, head_dim, d_state, rank, groups, chunk, disc, rotational, has_norm, post_norm, path, reverse_heads;
 };
+void mixer_inputs(m3_mixer_desc& d, const Tensor& proj, const Tensor* p) {
+  d.proj = ptr(proj);
+  d.conv_weight = fptr(p[0]); d.conv_bias = fptr(p[1]); d.dt_bias = fptr(p[2]); d.a_log = fptr(p[3]); d.d_skip = fptr(p[4]);
+  d.b_bias = fptr(p[5]); d.c_bias = fptr(p[6]); d.norm_weight = fptr(p[7]); d.post_weight = fptr(p[8]);
+}
 m3_mixer_desc mixer_desc(const Tensor& proj, const Tensor (&p)[kMixerParams], const Spec& s, double eps) {
   m3_mixer_desc d{};
   d.batch = proj.size(0); d.seq = proj.size(1);
@@ -185,9 +226,7 @@ m3_mixer_desc mixer_desc(const Tensor& proj, const Tensor (&p)[kMixerParams], co
   d.dtype = dtype_code(proj); d.discretization = s.disc; d.dynamics = s.rotational ? M3_ROTATIONAL : M3_REAL;
   d.conv_kernel = p[0].size(0); d.has_norm = s.has_norm; d.post_norm = s.post_norm; d.path = s.path;
   d.reverse_heads = s.reverse_heads; d.eps = static_cast<float>(eps);
-  d.proj = ptr(proj);
-  d.conv_weight = fptr(p[0]); d.conv_bias = fptr(p[1]); d.dt_bias = fptr(p[2]); d.a_log = fptr(p[3]); d.d_skip = fptr(p[4]);
-  d.b_bias = fptr(p[5]); d.c_bias = fptr(p[6]); d.norm_weight = fptr(p[7]); d.post_weight = fptr(p[8]);
+  mixer_inputs(d, proj, p);
   return d;
 }
 Spec spec_of(const std::vector<int64_t>& v) {
@@ -199,10 +238,9 @@ Spec spec_of(const std::vector<int64_t>& v) {
 struct MixerNode : public torch::autograd::Node {
   m3_ctx* ctx = nullptr;
   m3_saved* handle = nullptr;
-  m3_mixer_desc desc{};
+  m3_mixer_desc desc{};    // extents and options
   Tensor act;
-  torch::autograd::SavedVariable in[1 + kMixerParams];   // proj, then the parameters
-  bool present[1 + kMixerParams] = {};
+  Saved in[1 + kMixerParams];   // proj, then the parameters
 
   ~MixerNode() override { free_handle(); }
   void free_handle() {
@@ -212,7 +250,7 @@ struct MixerNode : public torch::autograd::Node {
     handle = nullptr;
   }
   void release_variables() override {
-    for (auto& v : in) v.reset_data();
+    for (auto& v : in) v.var.reset_data();
     free_handle();
     act = Tensor();
   }
@@ -221,20 +259,21 @@ struct MixerNode : public torch::autograd::Node {
   variable_list apply(variable_list&& up) override {
     variable_list g(1 + kMixerParams);
     Tensor t[1 + kMixerParams];
-    for (int i = 0; i <= kMixerParams; ++i)
-      if (present[i]) t[i] = in[i].unpack(shared_from_this());   // refuses a second pass unless the graph is retained
+    for (int i = 0; i <= kMixerParams; ++i) t[i] = in[i].unpack(shared_from_this());
     if (!up[0].defined()) return g;
+    m3_mixer_desc d = desc;
+    mixer_inputs(d, t[0], t + 1);
     const Tensor dout = up[0].contiguous();
     for (int i = 0; i <= kMixerParams; ++i)
-      if (present[i]) g[i] = at::empty_like(t[i], at::MemoryFormat::Contiguous);
+      if (in[i].present) g[i] = at::empty_like(t[i], at::MemoryFormat::Contiguous);
     const m3_mixer_grads out{mut(g[0]), fmut(g[1]), fmut(g[2]), fmut(g[3]), fmut(g[4]), fmut(g[5]),
                              fmut(g[6]), fmut(g[7]), fmut(g[8]), fmut(g[9])};
-    const Tensor work = at::empty({(int64_t)m3_mixer_backward_bytes(&desc)}, act.options());
+    const Tensor work = at::empty({(int64_t)m3_mixer_backward_bytes(&d)}, act.options());
     int rc;
     {
       std::lock_guard<std::mutex> lock(lock_of(ctx));
       bind(ctx, t[0]);
-      rc = m3_mixer_backward(ctx, &desc, handle, ptr(act), ptr(dout), &out, mut(work));
+      rc = m3_mixer_backward(ctx, &d, handle, ptr(act), ptr(dout), &out, mut(work));
     }
     if (rc != M3_OK) raise_status(ctx, rc);
     return g;
@@ -272,13 +311,8 @@ Tensor mixer(uintptr_t handle, const Tensor& proj0, const std::vector<OptTensor>
     node->handle = saved;
     node->desc = d;
     node->act = act;
-    node->in[0] = torch::autograd::SavedVariable(proj, false);
-    node->present[0] = true;
-    for (int i = 0; i < kMixerParams; ++i)
-      if (p[i].defined()) {
-        node->in[1 + i] = torch::autograd::SavedVariable(p[i], false);
-        node->present[1 + i] = true;
-      }
+    node->in[0].set(proj);
+    for (int i = 0; i < kMixerParams; ++i) node->in[1 + i].set(p[i]);
     node->set_next_edges(torch::autograd::collect_next_edges(proj, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8]));
     torch::autograd::set_history(out, node);
   }

@@ -193,19 +193,34 @@ def _ptr(t: Optional[torch.Tensor]):
     return C.c_void_p(t.data_ptr()) if t is not None else None
 
 
+def _placed(t: torch.Tensor, like) -> torch.Tensor:
+    """A saved tensor as hooks gave it back, with the element type, density and alignment it had in the forward pass."""
+    dtype, device, align = like
+    t = t.detach().to(device=device, dtype=dtype).contiguous()
+    if t.data_ptr() % 16 == align:
+        return t
+    n, es = t.numel(), t.element_size()
+    return torch.empty(n + 16 // es, dtype=dtype, device=device)[align // es:align // es + n].view(t.shape).copy_(t)
+
+
 class _FusedSsd(torch.autograd.Function):
     """`ssd_chunked` as one node: the caller's own a, g, w (src/ssm/scan.rs:116-291)."""
+
+    @staticmethod
+    def _desc(opts, x, b, c, a, g, w, h0):
+        B, T, H, P = x.shape
+        return _ffi.ScanDesc(
+            batch=B, seq=T, heads=H, head_dim=P, d_state=b.shape[3], rank=1, chunk=int(opts["chunk"]),
+            dtype=_DTYPES[x.dtype], discretization=int(Discretization.LearnedTrapezoid), dynamics=0,
+            want_state=1 if opts["want_state"] else 0, path=_ffi.PATH_GENERIC,
+            x=_ptr(x), b=_ptr(b), c=_ptr(c), h0=_ptr(h0), a_raw=_ptr(a), g_raw=_ptr(g), w_raw=_ptr(w))
 
     @staticmethod
     def forward(fctx, opts, x, b, c, a, g, w, h0):
         ctx = Context.for_device(x.device)
         B, T, H, P = x.shape
         N = b.shape[3]
-        desc = _ffi.ScanDesc(
-            batch=B, seq=T, heads=H, head_dim=P, d_state=N, rank=1, chunk=int(opts["chunk"]),
-            dtype=_DTYPES[x.dtype], discretization=int(Discretization.LearnedTrapezoid), dynamics=0,
-            want_state=1 if opts["want_state"] else 0, path=_ffi.PATH_GENERIC,
-            x=_ptr(x), b=_ptr(b), c=_ptr(c), h0=_ptr(h0), a_raw=_ptr(a), g_raw=_ptr(g), w_raw=_ptr(w))
+        desc = _FusedSsd._desc(opts, x, b, c, a, g, w, h0)
         y = torch.empty_like(x)
         h = torch.empty((B, H, P, N), device=x.device, dtype=torch.float32) if opts["want_state"] else None
         out = _ffi.ScanOut(y=_ptr(y), h=_ptr(h))
@@ -218,7 +233,8 @@ class _FusedSsd(torch.autograd.Function):
             fctx.saved = _Saved(ctx, saved)
             tensors = (x, b, c, a, g, w, h0)
             fctx.save_for_backward(*[t for t in tensors if t is not None])
-            fctx.present = [t is not None for t in tensors]
+            fctx.opts = opts
+            fctx.like = [(t.dtype, t.device, t.data_ptr() % 16) if t is not None else None for t in tensors]
             fctx.set_materialize_grads(False)
         return (y, h) if h is not None else (y,)
 
@@ -227,11 +243,13 @@ class _FusedSsd(torch.autograd.Function):
         ctx = fctx.m3
         ctx.bind_current_stream()
         it = iter(fctx.saved_tensors)
-        x, b, c, a, g, w, h0 = (next(it) if p else None for p in fctx.present)
+        # saved-tensor hooks may have dropped the forward's tensors: the adjoint reads these
+        tensors = tuple(_placed(next(it), p) if p else None for p in fctx.like)
+        x = tensors[0]
+        desc = _FusedSsd._desc(fctx.opts, *tensors)
         if dy is None:
             dy = torch.zeros_like(x)
         need = fctx.needs_input_grad[1:]
-        tensors = (x, b, c, a, g, w, h0)
         grads = [torch.empty_like(t) if (t is not None and need[i]) else None for i, t in enumerate(tensors)]
         mask = sum(bit for bit, gr in zip((_ffi.GRAD_X, _ffi.GRAD_B, _ffi.GRAD_C, _ffi.GRAD_DT, _ffi.GRAD_DT,
                                            _ffi.GRAD_DT, _ffi.GRAD_H0), grads) if gr is not None)
@@ -240,8 +258,8 @@ class _FusedSsd(torch.autograd.Function):
         bin_ = _ffi.ScanBwdIn(dy=_ptr(dy), dh=_ptr(dh))
         gout = _ffi.ScanGrads(dx=_ptr(grads[0]), db=_ptr(grads[1]), dc=_ptr(grads[2]), da_raw=_ptr(grads[3]),
                               dg_raw=_ptr(grads[4]), dw_raw=_ptr(grads[5]), dh0=_ptr(grads[6]))
-        ctx.check(ctx.lib.m3_scan_backward(ctx.handle, fctx.saved.handle, C.byref(bin_), C.c_uint32(mask | 0xFF),
-                                           C.byref(gout)))
+        ctx.check(ctx.lib.m3_scan_backward_moved(ctx.handle, fctx.saved.handle, C.byref(desc), C.byref(bin_),
+                                                 C.c_uint32(mask | 0xFF), C.byref(gout)))
         return (None,) + tuple(grads)
 
 

@@ -1,0 +1,114 @@
+"""The autograd nodes around the library (csrc/m3_torch.cpp, ssm/scan.py): what torch may do to a node between its
+forward and its backward pass, and to the module that holds the parameters."""
+import pytest
+import torch
+
+from mamba_trainer_b200.nn import MixerCore, MixerShape
+from mamba_trainer_b200.ssm import ScanInputs, mamba3_scan, ssd_chunked
+
+pytestmark = pytest.mark.gpu
+
+
+def _scan_case(dtype, head_dim, d_state, T=200):
+    """(function of leaves, leaves, upstream gradient); the scan's own inputs are intermediate results."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    B, H, R = 1, 2, 1
+    leaves = [r(B, T, H, head_dim, R).to(dtype), (r(B, T, H, d_state, R) / d_state ** 0.5).to(dtype),
+              (r(B, T, H, d_state, R) / d_state ** 0.5).to(dtype), (0.05 + 0.1 * r(B, T, H).abs()).to(dtype), r(H).abs(),
+              torch.sigmoid(r(B, T, H)).to(dtype), r(B, T, H, d_state // 2).to(dtype), r(H)]
+
+    def f(*v):
+        x, b, c, dt, a_log, lam, theta, d_skip = (t * 0.5 for t in v)
+        return mamba3_scan(ScanInputs.new(x, b, c, dt, a_log, lam).with_theta(theta).with_skip(d_skip).with_chunk_size(64)).y
+    return f, leaves, r(B, T, H, head_dim, R).to(dtype)
+
+
+def _ssd_case():
+    g = torch.Generator(device="cuda").manual_seed(2)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    leaves = [r(2, 50, 2, 16), r(2, 50, 2, 24), r(2, 50, 2, 24), -r(2, 50, 2).abs(), r(2, 50, 2), r(2, 50, 2), r(2, 2, 16, 24)]
+    return (lambda *v: ssd_chunked(*(t * 0.5 for t in v), chunk_size=16)[0]), leaves, r(2, 50, 2, 16)
+
+
+def _mixer_case(dtype, head_dim=64, d_state=128, T=200):
+    shape = MixerShape(2, head_dim, d_state, 1)
+    torch.manual_seed(3)
+    core = MixerCore(shape, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(4)
+    proj = torch.randn(2, T, shape.in_proj_width, device="cuda", generator=g).to(dtype)
+    names = [n for n, _ in core.named_parameters()]
+
+    def f(p, *params):
+        return torch.func.functional_call(core, {n: q * 0.5 for n, q in zip(names, params)}, (p * 0.5,))
+    return f, [proj] + [q.detach().clone() for q in core.parameters()], \
+        torch.randn(2, T, shape.d_inner, device="cuda", generator=g).to(dtype)
+
+
+CASES = {
+    "scan_tensor_core": lambda: _scan_case(torch.bfloat16, 64, 128),
+    "scan_chunk_parallel": lambda: _scan_case(torch.float32, 64, 64),
+    "scan_generic": lambda: _scan_case(torch.float32, 24, 40),
+    "ssd": _ssd_case,
+    "mixer_bf16": lambda: _mixer_case(torch.bfloat16),
+    "mixer_f32": lambda: _mixer_case(torch.float32),
+    "mixer_f32_separate_steps": lambda: _mixer_case(torch.float32, 24, 40),
+}
+
+
+def _gradients(f, leaves, dout, around=None, apply=None):
+    leaves = [t.clone().requires_grad_(True) for t in leaves]
+    if around is None:
+        out = (apply or (lambda fn, *a: fn(*a)))(f, *leaves)
+    else:
+        with around:
+            out = f(*leaves)
+    # whatever the forward pass let go of is taken over by others before the backward pass runs
+    junk = [torch.full((n,), float("nan"), device="cuda") for n in (64, 1024, 16384, 1 << 18, 1 << 20) for _ in range(12)]
+    grads = torch.autograd.grad(out, leaves, dout)
+    del junk
+    return (out.detach(),) + grads
+
+
+@pytest.mark.parametrize("how", ["checkpoint", "offload", "moved"])
+@pytest.mark.parametrize("case", CASES)
+def test_gradients_under_saved_tensor_hooks(case, how):
+    """Activation checkpointing and offloading drop what a node saved and bring back other tensors - in `moved`, at another
+    alignment: the adjoint reads those, and the gradients are the plain run's."""
+    from torch.utils.checkpoint import checkpoint
+    f, leaves, dout = CASES[case]()
+    want = _gradients(f, leaves, dout)
+    if how == "checkpoint":
+        got = _gradients(f, leaves, dout, apply=lambda fn, *a: checkpoint(fn, *a, use_reentrant=False))
+    elif how == "offload":
+        got = _gradients(f, leaves, dout, torch.autograd.graph.save_on_cpu())
+    else:
+        def unpack(t):
+            return torch.empty(t.numel() + 3, dtype=t.dtype, device="cuda")[3:].view(t.shape).copy_(t)
+        got = _gradients(f, leaves, dout, torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach().cpu().contiguous(), unpack))
+    for i, (a, e) in enumerate(zip(got, want)):
+        assert torch.equal(a, e), (i, float((a.float() - e.float()).abs().max()))
+
+
+def test_moved_inputs_are_checked():
+    """The C entry that takes the inputs' new addresses refuses another shape, another alignment and an absent input."""
+    import ctypes as C
+    from mamba_trainer_b200 import _ffi
+    from mamba_trainer_b200.ssm import Context
+    ctx = Context.for_device(torch.device("cuda"))
+    B, T, H, P, N = 1, 70, 2, 24, 40
+    n = {"x": B * T * H * P, "b": B * T * H * N, "c": B * T * H * N, "dt": B * T * H, "lambda_": B * T * H, "a_log": H}
+    t = {k: torch.rand(v + 4, device="cuda") for k, v in n.items()}
+    at = lambda off: {k: C.c_void_p(v.data_ptr() + 4 * off) for k, v in t.items()}
+    make = lambda off=0, **kw: _ffi.ScanDesc(**{**dict(batch=B, seq=T, heads=H, head_dim=P, d_state=N, rank=1, chunk=16,
+                                                       discretization=2), **at(off), **kw})
+    y, saved = torch.empty(n["x"], device="cuda"), C.c_void_p()
+    ctx.check(ctx.lib.m3_scan_forward(ctx.handle, C.byref(make()), C.byref(_ffi.ScanOut(y=C.c_void_p(y.data_ptr()))), C.byref(saved)))
+    dx = torch.empty_like(y)
+    run = lambda d: ctx.lib.m3_scan_backward_moved(ctx.handle, saved, C.byref(d), C.byref(_ffi.ScanBwdIn(dy=C.c_void_p(y.data_ptr()))),
+                                                   _ffi.GRAD_X, C.byref(_ffi.ScanGrads(dx=C.c_void_p(dx.data_ptr()))))
+    assert run(make()) == _ffi.OK
+    assert run(make(heads=1)) == _ffi.ERR_CONFIG
+    assert run(make(off=1)) == _ffi.ERR_UNSUPPORTED
+    assert run(make(lambda_=None)) == _ffi.ERR_NULL
+    ctx.check(ctx.lib.m3_saved_free(ctx.handle, saved))
