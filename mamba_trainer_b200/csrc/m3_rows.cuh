@@ -4,16 +4,17 @@
 // A CTA works on one chunk of 64 rows rho = (t, r) (64 / R time steps) of one (batch, head); all chunks of all stripes
 // run at once and only the pass over chunk states is sequential (m3_rows_fwd.cu says which kernels there are).
 //
-// Contractions run on the tensor cores in split TF32: an operand x is hi + lo, hi = x cut to TF32's 11 significant
-// bits, lo = the rest rounded to as many, and a product is lo hi + hi lo + hi hi with float32 accumulation: what is
-// dropped (lo lo, and the rounding of lo) is below 2^-20 of a product and unbiased, as a float32 sum's own rounding is.
-// Fragments come four words at a time by ldmatrix where the operand is stored along the contraction (a word at a time,
-// with four operations for the split, the kernels were bound by issue: float32, 8 x 1024 x 16 heads, d_state 128: the
-// adjoint 478 -> 472 us, the outputs 166 -> 159 us; what bounds them now is the phases between block barriers).  mma.sync m16n8k8 runs 278 TFLOP/s
-// on a B200, so 93 after the threefold product, against 51 measured for float32 FMAs from registers (and half of that
-// in the 64 x 64 block products of the generic family).  tcgen05's kind::tf32 would be faster still, but wants every
-// operand K-major in shared memory: half of the operands here are contracted along their rows.  An operand whose values
-// are bf16 already is its own hi part and needs no lo product.
+// Contractions run on the tensor cores in split TF32: an operand x is hi + lo, hi = x rounded to TF32's 11 significant bits,
+// lo = the rest cut to as many, and a product is lo hi + hi lo + hi hi; what is dropped (lo lo, and what is cut from lo) is
+// below 2^-22 of it.  For float32 tensors the sum over the contraction is kept by the float32 units (warp_mma says why): with
+// hi cut and the whole sum left to the tensor core, y, d x, d B and d C were 2.7 to 4.6 times as far from 64-bit results as
+// the generic family's, now 0.6 to 0.9 times, for 2 % of the time (8 x 1024 tokens x 16 heads, d_state 128, mixer forward +
+// backward: 1125 -> 1149 us; the double sums of the log decay, SumOf, and the skip's place in d x: 1165 us).  mma.sync m16n8k8
+// runs 278 TFLOP/s on a B200, so 93 after the threefold product, against 51 measured for float32 FMAs from registers (and half
+// of that in the 64 x 64 block products of the generic family).  Fragments come four words at a time by ldmatrix where the
+// operand is stored along the contraction.  tcgen05's kind::tf32 would be faster still, but wants every operand K-major in
+// shared memory: half of the operands here are contracted along their rows.  An operand whose values are bf16 already is its
+// own hi part and needs no lo product.
 //
 // Operands lie in shared memory as [row][col] floats with leading dimension N or 64, columns XOR-swizzled by fsw(row),
 // so that fragments along either index come without bank conflicts: eight rows x four columns (an operand contracted
@@ -32,11 +33,12 @@ __host__ __device__ __forceinline__ constexpr int fsw(int row) { return ((row & 
 template <int LD>
 __device__ __forceinline__ int at(int row, int col) { return row * LD + (col ^ fsw(row)); }
 
-// The tensor core reads the upper 19 bits of a TF32 operand, so x as it stands is its own hi part (truncated); lo is what
-// truncation leaves, rounded to the bits that will be read (half of the last one added): three operations.
+// hi is x rounded to the 19 bits that the tensor core reads of a TF32 operand, lo the rest (exact; the tensor core reads its
+// upper 19 bits, which cuts it below 2^-23 of x).  Rounding hi makes lo's sign independent of x's, so that neither what is
+// cut from lo nor the dropped lo lo pulls a sum one way.
 __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = __float_as_uint(x);
-  lo = __float_as_uint(x - __uint_as_float(hi & 0xffffe000u)) + 0x1000u;
+  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  lo = __float_as_uint(x - __uint_as_float(hi));
 }
 // Four 8-row x 4-column pieces of float32 by one instruction: word q of row g of each is this lane's.
 __device__ __forceinline__ void ldm4f(uint32_t (&r)[4], const float* p) {
@@ -56,7 +58,10 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
 // AKC: A is stored [m][k], else [k][m]; BKC: B is stored [n][k], else [k][n].  AEX / BEX: that operand's values are
 // exact in TF32.  Accumulator layout: element e of a tile is row g + 8 (e >> 1), column 2 q + (e & 1), with g = lane / 4,
 // q = lane % 4.
-template <int MT, int NT, bool AKC, bool BKC, bool AEX, bool BEX, int LDA, int LDB>
+// SUM: the products of every eight k are summed in the tensor core and added to acc by the float32 units, whose additions
+// round to nearest; the tensor core's own cut, which over a sum of 64 to 128 would be most of the error (float32).  Tensors of
+// bf16 leave the whole sum to the tensor core.
+template <int MT, int NT, bool AKC, bool BKC, bool AEX, bool BEX, int LDA, int LDB, bool SUM>
 __device__ __forceinline__ void warp_mma(float (&acc)[MT][NT][4], const float* sA, int m0, const float* sB, int n0, int k0,
                                          int k1) {
   static_assert(!BKC || NT % 2 == 0, "a load brings two column tiles");
@@ -107,22 +112,36 @@ __device__ __forceinline__ void warp_mma(float (&acc)[MT][NT][4], const float* s
 #pragma unroll
         for (int i = 0; i < 2; ++i) split_tf32(__uint_as_float(bh[nt][i]), bh[nt][i], bl[nt][i]);
     }
-    if (!AEX) {
+    if constexpr (SUM) {
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) mma_tf32(acc[mt][nt], al[mt], bh[nt]);
-    }
-    if (!BEX) {
+        for (int nt = 0; nt < NT; ++nt) {
+          float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          if (!AEX) mma_tf32(t, al[mt], bh[nt]);
+          if (!BEX) mma_tf32(t, ah[mt], bl[nt]);
+          mma_tf32(t, ah[mt], bh[nt]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[mt][nt][e] += t[e];
+        }
+    } else {
+      if (!AEX) {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) mma_tf32(acc[mt][nt], al[mt], bh[nt]);
+      }
+      if (!BEX) {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) mma_tf32(acc[mt][nt], ah[mt], bl[nt]);
+      }
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) mma_tf32(acc[mt][nt], ah[mt], bl[nt]);
+        for (int nt = 0; nt < NT; ++nt) mma_tf32(acc[mt][nt], ah[mt], bh[nt]);
     }
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) mma_tf32(acc[mt][nt], ah[mt], bh[nt]);
   }
 }
 template <int MT, int NT>
@@ -182,12 +201,28 @@ __device__ __forceinline__ Chunk this_chunk(const Dims& d) {
 }
 
 // Per-token scalars of a chunk in shared memory: dt, lambda (one step of look-ahead), cumulative log decay, weights,
-// exp(ac), exp(cd - ac) w.
+// exp(ac), exp(cd - ac) and that times w.
 template <int R>
 struct Scal {
   static constexpr int LT = kRows / R;
-  float dt[LT + 1], lam[LT + 1], ac[LT], g[LT], w[LT], eac[LT], sw[LT];
+  float dt[LT + 1], lam[LT + 1], ac[LT], g[LT], w[LT], eac[LT], dte[LT], sw[LT];
 };
+// What the sums of the log decay and of its gradient over a chunk are kept in.  Sums by a tree do not share their roundings
+// as sequential ones do, and the differences of two of them near the chunk's end, which weigh most, would carry those of the
+// whole sum: double for float32 tensors.  (Far below the rounding of bf16 tensors.)
+template <class T>
+using SumOf = std::conditional_t<sizeof(T) == 4, double, float>;
+// Inclusive prefix sum over the lanes (SUFFIX: over this lane and those behind it).
+template <bool SUFFIX, class S>
+__device__ __forceinline__ S lane_scan(S v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const S n = SUFFIX ? __shfl_down_sync(0xffffffffu, v, o) : __shfl_up_sync(0xffffffffu, v, o);
+    if (SUFFIX ? lane + o < 32 : lane >= o) v += n;
+  }
+  return v;
+}
 // Contains two block barriers; complete after the caller's next one.
 template <class T, int R>
 __device__ __forceinline__ void chunk_scalars(Scal<R>& s, const Dims& d, const Chunk& c, const m3_scan_desc& in) {
@@ -208,11 +243,12 @@ __device__ __forceinline__ void chunk_scalars(Scal<R>& s, const Dims& d, const C
   if (tid < 32) {
     constexpr int EPL = LT >= 32 ? LT / 32 : 1;
     const float A = d.raw ? 0.0f : -expf(in.a_log[c.h]);
-    float loc[EPL], run = 0.0f;
+    SumOf<T> loc[EPL], run = 0;
 #pragma unroll
     for (int i = 0; i < EPL; ++i) {
       const int l = tid * EPL + i, t = c.t0 + l;
-      float gv = 0.0f, wv = 0.0f, av = 0.0f;
+      float gv = 0.0f, wv = 0.0f;
+      SumOf<T> av = 0;
       if (l < LT && t < d.T) {
         if (d.raw) {  // scan.rs:116-126: the caller's own a, g, w
           const size_t o = tok_index(d, c.b, t, c.h);
@@ -220,7 +256,7 @@ __device__ __forceinline__ void chunk_scalars(Scal<R>& s, const Dims& d, const C
           gv = ldf(static_cast<const T*>(in.g_raw), o);
           wv = ldf(static_cast<const T*>(in.w_raw), o);
         } else {
-          av = s.dt[l] * A;
+          av = (SumOf<T>)s.dt[l] * A;
           gv = s.lam[l] * s.dt[l];
           wv = gv + (t + 1 < d.T ? (1.0f - s.lam[l + 1]) * s.dt[l + 1] : 0.0f);
         }
@@ -229,21 +265,16 @@ __device__ __forceinline__ void chunk_scalars(Scal<R>& s, const Dims& d, const C
       run += av;
       loc[i] = run;
     }
-    float tot = run;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float n = __shfl_up_sync(0xffffffffu, tot, o);
-      if (tid >= o) tot += n;
-    }
-    const float base = tot - run, cd = __shfl_sync(0xffffffffu, tot, 31);
+    const SumOf<T> tot = lane_scan<false>(run), base = tot - run, cd = __shfl_sync(0xffffffffu, tot, 31);
 #pragma unroll
     for (int i = 0; i < EPL; ++i) {
       const int l = tid * EPL + i;
       if (l < LT) {
-        const float ac = base + loc[i];
-        s.ac[l] = l == LT - 1 ? cd : ac;
-        s.eac[l] = exp_decay(ac);
-        s.sw[l] = exp_decay(cd - ac) * s.w[l];
+        const SumOf<T> ac = base + loc[i];
+        s.ac[l] = (float)(l == LT - 1 ? cd : ac);
+        s.eac[l] = exp_decay((float)ac);
+        s.dte[l] = exp_decay((float)(cd - ac));
+        s.sw[l] = s.dte[l] * s.w[l];
       }
     }
   }

@@ -166,12 +166,13 @@ __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoin
   constexpr int NX = 8 / WC;         // [64 x 64] results: warps 4 (16 rows) x WC
   const int m0 = 16 * (warp & 3), n0 = 8 * NX * (warp >> 2);
   float dc[2][NT][4], db[2][NT][4], dx[1][NX][4];
+  const float dsk = in.d_skip ? in.d_skip[c.h] : 0.0f;
   zero(dc);
   zero(db);
   zero(dx);
-  warp_mma<2, NT, true, false, EX, false, kP, N>(dc, sm.dy, M0, sH, N0, 0, kP);   // T1 = dY~ H_k
-  warp_mma<2, NT, true, false, EX, false, kP, N>(db, sm.x, M0, sS, N0, 0, kP);    // X~ dS_k
-  warp_mma<1, NX, true, true, false, false, N, N>(dx, sm.b, m0, sS, n0, 0, N);     // U = B^ dS_k^T
+  warp_mma<2, NT, true, false, EX, false, kP, N, !EX>(dc, sm.dy, M0, sH, N0, 0, kP);   // T1 = dY~ H_k
+  warp_mma<2, NT, true, false, EX, false, kP, N, !EX>(db, sm.x, M0, sS, N0, 0, kP);    // X~ dS_k
+  warp_mma<1, NX, true, true, false, false, N, N, !EX>(dx, sm.b, m0, sS, n0, 0, N);     // U = B^ dS_k^T
   {
     float t1[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};   // <T1, C^> of the rows
     for_acc(dc, M0, N0, [&](int row, int col, float& a, float& b) {
@@ -192,15 +193,18 @@ __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoin
       const float v = quad_sum(t1[i >> 1][i & 1]);
       if (q4 == 0) sm.t1[wn][M0 + 8 * i + g] = v;
     }
-    float qs[2] = {0.0f, 0.0f};   // q = <U, x> of the rows; dX~ starts as sw U + D dy
-    const float dsk = in.d_skip ? in.d_skip[c.h] : 0.0f;
+    float qs[2] = {0.0f, 0.0f};   // q = <U, x> of the rows; dX~ starts as sw U (+ D dy)
     for_acc(dx, m0, n0, [&](int row, int col, float& a, float& b) {
       const float2 xv = *reinterpret_cast<const float2*>(sm.x + at<kP>(row, col));
-      const float2 gv = *reinterpret_cast<const float2*>(sm.dy + at<kP>(row, col));
       qs[(row - m0 - g) >> 3] += a * xv.x + b * xv.y;
       const float e = ts.sw[row / R];
-      a = fmaf(e, a, dsk * gv.x);
-      b = fmaf(e, b, dsk * gv.y);
+      a *= e;
+      b *= e;
+      if (EX) {
+        const float2 gv = *reinterpret_cast<const float2*>(sm.dy + at<kP>(row, col));
+        a = fmaf(dsk, gv.x, a);
+        b = fmaf(dsk, gv.y, b);
+      }
     });
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -225,8 +229,8 @@ __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoin
   zero(dm);
   const bool below = n0 < m0 + 16;
   if (below) {
-    warp_mma<1, NX, true, true, false, false, N, N>(gm, sm.c, m0, sm.b, n0, 0, N);
-    warp_mma<1, NX, true, true, EX, EX, kP, kP>(dm, sm.dy, m0, sm.x, n0, 0, kP);
+    warp_mma<1, NX, true, true, false, false, N, N, !EX>(gm, sm.c, m0, sm.b, n0, 0, N);
+    warp_mma<1, NX, true, true, EX, EX, kP, kP, !EX>(dm, sm.dy, m0, sm.x, n0, 0, kP);
   }
   dcd = adj_sum<kAdj>(dcd, sm.red);   // the states have been read by everyone: M and dG take their place
   dD = adj_sum<kAdj>(dD, sm.red);
@@ -285,11 +289,18 @@ __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoin
   }
   __syncthreads();
   // ---- dX~ += M^T dY~, dB^ += dG^T C^, dC^ += dG B^ (only the triangle's half of each sum) ---------------------
-  warp_mma<1, NX, false, false, false, EX, kRows, kP>(dx, sM, m0, sm.dy, n0, m0, kRows);
-  warp_mma<2, NT, false, false, false, false, kRows, N>(db, sG, M0, sm.c, N0, M0, kRows);
-  warp_mma<2, NT, true, false, false, false, kRows, N>(dc, sG, M0, sm.b, N0, 0, M0 + 32);
-  __syncthreads();   // M, dG and dY~ are spent
-  store_acc<kP>(dx, m0, n0, sm.dy);
+  warp_mma<1, NX, false, false, false, EX, kRows, kP, !EX>(dx, sM, m0, sm.dy, n0, m0, kRows);
+  warp_mma<2, NT, false, false, false, false, kRows, N, !EX>(db, sG, M0, sm.c, N0, M0, kRows);
+  warp_mma<2, NT, true, false, false, false, kRows, N, !EX>(dc, sG, M0, sm.b, N0, 0, M0 + 32);
+  __syncthreads();   // M and dG are spent, and dY~ but for the words that a thread's own share of dX~ replaces
+  if constexpr (EX) {
+    store_acc<kP>(dx, m0, n0, sm.dy);
+  } else {   // float32: the skip's share last, as all that is added behind it is rounded at its size
+    for_acc(dx, m0, n0, [&](int row, int col, float& a, float& b) {
+      float2* const to = reinterpret_cast<float2*>(sm.dy + at<kP>(row, col));
+      *to = make_float2(fmaf(dsk, to->x, a), fmaf(dsk, to->y, b));
+    });
+  }
   store_acc<N>(db, M0, N0, sDB);
   store_acc<N>(dc, M0, N0, sDC);
   __syncthreads();
@@ -399,7 +410,7 @@ __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoin
 #pragma unroll
       for (int i = 0; i < WN; ++i) t1 += sm.t1[i][ro];
     }
-    const float ac = ts.ac[l], raw = cd - ac, sg = exp_decay(raw);
+    const float ac = ts.ac[l], raw = cd - ac, sg = ts.dte[l];
     const float dast = sg * ts.w[l] * q * clamp_inside(raw);
     sm.dac[l] = rows_ - col + ts.eac[l] * clamp_inside(ac) * t1 - dast;
     sm.dast[l] = dast;
@@ -415,25 +426,20 @@ __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoin
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tail += __shfl_xor_sync(0xffffffffu, tail, o);
     tail += exp_decay(cd) * clamp_inside(cd) * dcd;
-    float loc[EPL], run = 0.0f;
+    SumOf<T> loc[EPL], run = 0;
 #pragma unroll
     for (int i = EPL - 1; i >= 0; --i) {
       const int l = lane * EPL + i;
-      if (l < LT) run += sm.dac[l] + (l == LT - 1 ? tail : 0.0f);
+      if (l < LT) run += (SumOf<T>)sm.dac[l] + (l == LT - 1 ? tail : 0.0f);
       loc[i] = run;
     }
-    float tot = run;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float n = __shfl_down_sync(0xffffffffu, tot, o);
-      if (lane + o < 32) tot += n;
-    }
+    const SumOf<T> tot = lane_scan<true>(run);
     float pa = 0.0f;
 #pragma unroll
     for (int i = 0; i < EPL; ++i) {
       const int l = lane * EPL + i;
       if (l < LT) {
-        const float da = tot - run + loc[i];
+        const float da = (float)(tot - run + loc[i]);
         out.da[(size_t)c.bh * d.Tp + c.t0 + l] = da;
         pa += da * ts.dt[l];
       }

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256, N == 64 ? 4 : 3) k_rows_state(Dims d, m3_
   const int warp = threadIdx.x >> 5, m0 = 32 * (warp & 1), n0 = 8 * NT * (warp >> 1);
   float acc[2][NT][4];
   zero(acc);
-  warp_mma<2, NT, false, false, EX, false, kP, N>(acc, sm.x, m0, sm.b, n0, 0, kRows);
+  warp_mma<2, NT, false, false, EX, false, kP, N, !EX>(acc, sm.x, m0, sm.b, n0, 0, kRows);
   store_acc<N>(acc, m0, n0, dst + ((size_t)c.bh * (BWD ? d.C + 1 : d.C) + c.k) * kP * N);
 }
 
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256, N == 64 ? 3 : 2) k_rows_out(Dims d, m3_sc
   {
     float g[2][2][4];
     zero(g);
-    if (n0 < m0 + 32) warp_mma<2, 2, true, true, false, false, N, N>(g, sm.c, m0, sm.b, n0, 0, N);
+    if (n0 < m0 + 32) warp_mma<2, 2, true, true, false, false, N, N, !EX>(g, sm.c, m0, sm.b, n0, 0, N);
     for_acc(g, m0, n0, [&](int row, int col, float& a, float& b) {
       const int l = row / R;
       const float ac = sm.s.ac[l];
@@ -191,13 +191,13 @@ __global__ void __launch_bounds__(256, N == 64 ? 3 : 2) k_rows_out(Dims d, m3_sc
   // Y = exp(acum) C~ H^T + M X~
   float acc[2][2][4];
   zero(acc);
-  warp_mma<2, 2, true, true, false, false, N, N>(acc, sm.c, m0, sm.b, n0, 0, N);
+  warp_mma<2, 2, true, true, false, false, N, N, !EX>(acc, sm.c, m0, sm.b, n0, 0, N);
   for_acc(acc, m0, n0, [&](int row, int, float& a, float& b) {
     const float e = sm.s.eac[row / R];
     a *= e;
     b *= e;
   });
-  warp_mma<2, 2, true, false, false, EX, kP, kP>(acc, sm.m, m0, sm.x, n0, 0, m0 + 32);
+  warp_mma<2, 2, true, false, false, EX, kP, kP, !EX>(acc, sm.m, m0, sm.x, n0, 0, m0 + 32);
   __syncthreads();   // M is spent: its buffer stages y
   const float dsk = in.d_skip ? in.d_skip[c.h] : 0.0f;
   for_acc(acc, m0, n0, [&](int row, int col, float& a, float& b) {

@@ -66,6 +66,29 @@ def test_chunk_parallel_family_matches_the_oracle(dtype, B, T, H, N, R, rot, sta
     compare_all(t, 64, check_f32 if dtype == torch.float32 else check_bf16, True, ds, discretization=d, reverse_heads=rev)
 
 
+@pytest.mark.parametrize("B,T,H,N,R,rot", [(2, 256, 4, 64, 1, False), (1, 2000, 4, 128, 1, True), (2, 513, 4, 128, 2, True),
+                                          (2, 300, 4, 64, 4, False)])
+def test_chunk_parallel_float32_is_as_accurate_as_float32_sums(B, T, H, N, R, rot):
+    """Split TF32 against float32 multiply-adds, on inputs as models have them: the chunk-parallel family's distance from
+    the float64 oracle is at most the generic family's, which an x that starts off 16 bytes takes.  (1.1: the rounding
+    noise of the smallest tensors here, a few thousand values.)"""
+    from _util import fused_run, oracle_run
+    from mamba_trainer_b200 import synthetic
+    w = synthetic.Workload("float32", B, T, H, 64, N, 64, R, torch.float32, Discretization.LearnedTrapezoid, rot,
+                           "rms" if R == 1 else "scaled")
+    t = synthetic.make_inputs(w, seed=T)
+    y, _, exact = oracle_run(t, 64, False)
+    exact["y"] = y
+    dev = {k: v.cuda() if v is not None else None for k, v in t.items()}
+    buf = torch.empty(t["x"].numel() + 1, device="cuda")
+    off = dict(dev, x=buf[1:].view(t["x"].shape).copy_(t["x"]))
+    (y, _, got), (yg, _, generic) = fused_run(dev, 64, False), fused_run(off, 64, False)
+    got["y"], generic["y"] = y, yg
+    for n in ("y", "x", "b", "c", "dt", "lam") + (("theta",) if rot else ()):
+        a, e = norm_rel(got[n], exact[n]), norm_rel(generic[n], exact[n])
+        assert a <= 1.1 * e, (n, a, e)
+
+
 def test_chunk_parallel_backward_takes_unaligned_gradients():
     """dy and the gradient buffers of the C ABI may start anywhere; aligned ones give the same bits."""
     import ctypes as C
