@@ -54,8 +54,9 @@ typedef enum { M3_EULER = 0, M3_TRAPEZOID = 1, M3_LEARNED_TRAPEZOID = 2 } m3_dis
 /* StateDynamics, src/ssm/config.rs:45-56.  Rotational needs theta and even d_state. */
 typedef enum { M3_REAL = 0, M3_ROTATIONAL = 1 } m3_dynamics;
 
-/* Which kernel family runs.  AUTO picks the tensor-core family when the shape is
- * one it serves and the generic family otherwise. */
+/* Which kernel family runs.  AUTO picks the tensor-core family when the shape is one it serves, the chunk-parallel
+ * family (head_dim 64, d_state 64 or 128, rank 1, 2 or 4, four elements at a time aligned) where that does, and the
+ * generic family otherwise.  GENERIC and TENSOR run the family they name. */
 typedef enum { M3_PATH_AUTO = 0, M3_PATH_GENERIC = 1, M3_PATH_TENSOR = 2 } m3_path;
 
 /* ScanInputs, src/ssm/scan.rs:361-385.  rank is SsmMode::rank() (config.rs:74-79). */
@@ -92,7 +93,7 @@ typedef struct {
    * diagonal / off-diagonal weights g, w themselves, all [batch, seq, heads].  When a_raw is
    * set (then g_raw and w_raw must be too) dt, lambda and a_log are not read, theta must be
    * NULL, h0 alone is the boundary value carried in (last_u0 is not read) and no last_u is
-   * produced.  The generic kernel family serves this form. */
+   * produced.  The tensor-core family does not serve this form. */
   const void *a_raw, *g_raw, *w_raw;
 } m3_scan_desc;
 
@@ -175,7 +176,7 @@ int m3_download(m3_ctx *ctx, void *dst_host, const void *src_device, size_t byte
  * The saved context refers to the input buffers of `desc`: keep them alive and
  * unchanged until then (the reference's closure holds clones, var.rs:210-216).
  * The tensor-core kernel family moves rows as 16-byte vectors: with M3_PATH_AUTO a call whose
- * x, b, c, theta or y is not 16-byte aligned runs the generic family instead (M3_PATH_TENSOR
+ * x, b, c, theta or y is not 16-byte aligned runs another family instead (M3_PATH_TENSOR
  * refuses it), and the backward of a forward that ran the tensor-core family needs 16-byte
  * aligned dy, dx, db, dc and dtheta (M3_ERR_UNSUPPORTED otherwise). */
 int m3_scan_forward(m3_ctx *ctx, const m3_scan_desc *desc, const m3_scan_out *out,
@@ -224,7 +225,7 @@ int m3_step_forward(m3_ctx *ctx, const m3_step_desc *desc, const m3_step_out *ou
  * M3_ERR_UNSUPPORTED.  Shapes the tensor-core family serves run there unless
  * desc->path says M3_PATH_GENERIC: with nothing kept for a backward pass that family
  * needs no scratch at all (few long stripes are cut into segments while what that takes fits the block);
- * everything else runs the generic family on the block.
+ * everything else runs the chunk-parallel or the generic family on the block.
  * The first call on each device looks up the block's device address (with that
  * device current), and - CUDA loads a library's kernels and file-scope device arrays
  * when they are first touched - it is also the call during which the driver maps the

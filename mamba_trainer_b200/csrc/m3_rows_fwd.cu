@@ -247,8 +247,10 @@ cudaError_t dh_local(cudaStream_t st, const Dims& d, const m3_scan_desc& in, con
 
 }  // namespace rows
 
-// Vector accesses of 4 elements: every tensor and theta-free row start aligned to that.
+// Vector accesses of 4 elements: every tensor and theta-free row start aligned to that.  A caller who names the generic family
+// gets it.
 bool rows_supported(const m3_scan_desc& s, const void* y) {
+  if (s.path == M3_PATH_GENERIC) return false;
   if (s.head_dim != rows::kP || (s.d_state != 64 && s.d_state != 128) || (s.rank != 1 && s.rank != 2 && s.rank != 4)) return false;
   const uintptr_t a = s.dtype == M3_F32 ? 15 : 7;
   for (const void* p : {s.x, s.b, s.c, y})

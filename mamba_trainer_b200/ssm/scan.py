@@ -212,7 +212,7 @@ class _FusedSsd(torch.autograd.Function):
         return _ffi.ScanDesc(
             batch=B, seq=T, heads=H, head_dim=P, d_state=b.shape[3], rank=1, chunk=int(opts["chunk"]),
             dtype=_DTYPES[x.dtype], discretization=int(Discretization.LearnedTrapezoid), dynamics=0,
-            want_state=1 if opts["want_state"] else 0, path=_ffi.PATH_GENERIC,
+            want_state=1 if opts["want_state"] else 0, path=_ffi.PATH_AUTO,
             x=_ptr(x), b=_ptr(b), c=_ptr(c), h0=_ptr(h0), a_raw=_ptr(a), g_raw=_ptr(g), w_raw=_ptr(w))
 
     @staticmethod

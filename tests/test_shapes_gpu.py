@@ -89,6 +89,66 @@ def test_chunk_parallel_float32_is_as_accurate_as_float32_sums(B, T, H, N, R, ro
         assert a <= 1.1 * e, (n, a, e)
 
 
+@pytest.mark.parametrize("dtype,N,R,rot", [(torch.float32, 64, 1, True), (torch.float32, 128, 2, False), (torch.bfloat16, 64, 1, True)])
+def test_the_generic_path_runs_the_generic_kernels(dtype, N, R, rot):
+    """A caller who names the generic family gets it at shapes the chunk-parallel one serves, in the scan and in the mixer:
+    the oracle's results, from more launches."""
+    from test_scan_gpu import check_bf16, check_f32, compare_all, small_inputs
+    from _util import fused_run
+    from mamba_trainer_b200 import _ffi
+    from mamba_trainer_b200.nn import MixerCore, MixerShape
+    from mamba_trainer_b200.ssm import Context
+    t, ds = small_inputs(2, 150, 2, 64, N, R, rot, True, seed=N + R)
+    for k in ("x", "b", "c", "dt", "lam", "theta", "dy"):
+        if t[k] is not None:
+            t[k] = (t[k] / (N ** 0.5 if k in "bc" else 1)).to(dtype)
+    ctx = Context.for_device(torch.device("cuda"))
+
+    def launches(f):
+        before = ctx.lib.m3_launch_count(ctx.handle)
+        f()
+        return ctx.lib.m3_launch_count(ctx.handle) - before
+    check = check_f32 if dtype == torch.float32 else check_bf16
+    n = {p: launches(lambda: fused_run(t, 64, True, True, ds, path=p)) for p in (_ffi.PATH_AUTO, _ffi.PATH_GENERIC)}
+    assert n[_ffi.PATH_GENERIC] > n[_ffi.PATH_AUTO], n
+    compare_all(t, 64, check, True, ds, path=_ffi.PATH_GENERIC)
+    shape = MixerShape(2, 64, N, R, None, True, rot)
+    torch.manual_seed(1)
+    core = MixerCore(shape, device="cuda")
+    proj = torch.randn(2, 150, shape.in_proj_width, device="cuda").to(dtype).requires_grad_(True)
+    outs = []
+    m = {p: launches(lambda: outs.append(core(proj, path=p))) for p in (_ffi.PATH_AUTO, _ffi.PATH_GENERIC)}
+    assert m[_ffi.PATH_GENERIC] > m[_ffi.PATH_AUTO], m
+    (a,), (b,) = (torch.autograd.grad(o.float().square().sum(), [proj]) for o in outs)
+    assert norm_rel(outs[0], outs[1]) <= (1e-5 if dtype == torch.float32 else 2e-2)
+    assert norm_rel(a, b) <= (1e-5 if dtype == torch.float32 else 2e-2)
+
+
+@pytest.mark.parametrize("dtype,B,T,H,N,state", [(torch.float32, 2, 64, 2, 128, True), (torch.float32, 1, 65, 3, 64, False),
+                                                (torch.float32, 1, 321, 2, 64, True), (torch.bfloat16, 1, 150, 2, 128, True)])
+def test_ssd_chunked_at_chunk_parallel_shapes(dtype, B, T, H, N, state):
+    """The entry with the caller's own a, g, w takes the chunk-parallel kernels at head_dim 64: against the oracle."""
+    from test_scan_gpu import check_bf16, check_f32
+    from mamba_trainer_b200.ssm import ssd_chunked
+    from oracle import m3_oracle as O
+    g = torch.Generator().manual_seed(T)
+    r = lambda *s: torch.randn(*s, generator=g)
+    vals = [r(B, T, H, 64), r(B, T, H, N) / N ** 0.5, r(B, T, H, N) / N ** 0.5, -0.3 * r(B, T, H).abs(), r(B, T, H), r(B, T, H)]
+    vals = [v.to(dtype) for v in vals] + ([r(B, H, 64, N)] if state else [])
+    dy, dh = r(B, T, H, 64).to(dtype), r(B, H, 64, N)
+    cpu = [v.double().requires_grad_(True) for v in vals]
+    ey, eh = O.ssd_chunked(*cpu[:6], cpu[6] if state else None, 64, True)
+    eg = torch.autograd.grad((ey * dy.double()).sum() + (eh * dh.double()).sum(), cpu)
+    dev = [v.cuda().requires_grad_(True) for v in vals]
+    y, h = ssd_chunked(*dev[:6], dev[6] if state else None, 64, True)
+    gg = torch.autograd.grad((y.float() * dy.float().cuda()).sum() + (h * dh.cuda()).sum(), dev)
+    check = check_f32 if dtype == torch.float32 else check_bf16
+    check("y", y, ey.detach())
+    check("h", h, eh.detach())
+    for n, a, e in zip(("x", "b", "c", "a", "g", "w", "h0"), gg, eg):
+        check("d" + n, a, e)
+
+
 def test_chunk_parallel_backward_takes_unaligned_gradients():
     """dy and the gradient buffers of the C ABI may start anywhere; aligned ones give the same bits."""
     import ctypes as C
