@@ -440,7 +440,9 @@ int m3_mixer_backward(m3_ctx *ctx, const m3_mixer_desc *desc, const m3_saved *sa
                       const void *dout, const m3_mixer_grads *grads, void *workspace);
 
 /* Bytes of device scratch a forward with this descriptor allocates (kept until
- * m3_saved_free when `saved` is requested). */
+ * m3_saved_free when `saved` is requested), plus, for_backward, its backward's: of the chunk-parallel or the generic
+ * family, whichever desc->path and the alignment of x, b and c select (absent pointers and y count as aligned);
+ * for shapes of the tensor-core family what the generic family would need. */
 size_t m3_scan_scratch_bytes(const m3_scan_desc *desc, int for_backward);
 
 #ifdef __cplusplus

@@ -469,15 +469,17 @@ size_t m3_scan_scratch_bytes(const m3_scan_desc* desc, int for_backward) {
   if (!desc) return 0;
   m3::Dims d;
   m3_scan_desc s = *desc;
-  // Only the extents matter here: stand in for pointers the caller may not have yet.
+  // Stand in for pointers the caller may not have yet; those it has decide the family by their alignment.
   alignas(16) static const float dummy = 0.0f;
-  s.x = s.b = s.c = s.dt = &dummy; s.a_log = &dummy;
-  if (s.discretization == M3_LEARNED_TRAPEZOID) s.lambda = &dummy;
-  if (s.dynamics == M3_ROTATIONAL) s.theta = &dummy;
+  auto want = [](const auto*& p) { if (!p) p = &dummy; };
+  want(s.x); want(s.b); want(s.c); want(s.dt); want(s.a_log);
+  if (s.discretization == M3_LEARNED_TRAPEZOID) want(s.lambda);
+  if (s.dynamics == M3_ROTATIONAL) want(s.theta);
   s.h0 = s.last_u0 = nullptr;
-  if (s.a_raw) s.a_raw = s.g_raw = s.w_raw = &dummy;
+  if (s.a_raw) { want(s.g_raw); want(s.w_raw); }
   if (make_dims(nullptr, s, &d) != M3_OK || d.T == 0) return 0;
-  if (m3::rows_supported(s, &dummy)) {
+  const bool tensor = m3::tc_supported(s) && !d.raw && s.path != M3_PATH_GENERIC;
+  if (!tensor && m3::rows_supported(s, &dummy)) {
     d = m3::rows_dims(d);
     return m3::rows_ws_layout(d, nullptr, nullptr) + (for_backward ? m3::rows_bwd_ws_layout(d, nullptr, nullptr, nullptr) : 0);
   }

@@ -70,6 +70,24 @@ def test_scratch_size_query_needs_no_gpu():
     assert 0 < fwd < both
 
 
+def test_scratch_size_follows_the_family():
+    """The size answered is that of the family the call will take: the path and the addresses count, where there are any."""
+    lib = _ffi.load()
+
+    def size(path=_ffi.PATH_AUTO, dtype=_ffi.F32, d_state=64, x=None, backward=0):
+        d = _ffi.ScanDesc(batch=1, seq=300, heads=2, head_dim=64, d_state=d_state, rank=1, chunk=64, dtype=dtype,
+                          discretization=2, path=path, x=x)
+        return lib.m3_scan_scratch_bytes(ctypes.byref(d), backward)
+    for backward in (0, 1):
+        generic = size(_ffi.PATH_GENERIC, backward=backward)
+        assert size(backward=backward) != generic                      # the chunk-parallel family
+        assert size(x=4096, backward=backward) == size(backward=backward)
+        assert size(x=4100, backward=backward) == generic              # off the 16 bytes that one needs
+        assert size(_ffi.PATH_GENERIC, x=4096, backward=backward) == generic
+        # shapes of the tensor-core family: as the generic one
+        assert size(dtype=_ffi.BF16, d_state=128, backward=backward) == size(_ffi.PATH_GENERIC, _ffi.BF16, 128, backward=backward)
+
+
 def test_rust_sys_source_covers_the_header():
     """include/m3scan-sys/src/lib.rs (uncompiled here: the image has no Rust toolchain) declares every function
     of the header and nothing else, and lists every structure's fields in the header's order."""
