@@ -229,7 +229,7 @@ int m3_step_forward(m3_ctx *ctx, const m3_step_desc *desc, const m3_step_out *ou
  * The first call on each device looks up the block's device address (with that
  * device current), and - CUDA loads a library's kernels and file-scope device arrays
  * when they are first touched - it is also the call during which the driver maps the
- * block and the kernels it launches: make one warm-up call per device and element type
+ * block and the kernels of its element type, whichever shapes they serve: make one warm-up call per device and element type
  * at start-up, before the arena is sized and before any stream capture; from the
  * second call on nothing is allocated by anyone.  All calls on a device share the
  * block and it keeps the previous call's contents (nothing in it needs to start at

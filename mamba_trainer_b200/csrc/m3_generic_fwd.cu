@@ -392,6 +392,12 @@ static cudaError_t forward_t(cudaStream_t st, const Dims& d, const m3_scan_desc&
   return cudaGetLastError();
 }
 
+template <class T>
+static cudaError_t load_t() {
+  return load_kernels(k_angle_sum<T>, k_angle_prefix, k_prep<T>, k_chunk_state, k_state_pass<T>, k_chunk_out<T>, k_last_u);
+}
+cudaError_t generic_load(int dtype) { return dtype == M3_BF16 ? load_t<__nv_bfloat16>() : load_t<float>(); }
+
 cudaError_t generic_forward(cudaStream_t st, const Dims& d, const m3_scan_desc& desc,
                             const m3_scan_out& out, const GenericWs& ws, uint64_t* launches) {
   if (desc.dtype == M3_BF16) return forward_t<__nv_bfloat16>(st, d, desc, out, ws, launches);

@@ -31,6 +31,14 @@ namespace m3 {
 inline cudaError_t scratch_alloc(m3_ctx* ctx, void** out, size_t bytes, cudaStream_t st) {
   return ctx->pool ? cudaMallocFromPoolAsync(out, bytes, ctx->pool, st) : cudaMallocAsync(out, bytes, st);
 }
+// Have the driver load kernels now instead of at their first launch.
+template <class... K>
+inline cudaError_t load_kernels(K... kernels) {
+  cudaFuncAttributes a;
+  cudaError_t e = cudaSuccess;
+  ((e = e == cudaSuccess ? cudaFuncGetAttributes(&a, kernels) : e), ...);
+  return e;
+}
 // Report (and clear) a wait that gave up in an earlier call; M3_OK if none did.
 int take_device_flag(m3_ctx* ctx, const char* when);
 }  // namespace m3
@@ -84,6 +92,7 @@ size_t generic_bwd_ws_layout(const Dims& d, GenericBwdWs* ws, char* base);
 
 cudaError_t generic_forward(cudaStream_t st, const Dims& d, const m3_scan_desc& desc,
                             const m3_scan_out& out, const GenericWs& ws, uint64_t* launches);
+cudaError_t generic_load(int dtype);   // load_kernels of every kernel a forward pass of the element type may launch
 cudaError_t generic_backward(cudaStream_t st, const Dims& d, const m3_scan_desc& desc,
                              const GenericWs& ws, const GenericBwdWs& bw,
                              const m3_scan_bwd_in& in, uint32_t mask,

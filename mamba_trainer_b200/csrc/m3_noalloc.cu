@@ -44,6 +44,20 @@ cudaError_t scratch_address(int device, char** out) {
   return cudaSuccess;
 }
 
+// Every kernel that a call with this element type may launch, loaded once per device (which must be current): which of
+// them a call takes depends on its shape, and a caller warms up with one shape only.
+cudaError_t load_kernels_once(int device, int dtype) {
+  static bool loaded[kMaxDevices][2] = {};
+  std::lock_guard<std::mutex> lock(g_mu);
+  bool& done = loaded[device][dtype == M3_BF16 ? 1 : 0];
+  if (done) return cudaSuccess;
+  cudaError_t e = m3::generic_load(dtype);
+  if (e == cudaSuccess) e = m3::rows_load(dtype);
+  if (e == cudaSuccess && dtype == M3_BF16) e = m3::tc_load();
+  done = e == cudaSuccess;
+  return e;
+}
+
 }  // namespace
 
 extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* out) {
@@ -56,6 +70,11 @@ extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, co
   if (!out->y) return m3::fail(ctx, M3_ERR_NULL, "y is required");
   if (ctx->device < 0 || ctx->device >= kMaxDevices)
     return m3::fail(ctx, M3_ERR_UNSUPPORTED, "device ordinal %d outside the table of %d", ctx->device, kMaxDevices);
+  {
+    cudaError_t e = cudaSetDevice(ctx->device);
+    if (e == cudaSuccess) e = load_kernels_once(ctx->device, desc->dtype);
+    if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "loading kernels");
+  }
   // Shapes the tensor-core family serves need no scratch at all when nothing is kept for a backward
   // pass - or, for few long stripes, states at segment boundaries, which go to the block while they fit.
   if (m3::tc_supported(*desc) && !d.raw && desc->path != M3_PATH_GENERIC) {

@@ -487,6 +487,7 @@ Dims rows_dims(Dims d);
 size_t rows_ws_layout(const Dims& d, rows::RowsWs* ws, char* base);
 cudaError_t rows_forward(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const m3_scan_out& out,
                          const rows::RowsWs& ws, uint64_t* launches);
+cudaError_t rows_load(int dtype);   // load_kernels of every kernel a forward pass of the element type may launch
 // The last pass over tokens for the tensor-core family's side-by-side segments (bf16, d_state 128, rotational): d.L steps
 // per tile, `per_seg` tiles per segment.
 cudaError_t rows_final(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const float* dphi, const float* dpsum, int per_seg,

@@ -227,6 +227,19 @@ cudaError_t forward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, co
   return cudaGetLastError();
 }
 
+template <class T, int N, int R>
+cudaError_t load_t() {
+  return load_kernels(k_rows_state<T, N, R, true, false>, k_rows_state<T, N, R, false, false>, k_rows_pass<T, N, true>,
+                      k_rows_pass<T, N, false>, k_rows_out<T, N, R, true>, k_rows_out<T, N, R, false>);
+}
+template <class T>
+cudaError_t load_all() {
+  cudaError_t e = cudaSuccess;
+  for (cudaError_t (*f)() : {load_t<T, 64, 1>, load_t<T, 64, 2>, load_t<T, 64, 4>, load_t<T, 128, 1>, load_t<T, 128, 2>, load_t<T, 128, 4>})
+    if (e == cudaSuccess) e = f();
+  return e;
+}
+
 template <class T, int N, int R, bool ROT>
 cudaError_t dh_local_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const void* dy, const RowsWs& ws, float* dhs) {
   cudaError_t e = smem_limit(k_rows_state<T, N, R, ROT, true>, sizeof(StateSmem<N, R>));
@@ -282,6 +295,8 @@ size_t rows_ws_layout(const Dims& d, rows::RowsWs* ws, char* base) {
   if (ws) *ws = t;
   return off;
 }
+
+cudaError_t rows_load(int dtype) { return dtype == M3_BF16 ? rows::load_all<__nv_bfloat16>() : rows::load_all<float>(); }
 
 cudaError_t rows_forward(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const m3_scan_out& out,
                          const rows::RowsWs& ws, uint64_t* launches) {

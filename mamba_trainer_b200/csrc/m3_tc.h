@@ -84,6 +84,10 @@ cudaError_t tc_ahead(cudaStream_t st, const Dims& d, const m3_scan_desc& in, con
                      const float* ckpt_angle, const TcAhead& a);
 
 cudaError_t tc_forward(cudaStream_t st, const TcFwdParams& p, bool rotational);
+// load_kernels of every kernel that a forward pass may launch.
+cudaError_t tc_load();
+cudaError_t tc_direct_load();
+cudaError_t tc_ahead_load();
 // The direct form (rank 1, real dynamics, use_tma): m3_tc_fwd_direct.cu.
 cudaError_t tc_forward_direct(cudaStream_t st, const TcFwdParams& p);
 

@@ -422,6 +422,17 @@ cudaError_t ahead_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, cons
 
 }  // namespace
 
+template <int R>
+static cudaError_t load_r() {
+  return load_kernels(k_group_state<R, true, false>, k_group_state<R, false, false>);
+}
+cudaError_t tc_ahead_load() {
+  cudaError_t e = load_kernels(k_group_pass<true, false>, k_group_pass<false, false>);
+  for (cudaError_t (*f)() : {load_r<1>, load_r<2>, load_r<4>})
+    if (e == cudaSuccess) e = f();
+  return e;
+}
+
 // Whether to cut `BH` stripes of `tiles` tiles into segments that run side by side, and into how many.  Microseconds,
 // measured on a B200: a tile takes about 5.5 forward and 15 backward inside a stripe (5.2 and 11 in the direct form, which
 // whole stripes may have), an item costs about one more to start and finish; working out what a tile adds to the state

@@ -18,6 +18,7 @@
 // Warp roles, barriers and the distribution of stripes (or time segments of stripes) over CTAs:
 // m3_tc_roles.cuh.  Rank 1 with real dynamics has a second form (m3_tc_fwd_direct.cu) whose rows need no
 // conversion and land in operand layout by bulk TENSOR copies.
+#include "m3_internal.h"
 #include "m3_tc.h"
 #include "m3_tc_roles.cuh"
 
@@ -516,6 +517,18 @@ void tc_segment_plan(int BH, int tiles, bool allow_split, int* nseg, int* tps, i
   *grid = n == 1 ? BH : (int)(items < sms ? items : sms);
   if (scratch_bytes)
     *scratch_bytes = n > 1 ? (size_t)BH * n * ((size_t)kP * kN * 4 + kNH * 4 + 4) : 0;
+}
+
+template <int R>
+static cudaError_t load_r() {
+  return load_kernels(tc_fwd_kernel<R, true, 0>, tc_fwd_kernel<R, false, 0>, tc_fwd_kernel<R, true, 1>, tc_fwd_kernel<R, false, 1>,
+                      tc_fwd_kernel<R, true, 2>, tc_fwd_kernel<R, false, 2>);
+}
+cudaError_t tc_load() {
+  cudaError_t e = tc_direct_load();
+  for (cudaError_t (*f)() : {load_r<1>, load_r<2>, load_r<4>, tc_ahead_load})
+    if (e == cudaSuccess) e = f();
+  return e;
 }
 
 cudaError_t tc_forward(cudaStream_t st, const TcFwdParams& p, bool rot) {

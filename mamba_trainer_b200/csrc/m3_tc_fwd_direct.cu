@@ -9,6 +9,7 @@
 // tensors; everything else takes the role-split kernel of m3_tc_fwd.cu.  The arithmetic per tile is
 // the same (scan.rs:192-268): Yoff = C H, G = C B^T, M = G o band, Y += M x, H^T += B^T (sigma_w x).
 // 256 threads: warps 1-7 compute the next tile's scalars while thread 0 issues the products.
+#include "m3_internal.h"
 #include "m3_tc.h"
 #include "m3_tc_stage.cuh"
 
@@ -380,6 +381,8 @@ bool tc_make_row_map(CUtensorMap* map, const void* base, int B, int T, int H, in
                 CU_TENSOR_MAP_L2_PROMOTION_NONE,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+cudaError_t tc_direct_load() { return load_kernels(tc_fwd_direct_kernel); }
 
 cudaError_t tc_forward_direct(cudaStream_t st, const TcFwdParams& p) {
   auto kern = tc_fwd_direct_kernel;

@@ -117,3 +117,40 @@ def test_noalloc_refuses_what_does_not_fit():
         assert b"scratch" in lib.m3_last_error(ctx)
     finally:
         lib.m3_ctx_destroy(ctx)
+
+
+def test_one_warm_up_call_loads_every_kernel():
+    """In a process of its own: after one call per element type, calls of shapes that take other kernels (another rank,
+    d_state, dynamics, few long stripes) leave the device's free memory as it is."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    code = """
+import ctypes as C, torch
+from mamba_trainer_b200 import _ffi, synthetic
+from mamba_trainer_b200.ssm import Discretization
+from tests.test_zz_no_alloc import _desc, _outputs
+lib, ctx = _ffi.load(), C.c_void_p()
+assert lib.m3_ctx_create(0, C.byref(ctx)) == _ffi.OK
+def make(dtype, heads, seq, n, rank, rot, p=64):
+    w = synthetic.Workload('w', 1, seq, heads, p, n, 64, rank, dtype, Discretization.LearnedTrapezoid, rot, 'scaled')
+    t = {k: (v.cuda() if v is not None else None) for k, v in synthetic.make_inputs(w, seed=1).items()}
+    d = _desc(t, w)
+    d.path = _ffi.PATH_AUTO
+    return t, d, _outputs(t, w)
+warm = [make(torch.float32, 2, 100, 64, 1, True), make(torch.bfloat16, 2, 100, 128, 1, True)]
+other = [make(torch.float32, 2, 70, 128, 2, False), make(torch.float32, 2, 50, 40, 1, True, 24), make(torch.float32, 1, 90, 64, 4, True),
+         make(torch.bfloat16, 2, 256, 128, 1, False), make(torch.bfloat16, 2, 900, 128, 2, True), make(torch.bfloat16, 2, 90, 64, 2, True),
+         make(torch.bfloat16, 150, 64, 128, 4, False), make(torch.bfloat16, 2, 1000, 128, 4, False)]
+def run(c):
+    assert lib.m3_scan_forward_noalloc(ctx, C.byref(c[1]), C.byref(c[2][1])) == _ffi.OK, lib.m3_last_error(ctx)
+    assert lib.m3_sync(ctx) == _ffi.OK
+for c in warm: run(c)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+for c in other: run(c)
+assert torch.cuda.mem_get_info()[0] == free, (free, torch.cuda.mem_get_info()[0])
+"""
+    root = Path(__file__).resolve().parent.parent
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
