@@ -233,8 +233,10 @@ int m3_step_forward(m3_ctx *ctx, const m3_step_desc *desc, const m3_step_out *ou
  * at start-up, before the arena is sized and before any stream capture; from the
  * second call on nothing is allocated by anyone.  All calls on a device share the
  * block and it keeps the previous call's contents (nothing in it needs to start at
- * zero): two calls whose kernels overlap on the GPU race - keep them on one stream or
- * order them yourself. */
+ * zero): calls of different streams wait on the device for one another.  Calls enqueued
+ * into a stream capture are not ordered so; there the tensor-core family runs without
+ * the block (whole stripes: another rounding), and graphs of the other families' calls
+ * must not run beside other calls. */
 #define M3_NOALLOC_SCRATCH_BYTES (16u << 20)
 int m3_scan_forward_noalloc(m3_ctx *ctx, const m3_scan_desc *desc, const m3_scan_out *out);
 

@@ -10,7 +10,8 @@
 // device memory that is part of the library image instead.
 //
 // The price: every GPU that loads the library holds M3_NOALLOC_SCRATCH_BYTES until the
-// process exits, requests needing more are refused, and all calls share the block.
+// process exits, requests needing more are refused, and all calls share the block: those of
+// different streams are put one behind the other.
 #include <mutex>
 
 #include "m3_internal.h"
@@ -58,30 +59,48 @@ cudaError_t load_kernels_once(int device, int dtype) {
   return e;
 }
 
-}  // namespace
-
-extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* out) {
-  if (!ctx) return M3_ERR_NULL;
-  if (!desc || !out) return m3::fail(ctx, M3_ERR_NULL, "descriptor and outputs are required");
-  m3::Dims d;
-  int rc = m3::make_dims(ctx, *desc, &d);
-  if (rc != M3_OK) return rc;
-  if (d.T == 0) return m3_scan_forward(ctx, desc, out, nullptr);  // that branch only copies the state
-  if (!out->y) return m3::fail(ctx, M3_ERR_NULL, "y is required");
-  if (ctx->device < 0 || ctx->device >= kMaxDevices)
-    return m3::fail(ctx, M3_ERR_UNSUPPORTED, "device ordinal %d outside the table of %d", ctx->device, kMaxDevices);
-  {
-    cudaError_t e = cudaSetDevice(ctx->device);
-    if (e == cudaSuccess) e = load_kernels_once(ctx->device, desc->dtype);
-    if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "loading kernels");
+// Calls that use the block wait on the device for the one before them: a tensor-core call of one stream must not
+// write what a call of another is reading.  Held from before the first launch until the event behind the last one is
+// recorded, so that calls of several threads enter one at a time.
+struct BlockOrder {
+  std::mutex mu;
+  cudaEvent_t behind[kMaxDevices] = {};   // the last call's end
+};
+BlockOrder& block_order() {
+  static BlockOrder* o = new BlockOrder;   // (never destroyed: a stream may outlive the statics)
+  return *o;
+}
+class BlockUse {
+ public:
+  explicit BlockUse(m3_ctx* ctx) : ctx_(ctx), lock_(block_order().mu) {
+    cudaEvent_t& ev = block_order().behind[ctx->device];
+    if (ev) status = cudaStreamWaitEvent(ctx->stream, ev, 0);
+    else status = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   }
+  ~BlockUse() {
+    if (status == cudaSuccess) cudaEventRecord(block_order().behind[ctx_->device], ctx_->stream);
+  }
+  cudaError_t status;
+
+ private:
+  m3_ctx* ctx_;
+  std::lock_guard<std::mutex> lock_;
+};
+
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
+// One call, with the block's address in `base`; NULL: the block may not be used.
+int forward_on(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* out, m3::Dims d, char* base) {
   // Shapes the tensor-core family serves need no scratch at all when nothing is kept for a backward
   // pass - or, for few long stripes, states at segment boundaries, which go to the block while they fit.
   if (m3::tc_supported(*desc) && !d.raw && desc->path != M3_PATH_GENERIC) {
-    cudaError_t e = cudaSetDevice(ctx->device);
-    if (e == cudaSuccess) e = scratch_address(ctx->device, &ctx->fixed_scratch);
-    if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "cudaGetSymbolAddress");
-    ctx->fixed_bytes = M3_NOALLOC_SCRATCH_BYTES;
+    ctx->fixed_scratch = base;
+    ctx->fixed_bytes = base ? M3_NOALLOC_SCRATCH_BYTES : 0;
     ctx->no_scratch = true;
     const int rc = m3_scan_forward(ctx, desc, out, nullptr);
     ctx->no_scratch = false;
@@ -94,14 +113,10 @@ extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, co
     return m3::fail(ctx, M3_ERR_UNSUPPORTED,
                     "this scan needs %zu bytes of scratch; the built-in block holds %zu - use m3_scan_forward",
                     need, (size_t)M3_NOALLOC_SCRATCH_BYTES);
-  cudaError_t e = cudaSetDevice(ctx->device);
-  if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "cudaSetDevice");
-  char* base = nullptr;
-  e = scratch_address(ctx->device, &base);
-  if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "cudaGetSymbolAddress");
   // Every scratch region is written in full before it is read (padded rows are stored
   // as zeros, every chunk-state slot is produced by the chunk kernels), so nothing left
   // behind by the previous call needs clearing.
+  cudaError_t e;
   if (rows) {
     m3::rows::RowsWs ws;
     m3::rows_ws_layout(d, &ws, base);
@@ -113,4 +128,34 @@ extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, co
   }
   if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "forward on built-in scratch");
   return M3_OK;
+}
+
+}  // namespace
+
+extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* out) {
+  if (!ctx) return M3_ERR_NULL;
+  if (!desc || !out) return m3::fail(ctx, M3_ERR_NULL, "descriptor and outputs are required");
+  m3::Dims d;
+  int rc = m3::make_dims(ctx, *desc, &d);
+  if (rc != M3_OK) return rc;
+  if (d.T == 0) return m3_scan_forward(ctx, desc, out, nullptr);  // that branch only copies the state
+  if (!out->y) return m3::fail(ctx, M3_ERR_NULL, "y is required");
+  if (ctx->device < 0 || ctx->device >= kMaxDevices)
+    return m3::fail(ctx, M3_ERR_UNSUPPORTED, "device ordinal %d outside the table of %d", ctx->device, kMaxDevices);
+  cudaError_t e = cudaSetDevice(ctx->device);
+  if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "cudaSetDevice");
+  char* base = nullptr;
+  e = scratch_address(ctx->device, &base);
+  if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "cudaGetSymbolAddress");
+  e = load_kernels_once(ctx->device, desc->dtype);
+  if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "loading kernels");
+  if (capturing(ctx->stream)) {
+    // A graph's launches cannot be put behind other streams' here.  The tensor-core family runs whole stripes then, which
+    // need no scratch; the other families' calls have always shared the block.
+    const bool tensor = m3::tc_supported(*desc) && !d.raw && desc->path != M3_PATH_GENERIC;
+    return forward_on(ctx, desc, out, d, tensor ? nullptr : base);
+  }
+  const BlockUse use(ctx);
+  if (use.status != cudaSuccess) return m3::cuda_fail(ctx, use.status, "order of the calls on the built-in scratch");
+  return forward_on(ctx, desc, out, d, base);
 }

@@ -119,6 +119,57 @@ def test_noalloc_refuses_what_does_not_fit():
         lib.m3_ctx_destroy(ctx)
 
 
+def test_noalloc_calls_of_two_streams_keep_off_each_other():
+    """Few long stripes of the tensor-core family put segment states into the shared block: calls of two streams are put one
+    behind the other, and give what each gives alone; a call that is captured into a graph, whose launches cannot be, runs
+    whole stripes as one launch without the block."""
+    from tests._util import norm_rel
+    lib = _ffi.load()
+    ctxs = [C.c_void_p(), C.c_void_p()]
+    for c in ctxs:
+        assert lib.m3_ctx_create(0, C.byref(c)) == _ffi.OK
+    try:
+        w = synthetic.WORKLOADS[3].scaled(batch=1, heads=2, seq=1500)
+        ts = [{k: (v.cuda() if v is not None else None) for k, v in synthetic.make_inputs(w, seed=s).items()} for s in (5, 6)]
+        descs = [_desc(t, w) for t in ts]
+        for d in descs:
+            d.path = _ffi.PATH_AUTO
+
+        def call(i):
+            got, out = _outputs(ts[i], w)
+            torch.cuda.synchronize()
+            return got, lambda: lib.m3_scan_forward_noalloc(ctxs[i], C.byref(descs[i]), C.byref(out)), out
+        alone = []
+        for i in (0, 1):
+            got, run, _keep = call(i)
+            before = lib.m3_launch_count(ctxs[i])
+            assert run() == _ffi.OK, lib.m3_last_error(ctxs[i]).decode()
+            assert lib.m3_sync(ctxs[i]) == _ffi.OK
+            assert lib.m3_launch_count(ctxs[i]) - before > 1      # cut into segments
+            alone.append(got)
+        calls = [(i, call(i)) for _ in range(8) for i in (0, 1)]
+        for i, (_, run, _keep) in calls:
+            assert run() == _ffi.OK, lib.m3_last_error(ctxs[i]).decode()
+        for c in ctxs:
+            assert lib.m3_sync(c) == _ffi.OK
+        for i, (got, _, _keep) in calls:
+            for a, e in zip(got[:3], alone[i][:3]):
+                assert torch.equal(a, e)
+        got, run, _keep = call(0)
+        graph, side, before = torch.cuda.CUDAGraph(), torch.cuda.Stream(), lib.m3_launch_count(ctxs[0])
+        assert lib.m3_ctx_set_stream(ctxs[0], side.cuda_stream) == _ffi.OK
+        with torch.cuda.graph(graph, stream=side):
+            assert run() == _ffi.OK, lib.m3_last_error(ctxs[0]).decode()
+        assert lib.m3_launch_count(ctxs[0]) - before == 1
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, e in zip(got[:3], alone[0][:3]):   # bf16 operands either way
+            assert norm_rel(a.float(), e.float()) <= 2e-2
+    finally:
+        for c in ctxs:
+            lib.m3_ctx_destroy(c)
+
+
 def test_one_warm_up_call_loads_every_kernel():
     """In a process of its own: after one call per element type, calls of shapes that take other kernels (another rank,
     d_state, dynamics, few long stripes) leave the device's free memory as it is."""
