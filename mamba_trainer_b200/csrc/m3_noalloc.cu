@@ -94,11 +94,17 @@ bool capturing(cudaStream_t st) {
   return true;
 }
 
+// Whether m3_scan_forward will run the tensor-core family (or, asked for it by name, refuse): with a y that is not 16-byte
+// aligned it would take another family, and that one's scratch from the pool.
+bool tensor_core(const m3_scan_desc& s, const m3_scan_out& out, const m3::Dims& d) {
+  return m3::tc_supported(s) && !d.raw && s.path != M3_PATH_GENERIC && (s.path == M3_PATH_TENSOR || m3::tc_aligned(out.y));
+}
+
 // One call, with the block's address in `base`; NULL: the block may not be used.
 int forward_on(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* out, m3::Dims d, char* base) {
   // Shapes the tensor-core family serves need no scratch at all when nothing is kept for a backward
   // pass - or, for few long stripes, states at segment boundaries, which go to the block while they fit.
-  if (m3::tc_supported(*desc) && !d.raw && desc->path != M3_PATH_GENERIC) {
+  if (tensor_core(*desc, *out, d)) {
     ctx->fixed_scratch = base;
     ctx->fixed_bytes = base ? M3_NOALLOC_SCRATCH_BYTES : 0;
     ctx->no_scratch = true;
@@ -152,8 +158,7 @@ extern "C" int m3_scan_forward_noalloc(m3_ctx* ctx, const m3_scan_desc* desc, co
   if (capturing(ctx->stream)) {
     // A graph's launches cannot be put behind other streams' here.  The tensor-core family runs whole stripes then, which
     // need no scratch; the other families' calls have always shared the block.
-    const bool tensor = m3::tc_supported(*desc) && !d.raw && desc->path != M3_PATH_GENERIC;
-    return forward_on(ctx, desc, out, d, tensor ? nullptr : base);
+    return forward_on(ctx, desc, out, d, tensor_core(*desc, *out, d) ? nullptr : base);
   }
   const BlockUse use(ctx);
   if (use.status != cudaSuccess) return m3::cuda_fail(ctx, use.status, "order of the calls on the built-in scratch");

@@ -170,6 +170,34 @@ def test_noalloc_calls_of_two_streams_keep_off_each_other():
             lib.m3_ctx_destroy(c)
 
 
+def test_noalloc_with_a_misaligned_y_allocates_nothing():
+    """A y that the tensor-core family cannot write goes to a family that needs scratch: the block, not the pool."""
+    from tests._util import norm_rel
+    lib = _ffi.load()
+    ctx = C.c_void_p()
+    assert lib.m3_ctx_create(0, C.byref(ctx)) == _ffi.OK
+    try:
+        w = synthetic.WORKLOADS[3].scaled(batch=1, heads=2, seq=300)
+        t = {k: (v.cuda() if v is not None else None) for k, v in synthetic.make_inputs(w, seed=7).items()}
+        desc = _desc(t, w)
+        desc.path = _ffi.PATH_AUTO
+        (y, *_rest), out = _outputs(t, w)
+        off = torch.zeros(y.numel() + 8, device="cuda", dtype=y.dtype)[4:4 + y.numel()]   # 8 bytes
+        out2 = _ffi.ScanOut(y=C.c_void_p(off.data_ptr()), h=out.h, last_u=out.last_u, angle=out.angle)
+        assert lib.m3_scan_forward_noalloc(ctx, C.byref(desc), C.byref(out)) == _ffi.OK   # warm-up
+        assert lib.m3_sync(ctx) == _ffi.OK
+        torch.cuda.synchronize()
+        before = _free_bytes()
+        assert lib.m3_scan_forward_noalloc(ctx, C.byref(desc), C.byref(out2)) == _ffi.OK, lib.m3_last_error(ctx).decode()
+        assert lib.m3_sync(ctx) == _ffi.OK
+        assert _free_bytes() == before
+        assert norm_rel(off.view(y.shape).float(), y.float()) <= 2e-2   # bf16 operands on one side
+        desc.path = _ffi.PATH_TENSOR
+        assert lib.m3_scan_forward_noalloc(ctx, C.byref(desc), C.byref(out2)) == _ffi.ERR_UNSUPPORTED
+    finally:
+        lib.m3_ctx_destroy(ctx)
+
+
 def test_one_warm_up_call_loads_every_kernel():
     """In a process of its own: after one call per element type, calls of shapes that take other kernels (another rank,
     d_state, dynamics, few long stripes) leave the device's free memory as it is."""
