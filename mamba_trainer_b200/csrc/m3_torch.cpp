@@ -210,7 +210,7 @@ std::vector<OptTensor> scan(uintptr_t handle, const Tensor& x0, const Tensor& b0
 }
 
 // ---- the mixer ----------------------------------------------------------------------------------------------------
-constexpr int kMixerParams = 9;   // in the order of m3_mixer_desc
+constexpr int kMixerParams = 9, kNormWeight = 7, kPostWeight = 8;   // in the order of m3_mixer_desc
 struct Spec {   // the integers of m3_mixer_desc between its extents and its pointers
   int heads, head_dim, d_state, rank, groups, chunk, disc, rotational, has_norm, post_norm, path, reverse_heads;
 };
@@ -264,8 +264,10 @@ struct MixerNode : public torch::autograd::Node {
     m3_mixer_desc d = desc;
     mixer_inputs(d, t[0], t + 1);
     const Tensor dout = up[0].contiguous();
+    // (a gain whose norm was switched off is read by nothing: no gradient)
     for (int i = 0; i <= kMixerParams; ++i)
-      if (in[i].present) g[i] = at::empty_like(t[i], at::MemoryFormat::Contiguous);
+      if (in[i].present && (i != 1 + kNormWeight || d.has_norm) && (i != 1 + kPostWeight || d.post_norm))
+        g[i] = at::empty_like(t[i], at::MemoryFormat::Contiguous);
     const m3_mixer_grads out{mut(g[0]), fmut(g[1]), fmut(g[2]), fmut(g[3]), fmut(g[4]), fmut(g[5]),
                              fmut(g[6]), fmut(g[7]), fmut(g[8]), fmut(g[9])};
     const Tensor work = at::empty({(int64_t)m3_mixer_backward_bytes(&d)}, act.options());

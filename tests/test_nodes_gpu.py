@@ -112,3 +112,21 @@ def test_moved_inputs_are_checked():
     assert run(make(off=1)) == _ffi.ERR_UNSUPPORTED
     assert run(make(lambda_=None)) == _ffi.ERR_NULL
     ctx.check(ctx.lib.m3_saved_free(ctx.handle, saved))
+
+
+@pytest.mark.parametrize("head_dim,d_state", [(64, 64), (24, 40)])
+def test_switched_off_norms_have_no_gradient(head_dim, d_state):
+    """A norm that is switched off on a built module leaves its gain out of the graph: no gradient (not memory that nothing
+    wrote), and the other gradients are those of a module built without it."""
+    kw = dict(chunk=16, device="cuda")
+    shape = MixerShape(2, head_dim, d_state, 1)
+    torch.manual_seed(0)
+    off, without = MixerCore(shape, post_gate_norm=True, **kw), MixerCore(shape, bc_norm=False, **kw)
+    without.load_state_dict({k: v for k, v in off.state_dict().items() if k not in ("norm_w", "post_norm_w")})
+    off.use_norm = off.post_gate_norm = False
+    proj = torch.randn(2, 50, shape.in_proj_width, device="cuda")
+    for core in (off, without):
+        core(proj).square().sum().backward()
+    assert off.norm_w.grad is None and off.post_norm_w.grad is None
+    for n, q in without.named_parameters():
+        assert torch.equal(q.grad, getattr(off, n).grad), n
