@@ -113,10 +113,6 @@ class MixerCore(torch.nn.Module):
         # RmsNormConfig::new(d_inner) (mamba3.rs:245-247): a gain of ones over the scan's flattened output
         self.post_gate_norm = post_gate_norm
         self.post_norm_w = par(torch.ones(shape.d_inner)) if post_gate_norm else None
-        for name in _PARAMS:   # absent parameters are named all the same
-            if name not in self._parameters:
-                delattr(self, name)
-                self.register_parameter(name, None)
 
     def empty_cache(self, batch: int, device, dtype=torch.float32) -> MixerCache:
         s = self.shape
@@ -126,7 +122,8 @@ class MixerCore(torch.nn.Module):
     def _spec(self, path: int = _ffi.PATH_AUTO):
         """The parameters in _PARAMS' order, the integers of m3_mixer_desc, eps and d_inner: what the native node takes."""
         s, p = self.shape, self._parameters
-        return ([p[n] for n in _PARAMS],
+        # (what is no parameter of the module: absent, or parametrised, pruned, assigned, a view of a flattened one)
+        return ([getattr(self, n) if (v := p.get(n)) is None else v for n in _PARAMS],
                 (s.heads, s.head_dim, s.d_state, s.rank, s.n_groups, self.chunk, self.disc, s.rotational, self.use_norm,
                  self.post_gate_norm, path, s.heads // 2 if self.bidirectional else 0), self.eps, s.d_inner)
 
@@ -146,7 +143,8 @@ class MixerCore(torch.nn.Module):
         if cache is None:
             cache = self.empty_cache(B, proj.device, proj.dtype)
         st = cache.ssm
-        K = self._parameters["conv_w"].shape[0]
+        spec = self._spec()
+        K = spec[0][0].shape[0]
         if cache.conv.shape != (B, K - 1, s.conv_channels):
             raise ShapeError(f"the cache's convolution history has shape {tuple(cache.conv.shape)}, expected "
                              f"{(B, K - 1, s.conv_channels)}")
@@ -154,7 +152,7 @@ class MixerCore(torch.nn.Module):
                 s.rotational and st.angle is not None and st.angle.shape != (B, H, N // 2)):
             raise ShapeError(f"the cache's state does not match batch {B}, heads {H}, head_dim {P}, d_state {N}")
         out, conv, h, last_u, angle = _ffi.extension().window(
-            Context.of(proj.device).handle.value, proj, *self._spec(), cache.conv, st.h, st.last_u, st.angle)
+            Context.of(proj.device).handle.value, proj, *spec, cache.conv, st.h, st.last_u, st.angle)
         return out, MixerCache(conv, SsmState(h, last_u, angle))
 
     def forward(self, proj: torch.Tensor, path: int = _ffi.PATH_AUTO) -> torch.Tensor:

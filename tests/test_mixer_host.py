@@ -54,3 +54,30 @@ def test_conv_validates_before_touching_the_device():
         causal_conv1d(torch.zeros(1, 5, 6), w, history=torch.zeros(1, 2, 6))
     conv = CausalConv1d(6, 4)
     assert conv.empty_history(3).shape == (3, 3, 6) and conv.weight.shape == (4, 6)
+
+
+def test_mixer_core_takes_parameters_that_are_none_of_its_own():
+    """A parametrised or pruned weight, a plain tensor in the place of an absent parameter and functional_call's stand-ins
+    reach the native call as the module's attributes have them."""
+    import torch.nn.utils.parametrize as parametrize
+    import torch.nn.utils.prune as prune
+    names = ("conv_w", "conv_b", "dt_bias", "a_log", "d_skip", "b_bias", "c_bias", "norm_w", "post_norm_w")
+
+    class Twice(torch.nn.Module):
+        def forward(self, v):
+            return 2 * v
+    core = MixerCore(MixerShape(heads=2, head_dim=4, d_state=8), d_skip=False)
+    assert set(core.state_dict()) == set(names) - {"d_skip", "post_norm_w"}
+    before = core.conv_w.detach().clone()
+    parametrize.register_parametrization(core, "conv_w", Twice())
+    prune.random_unstructured(core, "b_bias", 0.5)
+    core.d_skip = torch.ones(2)
+    got = dict(zip(names, core._spec()[0]))
+    assert torch.equal(got["conv_w"], 2 * before) and got["conv_w"].requires_grad
+    assert got["b_bias"] is core.b_bias and got["d_skip"] is core.d_skip and got["post_norm_w"] is None
+    assert got["a_log"] is core.a_log
+    stand_in = torch.zeros(2)
+    seen = []
+    core.forward = lambda: seen.append(core._spec()[0][3])
+    torch.func.functional_call(core, {"a_log": stand_in}, ())
+    assert seen[0] is stand_in
