@@ -709,7 +709,7 @@ int m3_saved_free(m3_ctx* ctx, m3_saved* saved) {
   // Freed in the order of the stream the forward (and, by the tape's order, the backward) ran on: the
   // context may have been rebound to another stream since, and the pool must not hand this block
   // to a later allocation while kernels of the old stream still read it.
-  cudaError_t e = saved->ws_base ? cudaFreeAsync(saved->ws_base, saved->stream ? saved->stream : ctx->stream) : cudaSuccess;
+  cudaError_t e = saved->ws_base ? cudaFreeAsync(saved->ws_base, saved->stream) : cudaSuccess;   // (0 is a stream too)
   delete saved;
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaFreeAsync");
   return M3_OK;

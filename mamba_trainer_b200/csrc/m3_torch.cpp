@@ -12,6 +12,8 @@
 
 #include <map>
 #include <mutex>
+#include <optional>
+#include <string>
 
 #include "../../include/m3scan.h"
 
@@ -24,19 +26,36 @@ using OptTensor = c10::optional<Tensor>;
 PyObject* g_from_status = nullptr;   // error.from_status
 
 // A context is shared by the threads of a process (autograd runs backward passes on a thread of its own): binding the
-// stream and the calls that use it go together under its lock.
-std::mutex& lock_of(m3_ctx* ctx) {
+// stream, the calls that use it and the reading of their message go together under its lock.  Python code that calls the
+// library takes the same lock (ssm/scan.py) and needs the interpreter's to go on, so nobody waits here holding that; a
+// thread may take it again (a finaliser that runs in between).
+std::recursive_mutex& lock_of(m3_ctx* ctx) {
   static auto* mu = new std::mutex;   // never destroyed: nodes may outlive the statics of a process on its way out
-  static auto* locks = new std::map<m3_ctx*, std::mutex>;
+  static auto* locks = new std::map<m3_ctx*, std::recursive_mutex>;
   std::lock_guard<std::mutex> g(*mu);
   return (*locks)[ctx];
 }
+struct Status {
+  int rc = M3_OK;
+  std::string message;
+};
+// One call of the library on the current stream of `t`'s device.
+template <class F>
+Status locked(m3_ctx* ctx, const Tensor& t, F call) {
+  std::optional<py::gil_scoped_release> nogil;
+  if (PyGILState_Check()) nogil.emplace();
+  std::lock_guard<std::recursive_mutex> lock(lock_of(ctx));
+  m3_ctx_set_stream(ctx, c10::cuda::getCurrentCUDAStream(t.device().index()).stream());
+  Status s;
+  s.rc = call();
+  if (s.rc != M3_OK) s.message = m3_last_error(ctx);
+  return s;
+}
 
 // The library's error as the package's exception class; rethrown across the autograd engine's threads as it is.
-[[noreturn]] void raise_status(m3_ctx* ctx, int rc) {
-  const std::string msg = m3_last_error(ctx);
+[[noreturn]] void raise_status(const Status& s) {
   py::gil_scoped_acquire gil;
-  PyObject* exc = PyObject_CallFunction(g_from_status, "is", rc, msg.c_str());
+  PyObject* exc = PyObject_CallFunction(g_from_status, "is", s.rc, s.message.c_str());
   if (exc) {
     PyErr_SetObject(reinterpret_cast<PyObject*>(Py_TYPE(exc)), exc);
     Py_DECREF(exc);
@@ -44,10 +63,6 @@ std::mutex& lock_of(m3_ctx* ctx) {
   python_error e;
   e.persist();
   throw e;
-}
-
-void bind(m3_ctx* ctx, const Tensor& t) {
-  m3_ctx_set_stream(ctx, c10::cuda::getCurrentCUDAStream(t.device().index()).stream());
 }
 
 const void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
@@ -113,8 +128,7 @@ struct ScanNode : public torch::autograd::Node {
   ~ScanNode() override { free_handle(); }
   void free_handle() {
     if (!handle) return;
-    std::lock_guard<std::mutex> lock(lock_of(ctx));
-    m3_saved_free(ctx, handle);
+    m3_saved_free(ctx, handle);   // (on the stream that the handle remembers: no lock)
     handle = nullptr;
   }
   void release_variables() override {
@@ -143,13 +157,8 @@ struct ScanNode : public torch::autograd::Node {
     out.dx = mut(g[0]); out.db = mut(g[1]); out.dc = mut(g[2]); out.ddt = mut(g[3]); out.da_log = fmut(g[4]);
     out.dlambda = mut(g[5]); out.dtheta = mut(g[6]); out.dd_skip = fmut(g[7]);
     out.dh0 = fmut(g[8]); out.dlast_u0 = fmut(g[9]); out.dangle0 = fmut(g[10]);
-    int rc;
-    {
-      std::lock_guard<std::mutex> lock(lock_of(ctx));
-      bind(ctx, t[0]);
-      rc = m3_scan_backward_moved(ctx, handle, &d, &bin, mask, &out);
-    }
-    if (rc != M3_OK) raise_status(ctx, rc);
+    const Status s = locked(ctx, t[0], [&] { return m3_scan_backward_moved(ctx, handle, &d, &bin, mask, &out); });
+    if (s.rc != M3_OK) raise_status(s);
     return variable_list(g, g + kScanInputs);
   }
 };
@@ -183,14 +192,8 @@ std::vector<OptTensor> scan(uintptr_t handle, const Tensor& x0, const Tensor& b0
     for (const Tensor& v : t) track = track || (v.defined() && v.requires_grad());
   const m3_scan_out out{mut(y), fmut(h), fmut(lu), fmut(ang)};
   m3_saved* saved = nullptr;
-  int rc;
-  {
-    py::gil_scoped_release nogil;
-    std::lock_guard<std::mutex> lock(lock_of(ctx));
-    bind(ctx, x);
-    rc = m3_scan_forward(ctx, &d, &out, track ? &saved : nullptr);
-  }
-  if (rc != M3_OK) raise_status(ctx, rc);
+  const Status s = locked(ctx, x, [&] { return m3_scan_forward(ctx, &d, &out, track ? &saved : nullptr); });
+  if (s.rc != M3_OK) raise_status(s);
   if (track) {
     std::shared_ptr<ScanNode> node(new ScanNode(), torch::autograd::deleteNode);
     node->ctx = ctx;
@@ -245,8 +248,7 @@ struct MixerNode : public torch::autograd::Node {
   ~MixerNode() override { free_handle(); }
   void free_handle() {
     if (!handle) return;
-    std::lock_guard<std::mutex> lock(lock_of(ctx));
-    m3_saved_free(ctx, handle);
+    m3_saved_free(ctx, handle);   // (on the stream that the handle remembers: no lock)
     handle = nullptr;
   }
   void release_variables() override {
@@ -271,13 +273,8 @@ struct MixerNode : public torch::autograd::Node {
     const m3_mixer_grads out{mut(g[0]), fmut(g[1]), fmut(g[2]), fmut(g[3]), fmut(g[4]), fmut(g[5]),
                              fmut(g[6]), fmut(g[7]), fmut(g[8]), fmut(g[9])};
     const Tensor work = at::empty({(int64_t)m3_mixer_backward_bytes(&d)}, act.options());
-    int rc;
-    {
-      std::lock_guard<std::mutex> lock(lock_of(ctx));
-      bind(ctx, t[0]);
-      rc = m3_mixer_backward(ctx, &d, handle, ptr(act), ptr(dout), &out, mut(work));
-    }
-    if (rc != M3_OK) raise_status(ctx, rc);
+    const Status s = locked(ctx, t[0], [&] { return m3_mixer_backward(ctx, &d, handle, ptr(act), ptr(dout), &out, mut(work)); });
+    if (s.rc != M3_OK) raise_status(s);
     return g;
   }
 };
@@ -299,14 +296,8 @@ Tensor mixer(uintptr_t handle, const Tensor& proj0, const std::vector<OptTensor>
     for (const Tensor& v : p) track = track || (v.defined() && v.requires_grad());
   }
   m3_saved* saved = nullptr;
-  int rc;
-  {
-    py::gil_scoped_release nogil;
-    std::lock_guard<std::mutex> lock(lock_of(ctx));
-    bind(ctx, proj);
-    rc = m3_mixer_forward(ctx, &d, mut(out), mut(act), track ? &saved : nullptr);
-  }
-  if (rc != M3_OK) raise_status(ctx, rc);
+  const Status s = locked(ctx, proj, [&] { return m3_mixer_forward(ctx, &d, mut(out), mut(act), track ? &saved : nullptr); });
+  if (s.rc != M3_OK) raise_status(s);
   if (track) {
     std::shared_ptr<MixerNode> node(new MixerNode(), torch::autograd::deleteNode);
     node->ctx = ctx;
@@ -344,14 +335,8 @@ std::vector<OptTensor> window(uintptr_t handle, const Tensor& proj0, const std::
   const size_t bytes = m3_mixer_window_bytes(&d, &io);
   Tensor work;
   if (bytes) work = at::empty({(int64_t)bytes}, opt.dtype(at::kByte));
-  int rc;
-  {
-    py::gil_scoped_release nogil;
-    std::lock_guard<std::mutex> lock(lock_of(ctx));
-    bind(ctx, proj);
-    rc = m3_mixer_window(ctx, &d, &io, mut(work));
-  }
-  if (rc != M3_OK) raise_status(ctx, rc);
+  const Status done = locked(ctx, proj, [&] { return m3_mixer_window(ctx, &d, &io, mut(work)); });
+  if (done.rc != M3_OK) raise_status(done);
   return {out, conv2, h2, lu2, ang2.defined() ? OptTensor(ang2) : OptTensor()};
 }
 
@@ -359,6 +344,9 @@ std::vector<OptTensor> window(uintptr_t handle, const Tensor& proj0, const std::
 
 PYBIND11_MODULE(_m3torch, m) {
   m.def("set_from_status", [](py::object f) { g_from_status = f.release().ptr(); });
+  auto of = [](uintptr_t handle) -> std::recursive_mutex& { return lock_of(reinterpret_cast<m3_ctx*>(handle)); };
+  m.def("lock", [of](uintptr_t handle) { of(handle).lock(); }, py::call_guard<py::gil_scoped_release>());
+  m.def("unlock", [of](uintptr_t handle) { of(handle).unlock(); });
   m.def("scan", &scan);
   m.def("mixer", &mixer);
   m.def("window", &window);

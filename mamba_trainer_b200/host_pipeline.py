@@ -92,7 +92,7 @@ class HostScanPipeline:
         self._desc_args = dict(
             batch=B, seq=T, heads=H, head_dim=P, d_state=N, rank=R, chunk=int(chunk), dtype=_DTYPES[x.dtype],
             discretization=int(self.disc.value), dynamics=1 if self.rot else 0, want_state=0, path=int(path))
-        self._ctx = Context.for_device(self.dev)
+        self._ctx = Context.of(self.dev)
         self._pipe = None
         self._params = None
         self._runs = 0
@@ -108,7 +108,8 @@ class HostScanPipeline:
         self._params = (a_log, d_skip)   # kept alive: the native pipeline holds their addresses
         desc = _ffi.ScanDesc(a_log=_hp(a_log), d_skip=_hp(d_skip), **self._desc_args)
         handle = C.c_void_p()
-        self._ctx.check(self._ctx.lib.m3_host_pipe_create(self._ctx.handle, C.byref(desc), self.slices, C.byref(handle)))
+        with self._ctx as ctx:
+            ctx.check(ctx.lib.m3_host_pipe_create(ctx.handle, C.byref(desc), self.slices, C.byref(handle)))
         self._pipe = handle
 
     def run(self, host: Dict[str, Optional[torch.Tensor]], params: Dict[str, torch.Tensor],
@@ -121,7 +122,6 @@ class HostScanPipeline:
         elif params["a_log"].data_ptr() != self._params[0].data_ptr() or (
                 self._params[1] is not None and params["d_skip"].data_ptr() != self._params[1].data_ptr()):
             raise ValueError("the pipeline was created for other parameter tensors")
-        self._ctx.bind_current_stream()
         out = self._outs[self._runs % self.depth]
         hin = _ffi.HostIn(x=_hp(host["x"]), b=_hp(host["b"]), c=_hp(host["c"]), dt=_hp(host["dt"]),
                           lambda_=_hp(host.get("lam")) if "lam" in self.names else None,
@@ -130,7 +130,8 @@ class HostScanPipeline:
                             ddt=_hp(out["ddt"]), dlambda=_hp(out.get("dlam")), dtheta=_hp(out.get("dtheta")),
                             da_log=_hp(out["da_log"]), dd_skip=_hp(out["dd_skip"]) if self._params[1] is not None else None)
         ticket = C.c_uint64()
-        self._ctx.check(self._ctx.lib.m3_host_pipe_run(self._pipe, C.byref(hin), C.byref(hout), C.byref(ticket)))
+        with self._ctx as ctx:
+            ctx.check(ctx.lib.m3_host_pipe_run(self._pipe, C.byref(hin), C.byref(hout), C.byref(ticket)))
         self._tickets[id(out)] = ticket.value
         self._runs += 1
         if wait:

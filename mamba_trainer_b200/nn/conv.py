@@ -35,7 +35,7 @@ def _rows(t: torch.Tensor) -> int:
 class _FusedConv(torch.autograd.Function):
     @staticmethod
     def forward(fctx, x, weight, bias, history, activation, want_history):
-        ctx = Context.for_device(x.device)
+        ctx = Context.of(x.device)
         B, T, Cn = x.shape
         K = weight.shape[0]
         y = torch.empty((B, T, Cn), device=x.device, dtype=x.dtype)
@@ -43,7 +43,8 @@ class _FusedConv(torch.autograd.Function):
         desc = _ffi.ConvDesc(batch=B, seq=T, channels=Cn, kernel_size=K, dtype=_DTYPES[x.dtype],
                              activation=1 if activation else 0, x_stride=_rows(x), y_stride=Cn,
                              x=_ptr(x), history=_ptr(history), weight=_ptr(weight), bias=_ptr(bias))
-        ctx.check(ctx.lib.m3_conv_forward(ctx.handle, C.byref(desc), _ptr(y), _ptr(new_hist)))
+        with ctx:
+            ctx.check(ctx.lib.m3_conv_forward(ctx.handle, C.byref(desc), _ptr(y), _ptr(new_hist)))
         fctx.save_for_backward(x, weight, bias, history)
         fctx.activation = activation
         if want_history:
@@ -54,7 +55,7 @@ class _FusedConv(torch.autograd.Function):
     @staticmethod
     def backward(fctx, dy, *_unused):
         x, weight, bias, history = fctx.saved_tensors
-        ctx = Context.for_device(x.device)
+        ctx = Context.of(x.device)
         B, T, Cn = x.shape
         K = weight.shape[0]
         dy = dy.contiguous()
@@ -67,7 +68,8 @@ class _FusedConv(torch.autograd.Function):
         desc = _ffi.ConvDesc(batch=B, seq=T, channels=Cn, kernel_size=K, dtype=_DTYPES[x.dtype],
                              activation=1 if fctx.activation else 0, x_stride=_rows(xc), y_stride=Cn,
                              x=_ptr(xc), history=_ptr(history), weight=_ptr(weight), bias=_ptr(bias))
-        ctx.check(ctx.lib.m3_conv_backward(ctx.handle, C.byref(desc), _ptr(dy), _ptr(dx), _ptr(dw), _ptr(db), _ptr(dh)))
+        with ctx:
+            ctx.check(ctx.lib.m3_conv_backward(ctx.handle, C.byref(desc), _ptr(dy), _ptr(dx), _ptr(dw), _ptr(db), _ptr(dh)))
         return dx, dw, db, dh, None, None
 
 

@@ -28,7 +28,11 @@ _DTYPES = {torch.float32: _ffi.F32, torch.bfloat16: _ffi.BF16}
 
 
 class Context:
-    """One m3_ctx per CUDA device; work is enqueued on torch's current stream."""
+    """One m3_ctx per CUDA device; work is enqueued on torch's current stream.
+
+    The context is shared by the threads of the process.  `with ctx:` binds it to the thread's current stream and keeps
+    others (the native nodes' backward passes run on threads of autograd's) from binding it to theirs until the block's
+    calls have been made and their message read."""
 
     _by_device: dict = {}
 
@@ -58,6 +62,14 @@ class Context:
         if ctx is None:
             ctx = cls._by_device[idx] = Context(idx)
         return ctx
+
+    def __enter__(self) -> "Context":
+        _ffi.extension().lock(self.handle.value)
+        self.lib.m3_ctx_set_stream(self.handle, _current_stream(self.device_index))
+        return self
+
+    def __exit__(self, *exc) -> None:
+        _ffi.extension().unlock(self.handle.value)
 
     def bind_current_stream(self) -> None:
         # (every time: the native nodes bind the stream of their own calls)
@@ -217,7 +229,7 @@ class _FusedSsd(torch.autograd.Function):
 
     @staticmethod
     def forward(fctx, opts, x, b, c, a, g, w, h0):
-        ctx = Context.for_device(x.device)
+        ctx = Context.of(x.device)
         B, T, H, P = x.shape
         N = b.shape[3]
         desc = _FusedSsd._desc(opts, x, b, c, a, g, w, h0)
@@ -226,8 +238,9 @@ class _FusedSsd(torch.autograd.Function):
         out = _ffi.ScanOut(y=_ptr(y), h=_ptr(h))
         track = any(fctx.needs_input_grad)
         saved = C.c_void_p()
-        ctx.check(ctx.lib.m3_scan_forward(ctx.handle, C.byref(desc), C.byref(out),
-                                          C.byref(saved) if track else None))
+        with ctx:
+            ctx.check(ctx.lib.m3_scan_forward(ctx.handle, C.byref(desc), C.byref(out),
+                                              C.byref(saved) if track else None))
         if track:
             fctx.m3 = ctx
             fctx.saved = _Saved(ctx, saved)
@@ -241,7 +254,6 @@ class _FusedSsd(torch.autograd.Function):
     @staticmethod
     def backward(fctx, dy, dh=None):
         ctx = fctx.m3
-        ctx.bind_current_stream()
         it = iter(fctx.saved_tensors)
         # saved-tensor hooks may have dropped the forward's tensors: the adjoint reads these
         tensors = tuple(_placed(next(it), p) if p else None for p in fctx.like)
@@ -258,8 +270,9 @@ class _FusedSsd(torch.autograd.Function):
         bin_ = _ffi.ScanBwdIn(dy=_ptr(dy), dh=_ptr(dh))
         gout = _ffi.ScanGrads(dx=_ptr(grads[0]), db=_ptr(grads[1]), dc=_ptr(grads[2]), da_raw=_ptr(grads[3]),
                               dg_raw=_ptr(grads[4]), dw_raw=_ptr(grads[5]), dh0=_ptr(grads[6]))
-        ctx.check(ctx.lib.m3_scan_backward_moved(ctx.handle, fctx.saved.handle, C.byref(desc), C.byref(bin_),
-                                                 C.c_uint32(mask | 0xFF), C.byref(gout)))
+        with ctx:
+            ctx.check(ctx.lib.m3_scan_backward_moved(ctx.handle, fctx.saved.handle, C.byref(desc), C.byref(bin_),
+                                                     C.c_uint32(mask | 0xFF), C.byref(gout)))
         return (None,) + tuple(grads)
 
 
@@ -313,7 +326,7 @@ def mamba3_step(x, b, c, dt, lambda_, a_log, theta, d_skip, state: SsmState,
     disc = Discretization(discretization)
     if disc is Discretization.LearnedTrapezoid and lambda_ is None:
         raise NullError("LearnedTrapezoid needs a lambda tensor")
-    ctx = Context.for_device(x.device)
+    ctx = Context.of(x.device)
     el = x.dtype
     big = lambda t: None if t is None else t.detach().to(el).contiguous()
     f32 = lambda t: None if t is None else t.detach().to(torch.float32).contiguous()
@@ -329,7 +342,8 @@ def mamba3_step(x, b, c, dt, lambda_, a_log, theta, d_skip, state: SsmState,
                          lambda_=_ptr(lams) if disc is Discretization.LearnedTrapezoid else None, theta=_ptr(ths),
                          a_log=_ptr(al), d_skip=_ptr(dk), h=_ptr(h), last_u=_ptr(lu), angle=_ptr(ang))
     out = _ffi.StepOut(y=_ptr(y), h=_ptr(h2), last_u=_ptr(lu2), angle=_ptr(ang2))
-    ctx.check(ctx.lib.m3_step_forward(ctx.handle, C.byref(desc), C.byref(out)))
+    with ctx:
+        ctx.check(ctx.lib.m3_step_forward(ctx.handle, C.byref(desc), C.byref(out)))
     return y, SsmState(h2, lu2, ang2)
 
 

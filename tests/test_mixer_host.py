@@ -81,3 +81,28 @@ def test_mixer_core_takes_parameters_that_are_none_of_its_own():
     core.forward = lambda: seen.append(core._spec()[0][3])
     torch.func.functional_call(core, {"a_log": stand_in}, ())
     assert seen[0] is stand_in
+
+
+def test_the_contexts_lock_keeps_other_threads_out():
+    """What `with ctx:` holds: another thread waits for it without holding the interpreter's lock, and its owner may take it
+    again."""
+    import threading
+    from mamba_trainer_b200 import _ffi
+    ext, handle, order = _ffi.extension(), 4096, []   # (a key; nothing is read there)
+
+    def other():
+        ext.lock(handle)
+        order.append("other")
+        ext.unlock(handle)
+    ext.lock(handle)
+    ext.lock(handle)
+    t = threading.Thread(target=other)
+    t.start()
+    t.join(0.2)
+    order.append("owner")
+    ext.unlock(handle)
+    t.join(0.1)
+    assert t.is_alive() and order == ["owner"]
+    ext.unlock(handle)
+    t.join(10)
+    assert order == ["owner", "other"]

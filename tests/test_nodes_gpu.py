@@ -130,3 +130,43 @@ def test_switched_off_norms_have_no_gradient(head_dim, d_state):
     assert off.norm_w.grad is None and off.post_norm_w.grad is None
     for n, q in without.named_parameters():
         assert torch.equal(q.grad, getattr(off, n).grad), n
+
+
+def test_threads_with_streams_of_their_own():
+    """Native nodes, with their backward passes on autograd's threads, and the calls that go through ctypes, from threads
+    with streams of their own: each call's launches stay on its thread's stream, behind that stream's writes of its inputs."""
+    import threading
+    from mamba_trainer_b200.nn import causal_conv1d
+    from mamba_trainer_b200.ssm import SsmState, mamba3_step
+    cases = [_scan_case(torch.bfloat16, 64, 128), _scan_case(torch.float32, 64, 64), _ssd_case(), _mixer_case(torch.float32)]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    one = [r(4, 2, 64, 1), r(4, 2, 64, 1), r(4, 2, 64, 1), r(4, 2).abs(), torch.sigmoid(r(4, 2)), r(2).abs(), None, None]
+    state, img, w = (r(4, 2, 64, 64), r(4, 2, 64, 64)), r(4, 300, 96), r(4, 96)
+    step = lambda *v: mamba3_step(*v, None, None, SsmState(*state))[0]
+    work = [lambda c=c: _gradients_alone(*c) for c in cases]
+    work += [lambda: (step(*(t * 1.0 for t in one[:6])),), lambda: (causal_conv1d(img * 1.0, w),)]
+    want = [f() for f in work]
+    torch.cuda.synchronize()
+    failed = []
+
+    def loop(f, expected):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(40):
+                got = f()
+                torch.cuda.current_stream().synchronize()
+                if not all(torch.equal(a, e) for a, e in zip(got, expected)):
+                    failed.append(f)
+                    return
+    threads = [threading.Thread(target=loop, args=(f, e)) for f, e in zip(work, want)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+
+
+def _gradients_alone(f, leaves, dout):
+    leaves = [t.clone().requires_grad_(True) for t in leaves]
+    out = f(*leaves)
+    return (out.detach(),) + torch.autograd.grad(out, leaves, dout)
