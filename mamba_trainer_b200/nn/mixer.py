@@ -21,7 +21,7 @@ import torch
 from .. import _ffi
 from ..error import ConfigError, ShapeError, UnsupportedError
 from ..ssm.config import Discretization
-from ..ssm.scan import Context, SsmState, _DTYPES
+from ..ssm.scan import Context, SsmState, _DTYPES, native
 
 
 # The parameters in the order of m3_mixer_desc.
@@ -168,4 +168,6 @@ class MixerCore(torch.nn.Module):
         # reversed in memory.
         if proj.shape[1] == 0:                      # nothing to scan (scan.rs:134-144)
             return proj.new_zeros((proj.shape[0], 0, s.d_inner)) + 0.0 * proj.sum()
-        return _ffi.extension().mixer(Context.of(proj.device).handle.value, proj, *self._spec(path))
+        mixer, handle = _ffi.extension().mixer, Context.of(proj.device).handle.value
+        params, *spec = self._spec(path)
+        return native(lambda x, *p: (mixer(handle, x, p, *spec),), proj, *params)[0]

@@ -205,6 +205,50 @@ def _ptr(t: Optional[torch.Tensor]):
     return C.c_void_p(t.data_ptr()) if t is not None else None
 
 
+class _Traced(torch.autograd.Function):
+    """A native node inside torch.jit.trace.  The tracer does not see what a native call writes - it would record the buffers
+    of the traced run as the result - but it records a Python node as a call of it."""
+
+    @staticmethod
+    def forward(fctx, call, *tensors):
+        fctx.set_materialize_grads(False)
+        state = torch._C._get_tracing_state()
+        torch._C._set_tracing_state(None)
+        try:
+            leaves = [t if t is None else t.detach().requires_grad_(need)
+                      for t, need in zip(tensors, fctx.needs_input_grad[1:])]
+            with torch.enable_grad():
+                outs = [o for o in call(*leaves) if o is not None]
+            fctx.outs, fctx.leaves = outs, leaves
+            like = [(list(o.shape), o.dtype, o.device) for o in outs]
+        finally:
+            torch._C._set_tracing_state(state)
+        if state is None:   # a run of what was traced
+            return tuple(o.detach() for o in outs)
+        seen = [torch.empty(shape, dtype=dtype, device=device) for shape, dtype, device in like]   # known to the tracer
+        torch._C._set_tracing_state(None)
+        try:
+            for s, o in zip(seen, outs):
+                s.copy_(o.detach())
+        finally:
+            torch._C._set_tracing_state(state)
+        return tuple(seen)
+
+    @staticmethod
+    def backward(fctx, *up):
+        used = [(o, g) for o, g in zip(fctx.outs, up) if g is not None]
+        want = [i for i, t in enumerate(fctx.leaves) if t is not None and t.requires_grad]
+        got = torch.autograd.grad([o for o, _ in used], [fctx.leaves[i] for i in want], [g for _, g in used],
+                                  retain_graph=True, allow_unused=True) if used else [None] * len(want)
+        grads = dict(zip(want, got))
+        return (None,) + tuple(grads.get(i) for i in range(len(fctx.leaves)))
+
+
+def native(call, *tensors):
+    """`call` of a native node: the tuple of its results (without the absent ones when a trace is being recorded)."""
+    return call(*tensors) if torch._C._get_tracing_state() is None else _Traced.apply(call, *tensors)
+
+
 def _placed(t: torch.Tensor, like) -> torch.Tensor:
     """A saved tensor as hooks gave it back, with the element type, density and alignment it had in the forward pass."""
     dtype, device, align = like
@@ -411,10 +455,10 @@ def mamba3_scan(inputs: ScanInputs) -> ScanOutput:
         return ScanOutput(x, state)
 
     # the node is native (csrc/m3_torch.cpp): it brings the inputs to x's element type, parameters and states to float32
-    outs = _ffi.extension().scan(
-        Context.of(x.device).handle.value, x, b, c, inputs.dt, inputs.a_log, lam, theta, inputs.d_skip, st.h if st else None,
-        st.last_u if st else None, st.angle if (st and theta is not None) else None, inputs.chunk_size, int(disc),
-        bool(inputs.want_state), inputs.path, inputs.reverse_heads)
+    scan, handle = _ffi.extension().scan, Context.of(x.device).handle.value
+    options = (inputs.chunk_size, int(disc), bool(inputs.want_state), inputs.path, inputs.reverse_heads)
+    outs = native(lambda *t: scan(handle, *t, *options), x, b, c, inputs.dt, inputs.a_log, lam, theta, inputs.d_skip,
+                  st.h if st else None, st.last_u if st else None, st.angle if (st and theta is not None) else None)
     y = outs[0]
     state = None
     if inputs.want_state:

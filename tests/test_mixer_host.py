@@ -106,3 +106,31 @@ def test_the_contexts_lock_keeps_other_threads_out():
     ext.unlock(handle)
     t.join(10)
     assert order == ["owner", "other"]
+
+
+@pytest.mark.filterwarnings("ignore")
+def test_a_native_node_is_traced_as_a_call():
+    """What ssm.scan.native does under torch.jit.trace, with a stand-in whose arithmetic the tracer cannot see either."""
+    import numpy as np
+    from mamba_trainer_b200.ssm.scan import native
+
+    class Unseen(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x, w):
+            ctx.save_for_backward(x, w)
+            return torch.from_numpy(np.tanh(x.detach().numpy()) * w.detach().numpy())
+
+        @staticmethod
+        def backward(ctx, g):
+            x, w = ctx.saved_tensors
+            return g * w * (1 - x.tanh() ** 2), g * x.tanh()
+
+    def f(x, w):
+        return native(lambda a, b, absent: (Unseen.apply(a, b), None), x * 0.5, w * 2, None)[0] * 3
+    make = lambda: [torch.randn(3, 4, requires_grad=True) for _ in range(2)]
+    traced = torch.jit.trace(f, make(), check_trace=False)
+    for _ in range(2):
+        v = make()
+        assert torch.equal(traced(*v), f(*v))
+        for a, e in zip(torch.autograd.grad(traced(*v).sum(), v), torch.autograd.grad(f(*v).sum(), v)):
+            assert torch.equal(a, e)

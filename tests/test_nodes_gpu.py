@@ -170,3 +170,21 @@ def _gradients_alone(f, leaves, dout):
     leaves = [t.clone().requires_grad_(True) for t in leaves]
     out = f(*leaves)
     return (out.detach(),) + torch.autograd.grad(out, leaves, dout)
+
+
+@pytest.mark.filterwarnings("ignore")
+def test_traced_calls_compute():
+    """torch.jit.trace records a call of the node, not the buffers that the traced run happened to fill: other inputs give
+    their own results and gradients."""
+    for case in ("scan_tensor_core", "scan_chunk_parallel"):
+        f, leaves, dout = CASES[case]()
+        traced = torch.jit.trace(f, tuple(t.clone().requires_grad_(True) for t in leaves), check_trace=False)
+        other = [t * 0.75 for t in leaves]
+        for a, e in zip(_gradients_alone(traced, other, dout), _gradients_alone(f, other, dout)):
+            assert torch.equal(a, e), case
+    shape = MixerShape(2, 64, 128, 1)
+    core = MixerCore(shape, device="cuda")
+    proj, dout = torch.randn(2, 70, shape.in_proj_width, device="cuda"), torch.randn(2, 70, shape.d_inner, device="cuda")
+    traced = torch.jit.trace(core, (proj,), check_trace=False)
+    for a, e in zip(_gradients_alone(traced, [proj + 1], dout), _gradients_alone(core, [proj + 1], dout)):
+        assert torch.equal(a, e)
