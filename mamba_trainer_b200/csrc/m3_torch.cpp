@@ -110,6 +110,12 @@ struct Saved {
            static_cast<int64_t>(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16) == align;
   }
 };
+// The nodes have no forward-mode rule: an input with a tangent is refused, as torch refuses it for a Python node without one.
+void refuse_tangents(const Tensor* t, int n) {
+  for (int i = 0; i < n; ++i)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t[i].defined() || !t[i]._fw_grad(0).defined(),
+                                "forward-mode AD is not implemented for the fused scan and mixer");
+}
 int dtype_code(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? M3_BF16 : M3_F32; }
 
 // ---- the scan -----------------------------------------------------------------------------------------------------
@@ -173,6 +179,7 @@ std::vector<OptTensor> scan(uintptr_t handle, const Tensor& x0, const Tensor& b0
   const Tensor t[kScanInputs] = {as(x0, el), as(b0, el), as(c0, el), as(dt0, el), as(a_log0, at::kFloat), as(lam0, el),
                                  as(theta0, el), as(d_skip0, at::kFloat), as(h00, at::kFloat), as(lu00, at::kFloat),
                                  as(ang00, at::kFloat)};
+  refuse_tangents(t, kScanInputs);
   const Tensor& x = t[0];
   const int64_t B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), R = x.size(4), N = t[1].size(3);
   m3_scan_desc d{};
@@ -286,6 +293,8 @@ Tensor mixer(uintptr_t handle, const Tensor& proj0, const std::vector<OptTensor>
   const Tensor proj = proj0.contiguous();
   Tensor p[kMixerParams];
   for (int i = 0; i < kMixerParams; ++i) p[i] = as(params[i], at::kFloat);
+  refuse_tangents(&proj, 1);
+  refuse_tangents(p, kMixerParams);
   const m3_mixer_desc d = mixer_desc(proj, p, spec_of(ints), eps);
   const auto opt = proj.options().requires_grad(false);
   Tensor out = at::empty({proj.size(0), proj.size(1), d_inner}, opt);

@@ -134,3 +134,25 @@ def test_a_native_node_is_traced_as_a_call():
         assert torch.equal(traced(*v), f(*v))
         for a, e in zip(torch.autograd.grad(traced(*v).sum(), v), torch.autograd.grad(f(*v).sum(), v)):
             assert torch.equal(a, e)
+
+
+def test_forward_mode_is_refused():
+    """A tangent on an input of a native node (of either kind) is refused, not dropped."""
+    from torch.autograd import forward_ad
+    from mamba_trainer_b200 import _ffi
+    ext = _ffi.extension()
+    x, b, dt, a = torch.ones(1, 2, 1, 4, 1), torch.ones(1, 2, 1, 4, 1), torch.ones(1, 2, 1), torch.ones(1)
+    core = MixerCore(MixerShape(heads=1, head_dim=4, d_state=4))
+    proj = torch.ones(1, 2, core.shape.in_proj_width)
+    params, *spec = core._spec()
+    with forward_ad.dual_level():
+        for i, t in enumerate((x, b, b, dt, a)):
+            args = [x, b, b, dt, a]
+            args[i] = forward_ad.make_dual(t, torch.ones_like(t))
+            with pytest.raises(NotImplementedError):
+                ext.scan(0, *args, None, None, None, None, None, None, 64, 0, False, 0, 0)
+        with pytest.raises(NotImplementedError):
+            ext.mixer(0, forward_ad.make_dual(proj, proj), params, *spec)
+        dual = [forward_ad.make_dual(params[3].detach(), torch.ones(1)) if i == 3 else p for i, p in enumerate(params)]
+        with pytest.raises(NotImplementedError):
+            ext.mixer(0, proj, dual, *spec)
