@@ -124,8 +124,9 @@ class MixerCore(torch.nn.Module):
         s, p = self.shape, self._parameters
         # (what is no parameter of the module: absent, or parametrised, pruned, assigned, a view of a flattened one)
         return ([getattr(self, n) if (v := p.get(n)) is None else v for n in _PARAMS],
-                (s.heads, s.head_dim, s.d_state, s.rank, s.n_groups, self.chunk, self.disc, s.rotational, self.use_norm,
-                 self.post_gate_norm, path, s.heads // 2 if self.bidirectional else 0), self.eps, s.d_inner)
+                (s.heads, s.head_dim, s.d_state, s.rank, s.n_groups, min(int(self.chunk), 1 << 30), int(self.disc),
+                 1 if s.rotational else 0, 1 if self.use_norm else 0, 1 if self.post_gate_norm else 0, int(path),
+                 s.heads // 2 if self.bidirectional else 0), float(self.eps), s.d_inner)
 
     def forward_cached(self, proj: torch.Tensor, cache: Optional[MixerCache] = None):
         """Inference with a carried state (Mamba3Mixer::apply_with_state, src/models/mamba3.rs:486-560):

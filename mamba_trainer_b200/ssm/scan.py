@@ -456,7 +456,9 @@ def mamba3_scan(inputs: ScanInputs) -> ScanOutput:
 
     # the node is native (csrc/m3_torch.cpp): it brings the inputs to x's element type, parameters and states to float32
     scan, handle = _ffi.extension().scan, Context.of(x.device).handle.value
-    options = (inputs.chunk_size, int(disc), bool(inputs.want_state), inputs.path, inputs.reverse_heads)
+    # (the native call takes integers of 32 bits; a chunk longer than any sequence is the whole sequence)
+    options = (min(int(inputs.chunk_size), 1 << 30), int(disc), bool(inputs.want_state), int(inputs.path),
+               int(inputs.reverse_heads))
     outs = native(lambda *t: scan(handle, *t, *options), x, b, c, inputs.dt, inputs.a_log, lam, theta, inputs.d_skip,
                   st.h if st else None, st.last_u if st else None, st.angle if (st and theta is not None) else None)
     y = outs[0]

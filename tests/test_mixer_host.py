@@ -156,3 +156,23 @@ def test_forward_mode_is_refused():
         dual = [forward_ad.make_dual(params[3].detach(), torch.ones(1)) if i == 3 else p for i, p in enumerate(params)]
         with pytest.raises(NotImplementedError):
             ext.mixer(0, proj, dual, *spec)
+
+
+def test_options_of_other_number_types_reach_the_native_calls(monkeypatch):
+    """A chunk length that is a float or longer than 32 bits hold, and switches that are no bools of Python's own, are taken
+    as they have always been."""
+    import numpy as np
+    from mamba_trainer_b200.ssm import ScanInputs, mamba3_scan, scan
+    want = MixerCore(MixerShape(heads=2, head_dim=4, d_state=8), chunk=64)._spec()[1:]
+    odd = MixerCore(MixerShape(heads=2, head_dim=4, d_state=8, rotational=np.bool_(True)), chunk=64.0, bc_norm=np.bool_(True))
+    assert odd._spec(np.int64(0))[1:] == want and all(type(v) is int for v in odd._spec()[1])
+    assert MixerCore(MixerShape(heads=2, head_dim=4, d_state=8), chunk=10 ** 12)._spec()[1][5] == 1 << 30
+    seen = []
+    monkeypatch.setattr(scan, "native", lambda call, *t: seen.append(call) or (t[0], None, None, None))
+    monkeypatch.setattr(scan.Context, "of", lambda device: type("", (), {"handle": type("", (), {"value": 0})}))
+    monkeypatch.setattr(scan._ffi, "extension", lambda: type("", (), {"scan": staticmethod(lambda *a: a[-5:])}))
+    x, dt = torch.ones(1, 2, 1, 4, 1), torch.ones(1, 2, 1)
+    for chunk in (64.0, np.int64(64), 10 ** 12):
+        mamba3_scan(ScanInputs.new(x, x, x, dt, torch.ones(1), dt).with_chunk_size(chunk).with_state_output(False))
+        got = seen.pop()()
+        assert got[0] == min(int(chunk), 1 << 30) and all(type(v) in (int, bool) for v in got)
