@@ -175,6 +175,7 @@ int m3_download(m3_ctx *ctx, void *dst_host, const void *src_device, size_t byte
  * receives a handle the caller frees with m3_saved_free after the last backward.
  * The saved context refers to the input buffers of `desc`: keep them alive and
  * unchanged until then (the reference's closure holds clones, var.rs:210-216).
+ * Without `saved` the returned state may take the place of the one carried in (out->h == desc->h0 and so on).
  * The tensor-core kernel family moves rows as 16-byte vectors: with M3_PATH_AUTO a call whose
  * x, b, c, theta or y is not 16-byte aligned runs another family instead (M3_PATH_TENSOR
  * refuses it), and the backward of a forward that ran the tensor-core family needs 16-byte

@@ -539,7 +539,10 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     const int ntiles = m3::tc_tiles(d.T, d.R);
     int nseg = 1, tps = ntiles, bseg, btps;
     const bool direct = d.R == 1 && !d.rot && d.rev == 0 && d.T % 8 == 0;
-    bool ahead = m3::tc_ahead_plan((int)BH, ntiles, false, direct, &nseg, &tps);
+    // A state that is replaced in place is read by a stripe's first segment: its last one must not run beside that.
+    const bool in_place = p.h0 && ((p.h_out && p.h_out == p.h0) || (p.lu_out && p.lu_out == p.lu0) ||
+                                   (p.angle_out && p.angle_out == p.angle0));
+    bool ahead = !in_place && m3::tc_ahead_plan((int)BH, ntiles, false, direct, &nseg, &tps);
     if (ahead && ctx->no_scratch) {
       m3::TcAhead a{};
       a.nseg = nseg;

@@ -56,8 +56,7 @@ __global__ void __launch_bounds__(256, N == 64 ? 4 : 3) k_rows_state(Dims d, m3_
 
 // ---- the pass over chunk states: a thread owns planes (m, m + NH) of two rows p, p + 32 --------------------------
 template <class T, int N, bool ROT>
-__global__ void __launch_bounds__(256) k_rows_pass(Dims d, m3_scan_desc in, RowsWs ws, float* __restrict__ h_out,
-                                                   float* __restrict__ angle_out) {
+__global__ void __launch_bounds__(256) k_rows_pass(Dims d, m3_scan_desc in, RowsWs ws, float* h_out) {   // (h_out may be h0)
   constexpr int NH = N / 2, PN = kP * N, U = 4;
   const int bh = blockIdx.y, b = bh / d.H, h = bh - b * d.H;
   const int id = blockIdx.x * 256 + threadIdx.x, m = id % NH, p = id / NH;   // p < 32
@@ -113,7 +112,6 @@ __global__ void __launch_bounds__(256) k_rows_pass(Dims d, m3_scan_desc in, Rows
 #pragma unroll
     for (int i = 0; i < 4; ++i) h_out[(size_t)bh * PN + plain[i]] = carry[i];
   }
-  if (ROT && angle_out && p == 0) angle_out[(size_t)bh * NH + m] = ang;
 }
 
 // ---- outputs of a chunk ------------------------------------------------------------------------------------------
@@ -131,7 +129,7 @@ struct OutSmem {
 };
 template <class T, int N, int R, bool ROT>
 __global__ void __launch_bounds__(256, N == 64 ? 3 : 2) k_rows_out(Dims d, m3_scan_desc in, RowsWs ws, T* __restrict__ y,
-                                                     float* __restrict__ last_u) {
+                                                     float* __restrict__ last_u, float* __restrict__ angle_out) {
   extern __shared__ __align__(16) unsigned char smem[];
   OutSmem<N, R>& sm = *reinterpret_cast<OutSmem<N, R>*>(smem);
   constexpr int NH = N / 2, PN = kP * N;
@@ -141,6 +139,10 @@ __global__ void __launch_bounds__(256, N == 64 ? 3 : 2) k_rows_out(Dims d, m3_sc
   load_rows<T, R, kP, 256>(sm.x, static_cast<const T*>(in.x), d, c);
   chunk_scalars<T, R>(sm.s, d, c, in);
   if constexpr (ROT) {
+    if (angle_out && c.k == d.C - 1 && tid < NH) {   // (not in the pass, whose blocks all read an angle0 it may replace)
+      const size_t o = ((size_t)c.bh * d.C + c.k) * NH + tid;
+      angle_out[(size_t)c.bh * NH + tid] = wrap_angle(ws.abase[o] + ws.asum[o]);
+    }
     chunk_angles<T, N, R, 256>(sm.phi, sm.q, sm.s, d, c, static_cast<const T*>(in.theta),
                                ws.abase + ((size_t)c.bh * d.C + c.k) * NH, [](int, float) {});
     __syncthreads();
@@ -220,10 +222,9 @@ cudaError_t forward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, co
   if (e == cudaSuccess) e = smem_limit(k_rows_out<T, N, R, ROT>, sizeof(OutSmem<N, R>));
   if (e != cudaSuccess) return e;
   k_rows_state<T, N, R, ROT, false><<<grid, 256, sizeof(StateSmem<N, R>), st>>>(d, in, nullptr, ws, ws.hs);
-  k_rows_pass<T, N, ROT><<<dim3(32 * (N / 2) / 256, d.B * d.H), 256, 0, st>>>(d, in, ws, in.want_state ? out.h : nullptr,
-                                                                             in.want_state ? out.angle : nullptr);
+  k_rows_pass<T, N, ROT><<<dim3(32 * (N / 2) / 256, d.B * d.H), 256, 0, st>>>(d, in, ws, in.want_state ? out.h : nullptr);
   k_rows_out<T, N, R, ROT><<<grid, 256, sizeof(OutSmem<N, R>), st>>>(
-      d, in, ws, static_cast<T*>(out.y), in.want_state && !d.raw ? out.last_u : nullptr);
+      d, in, ws, static_cast<T*>(out.y), in.want_state && !d.raw ? out.last_u : nullptr, in.want_state ? out.angle : nullptr);
   return cudaGetLastError();
 }
 

@@ -282,3 +282,40 @@ def test_side_by_side_segments_match_the_oracle(B, H, R, rot, T, state, rev):
         else:
             check_bf16(name, a, e)
     compare_all(t, 64, check, True, ds, path=2, reverse_heads=rev)
+
+
+@pytest.mark.parametrize("dtype,H,N,R,T,rot", [(torch.float32, 40, 128, 1, 700, True), (torch.bfloat16, 40, 64, 2, 300, True),
+                                              (torch.bfloat16, 2, 128, 1, 1000, True), (torch.bfloat16, 3, 128, 2, 700, False),
+                                              (torch.bfloat16, 2, 128, 1, 1000, False), (torch.float32, 3, 40, 1, 90, True)])
+def test_a_state_replaced_in_place(dtype, H, N, R, T, rot):
+    """The C entry's returned state in the buffers of the one carried in gives what separate buffers give."""
+    import ctypes as C
+    from test_scan_gpu import small_inputs
+    from mamba_trainer_b200 import _ffi
+    from mamba_trainer_b200.ssm import Context
+    P = 24 if N == 40 else 64
+    t, _ = small_inputs(2, T, H, P, N, R, rot, True, seed=T)
+    for k in ("x", "b", "c", "dt", "lam", "theta"):
+        if t[k] is not None:
+            t[k] = (t[k] / (N ** 0.5 if k in "bc" else 1)).to(dtype)
+    t = {k: v.cuda() if v is not None else None for k, v in t.items()}
+    p = lambda v: C.c_void_p(v.data_ptr()) if v is not None else None
+    ctx, res = Context.for_device(torch.device("cuda")), []
+    for in_place in (False, True):
+        st = [v.clone() if v is not None else None for v in (t["h0"], t["last_u0"], t["angle0"])]
+        new = st if in_place else [torch.empty_like(v) if v is not None else None for v in st]
+        y = torch.empty_like(t["x"])
+        d = _ffi.ScanDesc(batch=2, seq=T, heads=H, head_dim=P, d_state=N, rank=R, chunk=64, discretization=2, want_state=1,
+                          dtype=_ffi.F32 if dtype == torch.float32 else _ffi.BF16, dynamics=int(rot), x=p(t["x"]), b=p(t["b"]),
+                          c=p(t["c"]), dt=p(t["dt"]), lambda_=p(t["lam"]), theta=p(t["theta"]), a_log=p(t["a_log"]),
+                          h0=p(st[0]), last_u0=p(st[1]), angle0=p(st[2]))
+        out = _ffi.ScanOut(y=p(y), h=p(new[0]), last_u=p(new[1]), angle=p(new[2]))
+        ctx.check(ctx.lib.m3_scan_forward(ctx.handle, C.byref(d), C.byref(out), None))
+        res.append([y] + [v for v in new if v is not None])
+    # (a tensor-core stripe runs whole in place and cut otherwise: bf16 operands either way)
+    tol = 2e-2 if dtype == torch.bfloat16 and N == 128 else 0.0
+    for n, a, e in zip(("y", "h", "last_u", "angle"), *res):
+        if n == "angle":
+            assert float((torch.sin(a) - torch.sin(e)).abs().max()) <= (2e-3 if tol else 0.0)
+        else:
+            assert norm_rel(a.float(), e.float()) <= tol, n
