@@ -122,11 +122,14 @@ class MixerCore(torch.nn.Module):
     def _spec(self, path: int = _ffi.PATH_AUTO):
         """The parameters in _PARAMS' order, the integers of m3_mixer_desc, eps and d_inner: what the native node takes."""
         s, p = self.shape, self._parameters
+        chunk = self.chunk
+        if type(chunk) is not int or chunk > 1 << 30:   # (the native call takes integers of 32 bits)
+            chunk = min(int(chunk), 1 << 30)
         # (what is no parameter of the module: absent, or parametrised, pruned, assigned, a view of a flattened one)
-        return ([getattr(self, n) if (v := p.get(n)) is None else v for n in _PARAMS],
-                (s.heads, s.head_dim, s.d_state, s.rank, s.n_groups, min(int(self.chunk), 1 << 30), int(self.disc),
-                 1 if s.rotational else 0, 1 if self.use_norm else 0, 1 if self.post_gate_norm else 0, int(path),
-                 s.heads // 2 if self.bidirectional else 0), float(self.eps), s.d_inner)
+        return ([p[n] if n in p else getattr(self, n) for n in _PARAMS],
+                (s.heads, s.head_dim, s.d_state, s.rank, s.n_groups, chunk, self.disc, 1 if s.rotational else 0,
+                 1 if self.use_norm else 0, 1 if self.post_gate_norm else 0, path, s.heads // 2 if self.bidirectional else 0),
+                self.eps, s.d_inner)
 
     def forward_cached(self, proj: torch.Tensor, cache: Optional[MixerCache] = None):
         """Inference with a carried state (Mamba3Mixer::apply_with_state, src/models/mamba3.rs:486-560):
