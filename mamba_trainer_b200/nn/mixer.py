@@ -172,6 +172,7 @@ class MixerCore(torch.nn.Module):
         # reversed in memory.
         if proj.shape[1] == 0:                      # nothing to scan (scan.rs:134-144)
             return proj.new_zeros((proj.shape[0], 0, s.d_inner)) + 0.0 * proj.sum()
-        mixer, handle = _ffi.extension().mixer, Context.of(proj.device).handle.value
-        params, *spec = self._spec(path)
-        return native(lambda x, *p: (mixer(handle, x, p, *spec),), proj, *params)[0]
+        mixer, handle, (params, *spec) = _ffi.extension().mixer, Context.of(proj.device).handle.value, self._spec(path)
+        if not torch._C._is_tracing():
+            return mixer(handle, proj, params, *spec)
+        return native(lambda h, x, *p: (mixer(h, x, p, *spec),), handle, (proj, *params), ())[0]

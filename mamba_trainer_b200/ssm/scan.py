@@ -244,9 +244,11 @@ class _Traced(torch.autograd.Function):
         return (None,) + tuple(grads.get(i) for i in range(len(fctx.leaves)))
 
 
-def native(call, *tensors):
-    """`call` of a native node: the tuple of its results (without the absent ones when a trace is being recorded)."""
-    return call(*tensors) if torch._C._get_tracing_state() is None else _Traced.apply(call, *tensors)
+def native(node, handle, tensors, options):
+    """A native node's call: the tuple of its results (without the absent ones when a trace is being recorded)."""
+    if not torch._C._is_tracing():
+        return node(handle, *tensors, *options)
+    return _Traced.apply(lambda *t: node(handle, *t, *options), *tensors)
 
 
 def _placed(t: torch.Tensor, like) -> torch.Tensor:
@@ -455,12 +457,12 @@ def mamba3_scan(inputs: ScanInputs) -> ScanOutput:
         return ScanOutput(x, state)
 
     # the node is native (csrc/m3_torch.cpp): it brings the inputs to x's element type, parameters and states to float32
-    scan, handle = _ffi.extension().scan, Context.of(x.device).handle.value
     # (the native call takes integers of 32 bits; a chunk longer than any sequence is the whole sequence)
     options = (min(int(inputs.chunk_size), 1 << 30), int(disc), bool(inputs.want_state), int(inputs.path),
                int(inputs.reverse_heads))
-    outs = native(lambda *t: scan(handle, *t, *options), x, b, c, inputs.dt, inputs.a_log, lam, theta, inputs.d_skip,
-                  st.h if st else None, st.last_u if st else None, st.angle if (st and theta is not None) else None)
+    outs = native(_ffi.extension().scan, Context.of(x.device).handle.value,
+                  (x, b, c, inputs.dt, inputs.a_log, lam, theta, inputs.d_skip, st.h if st else None,
+                   st.last_u if st else None, st.angle if (st and theta is not None) else None), options)
     y = outs[0]
     state = None
     if inputs.want_state:

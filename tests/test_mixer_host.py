@@ -126,7 +126,7 @@ def test_a_native_node_is_traced_as_a_call():
             return g * w * (1 - x.tanh() ** 2), g * x.tanh()
 
     def f(x, w):
-        return native(lambda a, b, absent: (Unseen.apply(a, b), None), x * 0.5, w * 2, None)[0] * 3
+        return native(lambda handle, a, b, absent, factor: (factor * Unseen.apply(a, b), None), 0, (x * 0.5, w * 2, None), (2,))[0] * 3
     make = lambda: [torch.randn(3, 4, requires_grad=True) for _ in range(2)]
     traced = torch.jit.trace(f, make(), check_trace=False)
     for _ in range(2):
@@ -168,11 +168,10 @@ def test_options_of_other_number_types_reach_the_native_calls(monkeypatch):
     assert odd._spec(np.int64(0))[1:] == want and type(odd._spec()[1][5]) is int
     assert MixerCore(MixerShape(heads=2, head_dim=4, d_state=8), chunk=10 ** 12)._spec()[1][5] == 1 << 30
     seen = []
-    monkeypatch.setattr(scan, "native", lambda call, *t: seen.append(call) or (t[0], None, None, None))
+    monkeypatch.setattr(scan, "native", lambda node, handle, t, options: seen.append(options) or (t[0], None, None, None))
     monkeypatch.setattr(scan.Context, "of", lambda device: type("", (), {"handle": type("", (), {"value": 0})}))
-    monkeypatch.setattr(scan._ffi, "extension", lambda: type("", (), {"scan": staticmethod(lambda *a: a[-5:])}))
     x, dt = torch.ones(1, 2, 1, 4, 1), torch.ones(1, 2, 1)
     for chunk in (64.0, np.int64(64), 10 ** 12):
         mamba3_scan(ScanInputs.new(x, x, x, dt, torch.ones(1), dt).with_chunk_size(chunk).with_state_output(False))
-        got = seen.pop()()
+        got = seen.pop()
         assert got[0] == min(int(chunk), 1 << 30) and all(type(v) in (int, bool) for v in got)
