@@ -340,10 +340,7 @@ __device__ __forceinline__ void load_rows(float* dst, const T* src, const Dims& 
 __device__ __forceinline__ void sincos_wrapped(float phi, float* sn, float* cs) { sincospif(phi * 0.31830988618379067f, sn, cs); }
 
 // Rows of B or C (two tensors at once share the sines), rotated by -phi; `scale` (per step, or NULL) multiplies them.
-// BF: the result is rounded to bf16 (exact in TF32: one product instead of three), as the tensor-core family's operands are.
-template <bool BF>
-__device__ __forceinline__ float operand(float v) { return BF ? __bfloat162float(__float2bfloat16_rn(v)) : v; }
-template <class T, int N, int R, int THREADS, int NTENS, bool BF = false>
+template <class T, int N, int R, int THREADS, int NTENS>
 __device__ __forceinline__ void load_rotated(float* const (&dst)[NTENS], const T* const (&src)[NTENS], const float* phi,
                                              const float* scale, const Dims& d, const Chunk& c) {
   constexpr int LT = kRows / R, NH = N / 2, PER = NH * R / 4, NA = R == 1 ? 4 : (R == 2 ? 2 : 1);
@@ -364,9 +361,7 @@ __device__ __forceinline__ void load_rotated(float* const (&dst)[NTENS], const T
     const float sc = scale ? scale[l] : 1.0f;
 #pragma unroll
     for (int j = 0; j < NA; ++j) {
-      // (the angle is wrapped: the special-function unit's sine is good to 2^-21 there, far below a bf16 operand)
-      if (BF) __sincosf(phi[l * NH + e / R + j], &sn[j], &cs[j]);
-      else sincos_wrapped(phi[l * NH + e / R + j], &sn[j], &cs[j]);
+      sincos_wrapped(phi[l * NH + e / R + j], &sn[j], &cs[j]);
       cs[j] *= sc;
       sn[j] *= sc;
     }
@@ -376,8 +371,8 @@ __device__ __forceinline__ void load_rotated(float* const (&dst)[NTENS], const T
       float o1[4], o2[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        o1[j] = operand<BF>(a[j] * cs[j / R] + b[j] * sn[j / R]);
-        o2[j] = operand<BF>(b[j] * cs[j / R] - a[j] * sn[j / R]);
+        o1[j] = a[j] * cs[j / R] + b[j] * sn[j / R];
+        o2[j] = b[j] * cs[j / R] - a[j] * sn[j / R];
       }
       if (R == 1) {
         *reinterpret_cast<float4*>(dst[w] + at<N>(l, e)) = make_float4(o1[0], o1[1], o1[2], o1[3]);
@@ -394,7 +389,7 @@ __device__ __forceinline__ void load_rotated(float* const (&dst)[NTENS], const T
   }
 }
 // The same without a rotation.
-template <class T, int N, int R, int THREADS, bool BF = false>
+template <class T, int N, int R, int THREADS>
 __device__ __forceinline__ void load_scaled(float* dst, const T* src, const float* scale, const Dims& d, const Chunk& c) {
   constexpr int LT = kRows / R, PER = N * R / 4;
 #pragma unroll
@@ -403,7 +398,7 @@ __device__ __forceinline__ void load_scaled(float* dst, const T* src, const floa
     float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (t < d.T) v = load4(src + tok_index(d, c.b, t, c.h) * N * R + e);
     const float sc = scale[l];
-    const float f[4] = {operand<BF>(v.x * sc), operand<BF>(v.y * sc), operand<BF>(v.z * sc), operand<BF>(v.w * sc)};
+    const float f[4] = {v.x * sc, v.y * sc, v.z * sc, v.w * sc};
     if (R == 1) {
       *reinterpret_cast<float4*>(dst + at<N>(l, e)) = make_float4(f[0], f[1], f[2], f[3]);
     } else {
