@@ -42,6 +42,17 @@ int cuda_fail(m3_ctx* ctx, cudaError_t e, const char* what) {
   return fail(ctx, M3_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+int sm_count() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0)
+      return n;
+    cudaGetLastError();
+    return 148;
+  }();
+  return sms;
+}
+
 int take_device_flag(m3_ctx* ctx, const char* when) {
   if (!ctx->err_host || !*ctx->err_host) return M3_OK;
   *ctx->err_host = 0;
@@ -205,7 +216,7 @@ cudaError_t plan_ahead(m3_ctx* ctx, Params& p, const m3::Dims& d, const m3_scan_
   p.ahead = 1;
   p.nseg = nseg;
   p.tps = tps;
-  p.grid = BH * nseg < 148 ? BH * nseg : 148;
+  p.grid = BH * nseg < m3::sm_count() ? BH * nseg : m3::sm_count();
   p.seg_state = a.seg_state;
   p.seg_angle = a.seg_angle;
   p.seg_flag = nullptr;

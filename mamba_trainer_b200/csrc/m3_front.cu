@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(1024) k_front_gain(const float* __restrict__ r
 
 // Steps per warp: a block of 128 steps amortises the window's start and the warps' parameters; a grid of fewer than four
 // such blocks per SM is cut finer so that every SM has work.
-bool front_long(const Front& f, int tiles) { return (long long)tiles * f.B * ((f.T + 127) / 128) >= 4 * 148; }
+bool front_long(const Front& f, int tiles) { return (long long)tiles * f.B * ((f.T + 127) / 128) >= 4 * sm_count(); }
 int bwd_steps(const Front& f, int tiles) { return kBwdWarps * (front_long(f, tiles) ? 32 : 8); }
 template <int N, int R>
 void front_tiles(const Front& f, int* nx, int* nb) {

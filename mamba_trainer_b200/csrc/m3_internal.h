@@ -31,6 +31,8 @@ namespace m3 {
 inline cudaError_t scratch_alloc(m3_ctx* ctx, void** out, size_t bytes, cudaStream_t st) {
   return ctx->pool ? cudaMallocFromPoolAsync(out, bytes, ctx->pool, st) : cudaMallocAsync(out, bytes, st);
 }
+// SMs of the device that was current when it was first asked for (148 where there is none): what grids and plans are cut by.
+int sm_count();
 // Have the driver load kernels now instead of at their first launch.
 template <class... K>
 inline cudaError_t load_kernels(K... kernels) {

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(256, 3) k_step_rows(const __grid_constant__ St
 // have about four CTAs per SM: a small step is all latency, and the chain inside a CTA grows with its rows.
 inline int step_rows_per_cta(int bh, int head_dim, int pass1) {
   int rows = head_dim < kStepMaxRows ? head_dim : kStepMaxRows;
-  while (rows > pass1 && (long long)bh * ((head_dim + rows - 1) / rows) < 4 * 148) rows = (rows + 1) / 2;
+  while (rows > pass1 && (long long)bh * ((head_dim + rows - 1) / rows) < 4 * sm_count()) rows = (rows + 1) / 2;
   return (rows + pass1 - 1) / pass1 * pass1;
 }
 

@@ -439,16 +439,16 @@ cudaError_t tc_ahead_load() {
 // takes about 4 per tile and SM, and the two launches and the pass some 12 more.  Beyond a third of the SMs it takes long
 // stripes to gain anything (96 stripes of 16 tiles: nothing; 64 of 248: forward + backward 3.47 -> 2.06 ms).
 bool tc_ahead_plan(int BH, int tiles, bool backward, bool direct, int* nseg, int* tps) {
-  constexpr int kSms = 148;
-  if (BH > kSms || tiles < (BH > kSms / 3 ? 24 : 3)) return false;
+  const int sms = sm_count();
+  if (BH > sms || tiles < (BH > sms / 3 ? 24 : 3)) return false;
   const float c = backward ? 15.0f : 5.5f, whole = direct ? (backward ? 11.0f : 5.2f) : c;
   float best = 0.92f * tiles * whole;
   bool found = false;
-  for (int n = 2; n <= tiles && n <= 4 * kSms; ++n) {
+  for (int n = 2; n <= tiles && n <= 4 * sms; ++n) {
     const int per = (tiles + n - 1) / n, segs = (tiles + per - 1) / per;
     if (segs != n) continue;
-    const int rounds = (BH * segs + kSms - 1) / kSms;
-    const float work = 4.0f * BH * (segs - 1) * per / kSms;
+    const int rounds = (BH * segs + sms - 1) / sms;
+    const float work = 4.0f * BH * (segs - 1) * per / sms;
     const float t = 12.0f + (work > 8.0f ? work : 8.0f) + rounds * (per + 1) * c;
     if (t < best) {
       best = t;
@@ -464,7 +464,7 @@ bool tc_ahead_plan(int BH, int tiles, bool backward, bool direct, int* nseg, int
 // tiles where there are fewer.
 static void ahead_groups(int BH, TcAhead* a) {
   a->gt = a->tps;
-  while (a->gt > 1 && (long long)BH * (a->nseg - 1) * ((a->tps + a->gt - 1) / a->gt) < 2 * 148) a->gt = (a->gt + 1) / 2;
+  while (a->gt > 1 && (long long)BH * (a->nseg - 1) * ((a->tps + a->gt - 1) / a->gt) < 2 * sm_count()) a->gt = (a->gt + 1) / 2;
   a->gps = (a->tps + a->gt - 1) / a->gt;
 }
 

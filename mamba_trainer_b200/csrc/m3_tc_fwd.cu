@@ -498,11 +498,7 @@ cudaError_t launch_r(cudaStream_t st, const TcFwdParams& p, bool rot) {
 }  // namespace
 
 void tc_segment_plan(int BH, int tiles, bool allow_split, int* nseg, int* tps, int* grid, size_t* scratch_bytes) {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
-    return n;
-  }();
+  const int sms = sm_count();
   int want = 1;
   // Segments of one stripe run one after the other, so cutting adds no parallelism: it only evens out the
   // last round when there are more stripes than SMs.
