@@ -284,6 +284,32 @@ def test_side_by_side_segments_match_the_oracle(B, H, R, rot, T, state, rev):
     compare_all(t, 64, check, True, ds, path=2, reverse_heads=rev)
 
 
+@pytest.mark.parametrize("T,H,R", [(8200, 2, 1), (9001, 3, 2)])
+def test_long_cut_stripes_match_the_oracle(T, H, R):
+    """Stripes of some hundred tiles cut into segments, inputs as models have them.  d theta, a difference of sums over the
+    sequence, is held to the reference's own bf16 matmul mode on the same inputs, as in the tests of whole stripes."""
+    from test_scan_gpu import check_bf16
+    from _util import fused_run, oracle_run, reference_mode_error
+    from mamba_trainer_b200 import synthetic
+    from mamba_trainer_b200.ssm import Context
+    w = synthetic.Workload("long", 1, T, H, 64, 128, 64, R, torch.bfloat16, Discretization.LearnedTrapezoid, True,
+                           "rms" if R == 1 else "scaled")
+    t = synthetic.make_inputs(w, seed=R)
+    ctx = Context.for_device(torch.device("cuda"))
+    before = ctx.lib.m3_launch_count(ctx.handle)
+    y, _, got = fused_run(t, 64, False, path=2)
+    # group states, pass and stripe kernel each way, then the joined sums of d phi and the per-head sums
+    assert ctx.lib.m3_launch_count(ctx.handle) - before >= 7
+    ey, _, exact = oracle_run(t, 64, False)
+    mode = reference_mode_error(t, 64, exact, ("theta",))
+    check_bf16("y", y, ey)
+    for n, e in exact.items():
+        if n == "theta":
+            assert norm_rel(got[n].float(), e) <= max(2e-2, mode[n]), (n, norm_rel(got[n].float(), e), mode)
+        else:
+            check_bf16("d" + n, got[n], e)
+
+
 @pytest.mark.parametrize("dtype,H,N,R,T,rot", [(torch.float32, 40, 128, 1, 700, True), (torch.bfloat16, 40, 64, 2, 300, True),
                                               (torch.bfloat16, 2, 128, 1, 1000, True), (torch.bfloat16, 3, 128, 2, 700, False),
                                               (torch.bfloat16, 2, 128, 1, 1000, False), (torch.float32, 3, 40, 1, 90, True)])
