@@ -200,7 +200,7 @@ cudaError_t plan_segments(m3_ctx* ctx, Params& p, int tiles, bool allow_split, c
 // `nseg` and `tps` come from tc_ahead_plan; dy, dh as in tc_ahead.
 template <class Params>
 cudaError_t plan_ahead(m3_ctx* ctx, Params& p, const m3::Dims& d, const m3_scan_desc& desc, int nseg, int tps, const void* dy,
-                       const float* dh, const float* ckpt_angle, char** scratch) {
+                       const float* dh, const float* ckpt_angle, bool full_angle, char** scratch) {
   *scratch = nullptr;
   const int BH = d.B * d.H;
   m3::TcAhead a{};
@@ -211,8 +211,7 @@ cudaError_t plan_ahead(m3_ctx* ctx, Params& p, const m3::Dims& d, const m3_scan_
   if (!ctx->no_scratch) e = m3::scratch_alloc(ctx, reinterpret_cast<void**>(scratch), bytes, ctx->stream);
   if (e != cudaSuccess) return e;
   m3::tc_ahead_bytes(BH, &a, ctx->no_scratch ? ctx->fixed_scratch : *scratch);
-  e = m3::tc_ahead(ctx->stream, d, desc, dy, dh, ckpt_angle, a);
-  ctx->launches += 2;
+  e = m3::tc_ahead(ctx->stream, d, desc, dy, dh, ckpt_angle, a, full_angle, &ctx->launches);
   p.ahead = 1;
   p.nseg = nseg;
   p.tps = tps;
@@ -295,7 +294,7 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
   if (ahead) {
     p.dphi = dphi;
     p.dpsum = dphi + per_tok * 64;
-    e = plan_ahead(ctx, p, d, desc, nseg, tps, in->dy, in->dh, saved->tc_ckpt_angle, &seg);
+    e = plan_ahead(ctx, p, d, desc, nseg, tps, in->dy, in->dh, saved->tc_ckpt_angle, false, &seg);
   } else {
     e = plan_segments(ctx, p, tiles, !p.use_tma, &seg);
   }
@@ -589,7 +588,7 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     }
     // a caller that must not allocate gets whole stripes: cutting them needs scratch
     char* seg = nullptr;
-    cudaError_t te = ahead ? plan_ahead(ctx, p, d, *desc, nseg, tps, nullptr, nullptr, nullptr, &seg)
+    cudaError_t te = ahead ? plan_ahead(ctx, p, d, *desc, nseg, tps, nullptr, nullptr, nullptr, saved != nullptr, &seg)
                            : plan_segments(ctx, p, ntiles, !p.use_tma && !ctx->no_scratch, &seg);
     if (te == cudaSuccess) te = m3::tc_forward(ctx->stream, p, d.rot != 0);
     if (seg) {

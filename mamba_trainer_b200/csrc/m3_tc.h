@@ -79,9 +79,10 @@ struct TcAhead {
 bool tc_ahead_plan(int BH, int tiles, bool backward, bool direct, int* nseg, int* tps);
 // nseg and tps given: fills in the rest; bytes of scratch.
 size_t tc_ahead_bytes(int BH, TcAhead* a, char* base);
-// dy NULL: forward; else the gradient of the state (dh: the one reaching the returned state, or NULL).
+// dy NULL: forward; else the gradient of the state (dh: the one reaching the returned state, or NULL).  full_angle: the
+// forward pass of a training step.
 cudaError_t tc_ahead(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const void* dy, const float* dh,
-                     const float* ckpt_angle, const TcAhead& a);
+                     const float* ckpt_angle, const TcAhead& a, bool full_angle, uint64_t* launches);
 
 cudaError_t tc_forward(cudaStream_t st, const TcFwdParams& p, bool rotational);
 // load_kernels of every kernel that a forward pass may launch.

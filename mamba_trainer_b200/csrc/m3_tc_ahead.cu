@@ -3,18 +3,22 @@
 // leaves SMs idle however long the sequence is (16 stripes of 14 tiles: 94 us on 16 of 148 SMs).  Two short launches
 // come first here:
 //   k_group_state  per group of tiles, all groups of all stripes at once: what the group adds to the state,
-//                  X~^T diag(sw) B^ decayed to its end (backward, to the state's gradient: (exp(acum) dY~)^T C^ from its
+//                  (sw X~)^T B^ decayed to its end (backward, to the state's gradient: (exp(acum) dY~)^T C^ from its
 //                  start), its decay and its angle
 //   k_group_pass   sequential over groups, parallel over state elements: the state (and the angle) at every segment
 //                  boundary, in the place where the stripe kernels expect what the segment before handed over
 // after which the segments are independent.  The last segment's groups (backward: the first one's) are needed by nobody and
-// not worked out.  Operands are rounded to bf16, like the stripe kernels' own; accumulation and states are float32.
+// not worked out.  Operands are rounded to bf16 where the stripe kernels' are - x or dY with its weight, the rotated B or C;
+// accumulation and states are float32.  (B is rotated by the angle since the group's start, unless a backward pass will
+// follow: k_group_angle.)
 //
 // k_group_state walks its group in half tiles (64 rows) with the rows of the next one in registers, the sum in registers
 // too, and leaves one state per group.  Its products are warp-level (mma.sync on bf16, operands by ldmatrix): a half tile
 // has one product of 1 MFLOP between two conversions, which is what it spends its time on.  An earlier form, a block per
 // half tile in TF32 with nothing requested ahead, took as long per tile as the whole forward kernel and a state per half
 // tile through memory: prefill of 1777 tokens, 16 heads: 25 + 12 us -> 14 + 9 us.
+#include <cuda_fp16.h>
+
 #include "m3_rows.cuh"
 #include "m3_tc.h"
 #include "m3_tc_common.cuh"
@@ -200,7 +204,38 @@ struct HalfAngles {
   }
 };
 
-template <int R, bool ROT, bool BWD>
+// FULL_ANGLE forward pass (one whose backward pass will follow): every group's angle ahead of k_group_state, so that B^ is
+// rotated by the angle since the start of the sequence and rounded as the stripe kernel's is.  A d theta sums the d phi of all
+// later steps, where the two sides of every pair of steps cancel - if both see the same B^ and C^: with B rotated by the angle
+// since the group's start, and rounded there, d theta was up to a third further from 64-bit results than that of whole stripes.
+// One launch of a few us; the pass then has nothing to rotate.
+template <int R>
+__global__ void __launch_bounds__(kThreads) k_group_angle(Dims d, m3_scan_desc in, TcAhead a, int tiles) {
+  __shared__ float2 part[8][32];
+  constexpr int LT = 2 * kRows / R;   // steps of a tile
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int bh = blockIdx.y, b = bh / d.H, h = bh - b * d.H;
+  const int seg = (int)blockIdx.x / a.gps, k0 = seg * a.tps + ((int)blockIdx.x % a.gps) * a.gt;
+  const int k1 = min(min(k0 + a.gt, (seg + 1) * a.tps), tiles), t1 = min(k1 * LT, d.T);
+  float2 s = make_float2(0.0f, 0.0f);
+#pragma unroll 4
+  for (int t = k0 * LT + warp; t < t1; t += 8) {
+    const float dt = ldf(static_cast<const __nv_bfloat16*>(in.dt), tok_index(d, b, t, h));
+    const uint32_t th = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const __nv_bfloat16*>(in.theta) + theta_index(d, b, t, h)) + lane);
+    s.x = fmaf(dt, bf16_lo(th), s.x);
+    s.y = fmaf(dt, bf16_hi(th), s.y);
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) { s.x += part[w][lane].x; s.y += part[w][lane].y; }
+    *reinterpret_cast<float2*>(a.asum + ((size_t)bh * gridDim.x + blockIdx.x) * kNH + 2 * lane) =
+        make_float2(wrap_angle(s.x), wrap_angle(s.y));
+  }
+}
+
+template <int R, bool ROT, bool BWD, bool FULL_ANGLE>
 __global__ void __launch_bounds__(kThreads, 2) k_group_state(Dims d, m3_scan_desc in, const __nv_bfloat16* __restrict__ dy,
                                                              const float* __restrict__ ckpt_angle, TcAhead a, int tiles) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -241,9 +276,26 @@ __global__ void __launch_bounds__(kThreads, 2) k_group_state(Dims d, m3_scan_des
   if (warp == 0) hl.load(in, d, b, h, (j0 + 2) * LT);
   if (ROT) {
     ha.load(theta, d, b, h, j0 * LT);
-    if (tid < 32)
+    if constexpr (FULL_ANGLE) {   // the angles of the groups before this one, a warp every eighth
+      const float* as = a.asum + (size_t)bh * gridDim.x * kNH + 2 * lane;
+      float2 v = make_float2(0.0f, 0.0f);
+      if (warp == 0 && in.angle0) v = make_float2(in.angle0[(size_t)bh * kNH + 2 * lane], in.angle0[(size_t)bh * kNH + 2 * lane + 1]);
+#pragma unroll 4
+      for (int g = warp; g < (int)blockIdx.x; g += 8) {
+        const float2 w = *reinterpret_cast<const float2*>(as + (size_t)g * kNH);
+        v = make_float2(wrap_angle(v.x + w.x), wrap_angle(v.y + w.y));
+      }
+      sm.q[warp * 32 + lane] = v;
+      __syncthreads();
+      if (warp == 0) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) v = make_float2(v.x + sm.q[w * 32 + lane].x, v.y + sm.q[w * 32 + lane].y);
+        sm.carry[0][lane] = make_float2(wrap_angle(v.x), wrap_angle(v.y));
+      }
+    } else if (tid < 32) {
       sm.carry[0][tid] = BWD && j0 < j1 ? *reinterpret_cast<const float2*>(ckpt_angle + ((size_t)bh * tiles + k0) * kNH + 2 * tid)
                                         : make_float2(0.0f, 0.0f);
+    }
   }
   __syncthreads();
   if (ROT) {
@@ -271,14 +323,22 @@ __global__ void __launch_bounds__(kThreads, 2) k_group_state(Dims d, m3_scan_des
       const float sc = s.scale[it.l] * before;
       float cs[IT::CW], sn[IT::CW];
 #pragma unroll
-      for (int c = 0; c < IT::CW; ++c) { cs[c] = sc; sn[c] = 0.0f; }
+      for (int c = 0; c < IT::CW; ++c) { cs[c] = 1.0f; sn[c] = 0.0f; }
       if (ROT) {
 #pragma unroll
         for (int c = 0; c < IT::CW; c += 4) {
           const float4 v = *reinterpret_cast<const float4*>(sm.phi + it.l * kNH + it.col + c);
           const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-          for (int k = 0; k < 4; ++k) { cs[c + k] = sc * __cosf(f[k]); sn[c + k] = sc * __sinf(f[k]); }
+          for (int k = 0; k < 4; ++k) {
+            cs[c + k] = __cosf(f[k]);
+            sn[c + k] = __sinf(f[k]);
+            if (BWD || FULL_ANGLE) {   // as in the stripe kernel's table, so that C^ (B^) is the one it has
+              const float2 h = __half22float2(__floats2half2_rn(cs[c + k], sn[c + k]));
+              cs[c + k] = h.x;
+              sn[c + k] = h.y;
+            }
+          }
         }
       }
 #pragma unroll
@@ -287,9 +347,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_group_state(Dims d, m3_scan_des
 #pragma unroll
         for (int c = 0; c < IT::CW; ++c) {
           const float v1 = item_el<R>(r1[i], c, r), v2 = item_el<R>(r2[i], c, r);
-          o1[c] = ROT ? v1 * cs[c] + v2 * sn[c] : v1 * sc;
-          o2[c] = ROT ? v2 * cs[c] - v1 * sn[c] : v2 * sc;
-          ox[c] = item_el<R>(xr[i], c, r);
+          o1[c] = ROT ? v1 * cs[c] + v2 * sn[c] : v1;
+          o2[c] = ROT ? v2 * cs[c] - v1 * sn[c] : v2;
+          ox[c] = item_el<R>(xr[i], c, r) * sc;
         }
         put<R, kN>(sm.b, it.l * R + r, it.col, o1);
         put<R, kN>(sm.b, it.l * R + r, it.col + kNH, o2);
@@ -340,13 +400,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_group_state(Dims d, m3_scan_des
     for (int e = 0; e < 4; e += 2)
       *reinterpret_cast<float2*>(dst + rows::at<kN>(p0 + g + 4 * e, n0 + 8 * t + 2 * q)) = make_float2(acc[t][e], acc[t][e + 1]);
   if (tid == 0) a.cd[slot] = total;
-  if (ROT && !BWD && tid < 32)
+  if (ROT && !BWD && !FULL_ANGLE && tid < 32)
     *reinterpret_cast<float2*>(a.asum + slot * kNH + 2 * tid) = j0 < j1 ? sm.carry[(j1 - j0) & 1][tid] : make_float2(0.0f, 0.0f);
 }
 
 // A thread owns planes (m, m + 64) of rows p, p + 32 and walks the groups in time (backward: against it); U of them are
 // requested before the first is used.  seg_state / seg_angle of segment s: what leaves it towards the next one walked.
-template <bool ROT, bool BWD>
+// ROT: the groups have angles; LOCAL: their states are those of B rotated by the angle since the group's start.
+template <bool ROT, bool BWD, bool LOCAL>
 __global__ void __launch_bounds__(256) k_group_pass(Dims d, m3_scan_desc in, const float* __restrict__ dh, TcAhead a, int count) {
   using T = __nv_bfloat16;
   constexpr int U = 8;
@@ -387,15 +448,15 @@ __global__ void __launch_bounds__(256) k_group_pass(Dims d, m3_scan_desc in, con
       const int k = BWD ? count - 1 - (i0 + u) : i0 + u;
       float sn = 0.0f, cs = 1.0f;
       if (ROT && !BWD) {
-        sincosf(ang, &sn, &cs);
+        if (LOCAL) sincosf(ang, &sn, &cs);
         ang = wrap_angle(ang + da[u]);
       }
       const float ec = exp_decay(e[u]);
 #pragma unroll
       for (int j = 0; j < 4; j += 2) {
         const float s1 = s[u][j], s2 = s[u][j + 1];
-        carry[j] = fmaf(ec, carry[j], ROT && !BWD ? s1 * cs + s2 * sn : s1);
-        carry[j + 1] = fmaf(ec, carry[j + 1], ROT && !BWD ? s2 * cs - s1 * sn : s2);
+        carry[j] = fmaf(ec, carry[j], LOCAL ? s1 * cs + s2 * sn : s1);
+        carry[j + 1] = fmaf(ec, carry[j + 1], LOCAL ? s2 * cs - s1 * sn : s2);
       }
       if (BWD ? k % a.gps == 0 : (k + 1) % a.gps == 0) {
         const size_t seg = (size_t)bh * a.nseg + k / a.gps + (BWD ? 1 : 0);
@@ -407,16 +468,17 @@ __global__ void __launch_bounds__(256) k_group_pass(Dims d, m3_scan_desc in, con
   }
 }
 
-template <int R, bool ROT, bool BWD>
+template <int R, bool ROT, bool BWD, bool FULL_ANGLE>
 cudaError_t ahead_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const void* dy, const float* dh, const float* ckpt_angle,
                     const TcAhead& a) {
-  auto kern = k_group_state<R, ROT, BWD>;
+  auto kern = k_group_state<R, ROT, BWD, FULL_ANGLE>;
   const int count = (a.nseg - 1) * a.gps;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmem<R>));
   if (e != cudaSuccess) return e;
+  if (FULL_ANGLE) k_group_angle<R><<<dim3(count, d.B * d.H), kThreads, 0, st>>>(d, in, a, tc_tiles(d.T, R));
   kern<<<dim3(count, d.B * d.H), kThreads, sizeof(GroupSmem<R>), st>>>(d, in, static_cast<const __nv_bfloat16*>(dy), ckpt_angle, a,
                                                                        tc_tiles(d.T, R));
-  k_group_pass<ROT, BWD><<<dim3(32 * kNH / 256, d.B * d.H), 256, 0, st>>>(d, in, dh, a, count);
+  k_group_pass<ROT, BWD, ROT && !BWD && !FULL_ANGLE><<<dim3(32 * kNH / 256, d.B * d.H), 256, 0, st>>>(d, in, dh, a, count);
   return cudaGetLastError();
 }
 
@@ -424,10 +486,10 @@ cudaError_t ahead_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, cons
 
 template <int R>
 static cudaError_t load_r() {
-  return load_kernels(k_group_state<R, true, false>, k_group_state<R, false, false>);
+  return load_kernels(k_group_state<R, true, false, false>, k_group_state<R, false, false, false>);
 }
 cudaError_t tc_ahead_load() {
-  cudaError_t e = load_kernels(k_group_pass<true, false>, k_group_pass<false, false>);
+  cudaError_t e = load_kernels(k_group_pass<true, false, true>, k_group_pass<false, false, false>);
   for (cudaError_t (*f)() : {load_r<1>, load_r<2>, load_r<4>})
     if (e == cudaSuccess) e = f();
   return e;
@@ -486,10 +548,14 @@ size_t tc_ahead_bytes(int BH, TcAhead* a, char* base) {
 }
 
 cudaError_t tc_ahead(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const void* dy, const float* dh,
-                     const float* ckpt_angle, const TcAhead& a) {
+                     const float* ckpt_angle, const TcAhead& a, bool full_angle, uint64_t* launches) {
+  const bool known = full_angle && d.rot && !dy;
+  *launches += known ? 3 : 2;
   auto go = [&](auto r, auto rot) {
-    return dy ? ahead_t<r.value, rot.value, true>(st, d, in, dy, dh, ckpt_angle, a)
-              : ahead_t<r.value, rot.value, false>(st, d, in, nullptr, nullptr, nullptr, a);
+    if (dy) return ahead_t<r.value, rot.value, true, false>(st, d, in, dy, dh, ckpt_angle, a);
+    if constexpr (rot.value)
+      if (known) return ahead_t<r.value, true, false, true>(st, d, in, nullptr, nullptr, nullptr, a);
+    return ahead_t<r.value, rot.value, false, false>(st, d, in, nullptr, nullptr, nullptr, a);
   };
   auto with_rot = [&](auto r) { return d.rot ? go(r, std::true_type{}) : go(r, std::false_type{}); };
   switch (d.R) {

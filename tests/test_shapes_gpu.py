@@ -284,6 +284,34 @@ def test_side_by_side_segments_match_the_oracle(B, H, R, rot, T, state, rev):
     compare_all(t, 64, check, True, ds, path=2, reverse_heads=rev)
 
 
+@pytest.mark.parametrize("T,H,R,copies", [(1670, 4, 1, 40), (1072, 6, 2, 27)])
+def test_cut_stripes_lose_no_accuracy(T, H, R, copies):
+    """Few stripes, cut into segments, against the same stripes among copies of themselves, which run whole: d theta, where
+    the two sides of every pair of steps have to cancel, is as close to the float64 oracle (1.08: what the segments' own
+    float32 sums may move)."""
+    from _util import fused_run, oracle_run
+    from mamba_trainer_b200 import synthetic
+    from mamba_trainer_b200.ssm import Context
+    w = synthetic.Workload("cut", 1, T, H, 64, 128, 64, R, torch.bfloat16, Discretization.LearnedTrapezoid, True,
+                           "rms" if R == 1 else "scaled")
+    ctx = Context.for_device(torch.device("cuda"))
+
+    def run(v):
+        before = ctx.lib.m3_launch_count(ctx.handle)
+        _, _, g = fused_run(v, 64, False, path=2)
+        return g["theta"], ctx.lib.m3_launch_count(ctx.handle) - before
+    errors = []
+    for seed in range(3):
+        t = synthetic.make_inputs(w, seed=seed)
+        _, _, exact = oracle_run(t, 64, False)
+        many = {k: v.repeat(copies, *[1] * (v.dim() - 1)) if v.dim() >= 3 else v for k, v in t.items() if v is not None}
+        (cut, n_cut), (whole, n_whole) = run(t), run(many)
+        assert n_cut > n_whole, (n_cut, n_whole)
+        errors.append((norm_rel(cut.float(), exact["theta"]), norm_rel(whole[:1].float(), exact["theta"])))
+    a, e = (sum(v) for v in zip(*errors))
+    assert a <= 1.08 * e, errors
+
+
 @pytest.mark.parametrize("T,H,R", [(8200, 2, 1), (9001, 3, 2)])
 def test_long_cut_stripes_match_the_oracle(T, H, R):
     """Stripes of some hundred tiles cut into segments, inputs as models have them.  d theta, a difference of sums over the
