@@ -9,7 +9,7 @@
 // and walks a run of time steps with the taps' window in registers and the rows of the next four steps already
 // requested; the norm's row sums are shuffles.  The warps of a block are neighbours in time (and, for ranks 2 and 4, the
 // ranks of one group, whose results are interleaved through shared memory on their way out).
-// bf16, 8 x 2048 tokens, 12 heads, d_state 128: forward 184 -> 100 us, backward 343 -> 270 us.
+// bf16, 8 x 2048 tokens, 12 heads, d_state 128, device time: forward 184 -> 69 us, backward 343 -> 174 us (and 12 us of sums).
 #include <cuda_bf16.h>
 
 #include <type_traits>

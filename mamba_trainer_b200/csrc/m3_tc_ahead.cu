@@ -1,7 +1,7 @@
 // States at segment boundaries, ahead of the tensor-core stripe kernels: what lets the segments of ONE stripe run side by
 // side.  The stripe kernels keep the state in TMEM and walk a stripe tile by tile, so a launch of fewer stripes than SMs
 // leaves SMs idle however long the sequence is (16 stripes of 14 tiles: 94 us on 16 of 148 SMs).  Two short launches
-// come first here:
+// come first here (three in a training step with rotation: k_group_angle):
 //   k_group_state  per group of tiles, all groups of all stripes at once: what the group adds to the state,
 //                  (sw X~)^T B^ decayed to its end (backward, to the state's gradient: (exp(acum) dY~)^T C^ from its
 //                  start), its decay and its angle
@@ -207,8 +207,10 @@ struct HalfAngles {
 // FULL_ANGLE forward pass (one whose backward pass will follow): every group's angle ahead of k_group_state, so that B^ is
 // rotated by the angle since the start of the sequence and rounded as the stripe kernel's is.  A d theta sums the d phi of all
 // later steps, where the two sides of every pair of steps cancel - if both see the same B^ and C^: with B rotated by the angle
-// since the group's start, and rounded there, d theta was up to a third further from 64-bit results than that of whole stripes.
-// One launch of a few us; the pass then has nothing to rotate.
+// since the group's start, rounded there, and the weights rounded with it, d theta was 1.4 to 1.5 times as far from 64-bit
+// results as that of whole stripes (4 stripes of 1670 steps, rank 1; 6 of 1072, rank 2); it is at most 1.07 times now.  One
+// launch of 4 us (forward + backward of a 2 x 509-token mixer, 8 heads, rank 2: 168.6 -> 173.1 us); the pass then has nothing
+// to rotate.
 template <int R>
 __global__ void __launch_bounds__(kThreads) k_group_angle(Dims d, m3_scan_desc in, TcAhead a, int tiles) {
   __shared__ float2 part[8][32];
