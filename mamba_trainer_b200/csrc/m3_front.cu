@@ -52,7 +52,8 @@ struct Four<__nv_bfloat16> {
   __device__ __forceinline__ void store(__nv_bfloat16* p) const { *reinterpret_cast<uint2*>(p) = v; }
 };
 
-// Two floats per instruction (packed fp32): these kernels are bound by instruction issue.
+// Two floats per instruction (packed fp32): of all resources these kernels use instruction issue most (64 % of the slots
+// forward, 47 % backward, where the chains of a step take the rest; DRAM 38 and 26 %).
 __device__ __forceinline__ void mul4(const float (&a)[4], const float (&b)[4], float (&c)[4]) {
   const float2 lo = __fmul2_rn(make_float2(a[0], a[1]), make_float2(b[0], b[1]));
   const float2 hi = __fmul2_rn(make_float2(a[2], a[3]), make_float2(b[2], b[3]));
