@@ -33,12 +33,53 @@ namespace {
 
 constexpr uint32_t OFF_C = 0, OFF_B = 32768, OFF_X = 65536, OFF_DY = 81920, OFF_XW = 98304, OFF_DYE = 114688,
                    OFF_M = 131072, OFF_DG = 163840, OFF_HS = 196608, OFF_SC = 212992;
-constexpr int kScalFloats = 2 * kNumScal * kScal + 256 * 4 + 512 + 256 + 132 + 132 + 16 + 64 + 256;
+constexpr int kScalFloats = 2 * kNumScal * kScal + 256 * 4 + 512 + 132 + 132 + 16 + 64 + 512;
 static_assert(OFF_SC + kScalFloats * 4 + 64 <= 232448, "backward shared memory exceeds the 227 KB a CTA can have");
 constexpr uint32_t kSmemBytes = OFF_SC + kScalFloats * 4 + 64;
 constexpr uint32_t TM_G = 0, TM_DM = 128, TM_T1 = 256, TM_DH = 384, TM_TAB = 448, TM_COLS = 512;
 // phase B reuse: dB^ accumulates over G's columns, dX~ and U over dM's.
 constexpr uint32_t TM_DB = 0, TM_DX = 128, TM_U = 192;
+
+// The gradient through last_u = sum_r x (x) B^ at the final token, added to accumulators in TMEM before their epilogue reads
+// them: out of line (whole warps), as few calls have one and the epilogues' code is what instruction fetch pays for.
+// `mine`: this thread's row is one of the final token's.  d x (columns from col0): += dlu B^.
+__device__ __noinline__ void add_dlu_x(uint32_t addr, const float* dlu, const uint8_t* sB, int row, bool mine) {
+  float v[16], s[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) s[j] = 0.0f;
+  if (mine) {
+#pragma unroll 1
+    for (int n = 0; n < kN; ++n) {
+      const float bv = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sB + tile_off(row, n, kN)));
+#pragma unroll
+      for (int j = 0; j < 16; ++j) s[j] += dlu[(size_t)j * kN + n] * bv;
+    }
+  }
+  tmem_ld16(addr, v);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] += s[j];
+  tmem_st16(addr, v);
+  tmem_wait_st();
+}
+// d B^: += dlu^T x.
+__device__ __noinline__ void add_dlu_b(uint32_t addr, const float* dlu, const uint8_t* sX, int row, bool mine) {
+  float v[16], s[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) s[j] = 0.0f;
+  if (mine) {
+#pragma unroll 1
+    for (int pp = 0; pp < kP; ++pp) {
+      const float xv = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sX + tile_off(row, pp, kP)));
+#pragma unroll
+      for (int j = 0; j < 16; ++j) s[j] += dlu[(size_t)pp * kN + j] * xv;
+    }
+  }
+  tmem_ld16(addr, v);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] += s[j];
+  tmem_st16(addr, v);
+  tmem_wait_st();
+}
 
 // MODE as in m3_tc_fwd.cu.
 template <int R, bool ROT, int MODE>
@@ -65,15 +106,14 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
   float* part_q = part_t1 + 256;      // [2][128]
   float* part_dg = part_q + 256;      // [2][128]
   float* part_col = part_dg + 256;    // [4][128]
-  float* part_rot = part_col + 512;   // [2][128]
-  float* s_dacum = part_rot + 256;    // [132]
+  float* s_dacum = part_col + 512;    // [132]
   float* s_dast = s_dacum + 132;      // [132]
-  float* s_red = s_dast + 132;        // [16]
+  float* s_red = s_dast + 132;        // [16] the warps' shares of <dH, H_k> and of d D (and epi_sum's scratch)
   float* s_dcar = s_red + 16;         // [64] sum of d phi over later tiles
-  float* s_q = s_dcar + 64;           // [4][64]
+  float* s_q = s_dcar + 64;           // [8][64]
   // [0]: phase A; [1]: the first three products of phase B, [4]: the rest of it; [2]: arrival of a tile's raw
   // rows; [3]: of its state checkpoint
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_q + 256);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_q + 512);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
   int* s_ok = reinterpret_cast<int*>(tmem_slot + 1);  // outcome of a hand-over wait, for the epilogue warps
 
@@ -521,8 +561,9 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
       fence_async_smem();
       tc_fence_before();
       epi_signal(BAR_MID, kPairCount, dead);
-      // (the sum behind d cd is wanted by the tile's last step only: it is taken while phase B runs)
-      const float dcd = ecd * inside(cd) * epi_sum(dcd_part, s_red);
+      // (the sum behind d cd is wanted by the tile's last step only: the warps' shares wait for it)
+      dcd_part = warp_sum(dcd_part);
+      if (lane == 0) s_red[warp] = dcd_part;
       // ---- 4. epilogue B -------------------------------------------------------------------------
       if (!dead) dead = !warp_all(mbar_wait(&bars[1], it & 1, wait_limit));
       const int t = t0 + rl;
@@ -537,6 +578,11 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
       for (int j = 0; j < 32; ++j) dphi[j] = 0.0f;
       if (!dead) {
         tc_fence_after();
+        if (last_tile && p.dlu) {
+#pragma unroll 1
+          for (int cc = 0; cc < 2; ++cc)
+            add_dlu_x(tmem_addr(tm, quad * 32, TM_DX + 32 * ch + 16 * cc), p.dlu + ((size_t)bh * kP + 32 * ch + 16 * cc) * kN, sB, row, at_end);
+        }
         float acc[2][16], u[2][16];
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
@@ -567,20 +613,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
               const float2 a2 = __ffma2_rn(sw2, u2, __ffma2_rn(dsk2, dy2, make_float2(acc[cc][j], acc[cc][j + 1])));
               acc[cc][j] = a2.x; acc[cc][j + 1] = a2.y;
             }
-            if (at_end && p.dlu) {  // gradient through last_u = sum_r x (x) B^ at the final token
-#pragma unroll 1
-              for (int j = 0; j < 16; ++j) {
-                const float* gl = p.dlu + ((size_t)bh * kP + p0 + j) * kN;
-                float s_ = 0.0f;
-                for (int n = 0; n < kN; ++n)
-                  s_ += gl[n] * __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sB + tile_off(row, n, kN)));
-                float add[16];
-#pragma unroll
-                for (int jj = 0; jj < 16; ++jj) add[jj] = (jj == j) ? s_ : 0.0f;
-#pragma unroll
-                for (int jj = 0; jj < 16; ++jj) acc[cc][jj] += add[jj];
-              }
-            }
             if constexpr (R != 2) stage_out16<R>(sHS, row, p0, acc[cc], rev);  // dS is spent: its buffer stages dx
           }
           if constexpr (R == 2) stage_out32<R>(sHS, row, 32 * ch, acc[0], acc[1], rev);  // rank 2: both halves at once
@@ -591,6 +623,11 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
       if (!dead) dead = !warp_all(mbar_wait(&bars[4], it & 1, wait_limit));  // the other four products
       if (!dead) {
         tc_fence_after();
+        if (last_tile && p.dlu) {
+#pragma unroll 1
+          for (int q4 = 0; q4 < 4; ++q4)
+            add_dlu_b(tmem_addr(tm, quad * 32, TM_DB + gcol(q4)), p.dlu + (size_t)bh * kP * kN + gcol(q4), sX, row, at_end);
+        }
         // dB^ (TM_DB, operand sB, out db), then dC^ (TM_T1, operand sC, out dc).  As two copies of this body rank 4 spilled
         // some 300 bytes a thread; as a loop 12, and its second pass finds its code in the instruction caches (cfg3 forward
         // + backward 9.32 -> 8.95 ms).  The lower ranks, which spill less, lose 1 to 3 % as a loop.
@@ -612,22 +649,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) tmem_ld_fence(g[q4]);
           if (ROT) { tmem_ld_fence(tabv[0]); tmem_ld_fence(tabv[1]); }
-          if (is_b && at_end && p.dlu) {  // d last_u reaches B^ of the final token: += dlu^T x
-#pragma unroll 1
-            for (int q4 = 0; q4 < 4; ++q4)
-#pragma unroll 1
-              for (int j = 0; j < 16; ++j) {
-                const int n = gcol(q4) + j;
-                float s_ = 0.0f;
-                for (int pp = 0; pp < kP; ++pp)
-                  s_ += p.dlu[((size_t)bh * kP + pp) * kN + n] *
-                        __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sX + tile_off(row, pp, kP)));
-#pragma unroll
-                for (int a4 = 0; a4 < 4; ++a4)
-#pragma unroll
-                  for (int jj = 0; jj < 16; ++jj) g[a4][jj] += (a4 == q4 && jj == j) ? s_ : 0.0f;
-              }
-          }
           if (ROT) {
 #pragma unroll
             for (int mc = 0; mc < 2; ++mc) {
@@ -640,13 +661,16 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
               load_chunk(sop, tile_off(row, kNH + m0, kN), *reinterpret_cast<float(*)[8]>(&o2[0]));
               load_chunk(sop, tile_off(row, kNH + m0 + 8, kN), *reinterpret_cast<float(*)[8]>(&o2[8]));
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                dphi[16 * mc + j] += g1[j] * o2[j] - g2[j] * o1[j];
-                const uint32_t cw = __float_as_uint(tabv[mc][j]);
-                const float2 csn = __half22float2(*reinterpret_cast<const __half2*>(&cw));
-                const float cs = csn.x, sn = csn.y;
-                const float u1 = g1[j] * cs - g2[j] * sn, u2 = g1[j] * sn + g2[j] * cs;
-                g1[j] = u1; g2[j] = u2;
+              for (int j = 0; j < 16; j += 2) {   // packed fp32 pairs
+                const float2 a = make_float2(g1[j], g1[j + 1]), b = make_float2(g2[j], g2[j + 1]), nb = make_float2(-b.x, -b.y);
+                const float2 d2 = __ffma2_rn(nb, make_float2(o1[j], o1[j + 1]),
+                                             __ffma2_rn(a, make_float2(o2[j], o2[j + 1]), make_float2(dphi[16 * mc + j], dphi[16 * mc + j + 1])));
+                dphi[16 * mc + j] = d2.x; dphi[16 * mc + j + 1] = d2.y;
+                const uint32_t w0 = __float_as_uint(tabv[mc][j]), w1 = __float_as_uint(tabv[mc][j + 1]);
+                const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w0)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&w1));
+                const float2 cs = make_float2(f0.x, f1.x), sn = make_float2(f0.y, f1.y);
+                const float2 u1 = __ffma2_rn(a, cs, __fmul2_rn(nb, sn)), u2 = __ffma2_rn(b, cs, __fmul2_rn(a, sn));
+                g1[j] = u1.x; g1[j + 1] = u1.y; g2[j] = u2.x; g2[j + 1] = u2.y;
               }
             }
           }
@@ -682,102 +706,80 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
           for (int o = 1; o < R; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
           dphi[j] = v;
         }
-        // Ranks 1 and 4 store four planes (16 bytes) at a time - the buffer's swizzle moves whole 16-byte pieces -
-        // and keep the scan's running sums in registers; on rank 2 both measured slower (backward + 1.8 % on the
-        // scaling workload: the kernel's timing follows its code layout more than its instruction count), so
-        // rank 2 keeps the plane-by-plane stores and the second pass over shared memory.
-        if constexpr (R == 2) {
-          if (rr == 0) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              float v = live ? dphi[j] : 0.0f;
-              if (at_end && p.dangle) v += p.dangle[(size_t)bh * kNH + 32 * ch + j];
-              sDphi[phi_idx(rl, 32 * ch + j)] = v;
-            }
-          }
-        } else if (rr == 0) {
+        if (rr == 0) {   // four planes (16 bytes) at a time: the buffer's swizzle moves whole 16-byte pieces
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
             float v[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              v[c] = live ? dphi[j + c] : 0.0f;
-              if (at_end && p.dangle) v[c] += p.dangle[(size_t)bh * kNH + 32 * ch + j + c];
-            }
+            for (int c = 0; c < 4; ++c) v[c] = live ? dphi[j + c] : 0.0f;
             *reinterpret_cast<float4*>(&sDphi[phi_idx(rl, 32 * ch + j)]) = make_float4(v[0], v[1], v[2], v[3]);
           }
         }
+        if (last_tile && p.dangle && at_end && rr == 0) {   // the gradient reaching the returned angle
+#pragma unroll 1
+          for (int j = 0; j < 32; ++j) sDphi[phi_idx(rl, 32 * ch + j)] += p.dangle[(size_t)bh * kNH + 32 * ch + j];
+        }
       }
-      const float dD_tile = epi_sum(dD_part, s_red);  // also orders part_* and sDphi for what follows
-      if (tid == 0) p.partD[(size_t)bh * ntiles + k] = dD_tile;
+      dD_part = warp_sum(dD_part);
+      if (lane == 0) s_red[8 + warp] = dD_part;
+      // theta and d theta of scan step t0 + l (they may be column bands of a wider row): warp o = the o-th eighth of the
+      // steps, lane m2 = planes 2 m2 and 2 m2 + 1, requested ahead of the barrier
+      constexpr int LO = LT / 8;
+      const ptrdiff_t th_step = rev ? -(ptrdiff_t)p.ths : (ptrdiff_t)p.ths;
+      const ptrdiff_t th0 = (ptrdiff_t)((size_t)b * T + (rev ? T - 1 - t0 : t0)) * p.ths + (ptrdiff_t)h * kNH + warp * LO * th_step + 2 * lane;
+      uint32_t thw[ROT && !AHEAD ? LO : 1];
+      if (ROT && !AHEAD) {
+#pragma unroll
+        for (int i = 0; i < LO; ++i)
+          thw[i] = t0 + warp * LO + i < T ? __ldg(reinterpret_cast<const uint32_t*>(p.theta + th0 + i * th_step)) : 0u;
+      }
+      epi_sync();  // part_* and sDphi are complete
       // ---- 5. reverse cumulative sum of d phi over time -> d theta, and the dt term -----------------
       if (ROT) {
-        constexpr int LQ = LT / 4, NV = 4 / R;  // NV: (time step, 8-plane group) items per thread
-        const int q = tid >> 6, m = tid & 63;
-        // theta and d theta of scan step t0 + l (they may be column bands of a wider row)
-        const ptrdiff_t th_step = rev ? -(ptrdiff_t)p.ths : (ptrdiff_t)p.ths;
-        const ptrdiff_t th0 = (ptrdiff_t)((size_t)b * T + (rev ? T - 1 - t0 : t0)) * p.ths + (ptrdiff_t)h * kNH;
-        uint4 thq[NV];  // theta of this thread's items of the vector pass below, requested early
+        float2 loc[LO], run = make_float2(0.0f, 0.0f);
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          const int iv = tid + 256 * i, l = iv >> 3, mg = iv & 7;
-          thq[i] = (t0 + l < T) ? __ldg(reinterpret_cast<const uint4*>(p.theta + th0 + l * th_step + mg * 8))
-                                : make_uint4(0u, 0u, 0u, 0u);
+        for (int i = LO - 1; i >= 0; --i) {
+          const float2 v = *reinterpret_cast<const float2*>(&sDphi[phi_idx(warp * LO + i, 2 * lane)]);
+          run.x += v.x;
+          run.y += v.y;
+          loc[i] = run;
         }
-        float run = 0.0f, loc[R == 2 ? 1 : LQ];  // (not rank 2:) the quarter's running sums wait in registers
-#pragma unroll
-        for (int i = LQ - 1; i >= 0; --i) {
-          run += sDphi[phi_idx(q * LQ + i, m)];
-          if constexpr (R == 2) sDphi[phi_idx(q * LQ + i, m)] = run;
-          else loc[i] = run;
-        }
-        s_q[q * 64 + m] = run;
+        float2* q2 = reinterpret_cast<float2*>(s_q);
+        q2[warp * 32 + lane] = run;
+        float2 off = *reinterpret_cast<const float2*>(&s_dcar[2 * lane]);
         epi_sync();
-        float off = s_dcar[m];
-        for (int qq = 3; qq > q; --qq) off += s_q[qq * 64 + m];
-#pragma unroll
-        for (int i = 0; i < LQ; ++i) {  // d step: sum of d phi from here on
-          if constexpr (R == 2) sDphi[phi_idx(q * LQ + i, m)] += off;
-          else sDphi[phi_idx(q * LQ + i, m)] = loc[i] + off;
+#pragma unroll 1
+        for (int j = 7; j > warp; --j) {
+          const float2 v = q2[j * 32 + lane];
+          off.x += v.x;
+          off.y += v.y;
         }
-        const float total = off + s_q[0 * 64 + m];  // for q == 0: carry + all four quarters
-        epi_sync();
-        if (q == 0) {
-          s_dcar[m] = total;
-          if (!AHEAD && k == 0 && p.dangle0) p.dangle0[(size_t)bh * kNH + m] = total;
+        if (warp == 0) {   // carry + all eight eighths (everyone has read the old carry)
+          const float2 total = make_float2(off.x + run.x, off.y + run.y);
+          *reinterpret_cast<float2*>(&s_dcar[2 * lane]) = total;
+          if (!AHEAD && k == 0 && p.dangle0) {
+            p.dangle0[(size_t)bh * kNH + 2 * lane] = total.x;
+            p.dangle0[(size_t)bh * kNH + 2 * lane + 1] = total.y;
+          }
         }
-        // vector pass: d theta = d step * dt (16-byte stores) and the rotation's share of d dt
+        // d step = sum of d phi from here on; d theta = d step * dt and the rotation's share of d dt
+        if constexpr (AHEAD) {   // later segments' share is not known yet
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          const int iv = tid + 256 * i, l = iv >> 3, mg = iv & 7;
-          const float4 d0 = *reinterpret_cast<const float4*>(&sDphi[phi_idx(l, mg * 8)]);
-          const float4 d1 = *reinterpret_cast<const float4*>(&sDphi[phi_idx(l, mg * 8 + 4)]);
-          if constexpr (AHEAD) {   // later segments' share is not known yet
-            float4* dst = reinterpret_cast<float4*>(p.dphi + ((size_t)bh * Tp + t0 + l) * kNH + mg * 8);
-            dst[0] = d0;
-            dst[1] = d1;
-            continue;
-          }
-          const float ds[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-          const uint32_t tw[4] = {thq[i].x, thq[i].y, thq[i].z, thq[i].w};
-          const float dtl = ts.dt[l];
-          float prod = 0.0f, o[8];
+          for (int i = 0; i < LO; ++i)
+            *reinterpret_cast<float2*>(p.dphi + ((size_t)bh * Tp + t0 + warp * LO + i) * kNH + 2 * lane) =
+                make_float2(loc[i].x + off.x, loc[i].y + off.y);
+        } else {
+          float prod[LO];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            prod += ds[2 * j] * bf16_lo(tw[j]) + ds[2 * j + 1] * bf16_hi(tw[j]);
-            o[2 * j] = ds[2 * j] * dtl;
-            o[2 * j + 1] = ds[2 * j + 1] * dtl;
+          for (int i = 0; i < LO; ++i) {
+            const float dx = loc[i].x + off.x, dy = loc[i].y + off.y, dtl = ts.dt[warp * LO + i];
+            prod[i] = fmaf(dx, bf16_lo(thw[i]), dy * bf16_hi(thw[i]));
+            if (t0 + warp * LO + i < T && p.dtheta)
+              *reinterpret_cast<uint32_t*>(p.dtheta + th0 + i * th_step) = pack_bf16(dx * dtl, dy * dtl);
           }
-          if (t0 + l < T && p.dtheta) {
-            uint4 qv;
-            qv.x = pack_bf16(o[0], o[1]); qv.y = pack_bf16(o[2], o[3]); qv.z = pack_bf16(o[4], o[5]); qv.w = pack_bf16(o[6], o[7]);
-            *reinterpret_cast<uint4*>(p.dtheta + th0 + l * th_step + mg * 8) = qv;
-          }
-#pragma unroll
-          for (int o_ = 1; o_ < 8; o_ <<= 1) prod += __shfl_xor_sync(0xffffffffu, prod, o_);
-          if (mg == 0) part_rot[l] = prod;
+          const float sum = warp_sums<LO>(prod);
+          if (lane % (32 / LO) == 0) p.ddt_rot[(size_t)bh * Tp + t0 + warp * LO + lane / (32 / LO)] = sum;
         }
-        epi_sync();
       }
       // ---- 6. per-token scalars of the tile ---------------------------------------------------------
       if (tid < LT) {
@@ -802,16 +804,16 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
         const size_t o = (size_t)bh * Tp + t0 + l;
         p.dw[o] = col + sg * q;
         p.dg[o] = dgv;
-        if (ROT && !AHEAD) p.ddt_rot[o] = part_rot[l];
       }
       epi_sync();
       if (warp == 0) {  // reverse inclusive scan of d acum (+ the chunk-decay terms on the last step)
         constexpr int EPL = LT / 32;
-        float tail = 0.0f;
+        float tail = 0.0f, dcd = 0.0f, dD = 0.0f;
         for (int i = lane; i < LT; i += 32) tail += s_dast[i];
+        tail = warp_sum(tail);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) tail += __shfl_xor_sync(0xffffffffu, tail, o);
-        tail += dcd;
+        for (int i = 0; i < 8; ++i) { dcd += s_red[i]; dD += s_red[8 + i]; }
+        tail += ecd * inside(cd) * dcd;
         float loc[EPL];
         float run = 0.0f;
 #pragma unroll
@@ -837,12 +839,15 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) pa += __shfl_xor_sync(0xffffffffu, pa, o);
-        if (lane == 0) p.partA[(size_t)bh * ntiles + k] = pa;
+        if (lane == 0) {
+          p.partA[(size_t)bh * ntiles + k] = pa;
+          p.partD[(size_t)bh * ntiles + k] = dD;
+        }
       }
       // this tile's scalars are spent: the look-ahead warp may overwrite their set
       if (it + 2 < total) epi_signal(bar_free(it), kPairCount, dead);
-      epi_sync();
       }
+      epi_sync();
       {
         // ---- the item's first tile is done: the gradient of the seed state, or the hand-over to the
         //      segment before this one ------------------------------------------------------------------

@@ -34,10 +34,10 @@ struct FwdSmem {
   static constexpr uint32_t kTheta = (kRows / R) * kNH * 2;                // raw theta rows, at the table's start
   static constexpr uint32_t kRaw = RawTile<R>::bytes(kN);                  // staged raw rows of B (and again of C)
   static constexpr uint32_t off_raw_b = OFF_TAB + kTab, off_raw_c = off_raw_b + kRaw, off_sc = off_raw_c + kRaw;
-  // two sets of per-token scalars, the angle pass's exchange space ([4][64] sums, [64] running angle),
+  // two sets of per-token scalars, the angle pass's exchange space ([8][64] sums, [64] running angle),
   // then mbarriers and the TMEM slot
   static constexpr uint32_t off_q = off_sc + 2 * kNumScal * kScal * 4;
-  static constexpr uint32_t bytes = off_q + (4 * kNH + kNH) * 4 + 64;   // bars, TMEM slot, hand-over outcome
+  static constexpr uint32_t bytes = off_q + (8 * kNH + kNH) * 4 + 64;   // bars, TMEM slot, hand-over outcome
   static_assert(bytes <= 232448, "forward shared memory exceeds the 227 KB a CTA can have");
 };
 constexpr uint32_t TM_G = 0, TM_Y = 128, TM_H = 192, TM_COLS = 256;
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_con
                        q + 7 * kScal, q + 8 * kScal};
   };
   float* s_q = reinterpret_cast<float*>(smem + SM::off_q);
-  float* s_carry = s_q + 4 * kNH;
+  float* s_carry = s_q + 8 * kNH;
   // [0], [1]: tensor-core phases; [2]: arrival of a tile's raw rows of B and C; [3]: of its theta rows
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_carry + kNH);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);

@@ -112,86 +112,76 @@ __device__ __forceinline__ void raise_handover(int* flag) {
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok); }
 
 // ---------------------------------------------------------------------------------------
-// Per-token scalars of one tile, by ONE warp (the arithmetic of tile_scalars): g, w (shifted add),
-// a = dt A, inclusive cumulative sum ac, sw = exp(cd - ac) w, eac = exp(ac), column factors cf.
-// Lane i owns the EPL consecutive steps i*EPL .. i*EPL + EPL - 1.
+// Per-token scalars of one tile, by ONE warp (the arithmetic of tile_scalars): g, w (shifted add), inclusive cumulative sum
+// ac of a = dt A, sw = exp(cd - ac) w, eac = exp(ac), column factors cf.  32 steps at a time, in loops that stay rolled:
+// the warp finds its code cold every tile and pays for its length (with the EPL steps of a lane unrolled it took up to
+// 24 K cycles of a 27 K cycle backward tile).
 // ---------------------------------------------------------------------------------------
 template <int R>
 struct ScalarLoads {
   static constexpr int EPL = (kRows / R) / 32;
-  float dt[EPL + 1], lam[EPL + 1];
+  float dt[EPL], lam[EPL], dt_next, lam_next;   // steps 32 i + lane; the step after the tile
 };
-// dt and lambda of the steps lane * EPL .. lane * EPL + EPL of the tile at t0 (one step of look-ahead),
-// requested a whole tile before they are used: the loads are few but each is a sector of its own.
+// dt and lambda of the tile at t0 and of one step beyond, requested a whole tile before they are used: the loads are few
+// but each is a sector of its own.
 template <int R>
 __device__ __forceinline__ void lookahead_load(ScalarLoads<R>& v, const __nv_bfloat16* dt, const __nv_bfloat16* lam,
                                                int disc, int b, int h, int H, int T, int t0, bool rev) {
   constexpr int EPL = ScalarLoads<R>::EPL;
   const int lane = threadIdx.x & 31;
+  const float lam0 = disc == 1 ? 0.5f : 1.0f;
 #pragma unroll
   for (int i = 0; i <= EPL; ++i) {
-    const int t = t0 + lane * EPL + i;
-    v.dt[i] = 0.0f;
-    v.lam[i] = 1.0f;
+    const int t = t0 + 32 * i + (i < EPL ? lane : 0);
+    float d = 0.0f, la = lam0;
     if (t < T) {
       const size_t idx = ((size_t)b * T + (rev ? T - 1 - t : t)) * H + h;
-      v.dt[i] = bf(dt, idx);
-      v.lam[i] = disc == 0 ? 1.0f : (disc == 1 ? 0.5f : bf(lam, idx));
+      d = bf(dt, idx);
+      if (disc > 1) la = bf(lam, idx);
     }
+    if (i < EPL) { v.dt[i] = d; v.lam[i] = la; } else { v.dt_next = d; v.lam_next = la; }
   }
 }
 template <int R>
 __device__ __forceinline__ void lookahead_scalars(const TileScalars& s, const ScalarLoads<R>& v, float A, int T, int t0) {
   constexpr int LT = kRows / R, EPL = LT / 32, SPC = 16 / R;
   const int lane = threadIdx.x & 31;
-  float loc[EPL], wv[EPL];
-  float run = 0.0f;
 #pragma unroll
-  for (int i = 0; i < EPL; ++i) {
-    const int l = lane * EPL + i, t = t0 + l;
-    float gv = 0.0f, w = 0.0f, av = 0.0f;
-    if (t < T) {
-      gv = v.lam[i] * v.dt[i];
-      const float f = (t + 1 < T) ? (1.0f - v.lam[i + 1]) * v.dt[i + 1] : 0.0f;
-      w = gv + f;
-      av = v.dt[i] * A;
+  for (int i = 0; i < EPL; ++i) { s.dt[32 * i + lane] = v.dt[i]; s.lam[32 * i + lane] = v.lam[i]; }
+  if (lane == 0) { s.dt[LT] = v.dt_next; s.lam[LT] = v.lam_next; }
+  __syncwarp();
+  float cd = 0.0f;
+#pragma unroll 1
+  for (int l = lane; l < LT; l += 32) {
+    const float d = s.dt[l], gv = s.lam[l] * d;   // (dt is zero from T on)
+    const float f = t0 + l + 1 < T ? (1.0f - s.lam[l + 1]) * s.dt[l + 1] : 0.0f;
+    float ac = d * A;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float n = __shfl_up_sync(0xffffffffu, ac, o);
+      if (lane >= o) ac += n;
     }
-    s.dt[l] = v.dt[i]; s.lam[l] = v.lam[i]; s.g[l] = gv; s.w[l] = w; s.a[l] = av;
-    wv[i] = w;
-    run += av;
-    loc[i] = run;
-  }
-  if (lane == 31) { s.dt[LT] = v.dt[EPL]; s.lam[LT] = v.lam[EPL]; }
-  float tot = run;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float n = __shfl_up_sync(0xffffffffu, tot, o);
-    if (lane >= o) tot += n;
-  }
-  const float base = tot - run;
-  const float cd = __shfl_sync(0xffffffffu, tot, 31);
-#pragma unroll
-  for (int i = 0; i < EPL; ++i) {
-    loc[i] += base;
-    s.ac[lane * EPL + i] = loc[i];
+    ac += cd;
+    s.g[l] = gv; s.w[l] = t0 + l < T ? gv + f : 0.0f; s.ac[l] = ac;
+    cd = __shfl_sync(0xffffffffu, ac, 31);
   }
   __syncwarp();
-#pragma unroll
-  for (int i = 0; i < EPL; ++i) {
-    const int l = lane * EPL + i;
-    s.sw[l] = expc(cd - loc[i]) * wv[i];
-    s.eac[l] = expc(loc[i]);
-    s.cf[l] = __expf(fmaxf(s.ac[(l / SPC) * SPC + SPC - 1] - loc[i], -87.0f));
+#pragma unroll 1
+  for (int l = lane; l < LT; l += 32) {
+    const float ac = s.ac[l];
+    s.sw[l] = expc(cd - ac) * s.w[l];
+    s.eac[l] = expc(ac);
+    s.cf[l] = __expf(fmaxf(s.ac[(l / SPC) * SPC + SPC - 1] - ac, -87.0f));
   }
 }
 
 // Wrapped cumulative angle of one tile as a table of half2(cos phi, sin phi) words, [LT][64] at
-// phi_idx(l, m), by the 256 threads of the epilogue warps: thread (q, m) owns plane m over the quarter q
-// of the tile's steps.  The tile's raw theta rows ([LT][64] bf16, landed by a bulk tensor copy; for a head
+// phi_idx(l, m), by the eight epilogue warps: warp o takes the o-th eighth of the tile's steps, lane m2 planes 2 m2 and
+// 2 m2 + 1.  The tile's raw theta rows ([LT][64] bf16, landed by a bulk tensor copy; for a head
 // that walks right to left in memory order, i.e. step l in row LT - 1 - l) sit at the start of the table's
 // own buffer and are consumed before any table word is written (one barrier separates the passes).
-// `carry_in` [64] holds the angle entering the tile (shared or global memory), `carry_out` (may be NULL,
-// may alias carry_in) receives the wrapped angle leaving it; `s_q` is [4][64] floats of exchange space; dt
+// `carry_in` [64] holds the angle entering the tile (shared or global memory, 8-byte aligned), `carry_out` (may be NULL,
+// may alias carry_in) receives the wrapped angle leaving it; `s_q` is [8][64] floats of exchange space; dt
 // comes from the tile's scalars.  sin / cos come from the
 // special-function unit (the argument is wrapped into [-pi, pi] first, where its error is far below the
 // half-precision table's).  Contains one barrier of the epilogue warps; the caller's next one publishes
@@ -200,46 +190,79 @@ template <int R>
 __device__ __forceinline__ void epi_angle_table(float* tab, float* s_q, const float* carry_in, float* carry_out,
                                                 const float* s_dt, int T, int t0, bool rev, float* ckpt_slot,
                                                 float* angle_out_bh) {
-  constexpr int LT = kRows / R, LQ = LT / 4;
-  const __nv_bfloat16* raw = reinterpret_cast<const __nv_bfloat16*>(tab);
-  const int tid = threadIdx.x, q = tid >> 6, m = tid & 63;
-  float loc[LQ];
-  float run = 0.0f;
+  constexpr int LT = kRows / R, LO = LT / 8;
+  const int o = threadIdx.x >> 5, m2 = threadIdx.x & 31;
+  const uint8_t* raw = reinterpret_cast<const uint8_t*>(tab) + (rev ? LT - 1 - o * LO : o * LO) * (kNH * 2) + m2 * 4;
+  const int step = rev ? -kNH * 2 : kNH * 2;
+  float2* q2 = reinterpret_cast<float2*>(s_q);
+  float2 loc[LO], run = make_float2(0.0f, 0.0f);
 #pragma unroll
-  for (int i = 0; i < LQ; ++i) {
-    const int l = q * LQ + i;
-    run = fmaf(s_dt[l], __bfloat162float(raw[(rev ? LT - 1 - l : l) * kNH + m]), run);
-    loc[i] = run;
+  for (int i = 0; i < LO; i += 4) {
+    const float4 d4 = *reinterpret_cast<const float4*>(s_dt + o * LO + i);
+    const float d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t th = *reinterpret_cast<const uint32_t*>(raw + (i + u) * step);
+      run.x = fmaf(d[u], bf16_lo(th), run.x);
+      run.y = fmaf(d[u], bf16_hi(th), run.y);
+      loc[i + u] = run;
+    }
   }
-  s_q[q * 64 + m] = run;
-  const float cin = carry_in[m];
-  if (ckpt_slot && q == 0) ckpt_slot[m] = cin;
+  q2[o * 32 + m2] = run;
+  float2 off = *reinterpret_cast<const float2*>(carry_in + 2 * m2);
+  if (ckpt_slot && o == 0) *reinterpret_cast<float2*>(ckpt_slot + 2 * m2) = off;
   epi_sync();
-  float off = cin;
-  for (int qq = 0; qq < q; ++qq) off += s_q[qq * 64 + m];
-  if (carry_out && q == 3) carry_out[m] = wrap2pi(off + run);
+#pragma unroll 1
+  for (int j = 0; j < o; ++j) {
+    const float2 v = q2[j * 32 + m2];
+    off.x += v.x;
+    off.y += v.y;
+  }
+  if (carry_out && o == 7) *reinterpret_cast<float2*>(carry_out + 2 * m2) = make_float2(wrap2pi(off.x + run.x), wrap2pi(off.y + run.y));
 #pragma unroll
-  for (int i = 0; i < LQ; ++i) {
-    const int l = q * LQ + i;
-    const float wv = wrap2pi(loc[i] + off);
-    const __half2 h2 = __floats2half2_rn(__cosf(wv), __sinf(wv));
-    tab[phi_idx(l, m)] = __uint_as_float(*reinterpret_cast<const uint32_t*>(&h2));
-    if (angle_out_bh && t0 + l == T - 1) angle_out_bh[m] = wv;
+  for (int i = 0; i < LO; ++i) {
+    const float wx = wrap2pi_add(loc[i].x + off.x), wy = wrap2pi_add(loc[i].y + off.y);
+    const __half2 hx = __floats2half2_rn(__cosf(wx), __sinf(wx)), hy = __floats2half2_rn(__cosf(wy), __sinf(wy));
+    *reinterpret_cast<uint2*>(&tab[phi_idx(o * LO + i, 2 * m2)]) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&hx), *reinterpret_cast<const uint32_t*>(&hy));
+  }
+  if (angle_out_bh && t0 + LT >= T) {   // the stripe's last tile
+#pragma unroll
+    for (int i = 0; i < LO; ++i)
+      if (t0 + o * LO + i == T - 1) {
+        angle_out_bh[2 * m2] = wrap2pi(loc[i].x + off.x);
+        angle_out_bh[2 * m2 + 1] = wrap2pi(loc[i].y + off.y);
+      }
   }
 }
 
 // (cos, sin) of the eight planes [m0, m0 + 8) of step l from the table (m0 a multiple of 8).
-__device__ __forceinline__ void table_cos_sin(const float* tab, int l, int m0, float (&cs)[8], float (&sn)[8]) {
+__device__ __forceinline__ void table_cos_sin(const float* tab, int l, int m0, float2 (&cs)[4], float2 (&sn)[4]) {
   const float4 a = *reinterpret_cast<const float4*>(&tab[phi_idx(l, m0)]);
   const float4 b = *reinterpret_cast<const float4*>(&tab[phi_idx(l, m0 + 4)]);
   const uint32_t w[8] = {__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w),
                          __float_as_uint(b.x), __float_as_uint(b.y), __float_as_uint(b.z), __float_as_uint(b.w)};
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-    cs[j] = f.x;
-    sn[j] = f.y;
+  for (int k = 0; k < 4; ++k) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[2 * k]));
+    const float2 g = __half22float2(*reinterpret_cast<const __half2*>(&w[2 * k + 1]));
+    cs[k] = make_float2(f.x, g.x);
+    sn[k] = make_float2(f.y, g.y);
   }
+}
+// Eight columns of both halves (m, m + 64) of rank r, rotated by -phi.
+template <int R, bool ROT, int NREG>
+__device__ __forceinline__ void rotate_store(uint8_t* dst, int row, int n0, const uint32_t (&v0)[NREG], const uint32_t (&v1)[NREG], int r,
+                                             const float2 (&cs)[4], const float2 (&sn)[4]) {
+  float2 o1[4], o2[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 a = pair_rank<R>(v0, k, r), b = pair_rank<R>(v1, k, r);
+    o1[k] = __ffma2_rn(a, cs[k], __fmul2_rn(b, sn[k]));
+    o2[k] = __ffma2_rn(b, cs[k], __fmul2_rn(a, make_float2(-sn[k].x, -sn[k].y)));
+  }
+  store_pairs(dst, tile_off(row, n0, kN), o1);
+  store_pairs(dst, tile_off(row, n0 + kNH, kN), o2);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -436,7 +459,7 @@ __device__ __forceinline__ void convert_bc(const uint8_t* rawB, const uint8_t* r
     convert_coords<RB::GB, R>(i, l, grp);
     const int n0 = grp * 8;
     const int rot = rank_rotation<R>();  // the order of the ranks differs by lane: see rank_rotation
-    float cs[8], sn[8];
+    float2 cs[4], sn[4];
     if (ROT) table_cos_sin(tab, l, n0, cs, sn);
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
@@ -449,21 +472,13 @@ __device__ __forceinline__ void convert_bc(const uint8_t* rawB, const uint8_t* r
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
         const int r = rr ^ rot;
-        if (ROT) {
-          float o1[8], o2[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float v1 = elem_rank<R>(v[0], j, r), v2 = elem_rank<R>(v[RB::NP - 1], j, r);
-            o1[j] = v1 * cs[j] + v2 * sn[j];
-            o2[j] = v2 * cs[j] - v1 * sn[j];
-          }
-          store_chunk(dst, tile_off(l * R + r, n0, kN), o1);
-          store_chunk(dst, tile_off(l * R + r, n0 + kNH, kN), o2);
+        if constexpr (ROT) {
+          rotate_store<R, ROT>(dst, l * R + r, n0, v[0], v[RB::NP - 1], r, cs, sn);
         } else {
-          float o[8];
+          float2 o[4];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = elem_rank<R>(v[0], j, r);
-          store_chunk(dst, tile_off(l * R + r, n0, kN), o);
+          for (int k = 0; k < 4; ++k) o[k] = pair_rank<R>(v[0], k, r);
+          store_pairs(dst, tile_off(l * R + r, n0, kN), o);
         }
       }
     }
@@ -495,11 +510,11 @@ __device__ __forceinline__ void store_px(const RawPX<R>& raw, uint8_t* s_plain, 
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) {
       const int r = rr ^ rot;
-      float o[8], ow[8];
+      float2 o[4], ow[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { o[j] = elem_rank<R>(raw.v[i], j, r); ow[j] = o[j] * sv; }
-      store_chunk(s_plain, tile_off(l * R + r, grp * 8, kP), o);
-      store_chunk(s_scaled, tile_off(l * R + r, grp * 8, kP), ow);
+      for (int k = 0; k < 4; ++k) { o[k] = pair_rank<R>(raw.v[i], k, r); ow[k] = __fmul2_rn(o[k], make_float2(sv, sv)); }
+      store_pairs(s_plain, tile_off(l * R + r, grp * 8, kP), o);
+      store_pairs(s_scaled, tile_off(l * R + r, grp * 8, kP), ow);
     }
   }
 }
@@ -527,7 +542,7 @@ __device__ __forceinline__ void store_bc(const RawBC<R, ROT>& raw, uint8_t* sB, 
     convert_coords<RB::GB, R>(i, l, grp);
     const int n0 = grp * 8;
     const int rot = rank_rotation<R>();  // the order of the ranks differs by lane: see rank_rotation
-    float cs[8], sn[8];
+    float2 cs[4], sn[4];
     if (ROT) table_cos_sin(tab, l, n0, cs, sn);
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
@@ -535,25 +550,47 @@ __device__ __forceinline__ void store_bc(const RawBC<R, ROT>& raw, uint8_t* sB, 
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
         const int r = rr ^ rot;
-        if (ROT) {
-          float o1[8], o2[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float v1 = elem_rank<R>(raw.v[i][which][0], j, r), v2 = elem_rank<R>(raw.v[i][which][RB::NP - 1], j, r);
-            o1[j] = v1 * cs[j] + v2 * sn[j];
-            o2[j] = v2 * cs[j] - v1 * sn[j];
-          }
-          store_chunk(dst, tile_off(l * R + r, n0, kN), o1);
-          store_chunk(dst, tile_off(l * R + r, n0 + kNH, kN), o2);
+        if constexpr (ROT) {
+          rotate_store<R, ROT>(dst, l * R + r, n0, raw.v[i][which][0], raw.v[i][which][RB::NP - 1], r, cs, sn);
         } else {
-          float o[8];
+          float2 o[4];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = elem_rank<R>(raw.v[i][which][0], j, r);
-          store_chunk(dst, tile_off(l * R + r, n0, kN), o);
+          for (int k = 0; k < 4; ++k) o[k] = pair_rank<R>(raw.v[i][which][0], k, r);
+          store_pairs(dst, tile_off(l * R + r, n0, kN), o);
         }
       }
     }
   }
+}
+
+// Sum over a warp, on every lane.
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// v[V] per lane (V = 4, 8 or 16) -> the sum over the warp's lanes of v[lane / (32 / V)]: the halves of the warp split the
+// values between them until one is left.
+template <int V>
+__device__ __forceinline__ float warp_sums(float (&v)[V]) {
+  const int lane = threadIdx.x & 31;
+  int nv = V;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (nv > 1) {
+      nv >>= 1;
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i)
+        if (i < nv) {
+          const float send = up ? v[i] : v[i + nv], keep = up ? v[i + nv] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return v[0];
 }
 
 // Sum over the 256 threads of the epilogue warps; red: >= 8 floats of shared scratch.  Contains two of

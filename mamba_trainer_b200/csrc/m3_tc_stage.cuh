@@ -14,6 +14,12 @@ constexpr float kInvTwoPi = 0.15915494309189535f, kTwoPiF = 6.283185307179586f;
 
 __device__ __forceinline__ float bf(const __nv_bfloat16* p, size_t i) { return __bfloat162float(p[i]); }
 __device__ __forceinline__ float wrap2pi(float v) { return v - rintf(v * kInvTwoPi) * kTwoPiF; }
+// wrap2pi with the addition that leaves no fraction in place of rintf, a conversion instruction that would queue with the
+// sines and cosines; angles are far below the 2^22 turns this is exact for.
+__device__ __forceinline__ float wrap2pi_add(float v) {
+  const float turns = __fadd_rn(fmaf(v, kInvTwoPi, 12582912.0f), -12582912.0f);
+  return fmaf(turns, -kTwoPiF, v);
+}
 __device__ __forceinline__ float expc(float d) { return __expf(fmaxf(d, -60.0f)); }
 __device__ __forceinline__ float inside(float d) { return (d > -60.0f && d < 0.0f) ? 1.0f : 0.0f; }
 
@@ -65,6 +71,15 @@ __device__ __forceinline__ float elem_rank(const uint32_t (&raw)[NREG], int j, i
     const uint32_t w = (r & 2) ? raw[2 * j + 1] : raw[2 * j];
     return __uint_as_float(__byte_perm(w, 0u, (r & 1) ? 0x3244u : 0x1044u));
   }
+}
+// Columns 2 k and 2 k + 1 of rank r: pairs for packed fp32 (two operations an instruction).
+template <int R, int NREG>
+__device__ __forceinline__ float2 pair_rank(const uint32_t (&raw)[NREG], int k, int r) {
+  return make_float2(elem_rank<R>(raw, 2 * k, r), elem_rank<R>(raw, 2 * k + 1, r));
+}
+__device__ __forceinline__ void store_pairs(uint8_t* base, uint32_t off, const float2 (&v)[4]) {
+  *reinterpret_cast<uint4*>(base + off) = make_uint4(pack_bf16(v[0].x, v[0].y), pack_bf16(v[1].x, v[1].y),
+                                                     pack_bf16(v[2].x, v[2].y), pack_bf16(v[3].x, v[3].y));
 }
 __device__ __forceinline__ void store_chunk(uint8_t* base, uint32_t off, const float (&v)[8]) {
   uint4 q;
@@ -227,11 +242,11 @@ __device__ __forceinline__ void commit_px(const RawPX<R>& raw, uint8_t* s_plain,
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) {
       const int r = rr ^ rot;
-      float o[8], ow[8];
+      float2 o[4], ow[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { o[j] = elem_rank<R>(raw.v[i], j, r); ow[j] = o[j] * sv; }
-      store_chunk(s_plain, tile_off(l * R + r, grp * 8, kP), o);
-      store_chunk(s_scaled, tile_off(l * R + r, grp * 8, kP), ow);
+      for (int k = 0; k < 4; ++k) { o[k] = pair_rank<R>(raw.v[i], k, r); ow[k] = __fmul2_rn(o[k], make_float2(sv, sv)); }
+      store_pairs(s_plain, tile_off(l * R + r, grp * 8, kP), o);
+      store_pairs(s_scaled, tile_off(l * R + r, grp * 8, kP), ow);
     }
   }
 }
