@@ -184,6 +184,18 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
       request_raw_tile<R>(l0, rawDY, &p.tm_dy, &bars[2], kP, b, h, T, t0, rev);
       __syncwarp();
     };
+    // The next tile's rows into L2 while this one is worked on: between a tile that lets go of the buffers and the next
+    // one's first use of them lies a third of a tile, too short for loads from DRAM queued behind 80 KB of stores.
+    auto prefetch_tile = [&](int b, int h, bool rev, int kk) {
+      const int t0 = kk * LT;
+      int l0 = prefetch_raw_tile<R>(0, &p.tm_c, kN, b, h, T, t0, rev);
+      l0 += prefetch_raw_tile<R>(l0, &p.tm_b, kN, b, h, T, t0, rev);
+      l0 += prefetch_raw_tile<R>(l0, &p.tm_x, kP, b, h, T, t0, rev);
+      l0 += prefetch_raw_tile<R>(l0, &p.tm_dy, kP, b, h, T, t0, rev);
+      const int t = rev ? T - t0 - LT : t0;
+      if (ROT && lane == l0 && t >= 0) tma_prefetch_rows(&p.tm_th, 0, h, t, b);
+      __syncwarp();
+    };
     // The staged gradients of a finished tile leave by bulk tensor stores, one box per lane: d x from the
     // checkpoint's buffer, d B from that of the scaled copies, d C from dG's.
     auto store_tile = [&](int b, int h, bool rev, int kk) {
@@ -218,6 +230,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
           request_ckpt(im.bh, k);                 // the checkpoint, where d x was staged
           request_xdy(b, h, rev, k);              // x and dy, where d C was staged (d B's buffer is the epilogue's)
           ++requested;
+          if (k > im.k_lo) prefetch_tile(b, h, rev, k - 1);
         }
         pb = b; ph = h; prev = rev; pk = k;
       }

@@ -132,6 +132,12 @@ __device__ __forceinline__ void tma_load_rows(void* dst, const void* tensor_map,
       : "memory");
 }
 
+// The same box into L2 only, for a tma_load_rows to come.
+__device__ __forceinline__ void tma_prefetch_rows(const void* tensor_map, int col, int h, int t, int b) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(tensor_map), "r"(col), "r"(h), "r"(t), "r"(b)
+               : "memory");
+}
+
 // The reverse direction: one box of a row map leaves shared memory (laid out as tma_load_rows would have
 // landed it) for the tensor; rows past the tensor's end are dropped.  `t` must not be negative.  The copy
 // joins the issuing thread's current bulk group (bulk_commit / bulk_wait_read / bulk_wait_all).

@@ -130,6 +130,13 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_con
           if (ROT && lane == l0) tma_load_rows(sTab, &p.tm_th, &bars[3], 0, h, rev ? T - k * LT - LT : k * LT, b);
           __syncwarp();
           ++requested;
+          if (k + 1 < it.k_hi) {   // the tile after it into L2
+            int q = prefetch_raw_tile<R>(0, &p.tm_b, kN, b, h, T, (k + 1) * LT, rev);
+            q += prefetch_raw_tile<R>(q, &p.tm_c, kN, b, h, T, (k + 1) * LT, rev);
+            const int t = rev ? T - (k + 2) * LT : (k + 1) * LT;
+            if (ROT && lane == q && t >= 0) tma_prefetch_rows(&p.tm_th, 0, h, t, b);
+            __syncwarp();
+          }
         }
       }
     }

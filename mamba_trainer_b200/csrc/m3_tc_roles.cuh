@@ -298,6 +298,16 @@ __device__ __forceinline__ int request_raw_tile(int lane0, uint8_t* dst, const v
   return (int)RT::panels(cols);
 }
 
+// The same rows into L2, for the request of a tile to come (its loads then take an L2 latency, not DRAM's).
+template <int R>
+__device__ __forceinline__ int prefetch_raw_tile(int lane0, const void* map, int cols, int b, int h, int T, int t0, bool rev) {
+  using RT = RawTile<R>;
+  const int t = rev ? T - t0 - RT::LT : t0;
+  const int pn = (int)(threadIdx.x & 31) - lane0;
+  if (t >= 0 && pn >= 0 && pn < (int)RT::panels(cols)) tma_prefetch_rows(map, pn * 64, h, t, b);
+  return (int)RT::panels(cols);
+}
+
 // ---------------------------------------------------------------------------------------
 // Results on their way out.  A thread owns a folded row (l, r) of an accumulator tile; the caller's tensor
 // wants rows [step][col * R + r].  The tile is staged in shared memory exactly as a bulk tensor copy of a
