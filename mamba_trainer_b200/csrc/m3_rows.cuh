@@ -54,6 +54,14 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+// The same into registers that need not be cleared first.
+__device__ __forceinline__ void mma_tf32_new(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.0f));
+}
+
 // acc[mt][nt] += A[m0 + 16 mt.., k] B[k, n0 + 8 nt..] over k in [k0, k1) (multiples of 8), by one warp.
 // AKC: A is stored [m][k], else [k][m]; BKC: B is stored [n][k], else [k][n].  AEX / BEX: that operand's values are
 // exact in TF32.  Accumulator layout: element e of a tile is row g + 8 (e >> 1), column 2 q + (e & 1), with g = lane / 4,
@@ -117,12 +125,16 @@ __device__ __forceinline__ void warp_mma(float (&acc)[MT][NT][4], const float* s
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-          float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-          if (!AEX) mma_tf32(t, al[mt], bh[nt]);
-          if (!BEX) mma_tf32(t, ah[mt], bl[nt]);
-          mma_tf32(t, ah[mt], bh[nt]);
+          float t[4];
+          if (!AEX) mma_tf32_new(t, al[mt], bh[nt]); else if (!BEX) mma_tf32_new(t, ah[mt], bl[nt]); else mma_tf32_new(t, ah[mt], bh[nt]);
+          if (!AEX && !BEX) mma_tf32(t, ah[mt], bl[nt]);
+          if (!AEX || !BEX) mma_tf32(t, ah[mt], bh[nt]);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[mt][nt][e] += t[e];
+          for (int e = 0; e < 4; e += 2) {   // two sums per instruction
+            const float2 v = __fadd2_rn(make_float2(acc[mt][nt][e], acc[mt][nt][e + 1]), make_float2(t[e], t[e + 1]));
+            acc[mt][nt][e] = v.x;
+            acc[mt][nt][e + 1] = v.y;
+          }
         }
     } else {
       if (!AEX) {
@@ -310,7 +322,11 @@ __device__ __forceinline__ void chunk_angles(float* phi, float* s_q, const Scal<
     float before = 0.0f;
     for (int j = 0; j < q; ++j) before += s_q[j * NH + m];
 #pragma unroll
-    for (int i = 0; i < LQ; ++i) phi[(q * LQ + i) * NH + m] = wrap_angle(off + before + loc[i]);
+    for (int i = 0; i < LQ; ++i) {
+      // wrap_angle without its division: for the sines only, where a whole turn more or less at the ends does not matter
+      const float v = off + before + loc[i];
+      phi[(q * LQ + i) * NH + m] = fmaf(rintf(v * 0.15915494309189535f), -kTwoPi, v);
+    }
     if (q == NQ - 1) total(m, before + run);
   }
 }
