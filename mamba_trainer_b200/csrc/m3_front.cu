@@ -343,6 +343,11 @@ __host__ __device__ inline PartLayout part_layout(const Front& f) {
   return l;
 }
 
+// Behind the blocks' sums: the gain's columns row by row of B and C, and how many of them k_front_sums has finished.
+__host__ __device__ inline unsigned* gain_count(const Front& f, const FrontGrads& g, size_t nblk) {
+  return reinterpret_cast<unsigned*>(g.part + part_layout(f).total * nblk + 2 * (size_t)f.bc);
+}
+
 // d dt_raw, d lambda_raw and the dt bias's partial sums of the block's steps: thread (head, time lane).
 template <class T>
 __device__ __forceinline__ void act_backward(const Front& f, const FrontGrads& g, int b, int t0, int steps, float* part, float* red) {
@@ -386,6 +391,7 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 3) k_front_bwd(Front f, FrontG
   const int b = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, bx = blockIdx.x;
   const PartLayout pl = part_layout(f);
   float* part = gr.part + ((size_t)b * gridDim.y + blockIdx.y) * pl.total;
+  if (bx == 0 && blockIdx.y == 0 && b == 0 && threadIdx.x == 0) *gain_count(f, gr, (size_t)gridDim.y * gridDim.z) = 0u;
   if (bx == nx + 2 * nb) {
     act_backward<T>(f, gr, b, blockIdx.y * (kBwdWarps * RUN), kBwdWarps * RUN, part + pl.act, &red[0][0]);
     return;
@@ -632,8 +638,9 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 3) k_front_bwd(Front f, FrontG
 
 // out[c] = sum over blocks (for the B / C bias over the ranks too) of the partial sums, in a fixed order: block (32, 8)
 // owns 32 columns, thread row y every 8th term, the 8 row sums are added in order.  The blocks of the gradients follow one
-// another (a grid with a row per gradient is mostly blocks with nothing to do); the gain's columns are summed row by row of
-// B and C here and over the rows by k_front_gain.
+// another (a grid with a row per gradient is mostly blocks with nothing to do).  The gain's columns are summed row by row of
+// B and C, and over the rows by whichever of their blocks finishes last (in a fixed order; k_front_bwd clears the count): as
+// a launch of its own that took 2 us and 3.5 us of the host's time.
 constexpr int kSumRows = 8;
 struct SumRange {
   float* out;
@@ -643,6 +650,9 @@ struct SumRange {
 struct SumPlan {
   SumRange r[6];
   int n, blocks;
+  float *gain_rows, *gain;   // gain NULL: none
+  unsigned* gain_count;
+  int gain_blocks, nrows;
 };
 __global__ void __launch_bounds__(32 * kSumRows) k_front_sums(SumPlan plan, const float* __restrict__ part, size_t pitch, int nblk,
                                                              int N) {
@@ -670,6 +680,28 @@ __global__ void __launch_bounds__(32 * kSumRows) k_front_sums(SumPlan plan, cons
     for (int j = 0; j < kSumRows; ++j) tot += red[j][threadIdx.x];
     q.out[c] = tot;
   }
+  if (!plan.gain || q.out != plan.gain_rows) return;
+  __shared__ unsigned last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && threadIdx.y == 0) last = atomicAdd(plan.gain_count, 1u);
+  __syncthreads();
+  if (last != (unsigned)plan.gain_blocks - 1u) return;
+  __threadfence();
+  for (int c0 = 0; c0 < N; c0 += 32) {
+    float v = 0.0f;
+#pragma unroll 8
+    for (int t = threadIdx.y; t < plan.nrows; t += kSumRows) v += __ldcg(plan.gain_rows + (size_t)t * N + c0 + threadIdx.x);
+    red[threadIdx.y][threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.y == 0) {
+      float tot = 0.0f;
+#pragma unroll
+      for (int j = 0; j < kSumRows; ++j) tot += red[j][threadIdx.x];
+      plan.gain[c0 + threadIdx.x] = tot;
+    }
+    __syncthreads();
+  }
 }
 SumPlan sum_plan(const Front& f, const FrontGrads& g, int nblk) {
   const PartLayout pl = part_layout(f);
@@ -684,24 +716,16 @@ SumPlan sum_plan(const Front& f, const FrontGrads& g, int nblk) {
   add(g.dconv_b, pl.conv + (size_t)KT * C, C, 1, 0);
   add(g.db_bias, pl.bias, f.H * f.N, f.R, f.N);
   add(g.dc_bias, pl.bias + f.bc, f.H * f.N, f.R, f.N);
-  add(g.dgain ? g.part + (size_t)nblk * pl.total : nullptr, pl.gain, 2 * f.bc, 1, 0);
+  if (g.dgain) {
+    p.gain = g.dgain;
+    p.gain_rows = g.part + (size_t)nblk * pl.total;
+    p.gain_count = gain_count(f, g, nblk);
+    p.gain_blocks = (2 * f.bc + 31) / 32;
+    p.nrows = 2 * f.bc / f.N;
+    add(p.gain_rows, pl.gain, 2 * f.bc, 1, 0);
+  }
   add(g.ddt_bias, pl.act, f.H, 1, 0);
   return p;
-}
-
-__global__ void __launch_bounds__(1024) k_front_gain(const float* __restrict__ rows, int nrows, int N, float* __restrict__ out) {
-  __shared__ float red[32][33];
-  const int c = blockIdx.x * 32 + threadIdx.x;
-  float s = 0.0f;
-  for (int t = threadIdx.y; t < nrows; t += 32) s += rows[(size_t)t * N + c];
-  red[threadIdx.y][threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.y == 0) {
-    float tot = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) tot += red[i][threadIdx.x];
-    out[c] = tot;
-  }
 }
 
 // Steps per warp: a block of 128 steps amortises the window's start and the warps' parameters; a grid of fewer than four
@@ -737,8 +761,6 @@ cudaError_t backward_t(cudaStream_t st, const Front& f, const FrontGrads& g) {
   const SumPlan plan = sum_plan(f, g, nblk);
   if (plan.blocks)
     k_front_sums<<<plan.blocks, dim3(32, kSumRows), 0, st>>>(plan, g.part, part_layout(f).total, nblk, N);
-  if (g.dgain)
-    k_front_gain<<<N / 32, dim3(32, 32), 0, st>>>(g.part + part_layout(f).total * grid.y * grid.z, 2 * f.H * R, N, g.dgain);
   return cudaGetLastError();
 }
 
@@ -780,11 +802,11 @@ size_t front_part_floats(const Front& f) {
   int nx, nb;
   dispatch(M3_F32, f, [&](auto, auto n, auto r) { front_tiles<n.value, r.value>(f, &nx, &nb); return 0; });
   const int steps = bwd_steps(f, nx + 2 * nb);
-  return part_layout(f).total * f.B * ((f.T + steps - 1) / steps) + 2 * (size_t)f.bc;
+  return part_layout(f).total * f.B * ((f.T + steps - 1) / steps) + 2 * (size_t)f.bc + 4;
 }
 
 cudaError_t front_backward(cudaStream_t st, int dtype, const Front& f, const FrontGrads& g, uint64_t* launches) {
-  if (launches) *launches += g.dgain ? 3 : 2;
+  if (launches) *launches += 2;
   return dispatch(dtype, f, [&](auto t, auto n, auto r) { return backward_t<decltype(t), n.value, r.value>(st, f, g); });
 }
 
