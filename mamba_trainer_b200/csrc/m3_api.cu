@@ -310,11 +310,12 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
     float* dalog = want(M3_GRAD_A_LOG, g->da_log) ? g->da_log : nullptr;
     float* ddsk = (want(M3_GRAD_D_SKIP, g->dd_skip) && desc.d_skip) ? g->dd_skip : nullptr;
     if (ahead && d.rot) {
-      e = m3::rows_final(ctx->stream, d, desc, p.dphi, p.dpsum, tps, nseg, bw, ddt, dlam, p.dtheta, p.dangle0);
+      e = m3::rows_final(ctx->stream, d, desc, p.dphi, p.dpsum, tps, nseg, bw, ddt, dlam, p.dtheta, p.dangle0,
+                         m3::HeadSums{desc.a_log, dalog, ddsk});
       ctx->launches += 1;
+    } else {
+      e = m3::finalize_scalars(ctx->stream, d, desc, bw, ddt, dlam, dalog, ddsk, &ctx->launches);
     }
-    if (e == cudaSuccess)
-      e = m3::finalize_scalars(ctx->stream, d, desc, bw, ddt, dlam, dalog, ddsk, &ctx->launches, !(ahead && d.rot));
   }
   cudaError_t e2 = cudaFreeAsync(base, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor-core backward");

@@ -125,6 +125,36 @@ __device__ __forceinline__ void zero_acc(float (&acc)[4][4]) {
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
 }
 
+// Sum over a warp, on every lane.
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// v[V] per lane (V = 4, 8 or 16) -> the sum over the warp's lanes of v[lane / (32 / V)]: the halves of the warp split the
+// values between them until one is left.
+template <int V>
+__device__ __forceinline__ float warp_sums(float (&v)[V]) {
+  const int lane = threadIdx.x & 31;
+  int nv = V;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (nv > 1) {
+      nv >>= 1;
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i)
+        if (i < nv) {
+          const float send = up ? v[i] : v[i + nv], keep = up ? v[i + nv] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return v[0];
+}
+
 // Sum over the 256 threads of a block; red: 8 floats of shared scratch.
 __device__ __forceinline__ float block_sum_256(float v, float* red) {
 #pragma unroll

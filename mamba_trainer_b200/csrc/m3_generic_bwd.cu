@@ -35,6 +35,20 @@ size_t generic_bwd_ws_layout(const Dims& d, GenericBwdWs* ws, char* base) {
   return off;
 }
 
+// The last launch of any backward pass: per-token d dt / d lambda from (da, dg, dw, the rotation term, the
+// seed-state term) - or, for the a / g / w form, da, dg, dw as they are - and the per-head sums.  `d.Tp` and
+// `d.C` give the pitch of the per-token arrays and the number of partial sums per (batch, head).
+template <class T>
+static void final_tokens(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const GenericBwdWs& bw, void* ddt, void* dlam,
+                         float* dalog, float* ddsk, const m3_scan_grads* raw) {
+  const unsigned blocks = (unsigned)(((size_t)d.B * d.T * d.H + 255) / 256);
+  const HeadSums hs{desc.a_log, dalog, ddsk};
+  kb_final<T><<<blocks + (hs.any() ? d.H : 0), 256, 0, st>>>(
+      d, static_cast<const T*>(desc.dt), static_cast<const T*>(desc.lambda), desc.a_log, bw, (desc.h0 && !d.raw) ? 1 : 0,
+      static_cast<T*>(ddt), static_cast<T*>(dlam), raw ? static_cast<T*>(raw->da_raw) : nullptr,
+      raw ? static_cast<T*>(raw->dg_raw) : nullptr, raw ? static_cast<T*>(raw->dw_raw) : nullptr, hs, (int)blocks);
+}
+
 template <class T>
 static cudaError_t backward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const GenericWs& ws,
                               const GenericBwdWs& bw, const m3_scan_bwd_in& in, uint32_t mask,
@@ -94,50 +108,21 @@ static cudaError_t backward_t(cudaStream_t st, const Dims& d, const m3_scan_desc
     n += 3;
   }
   kb_dx<T><<<gchunk, 256, 0, st>>>(d, x, dy, desc.d_skip, bw, dx);
-  const size_t total = (size_t)d.B * d.T * d.H;
-  kb_final<T><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
-      d, dt, lam, desc.a_log, bw, (has_state && !d.raw) ? 1 : 0, ddt, dlam, static_cast<T*>(g.da_raw),
-      static_cast<T*>(g.dg_raw), static_cast<T*>(g.dw_raw));
+  final_tokens<T>(st, d, desc, bw, ddt, dlam, dalog, ddsk, &g);
   n += 2;
   if (dh0 || dlu0) {
     kb_state_grads<T><<<dim3((PN + 255) / 256, BH), 256, 0, st>>>(d, dt, lam, bw, dh0, dlu0);
-    n += 1;
-  }
-  if (dalog || ddsk) {
-    kb_reduce_heads<<<d.H, 256, 0, st>>>(d, desc.a_log, bw, dalog, ddsk);
     n += 1;
   }
   if (launches) *launches += n;
   return cudaGetLastError();
 }
 
-// The last two launches of any backward: per-token d dt / d lambda from (da, dg, dw, the rotation term, the
-// seed-state term) - or, for the a / g / w form, da, dg, dw as they are - and the per-head reductions.  `d.Tp` and
-// `d.C` give the pitch of the per-token arrays and the number of partial sums per (batch, head).  `tokens` false: the
-// per-token part has been done.
-template <class T>
-static void final_tokens(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const GenericBwdWs& bw, void* ddt, void* dlam,
-                         const m3_scan_grads* raw) {
-  const size_t total = (size_t)d.B * d.T * d.H;
-  kb_final<T><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
-      d, static_cast<const T*>(desc.dt), static_cast<const T*>(desc.lambda), desc.a_log, bw, (desc.h0 && !d.raw) ? 1 : 0,
-      static_cast<T*>(ddt), static_cast<T*>(dlam), raw ? static_cast<T*>(raw->da_raw) : nullptr,
-      raw ? static_cast<T*>(raw->dg_raw) : nullptr, raw ? static_cast<T*>(raw->dw_raw) : nullptr);
-}
 cudaError_t finalize_scalars(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const GenericBwdWs& bw,
-                             void* ddt, void* dlam, float* dalog, float* ddsk, uint64_t* launches, bool tokens,
-                             const m3_scan_grads* raw) {
-  uint64_t n = 0;
-  if (tokens) {
-    if (desc.dtype == M3_BF16) final_tokens<__nv_bfloat16>(st, d, desc, bw, ddt, dlam, raw);
-    else final_tokens<float>(st, d, desc, bw, ddt, dlam, raw);
-    n += 1;
-  }
-  if (dalog || ddsk) {
-    kb_reduce_heads<<<d.H, 256, 0, st>>>(d, desc.a_log, bw, dalog, ddsk);
-    n += 1;
-  }
-  if (launches) *launches += n;
+                             void* ddt, void* dlam, float* dalog, float* ddsk, uint64_t* launches, const m3_scan_grads* raw) {
+  if (desc.dtype == M3_BF16) final_tokens<__nv_bfloat16>(st, d, desc, bw, ddt, dlam, dalog, ddsk, raw);
+  else final_tokens<float>(st, d, desc, bw, ddt, dlam, dalog, ddsk, raw);
+  if (launches) *launches += 1;
   return cudaGetLastError();
 }
 

@@ -231,7 +231,12 @@ template <class T>
 __global__ void kb_final(Dims d, const T* __restrict__ dt, const T* __restrict__ lam,
                          const float* __restrict__ a_log, GenericBwdWs bw, int has_state,
                          T* __restrict__ ddt, T* __restrict__ dlam, T* __restrict__ da_raw, T* __restrict__ dg_raw,
-                         T* __restrict__ dw_raw) {
+                         T* __restrict__ dw_raw, HeadSums hs, int token_blocks) {
+  if ((int)blockIdx.x >= token_blocks) {   // the blocks behind those of the tokens: one per head
+    __shared__ float red[8];
+    head_sums(d, blockIdx.x - token_blocks, hs, bw, red);
+    return;
+  }
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t total = (size_t)d.B * d.T * d.H;
   if (i >= total) return;
@@ -276,28 +281,6 @@ __global__ void kb_state_grads(Dims d, const T* __restrict__ dt, const T* __rest
   const float v = bw.dHs[((size_t)bh * (d.C + 1) + d.C) * PN + e];
   if (dh0) dh0[(size_t)bh * PN + e] = v;
   if (dlu0) dlu0[(size_t)bh * PN + e] = first * v;
-}
-
-// ---- per head: d a_log = A * sum da dt (A = -exp(a_log), scan.rs:470-475) and dD,
-// summed over batch and chunks in a fixed order.
-__global__ void kb_reduce_heads(Dims d, const float* __restrict__ a_log, GenericBwdWs bw,
-                                float* __restrict__ da_log, float* __restrict__ dd_skip) {
-  __shared__ float red[8];
-  const int h = blockIdx.x;
-  float sa = 0.0f, sd = 0.0f;
-  const int n = d.B * d.C;
-  for (int e = threadIdx.x; e < n; e += 256) {
-    const int b = e / d.C, k = e % d.C;
-    const size_t o = ((size_t)b * d.H + h) * d.C + k;
-    sa += bw.partA[o];
-    if (dd_skip) sd += bw.partD[o];
-  }
-  sa = block_sum_256(sa, red);
-  sd = block_sum_256(sd, red);
-  if (threadIdx.x == 0) {
-    if (da_log) da_log[h] = -expf(a_log[h]) * sa;
-    if (dd_skip) dd_skip[h] = sd;
-  }
 }
 
 }  // namespace m3

@@ -502,7 +502,7 @@ cudaError_t rows_load(int dtype);   // load_kernels of every kernel a forward pa
 // The last pass over tokens for the tensor-core family's side-by-side segments (bf16, d_state 128, rotational): d.L steps
 // per tile, `per_seg` tiles per segment.
 cudaError_t rows_final(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const float* dphi, const float* dpsum, int per_seg,
-                       int nseg, const GenericBwdWs& bw, void* ddt, void* dlam, void* dtheta, float* dangle0);
+                       int nseg, const GenericBwdWs& bw, void* ddt, void* dlam, void* dtheta, float* dangle0, const HeadSums& hs);
 size_t rows_bwd_ws_layout(const Dims& d, rows::RowsBwdWs* rw, GenericBwdWs* bw, char* base);
 cudaError_t rows_backward(cudaStream_t st, const Dims& d, const m3_scan_desc& desc, const rows::RowsWs& ws,
                           const rows::RowsBwdWs& rw, const GenericBwdWs& bw, const m3_scan_bwd_in& in, uint32_t mask,

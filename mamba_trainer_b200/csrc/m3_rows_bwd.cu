@@ -456,15 +456,39 @@ __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoin
 // ---- rotational dynamics: the later chunks' d phi on top, then per token d theta, d dt and d lambda (the arithmetic of
 // kb_final).  A warp per step, lanes over planes; a block per d.L steps, `per_seg` blocks to a segment whose sums of d phi
 // are complete within it, `nseg` of those (here the chunks; the tensor-core family's segments are longer).
+// Behind these rows of blocks, one block per head for its sums.  A warp requests eight steps before it uses the first (as a
+// loop over steps it waited for each pair of loads: float32, 8 x 1024 tokens x 16 heads, 42 us; its bytes take 15).
 template <class T, int N>
 __global__ void __launch_bounds__(256) k_rows_final(Dims d, m3_scan_desc in, RowsBwdWs rw, GenericBwdWs bw, int has_state,
                                                     T* __restrict__ ddt, T* __restrict__ dlam, T* __restrict__ dtheta,
-                                                    float* __restrict__ dangle0, int per_seg, int nseg) {
-  constexpr int NH = N / 2, NQ = 256 / NH, PL = NH / 32;
-  __shared__ float s_off[NQ][NH], s_rot[128];
+                                                    float* __restrict__ dangle0, int per_seg, int nseg, HeadSums hs) {
+  constexpr int NH = N / 2, NQ = 256 / NH, PL = NH / 32, U = 8;
+  __shared__ float s_off[NQ][NH], s_rot[128], red[8];
+  if (blockIdx.z || (int)blockIdx.y >= d.B * d.H) {
+    const int h = ((int)blockIdx.y - (blockIdx.z ? 0 : d.B * d.H)) * (int)gridDim.x + (int)blockIdx.x;
+    if (h < d.H) head_sums(d, h, hs, bw, red);
+    return;
+  }
   const Chunk c = this_chunk(d);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const T* dt = static_cast<const T*>(in.dt);
+  const T* theta = static_cast<const T*>(in.theta);
+  float v[U][PL], th[U][PL], vdt[U];
+  auto load = [&](int l0) {   // steps l0, l0 + 8, ...
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int l = l0 + 8 * u, t = c.t0 + l;
+      const bool live = l < d.L && t < d.T;
+      const size_t ti = live ? theta_index(d, c.b, t, c.h) : 0, o = ((size_t)c.bh * d.Tp + (live ? t : c.t0)) * NH;
+      vdt[u] = live ? ldf(dt, tok_index(d, c.b, t, c.h)) : 0.0f;
+#pragma unroll
+      for (int i = 0; i < PL; ++i) {
+        v[u][i] = live ? rw.dphi[o + lane + 32 * i] : 0.0f;
+        th[u][i] = live ? ldf(theta, ti + lane + 32 * i) : 0.0f;
+      }
+    }
+  };
+  load(warp);
   {
     const int q = tid / NH, m = tid % NH;
     float s = 0.0f;
@@ -482,41 +506,51 @@ __global__ void __launch_bounds__(256) k_rows_final(Dims d, m3_scan_desc in, Row
     if (c.k == 0 && warp == 0 && dangle0)
       dangle0[(size_t)c.bh * NH + lane + 32 * i] = off[i] + rw.dpsum[(size_t)c.bh * nseg * NH + lane + 32 * i];
   }
-#pragma unroll 4
-  for (int l = warp; l < d.L; l += 8) {
-    const int t = c.t0 + l;
-    if (t >= d.T) break;
-    const size_t ti = theta_index(d, c.b, t, c.h);
-    const float vdt = ldf(dt, tok_index(d, c.b, t, c.h));
-    float s = 0.0f;
+  for (int l0 = warp; l0 < d.L; l0 += 8 * U) {
+    if (l0 != warp) load(l0);
+    float s[U];
 #pragma unroll
-    for (int i = 0; i < PL; ++i) {
-      const int m = lane + 32 * i;
-      const float v = rw.dphi[((size_t)c.bh * d.Tp + t) * NH + m] + off[i];
-      s += v * ldf(static_cast<const T*>(in.theta), ti + m);
-      if (dtheta) stf(dtheta, ti + m, v * vdt);
+    for (int u = 0; u < U; ++u) {
+      const int l = l0 + 8 * u, t = c.t0 + l;
+      s[u] = 0.0f;
+#pragma unroll
+      for (int i = 0; i < PL; ++i) {
+        const float g = v[u][i] + off[i];
+        s[u] += g * th[u][i];
+        if (dtheta && l < d.L && t < d.T) stf(dtheta, theta_index(d, c.b, t, c.h) + lane + 32 * i, g * vdt[u]);
+      }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) s_rot[l] = s;
+    const float sum = warp_sums<U>(s);
+    const int l = l0 + 8 * (lane / (32 / U));
+    if (lane % (32 / U) == 0 && l < d.L) s_rot[l] = sum;
   }
   __syncthreads();
   const int t = c.t0 + tid;
   if (tid < d.L && t < d.T && (ddt || dlam)) {
     const size_t o = (size_t)c.bh * d.Tp + t, ti = tok_index(d, c.b, t, c.h);
     const float A = -expf(in.a_log[c.h]);
-    const float vdt = ldf(dt, ti), vl = lambda_at(static_cast<const T*>(in.lambda), d.disc, ti);
+    const float vdt0 = ldf(dt, ti), vl = lambda_at(static_cast<const T*>(in.lambda), d.disc, ti);
     const float gw = bw.dg[o] + bw.dw[o], dwm1 = t > 0 ? bw.dw[o - 1] : 0.0f;
-    float vdl = gw * vdt - dwm1 * vdt;
+    float vdl = gw * vdt0 - dwm1 * vdt0;
     float vdd = bw.da[o] * A + gw * vl + dwm1 * (1.0f - vl) + s_rot[tid];
     if (has_state && t == 0) {
       const float ip = bw.ip0[c.bh];
-      vdl -= vdt * ip;
+      vdl -= vdt0 * ip;
       vdd += (1.0f - vl) * ip;
     }
     if (ddt) stf(ddt, ti, vdd);
     if (dlam) stf(dlam, ti, vdl);
   }
+}
+
+template <class T, int N>
+cudaError_t final_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const RowsBwdWs& rw, const GenericBwdWs& bw, void* ddt,
+                    void* dlam, void* dtheta, float* dangle0, int per_seg, int nseg, const HeadSums& hs) {
+  const int nx = (d.T + d.L - 1) / d.L, BH = d.B * d.H, ny = BH + (hs.any() ? (d.H + nx - 1) / nx : 0);
+  const dim3 grid = ny <= 65535 ? dim3(nx, ny) : dim3(nx, BH, 2);   // (a layer of its own where the rows are used up)
+  k_rows_final<T, N><<<grid, 256, 0, st>>>(d, in, rw, bw, in.h0 ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam),
+                                                   static_cast<T*>(dtheta), dangle0, per_seg, nseg, hs);
+  return cudaGetLastError();
 }
 
 template <class T, int N, int R, bool ROT>
@@ -543,30 +577,21 @@ cudaError_t backward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, c
   }
   void* ddt = want(M3_GRAD_DT, g.ddt);
   void* dlam = d.disc == M3_LEARNED_TRAPEZOID ? want(M3_GRAD_LAMBDA, g.dlambda) : nullptr;
-  if (ROT) {
-    k_rows_final<T, N><<<grid, 256, 0, st>>>(d, in, rw, bw, has_state ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam),
-                                             static_cast<T*>(want(M3_GRAD_THETA, g.dtheta)),
-                                             in.angle0 ? static_cast<float*>(want(M3_GRAD_ANGLE0, g.dangle0)) : nullptr, 1, d.C);
-    n += 1;
-  }
-  if (launches) *launches += n;
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   float* dalog = d.raw ? nullptr : static_cast<float*>(want(M3_GRAD_A_LOG, g.da_log));
   float* ddsk = in.d_skip ? static_cast<float*>(want(M3_GRAD_D_SKIP, g.dd_skip)) : nullptr;
-  return finalize_scalars(st, d, in, bw, ddt, dlam, dalog, ddsk, launches, !ROT, &g);
+  if (launches) *launches += n + (ROT ? 1 : 0);
+  if (!ROT) return finalize_scalars(st, d, in, bw, ddt, dlam, dalog, ddsk, launches, &g);
+  return final_t<T, N>(st, d, in, rw, bw, ddt, dlam, want(M3_GRAD_THETA, g.dtheta),
+                       in.angle0 ? static_cast<float*>(want(M3_GRAD_ANGLE0, g.dangle0)) : nullptr, 1, d.C, HeadSums{in.a_log, dalog, ddsk});
 }
 
 }  // namespace
 }  // namespace rows
 
 cudaError_t rows_final(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const float* dphi, const float* dpsum, int per_seg,
-                       int nseg, const GenericBwdWs& bw, void* ddt, void* dlam, void* dtheta, float* dangle0) {
-  using T = __nv_bfloat16;
+                       int nseg, const GenericBwdWs& bw, void* ddt, void* dlam, void* dtheta, float* dangle0, const HeadSums& hs) {
   const rows::RowsBwdWs rw{nullptr, const_cast<float*>(dphi), const_cast<float*>(dpsum)};
-  rows::k_rows_final<T, 128><<<dim3((d.T + d.L - 1) / d.L, d.B * d.H), 256, 0, st>>>(
-      d, in, rw, bw, in.h0 ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam), static_cast<T*>(dtheta), dangle0, per_seg, nseg);
-  return cudaGetLastError();
+  return rows::final_t<__nv_bfloat16, 128>(st, d, in, rw, bw, ddt, dlam, dtheta, dangle0, per_seg, nseg, hs);
 }
 
 size_t rows_bwd_ws_layout(const Dims& d, rows::RowsBwdWs* rw, GenericBwdWs* bw, char* base) {

@@ -21,9 +21,12 @@
 // helper warp or one epilogue warp taking a branch of its own (the scalars on an epilogue warp inside
 // the wait for the first products made every tile 2.4 K cycles longer).
 #pragma once
+#include "m3_common.cuh"
 #include "m3_tc_stage.cuh"
 
 namespace m3tc {
+using m3::warp_sum;
+using m3::warp_sums;
 
 constexpr int kEpiThreads = 256, kCtaThreads = 384, kPairCount = kEpiThreads + 32;
 constexpr int kIssuerWarp = 8, kScalarWarp = 9, kCopyWarp = 10;  // warp 11 idles
@@ -571,36 +574,6 @@ __device__ __forceinline__ void store_bc(const RawBC<R, ROT>& raw, uint8_t* sB, 
       }
     }
   }
-}
-
-// Sum over a warp, on every lane.
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-// v[V] per lane (V = 4, 8 or 16) -> the sum over the warp's lanes of v[lane / (32 / V)]: the halves of the warp split the
-// values between them until one is left.
-template <int V>
-__device__ __forceinline__ float warp_sums(float (&v)[V]) {
-  const int lane = threadIdx.x & 31;
-  int nv = V;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    if (nv > 1) {
-      nv >>= 1;
-      const bool up = (lane & o) != 0;
-#pragma unroll
-      for (int i = 0; i < V / 2; ++i)
-        if (i < nv) {
-          const float send = up ? v[i] : v[i + nv], keep = up ? v[i + nv] : v[i];
-          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    } else {
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-    }
-  }
-  return v[0];
 }
 
 // Sum over the 256 threads of the epilogue warps; red: >= 8 floats of shared scratch.  Contains two of
