@@ -51,7 +51,7 @@ def _build_extension(force: bool) -> None:
     tmp = EXT.with_suffix(".tmp")   # a process that has the old one loaded keeps its file
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_m3torch",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{i}" for i in inc], str(src), "-o", str(tmp),
-           f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{root / 'lib'}",
+           f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{root / 'lib'}",
            f"-L{PKG}", "-l:libm3scan.so", "-Wl,-rpath,$ORIGIN"]
     subprocess.run(cmd, check=True)
     tmp.replace(EXT)

@@ -3,6 +3,7 @@
 // gradient buffer at a time - cost 120 us of a scan's forward + backward whose library calls take 26 us; the small calls
 // (a 2 x 256-token scan, a decoding step) were bound by it.
 // The arithmetic stays in libm3scan; this extension allocates with torch and enqueues on torch's current stream.
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
@@ -69,6 +70,14 @@ const void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; 
 void* mut(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 const float* fptr(const Tensor& t) { return static_cast<const float*>(ptr(t)); }
 float* fmut(const Tensor& t) { return static_cast<float*>(mut(t)); }
+
+// Uninitialised memory for results and scratch, straight from the allocator behind at::empty: these calls are the larger part
+// of what a small call costs the host (a decoding step makes five of them).
+Tensor fresh(at::IntArrayRef sizes, at::ScalarType el, const Tensor& like) {
+  return Tensor(at::detail::empty_cuda(sizes, el, like.device(), c10::nullopt));
+}
+Tensor fresh_like(const Tensor& t) { return fresh(t.sizes(), t.scalar_type(), t); }
+Tensor fresh_bytes(size_t n, const Tensor& like) { return fresh({static_cast<int64_t>(n)}, at::kByte, like); }
 
 Tensor as(const Tensor& t, at::ScalarType el) {
   if (!t.defined()) return t;
@@ -151,7 +160,7 @@ struct ScanNode : public torch::autograd::Node {
     uint32_t mask = 0;
     for (int i = 0; i < kScanInputs; ++i)
       if (in[i].present && task_should_compute_output(i)) {
-        g[i] = at::empty_like(t[i], at::MemoryFormat::Contiguous);
+        g[i] = fresh_like(t[i]);
         mask |= 1u << i;
       }
     auto dense = [](const Tensor& v) { return v.defined() ? v.contiguous() : v; };
@@ -187,12 +196,11 @@ std::vector<OptTensor> scan(uintptr_t handle, const Tensor& x0, const Tensor& b0
   d.discretization = disc; d.dynamics = t[6].defined() ? M3_ROTATIONAL : M3_REAL; d.want_state = want_state; d.path = path;
   d.reverse_heads = rev;
   scan_inputs(d, t);
-  const auto f32 = x.options().dtype(at::kFloat).requires_grad(false);
-  Tensor y = at::empty(x.sizes(), x.options().requires_grad(false)), h, lu, ang;
+  Tensor y = fresh_like(x), h, lu, ang;
   if (want_state) {
-    h = at::empty({B, H, P, N}, f32);
-    lu = at::empty({B, H, P, N}, f32);
-    if (t[6].defined()) ang = at::empty({B, H, N / 2}, f32);
+    h = fresh({B, H, P, N}, at::kFloat, x);
+    lu = fresh({B, H, P, N}, at::kFloat, x);
+    if (t[6].defined()) ang = fresh({B, H, N / 2}, at::kFloat, x);
   }
   bool track = false;
   if (at::GradMode::is_enabled())
@@ -276,10 +284,10 @@ struct MixerNode : public torch::autograd::Node {
     // (a gain whose norm was switched off is read by nothing: no gradient)
     for (int i = 0; i <= kMixerParams; ++i)
       if (in[i].present && (i != 1 + kNormWeight || d.has_norm) && (i != 1 + kPostWeight || d.post_norm))
-        g[i] = at::empty_like(t[i], at::MemoryFormat::Contiguous);
+        g[i] = fresh_like(t[i]);
     const m3_mixer_grads out{mut(g[0]), fmut(g[1]), fmut(g[2]), fmut(g[3]), fmut(g[4]), fmut(g[5]),
                              fmut(g[6]), fmut(g[7]), fmut(g[8]), fmut(g[9])};
-    const Tensor work = at::empty({(int64_t)m3_mixer_backward_bytes(&d)}, act.options());
+    const Tensor work = fresh_bytes(m3_mixer_backward_bytes(&d), act);
     const Status s = locked(ctx, t[0], [&] { return m3_mixer_backward(ctx, &d, handle, ptr(act), ptr(dout), &out, mut(work)); });
     if (s.rc != M3_OK) raise_status(s);
     return g;
@@ -296,9 +304,8 @@ Tensor mixer(uintptr_t handle, const Tensor& proj0, const std::vector<OptTensor>
   refuse_tangents(&proj, 1);
   refuse_tangents(p, kMixerParams);
   const m3_mixer_desc d = mixer_desc(proj, p, spec_of(ints), eps);
-  const auto opt = proj.options().requires_grad(false);
-  Tensor out = at::empty({proj.size(0), proj.size(1), d_inner}, opt);
-  const Tensor act = at::empty({(int64_t)m3_mixer_activation_bytes(&d)}, opt.dtype(at::kByte));
+  Tensor out = fresh({proj.size(0), proj.size(1), d_inner}, proj.scalar_type(), proj);
+  const Tensor act = fresh_bytes(m3_mixer_activation_bytes(&d), proj);
   bool track = false;
   if (at::GradMode::is_enabled()) {
     track = proj.requires_grad();
@@ -335,15 +342,14 @@ std::vector<OptTensor> window(uintptr_t handle, const Tensor& proj0, const std::
   const m3_mixer_desc d = mixer_desc(proj, p, s, eps);
   const Tensor conv = as(conv0, proj.scalar_type()), h = as(h0, at::kFloat), lu = as(lu0, at::kFloat);
   const Tensor ang = s.rotational ? as(ang0, at::kFloat) : Tensor();
-  const auto opt = proj.options().requires_grad(false);
-  const Tensor out = at::empty({proj.size(0), proj.size(1), d_inner}, opt), conv2 = at::empty(conv.sizes(), opt);
-  const Tensor h2 = at::empty(h.sizes(), opt.dtype(at::kFloat)), lu2 = at::empty(lu.sizes(), opt.dtype(at::kFloat));
+  const Tensor out = fresh({proj.size(0), proj.size(1), d_inner}, proj.scalar_type(), proj), conv2 = fresh_like(conv);
+  const Tensor h2 = fresh_like(h), lu2 = fresh_like(lu);
   Tensor ang2;
-  if (s.rotational) ang2 = at::empty({proj.size(0), s.heads, s.d_state / 2}, opt.dtype(at::kFloat));
+  if (s.rotational) ang2 = fresh({proj.size(0), s.heads, s.d_state / 2}, at::kFloat, proj);
   const m3_mixer_window_io io{ptr(conv), fptr(h), fptr(lu), fptr(ang), mut(out), mut(conv2), fmut(h2), fmut(lu2), fmut(ang2)};
   const size_t bytes = m3_mixer_window_bytes(&d, &io);
   Tensor work;
-  if (bytes) work = at::empty({(int64_t)bytes}, opt.dtype(at::kByte));
+  if (bytes) work = fresh_bytes(bytes, proj);
   const Status done = locked(ctx, proj, [&] { return m3_mixer_window(ctx, &d, &io, mut(work)); });
   if (done.rc != M3_OK) raise_status(done);
   return {out, conv2, h2, lu2, ang2.defined() ? OptTensor(ang2) : OptTensor()};
