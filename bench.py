@@ -543,13 +543,11 @@ def main():
         per_th = traffic_per_token_head(w, torch.cuda.get_device_properties(dev).multi_processor_count)
         cfg = workload_config(gw, world, args.config)
         cfg["batch_per_gpu"] = w.batch
-        # rank 1 with real dynamics takes the direct form of the stripe kernels, float32 the generic family
-        direct = w.rank == 1 and not w.rotational
+        # float32 takes the chunk-parallel family
         if w.dtype != torch.bfloat16:
-            fwd_name, bwd_name = "generic family (k_chunk_state ... k_chunk_out)", "generic family (kb_* kernels)"
+            fwd_name, bwd_name = "chunk-parallel family (k_rows_state ... k_rows_out)", "chunk-parallel family (k_rows_* kernels)"
         else:
-            fwd_name = "tc_fwd_direct_kernel" if direct else "tc_fwd_kernel"
-            bwd_name = "tc_bwd_direct_kernel" if direct else "tc_bwd_kernel"
+            fwd_name, bwd_name = "tc_fwd_kernel", "tc_bwd_kernel"
         if fallback_note:
             cfg["fallback"] = fallback_note
         line = {

@@ -18,7 +18,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libm3scan.so"
 EXT = PKG / "_m3torch.so"
-SOURCES = ["m3_api.cu", "m3_generic_fwd.cu", "m3_generic_bwd.cu", "m3_noalloc.cu", "m3_rows_fwd.cu", "m3_rows_bwd.cu", "m3_tc_fwd.cu", "m3_tc_fwd_direct.cu", "m3_tc_bwd.cu", "m3_tc_bwd_direct.cu", "m3_tc_ahead.cu", "m3_step.cu", "m3_mixer_call.cu", "m3_front.cu",
+SOURCES = ["m3_api.cu", "m3_generic_fwd.cu", "m3_generic_bwd.cu", "m3_noalloc.cu", "m3_rows_fwd.cu", "m3_rows_bwd.cu", "m3_tc_fwd.cu", "m3_tc_bwd.cu", "m3_tc_ahead.cu", "m3_step.cu", "m3_mixer_call.cu", "m3_front.cu",
            "m3_host_pipe.cu", "m3_conv.cu", "m3_mixer.cu", "m3_reduce.cu"]
 
 

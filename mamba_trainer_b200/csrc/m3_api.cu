@@ -22,7 +22,6 @@ struct m3_saved {
   m3::rows::RowsWs rws;
   __nv_bfloat16* tc_ckpt_h = nullptr;  // tensor-core family: bf16 state entering each tile
   float* tc_ckpt_angle = nullptr;  // and the angle entering each tile
-  bool tc_direct = false;          // the forward ran the direct form: so does the backward (same tile maps)
   cudaStream_t stream = nullptr;   // the stream the forward ran on: the scratch is freed in its order
 };
 
@@ -179,11 +178,11 @@ void split_chain_leave(m3_ctx* ctx) {
 // cut - the hand-over scratch (state, angle, flags; the flags zeroed on the stream).  `*scratch` is null
 // when nothing is handed over; the caller frees it on the stream after the launch.
 template <class Params>
-cudaError_t plan_segments(m3_ctx* ctx, Params& p, int tiles, bool allow_split, char** scratch) {
+cudaError_t plan_segments(m3_ctx* ctx, Params& p, int tiles, bool allow_split, bool backward, bool rot, char** scratch) {
   *scratch = nullptr;
   p.ahead = 0;
   size_t bytes = 0;
-  m3::tc_segment_plan(p.B * p.H, tiles, allow_split, &p.nseg, &p.tps, &p.grid, &bytes);
+  m3::tc_segment_plan(p.B * p.H, tiles, allow_split, backward, rot, p.R, &p.nseg, &p.tps, &p.grid, &bytes);
   if (p.nseg == 1) return cudaSuccess;
   cudaError_t e = m3::scratch_alloc(ctx, reinterpret_cast<void**>(scratch), bytes, ctx->stream);
   if (e != cudaSuccess) return e;
@@ -234,7 +233,7 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
   const size_t per_tok = BH * d.Tp, per_tile = BH * tiles;
   // few stripes: segments that run side by side; their sums of d phi are completed afterwards
   int nseg = 1, tps = tiles;
-  const bool ahead = !saved->tc_direct && m3::tc_ahead_plan((int)BH, tiles, true, false, &nseg, &tps);
+  const bool ahead = m3::tc_ahead_plan((int)BH, tiles, true, d.rot != 0, d.R, &nseg, &tps);
   const size_t nphi = ahead && d.rot ? (per_tok + BH * nseg) * 64 : 0;
   const size_t nfloat = 4 * per_tok + 2 * per_tile + BH + 4 + nphi;
   float* base = nullptr;
@@ -269,26 +268,18 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
     cudaFreeAsync(base, ctx->stream);
     return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs 16-byte aligned dy and gradient buffers");
   }
-  p.use_tma = (saved->tc_direct && d.R == 1 && !d.rot && d.rev == 0 && d.T % 8 == 0 && !(reinterpret_cast<uintptr_t>(p.ckpt_h) & 15) &&
-               m3::tc_make_tile_map(&p.tm_b, p.b, d.B, d.T, d.H, 128) && m3::tc_make_tile_map(&p.tm_c, p.c, d.B, d.T, d.H, 128)) ? 1 : 0;
-  if (saved->tc_direct && !p.use_tma) {
+  if (!m3::tc_make_row_map(&p.tm_b, p.b, d.B, d.T, d.H, 128 * d.R, steps, true) ||
+      !m3::tc_make_row_map(&p.tm_c, p.c, d.B, d.T, d.H, 128 * d.R, steps, true) ||
+      !m3::tc_make_row_map(&p.tm_x, p.x, d.B, d.T, d.H, 64 * d.R, steps, true) ||
+      !m3::tc_make_row_map(&p.tm_dy, p.dy, d.B, d.T, d.H, 64 * d.R, steps, true) ||
+      (d.rot && !m3::tc_make_row_map(&p.tm_th, p.theta, d.B, d.T, d.H, 64, steps, false, d.ths))) {
     cudaFreeAsync(base, ctx->stream);
-    return fail(ctx, M3_ERR_UNSUPPORTED, "the forward pass ran the direct form; its backward pass cannot be set up");
+    return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs 16-byte aligned b, c, x, dy and theta");
   }
-  if (!p.use_tma) {
-    if (!m3::tc_make_row_map(&p.tm_b, p.b, d.B, d.T, d.H, 128 * d.R, steps, true) ||
-        !m3::tc_make_row_map(&p.tm_c, p.c, d.B, d.T, d.H, 128 * d.R, steps, true) ||
-        !m3::tc_make_row_map(&p.tm_x, p.x, d.B, d.T, d.H, 64 * d.R, steps, true) ||
-        !m3::tc_make_row_map(&p.tm_dy, p.dy, d.B, d.T, d.H, 64 * d.R, steps, true) ||
-        (d.rot && !m3::tc_make_row_map(&p.tm_th, p.theta, d.B, d.T, d.H, 64, steps, false, d.ths))) {
-      cudaFreeAsync(base, ctx->stream);
-      return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs 16-byte aligned b, c, x, dy and theta");
-    }
-    // the gradients asked for leave by bulk tensor stores where they can; by plain stores otherwise
-    p.out_maps = ((!p.dx || m3::tc_make_row_map(&p.tm_dx, p.dx, d.B, d.T, d.H, 64 * d.R, steps, true)) &&
-                  (!p.db || m3::tc_make_row_map(&p.tm_db, p.db, d.B, d.T, d.H, 128 * d.R, steps, true)) &&
-                  (!p.dc || m3::tc_make_row_map(&p.tm_dc, p.dc, d.B, d.T, d.H, 128 * d.R, steps, true))) ? 1 : 0;
-  }
+  // the gradients asked for leave by bulk tensor stores where they can; by plain stores otherwise
+  p.out_maps = ((!p.dx || m3::tc_make_row_map(&p.tm_dx, p.dx, d.B, d.T, d.H, 64 * d.R, steps, true)) &&
+                (!p.db || m3::tc_make_row_map(&p.tm_db, p.db, d.B, d.T, d.H, 128 * d.R, steps, true)) &&
+                (!p.dc || m3::tc_make_row_map(&p.tm_dc, p.dc, d.B, d.T, d.H, 128 * d.R, steps, true))) ? 1 : 0;
   char* seg = nullptr;
   cudaError_t e;
   if (ahead) {
@@ -296,7 +287,7 @@ int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* i
     p.dpsum = dphi + per_tok * 64;
     e = plan_ahead(ctx, p, d, desc, nseg, tps, in->dy, in->dh, saved->tc_ckpt_angle, false, &seg);
   } else {
-    e = plan_segments(ctx, p, tiles, !p.use_tma, &seg);
+    e = plan_segments(ctx, p, tiles, true, true, d.rot != 0, &seg);
   }
   if (e == cudaSuccess) e = m3::tc_backward(ctx->stream, p, d.rot != 0);
   if (seg) {
@@ -545,38 +536,28 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     p.err = ctx->dev_err;
     p.B = d.B; p.T = d.T; p.H = d.H; p.R = d.R; p.disc = d.disc; p.rev = d.rev; p.ths = d.ths;
     p.wait_limit = ctx->wait_limit ? ctx->wait_limit : (1u << 18);
-    // Few stripes: segments of them run side by side (the role-split kernels only, which the forward pass also takes
-    // when it is the backward pass that will be cut; a caller that must not allocate has a fixed block for them).
+    // Few stripes: segments of them run side by side (a caller that must not allocate has a fixed block for them).
     const int ntiles = m3::tc_tiles(d.T, d.R);
-    int nseg = 1, tps = ntiles, bseg, btps;
-    const bool direct = d.R == 1 && !d.rot && d.rev == 0 && d.T % 8 == 0;
+    int nseg = 1, tps = ntiles;
     // A state that is replaced in place is read by a stripe's first segment: its last one must not run beside that.
     const bool in_place = p.h0 && ((p.h_out && p.h_out == p.h0) || (p.lu_out && p.lu_out == p.lu0) ||
                                    (p.angle_out && p.angle_out == p.angle0));
-    bool ahead = !in_place && m3::tc_ahead_plan((int)BH, ntiles, false, direct, &nseg, &tps);
+    bool ahead = !in_place && m3::tc_ahead_plan((int)BH, ntiles, false, d.rot != 0, d.R, &nseg, &tps);
     if (ahead && ctx->no_scratch) {
       m3::TcAhead a{};
       a.nseg = nseg;
       a.tps = tps;
       ahead = m3::tc_ahead_bytes((int)BH, &a, nullptr) <= ctx->fixed_bytes;
     }
-    const bool bwd_ahead = saved && m3::tc_ahead_plan((int)BH, ntiles, true, direct, &bseg, &btps);
-    // Rank 1 with real dynamics needs no conversion of its rows: bulk tensor copies land them in
-    // operand layout (every head left to right, T a multiple of 8, 16-byte aligned tensors).
-    p.use_tma = (!ahead && !bwd_ahead && direct &&
-                 m3::tc_make_tile_map(&p.tm_b, p.b, d.B, d.T, d.H, 128) && m3::tc_make_tile_map(&p.tm_c, p.c, d.B, d.T, d.H, 128) &&
-                 m3::tc_make_tile_map(&p.tm_x, p.x, d.B, d.T, d.H, 64)) ? 1 : 0;
-    if (!p.use_tma) {
-      // every other shape: the raw rows of b and c are fetched by bulk tensor copies, a tile at a time
-      const int steps = m3::tc_tile_steps(d.R);
-      if (!m3::tc_make_row_map(&p.tm_b, p.b, d.B, d.T, d.H, 128 * d.R, steps, true) ||
-          !m3::tc_make_row_map(&p.tm_c, p.c, d.B, d.T, d.H, 128 * d.R, steps, true))
-        return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs 16-byte aligned b and c");
-      if (d.rot && !m3::tc_make_row_map(&p.tm_th, p.theta, d.B, d.T, d.H, 64, steps, false, d.ths))
-        return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs a 16-byte aligned theta");
-      // y leaves by bulk tensor stores where it can (a 16-byte aligned tensor); by plain stores otherwise
-      p.out_maps = m3::tc_make_row_map(&p.tm_y, p.y, d.B, d.T, d.H, 64 * d.R, steps, true) ? 1 : 0;
-    }
+    // the raw rows of b and c are fetched by bulk tensor copies, a tile at a time
+    const int steps = m3::tc_tile_steps(d.R);
+    if (!m3::tc_make_row_map(&p.tm_b, p.b, d.B, d.T, d.H, 128 * d.R, steps, true) ||
+        !m3::tc_make_row_map(&p.tm_c, p.c, d.B, d.T, d.H, 128 * d.R, steps, true))
+      return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs 16-byte aligned b and c");
+    if (d.rot && !m3::tc_make_row_map(&p.tm_th, p.theta, d.B, d.T, d.H, 64, steps, false, d.ths))
+      return fail(ctx, M3_ERR_UNSUPPORTED, "the tensor-core family needs a 16-byte aligned theta");
+    // y leaves by bulk tensor stores where it can (a 16-byte aligned tensor); by plain stores otherwise
+    p.out_maps = m3::tc_make_row_map(&p.tm_y, p.y, d.B, d.T, d.H, 64 * d.R, steps, true) ? 1 : 0;
     char* base = nullptr;
     size_t bytes = 0;
     if (saved) {  // the backward pass needs the state and the angle entering every tile
@@ -590,7 +571,7 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
     // a caller that must not allocate gets whole stripes: cutting them needs scratch
     char* seg = nullptr;
     cudaError_t te = ahead ? plan_ahead(ctx, p, d, *desc, nseg, tps, nullptr, nullptr, nullptr, saved != nullptr, &seg)
-                           : plan_segments(ctx, p, ntiles, !p.use_tma && !ctx->no_scratch, &seg);
+                           : plan_segments(ctx, p, ntiles, !ctx->no_scratch, false, d.rot != 0, &seg);
     if (te == cudaSuccess) te = m3::tc_forward(ctx->stream, p, d.rot != 0);
     if (seg) {
       if (!ahead) split_chain_leave(ctx);
@@ -614,7 +595,6 @@ int m3_scan_forward(m3_ctx* ctx, const m3_scan_desc* desc, const m3_scan_out* ou
       sv->ws_bytes = bytes;
       sv->tc_ckpt_h = p.ckpt_h;
       sv->tc_ckpt_angle = p.ckpt_angle;
-      sv->tc_direct = p.use_tma != 0;
       sv->stream = ctx->stream;
       *saved = sv;
     }

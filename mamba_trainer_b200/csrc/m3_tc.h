@@ -20,14 +20,6 @@ inline bool tc_supported(const m3_scan_desc& s) {
 inline int tc_tile_steps(int rank) { return 128 / rank; }
 inline int tc_tiles(int seq, int rank) { return (seq + tc_tile_steps(rank) - 1) / tc_tile_steps(rank); }
 
-// A tensor map that lands a [128 tokens x cols] bf16 tile of a dense [B, T, H, cols] tensor directly in
-// the kernels' operand layout (8 x 8 core matrices tiled [rows/8][cols/8]): dimensions
-// (8 elements, 8 tokens, H*cols/8 column groups, B*T/8 token groups), box (8, 8, cols/8, 16), so the
-// tile of (batch b, head h, first token t0) is the box at (0, 0, h*cols/8, (b*T + t0)/8).  Needs T % 8 == 0
-// and a 16-byte aligned base.  Returns false when the driver refuses (the caller then takes the
-// register path).
-bool tc_make_tile_map(CUtensorMap* map, const void* base, int B, int T, int H, int cols);
-
 // A tensor map over the rows of a dense [B, T, H, cols] bf16 tensor as the caller stores them:
 // dimensions (cols, H, T, B), box (64, 1, steps, 1), so 64 columns of `steps` consecutive time steps of
 // one (batch, head) land as a dense [steps][128 bytes] panel (one request per 64 columns), rows past
@@ -38,11 +30,10 @@ bool tc_make_tile_map(CUtensorMap* map, const void* base, int B, int T, int H, i
 bool tc_make_row_map(CUtensorMap* map, const void* base, int B, int T, int H, int cols, int steps, bool swizzle, int tok_stride = 0);
 
 struct TcFwdParams {
-  alignas(64) CUtensorMap tm_b, tm_c, tm_x;   // tile maps of the direct form when use_tma, else row maps of b and c
-  alignas(64) CUtensorMap tm_th;              // row map of theta (rotational dynamics, role-split kernel)
+  alignas(64) CUtensorMap tm_b, tm_c;         // row maps of b and c
+  alignas(64) CUtensorMap tm_th;              // row map of theta (rotational dynamics)
   alignas(64) CUtensorMap tm_y;               // row map of y: its tiles leave by bulk tensor stores when out_maps
   int out_maps;
-  int use_tma;        // rank 1, real dynamics, T % 8 == 0, no right-to-left heads
   const __nv_bfloat16 *x, *b, *c, *dt, *lam, *theta;
   const float *a_log, *d_skip, *h0, *lu0, *angle0;
   __nv_bfloat16* y;
@@ -54,17 +45,23 @@ struct TcFwdParams {
   int rev;            // the last `rev` heads walk time right to left
   int ths;            // elements between consecutive tokens of theta
   uint32_t wait_limit; // iteration limit of the bounded waits (m3_ctx_set_wait_limit)
-  // time segments of a stripe (role-split kernel; work distribution in m3_tc_roles.cuh): nseg == 1 hands nothing over
+  // time segments of a stripe (work distribution in m3_tc_roles.cuh): nseg == 1 hands nothing over
   int nseg, tps, grid;
   int ahead;          // 1: seg_state and seg_angle hold every boundary's state before the launch (m3_tc_ahead.cu)
   float *seg_state, *seg_angle;
   int* seg_flag;
 };
 
-// How a launch of the role-split kernels cuts its stripes in time: enough items to keep every SM busy to
-// the end (about six per SM), segments of at least four tiles.  Returns segments per stripe, tiles per
+// What a 128-row tile takes inside a stripe, microseconds measured on a B200: what plans weigh cuts by.
+inline float tc_tile_us(bool backward, bool rot, int rank) {
+  if (backward) return !rot ? 10.0f : (rank == 1 ? 14.2f : 13.2f);
+  return rank == 1 ? (rot ? 5.3f : 4.6f) : (rot ? 4.5f : 3.8f);
+}
+
+// How a launch of the stripe kernels cuts its stripes in time (m3_tc_fwd.cu).  Returns segments per stripe, tiles per
 // segment and the grid; bytes of hand-over scratch (state, angle, flags) through *scratch_bytes.
-void tc_segment_plan(int BH, int tiles, bool allow_split, int* nseg, int* tps, int* grid, size_t* scratch_bytes);
+void tc_segment_plan(int BH, int tiles, bool allow_split, bool backward, bool rot, int rank, int* nseg, int* tps, int* grid,
+                     size_t* scratch_bytes);
 
 // Segments that run side by side (m3_tc_ahead.cu): the state and angle at every boundary are worked out first, in the
 // seg_state / seg_angle the stripe kernels read, and nothing is handed over.
@@ -75,8 +72,7 @@ struct TcAhead {
   float *hs, *asum, *cd;          // per group
   float *seg_state, *seg_angle;   // per segment
 };
-// `direct`: whole stripes would run the direct form.
-bool tc_ahead_plan(int BH, int tiles, bool backward, bool direct, int* nseg, int* tps);
+bool tc_ahead_plan(int BH, int tiles, bool backward, bool rot, int rank, int* nseg, int* tps);
 // nseg and tps given: fills in the rest; bytes of scratch.
 size_t tc_ahead_bytes(int BH, TcAhead* a, char* base);
 // dy NULL: forward; else the gradient of the state (dh: the one reaching the returned state, or NULL).  full_angle: the
@@ -87,17 +83,11 @@ cudaError_t tc_ahead(cudaStream_t st, const Dims& d, const m3_scan_desc& in, con
 cudaError_t tc_forward(cudaStream_t st, const TcFwdParams& p, bool rotational);
 // load_kernels of every kernel that a forward pass may launch.
 cudaError_t tc_load();
-cudaError_t tc_direct_load();
 cudaError_t tc_ahead_load();
-// The direct form (rank 1, real dynamics, use_tma): m3_tc_fwd_direct.cu.
-cudaError_t tc_forward_direct(cudaStream_t st, const TcFwdParams& p);
-
 struct TcBwdParams {
-  alignas(64) CUtensorMap tm_b, tm_c;   // tile maps of the direct form when use_tma, else row maps of b and c
-  alignas(64) CUtensorMap tm_x, tm_dy, tm_th;  // row maps of x, dy and theta (role-split kernel)
+  alignas(64) CUtensorMap tm_b, tm_c, tm_x, tm_dy, tm_th;  // row maps of the inputs and dy
   alignas(64) CUtensorMap tm_dx, tm_db, tm_dc; // row maps of the gradients asked for: their tiles leave by bulk tensor stores when out_maps
   int out_maps;
-  int use_tma;
   const __nv_bfloat16 *x, *b, *c, *dt, *lam, *theta, *dy;
   const float *a_log, *d_skip, *h0, *lu0;
   const float *dh, *dlu, *dangle;        // gradients reaching the returned state, or NULL
@@ -121,7 +111,5 @@ struct TcBwdParams {
 };
 
 cudaError_t tc_backward(cudaStream_t st, const TcBwdParams& p, bool rotational);
-// The direct form (rank 1, real dynamics, use_tma): m3_tc_bwd_direct.cu.
-cudaError_t tc_backward_direct(cudaStream_t st, const TcBwdParams& p);
 
 }  // namespace m3

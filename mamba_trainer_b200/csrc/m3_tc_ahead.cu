@@ -498,15 +498,15 @@ cudaError_t tc_ahead_load() {
 }
 
 // Whether to cut `BH` stripes of `tiles` tiles into segments that run side by side, and into how many.  Microseconds,
-// measured on a B200: a tile takes about 5.5 forward and 15 backward inside a stripe (5.2 and 11 in the direct form, which
-// whole stripes may have), an item costs about one more to start and finish; working out what a tile adds to the state
+// measured on a B200: a tile takes tc_tile_us inside a stripe, an item about one more to start and finish; working out what
+// a tile adds to the state
 // takes about 4 per tile and SM, and the two launches and the pass some 12 more.  Beyond a third of the SMs it takes long
 // stripes to gain anything (96 stripes of 16 tiles: nothing; 64 of 248: forward + backward 3.47 -> 2.06 ms).
-bool tc_ahead_plan(int BH, int tiles, bool backward, bool direct, int* nseg, int* tps) {
+bool tc_ahead_plan(int BH, int tiles, bool backward, bool rot, int rank, int* nseg, int* tps) {
   const int sms = sm_count();
   if (BH > sms || tiles < (BH > sms / 3 ? 24 : 3)) return false;
-  const float c = backward ? 15.0f : 5.5f, whole = direct ? (backward ? 11.0f : 5.2f) : c;
-  float best = 0.92f * tiles * whole;
+  const float c = tc_tile_us(backward, rot, rank);
+  float best = 0.92f * tiles * c;
   bool found = false;
   for (int n = 2; n <= tiles && n <= 4 * sms; ++n) {
     const int per = (tiles + n - 1) / n, segs = (tiles + per - 1) / per;

@@ -22,7 +22,6 @@
 // the tile has finished with (d x over dS, d B over the scaled copies, d C over dG).
 // The (cos, sin) table of the tile's angles is computed once, used for the rotation, and kept in 64
 // TMEM columns for the un-rotation of the gradients (its shared-memory buffer becomes M in between).
-// Rank 1 with real dynamics has a second form (m3_tc_bwd_direct.cu).
 #include "m3_tc.h"
 #include "m3_tc_roles.cuh"
 
@@ -98,8 +97,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
   // Two sets of per-token scalars: the look-ahead warp fills the next tile's while this tile is worked on.
   auto scal_set = [&](int i) {
     float* q = sc + i * kNumScal * kScal;
-    return TileScalars{q, q + kScal, q + 2 * kScal, q + 3 * kScal, q + 4 * kScal, q + 5 * kScal, q + 6 * kScal,
-                       q + 7 * kScal, q + 8 * kScal};
+    return TileScalars{q, q + kScal, q + 2 * kScal, q + 3 * kScal, q + 4 * kScal, q + 5 * kScal, q + 6 * kScal, q + 7 * kScal};
   };
   float* part_row = sc + 2 * kNumScal * kScal;   // [2][128]
   float* part_t1 = part_row + 256;    // [2][128]
@@ -928,7 +926,6 @@ cudaError_t launch_r(cudaStream_t st, const TcBwdParams& p, bool rot) {
 }  // namespace
 
 cudaError_t tc_backward(cudaStream_t st, const TcBwdParams& p, bool rot) {
-  if (p.use_tma && p.R == 1 && !rot) return tc_backward_direct(st, p);
   switch (p.R) {
     case 1: return launch_r<1>(st, p, rot);
     case 2: return launch_r<2>(st, p, rot);

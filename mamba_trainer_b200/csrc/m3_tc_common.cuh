@@ -113,15 +113,6 @@ __device__ __forceinline__ void raise_flag(int* flag) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-// One box of a 4-D tiled tensor map whose two inner coordinates are zero (see tc_make_tile_map).
-__device__ __forceinline__ void tma_load_tile(void* dst, const void* tensor_map, uint64_t* bar, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(
-          smem_u32(dst)),
-      "l"(tensor_map), "r"(smem_u32(bar)), "r"(0), "r"(0), "r"(c2), "r"(c3)
-      : "memory");
-}
-
 // One box of a row map (tc_make_row_map): columns from `col`, head h, time steps from t (may be negative
 // or run past the end: those rows arrive as zeros), batch b.
 __device__ __forceinline__ void tma_load_rows(void* dst, const void* tensor_map, uint64_t* bar, int col, int h, int t, int b) {

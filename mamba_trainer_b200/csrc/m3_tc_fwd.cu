@@ -16,8 +16,7 @@
 //           of H refreshed for the next tile
 // bf16 operands, fp32 accumulation and state; shapes: head_dim 64, d_state 128, R in {1,2,4}.
 // Warp roles, barriers and the distribution of stripes (or time segments of stripes) over CTAs:
-// m3_tc_roles.cuh.  Rank 1 with real dynamics has a second form (m3_tc_fwd_direct.cu) whose rows need no
-// conversion and land in operand layout by bulk TENSOR copies.
+// m3_tc_roles.cuh.
 #include "m3_internal.h"
 #include "m3_tc.h"
 #include "m3_tc_roles.cuh"
@@ -56,8 +55,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_con
   float* sc = reinterpret_cast<float*>(smem + SM::off_sc);
   auto scal_set = [&](int i) {
     float* q = sc + i * kNumScal * kScal;
-    return TileScalars{q, q + kScal, q + 2 * kScal, q + 3 * kScal, q + 4 * kScal, q + 5 * kScal, q + 6 * kScal,
-                       q + 7 * kScal, q + 8 * kScal};
+    return TileScalars{q, q + kScal, q + 2 * kScal, q + 3 * kScal, q + 4 * kScal, q + 5 * kScal, q + 6 * kScal, q + 7 * kScal};
   };
   float* s_q = reinterpret_cast<float*>(smem + SM::off_q);
   float* s_carry = s_q + 8 * kNH;
@@ -504,14 +502,54 @@ cudaError_t launch_r(cudaStream_t st, const TcFwdParams& p, bool rot) {
 
 }  // namespace
 
-void tc_segment_plan(int BH, int tiles, bool allow_split, int* nseg, int* tps, int* grid, size_t* scratch_bytes) {
+bool tc_make_row_map(CUtensorMap* map, const void* base, int B, int T, int H, int cols, int steps, bool swizzle, int tok_stride) {
+  typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static EncodeFn encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess) fn = nullptr;
+    return reinterpret_cast<EncodeFn>(fn);
+  }();
+  if (!encode || cols % 64 || steps < 1 || steps > 256 || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
+  const cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)H, (cuuint64_t)T, (cuuint64_t)B};
+  const cuuint64_t tok = tok_stride ? (cuuint64_t)tok_stride * 2 : (cuuint64_t)H * cols * 2;
+  const cuuint64_t strides[3] = {(cuuint64_t)cols * 2, tok, (cuuint64_t)T * tok};
+  const cuuint32_t box[4] = {64, 1, (cuuint32_t)steps, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Segments of one stripe run one after the other, so cutting adds no parallelism: it evens out the last round when there
+// are more stripes than SMs.  What it costs is an item's start - the hand-over, rows and states that nothing has requested
+// ahead: some 9 us for a whole stripe's CTA, 16 forward and 12 backward for an item.  With segments of four tiles whatever
+// the rest (six items an SM were the only aim) 384 stripes of 16 tiles, rank 1, took 424 us forward and 729 backward,
+// whole 287 and 721; 256 of 12 tiles 233 and 391, whole 154 and 385.  192 of 32 tiles, rank 2, in three: 268 and 641, whole
+// 303 and 858.  The cut has to promise 4 %.
+void tc_segment_plan(int BH, int tiles, bool allow_split, bool backward, bool rot, int rank, int* nseg, int* tps, int* grid,
+                     size_t* scratch_bytes) {
   const int sms = sm_count();
-  int want = 1;
-  // Segments of one stripe run one after the other, so cutting adds no parallelism: it only evens out the
-  // last round when there are more stripes than SMs.
-  while (allow_split && BH > sms && (long long)BH * want < 6LL * sms && tiles / (want * 2) >= 4) want *= 2;
-  const int per = (tiles + want - 1) / want;
-  const int n = (tiles + per - 1) / per;
+  const float c = tc_tile_us(backward, rot, rank);
+  int n = 1, per = tiles;
+  if (allow_split && BH > sms) {
+    const float whole = (float)((BH + sms - 1) / sms) * (tiles * c + 9.0f);
+    float best = 0.96f * whole;
+    for (int want = 2; want <= 16 && want <= tiles; ++want) {
+      const int p = (tiles + want - 1) / want, segs = (tiles + p - 1) / p;
+      if (segs != want) continue;
+      const long long rounds = ((long long)BH * segs + sms - 1) / sms;
+      const float t = (float)rounds * (p * c + (backward ? 12.0f : 16.0f));
+      if (t < best) {
+        best = t;
+        n = segs;
+        per = p;
+      }
+    }
+  }
   *nseg = n;
   *tps = per;
   // whole stripes: one CTA each, handed out by the hardware; cut stripes: one CTA per SM at most, each
@@ -528,14 +566,13 @@ static cudaError_t load_r() {
                       tc_fwd_kernel<R, true, 2>, tc_fwd_kernel<R, false, 2>);
 }
 cudaError_t tc_load() {
-  cudaError_t e = tc_direct_load();
+  cudaError_t e = cudaSuccess;
   for (cudaError_t (*f)() : {load_r<1>, load_r<2>, load_r<4>, tc_ahead_load})
     if (e == cudaSuccess) e = f();
   return e;
 }
 
 cudaError_t tc_forward(cudaStream_t st, const TcFwdParams& p, bool rot) {
-  if (p.use_tma && p.R == 1 && !rot) return tc_forward_direct(st, p);
   switch (p.R) {
     case 1: return launch_r<1>(st, p, rot);
     case 2: return launch_r<2>(st, p, rot);

@@ -115,66 +115,78 @@ __device__ __forceinline__ void raise_handover(int* flag) {
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok); }
 
 // ---------------------------------------------------------------------------------------
-// Per-token scalars of one tile, by ONE warp (the arithmetic of tile_scalars): g, w (shifted add), inclusive cumulative sum
-// ac of a = dt A, sw = exp(cd - ac) w, eac = exp(ac), column factors cf.  32 steps at a time, in loops that stay rolled:
-// the warp finds its code cold every tile and pays for its length (with the EPL steps of a lane unrolled it took up to
-// 24 K cycles of a 27 K cycle backward tile).
+// Per-token scalars of one tile, by ONE warp: g, w (shifted add), inclusive cumulative sum ac of a = dt A,
+// sw = exp(cd - ac) w, eac = exp(ac), column factors cf.  (As rolled loops over 32 steps at a time, a third of the
+// instructions for a warp that finds its code cold: its longer chain showed where a tile is short - real dynamics,
+// rank 1, forward 359 -> 418 us for 64 stripes of 128 tiles.)
+// Lane i owns the EPL consecutive steps i*EPL .. i*EPL + EPL - 1.
 // ---------------------------------------------------------------------------------------
 template <int R>
 struct ScalarLoads {
   static constexpr int EPL = (kRows / R) / 32;
-  float dt[EPL], lam[EPL], dt_next, lam_next;   // steps 32 i + lane; the step after the tile
+  float dt[EPL + 1], lam[EPL + 1];
 };
-// dt and lambda of the tile at t0 and of one step beyond, requested a whole tile before they are used: the loads are few
-// but each is a sector of its own.
+// dt and lambda of the steps lane * EPL .. lane * EPL + EPL of the tile at t0 (one step of look-ahead),
+// requested a whole tile before they are used: the loads are few but each is a sector of its own.
 template <int R>
 __device__ __forceinline__ void lookahead_load(ScalarLoads<R>& v, const __nv_bfloat16* dt, const __nv_bfloat16* lam,
                                                int disc, int b, int h, int H, int T, int t0, bool rev) {
   constexpr int EPL = ScalarLoads<R>::EPL;
   const int lane = threadIdx.x & 31;
-  const float lam0 = disc == 1 ? 0.5f : 1.0f;
 #pragma unroll
   for (int i = 0; i <= EPL; ++i) {
-    const int t = t0 + 32 * i + (i < EPL ? lane : 0);
-    float d = 0.0f, la = lam0;
+    const int t = t0 + lane * EPL + i;
+    v.dt[i] = 0.0f;
+    v.lam[i] = 1.0f;
     if (t < T) {
       const size_t idx = ((size_t)b * T + (rev ? T - 1 - t : t)) * H + h;
-      d = bf(dt, idx);
-      if (disc > 1) la = bf(lam, idx);
+      v.dt[i] = bf(dt, idx);
+      v.lam[i] = disc == 0 ? 1.0f : (disc == 1 ? 0.5f : bf(lam, idx));
     }
-    if (i < EPL) { v.dt[i] = d; v.lam[i] = la; } else { v.dt_next = d; v.lam_next = la; }
   }
 }
 template <int R>
 __device__ __forceinline__ void lookahead_scalars(const TileScalars& s, const ScalarLoads<R>& v, float A, int T, int t0) {
   constexpr int LT = kRows / R, EPL = LT / 32, SPC = 16 / R;
   const int lane = threadIdx.x & 31;
+  float loc[EPL], wv[EPL];
+  float run = 0.0f;
 #pragma unroll
-  for (int i = 0; i < EPL; ++i) { s.dt[32 * i + lane] = v.dt[i]; s.lam[32 * i + lane] = v.lam[i]; }
-  if (lane == 0) { s.dt[LT] = v.dt_next; s.lam[LT] = v.lam_next; }
-  __syncwarp();
-  float cd = 0.0f;
-#pragma unroll 1
-  for (int l = lane; l < LT; l += 32) {
-    const float d = s.dt[l], gv = s.lam[l] * d;   // (dt is zero from T on)
-    const float f = t0 + l + 1 < T ? (1.0f - s.lam[l + 1]) * s.dt[l + 1] : 0.0f;
-    float ac = d * A;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float n = __shfl_up_sync(0xffffffffu, ac, o);
-      if (lane >= o) ac += n;
+  for (int i = 0; i < EPL; ++i) {
+    const int l = lane * EPL + i, t = t0 + l;
+    float gv = 0.0f, w = 0.0f, av = 0.0f;
+    if (t < T) {
+      gv = v.lam[i] * v.dt[i];
+      const float f = (t + 1 < T) ? (1.0f - v.lam[i + 1]) * v.dt[i + 1] : 0.0f;
+      w = gv + f;
+      av = v.dt[i] * A;
     }
-    ac += cd;
-    s.g[l] = gv; s.w[l] = t0 + l < T ? gv + f : 0.0f; s.ac[l] = ac;
-    cd = __shfl_sync(0xffffffffu, ac, 31);
+    s.dt[l] = v.dt[i]; s.lam[l] = v.lam[i]; s.g[l] = gv; s.w[l] = w;
+    wv[i] = w;
+    run += av;
+    loc[i] = run;
+  }
+  if (lane == 31) { s.dt[LT] = v.dt[EPL]; s.lam[LT] = v.lam[EPL]; }
+  float tot = run;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float n = __shfl_up_sync(0xffffffffu, tot, o);
+    if (lane >= o) tot += n;
+  }
+  const float base = tot - run;
+  const float cd = __shfl_sync(0xffffffffu, tot, 31);
+#pragma unroll
+  for (int i = 0; i < EPL; ++i) {
+    loc[i] += base;
+    s.ac[lane * EPL + i] = loc[i];
   }
   __syncwarp();
-#pragma unroll 1
-  for (int l = lane; l < LT; l += 32) {
-    const float ac = s.ac[l];
-    s.sw[l] = expc(cd - ac) * s.w[l];
-    s.eac[l] = expc(ac);
-    s.cf[l] = __expf(fmaxf(s.ac[(l / SPC) * SPC + SPC - 1] - ac, -87.0f));
+#pragma unroll
+  for (int i = 0; i < EPL; ++i) {
+    const int l = lane * EPL + i;
+    s.sw[l] = expc(cd - loc[i]) * wv[i];
+    s.eac[l] = expc(loc[i]);
+    s.cf[l] = __expf(fmaxf(s.ac[(l / SPC) * SPC + SPC - 1] - loc[i], -87.0f));
   }
 }
 

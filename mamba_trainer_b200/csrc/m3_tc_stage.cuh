@@ -27,8 +27,6 @@ __device__ __forceinline__ float inside(float d) { return (d > -60.0f && d < 0.0
 // l & 7: threads that own different rows read the same plane group without bank conflicts.
 __device__ __forceinline__ int phi_idx(int l, int m) { return l * kNH + ((((m >> 2) ^ (l & 7)) << 2) | (m & 3)); }
 
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
 template <int R>
 __device__ __forceinline__ void load_row_group(const __nv_bfloat16* src, bool live, uint32_t (&raw)[4 * R]) {
   if (live) {
@@ -103,10 +101,10 @@ __device__ __forceinline__ void load_chunk(const uint8_t* base, uint32_t off, fl
 
 // Scalar arrays of one tile, all [kScal] floats in shared memory.
 struct TileScalars {
-  float *dt, *lam, *a, *ac, *g, *w, *sw, *eac;
+  float *dt, *lam, *ac, *g, *w, *sw, *eac;   // step; lambda; cumulative log decay; diagonal and off-diagonal weight; exp(cd - ac) w; exp(ac)
   float *cf;   // cf[s] = exp(ac[e(s)] - ac[s]) <= 1, e(s) = last time step of s's 16-column chunk
 };
-constexpr int kNumScal = 9;  // arrays in a TileScalars block
+constexpr int kNumScal = 8;  // arrays in a TileScalars block
 
 // Decay between a row's step l and the columns of one 16-column chunk, factorised so that a
 // thread pays ONE exponential per chunk: exp(ac_l - ac_s) = exp(ac_l - ac_e) * cf[s].  The row
@@ -115,79 +113,6 @@ constexpr int kNumScal = 9;  // arrays in a TileScalars block
 // representable contribution left) and at e^-87 below.
 __device__ __forceinline__ float row_factor(float ac_l, float ac_e) {
   return __expf(fminf(fmaxf(ac_l - ac_e, -87.0f), 80.0f));
-}
-
-// dt and lambda of step t0 + i in thread 32 + i (i <= LT: one step of look-ahead), as registers, so
-// the loads of the NEXT tile can be in flight while the current one computes.
-template <int R>
-__device__ __forceinline__ void load_dt_lam(float& vdt, float& vl, const __nv_bfloat16* dt, const __nv_bfloat16* lam,
-                                            int disc, int b, int h, int H, int T, int t0, bool rev) {
-  constexpr int LT = kRows / R;
-  const int tid = (int)threadIdx.x - 32, t = t0 + tid;
-  vdt = 0.0f;
-  vl = 1.0f;
-  if (tid >= 0 && tid <= LT && t >= 0 && t < T) {
-    const size_t i = ((size_t)b * T + (rev ? T - 1 - t : t)) * H + h;  // t is a scan position
-    vdt = bf(dt, i);
-    vl = disc == 0 ? 1.0f : (disc == 1 ? 0.5f : bf(lam, i));
-  }
-}
-
-// In the direct kernels the per-tile scalars are the work of warps 1-7: warp 0 holds the thread that issues
-// the tensor-core products, and that thread is held up by the tensor pipe for as long as the products run, so
-// it must not be needed at a barrier meanwhile.  Warps 1-7 meet at named barrier 1 (224 threads); every one
-// of their threads must reach each of its uses.
-__device__ __forceinline__ void scalar_warps_sync() { asm volatile("bar.sync 1, 224;" ::: "memory"); }
-
-// g, w (shifted add), a = dt A, its inclusive cumulative sum ac, sw = exp(cd - ac) w,
-// eac = exp(ac) and the column factors cf, from the (dt, lambda) registers of load_dt_lam.
-// The caller's next __syncthreads makes them visible to everyone (warp 0 included).
-template <int R>
-__device__ __forceinline__ void tile_scalars(const TileScalars& s, float vdt, float vl, float A, int T, int t0) {
-  constexpr int LT = kRows / R;
-  if (threadIdx.x < 32) return;  // warp 0 takes no part (see scalar_warps_sync)
-  const int tid = (int)threadIdx.x - 32, warp = tid >> 5, lane = tid & 31;
-  if (tid <= LT) {
-    s.dt[tid] = vdt;
-    s.lam[tid] = vl;
-  }
-  scalar_warps_sync();
-  if (tid < LT) {
-    const int t = t0 + tid;
-    float gv = 0.0f, wv = 0.0f, av = 0.0f;
-    if (t < T) {
-      gv = s.lam[tid] * s.dt[tid];
-      const float f = (t + 1 < T) ? (1.0f - s.lam[tid + 1]) * s.dt[tid + 1] : 0.0f;
-      wv = gv + f;
-      av = s.dt[tid] * A;
-    }
-    s.g[tid] = gv; s.w[tid] = wv; s.a[tid] = av;
-  }
-  scalar_warps_sync();
-  if (warp == 0) {  // the first of the seven
-    constexpr int EPL = LT / 32;
-    float loc[EPL];
-    float run = 0.0f;
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) { run += s.a[lane * EPL + i]; loc[i] = run; }
-    float tot = run;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float n = __shfl_up_sync(0xffffffffu, tot, o);
-      if (lane >= o) tot += n;
-    }
-    const float base = tot - run;
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) s.ac[lane * EPL + i] = base + loc[i];
-  }
-  scalar_warps_sync();
-  if (tid < LT) {
-    constexpr int SPC = 16 / R;  // time steps per 16-column chunk
-    const float cd = s.ac[LT - 1], ac = s.ac[tid];
-    s.sw[tid] = expc(cd - ac) * s.w[tid];
-    s.eac[tid] = expc(ac);
-    s.cf[tid] = __expf(fmaxf(s.ac[(tid / SPC) * SPC + SPC - 1] - ac, -87.0f));
-  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -272,69 +197,6 @@ __device__ __forceinline__ void load_col_scalars(ColScalars<R>& c, const TileSca
     c.w[4 * i] = b.x; c.w[4 * i + 1] = b.y; c.w[4 * i + 2] = b.z; c.w[4 * i + 3] = b.w;
     c.g[4 * i] = d.x; c.g[4 * i + 1] = d.y; c.g[4 * i + 2] = d.z; c.g[4 * i + 3] = d.w;
   }
-}
-
-// ---------------------------------------------------------------------------------------
-// Output staging: a thread owns a ROW of an accumulator tile, but the caller's tensors want
-// whole rows written by neighbouring lanes.  Rows go to shared memory first ([128][C] bf16,
-// 16-byte chunks XOR-swizzled by row & 7 so that both the row-owner writes and the
-// row-spanning reads are conflict-free), then leave as coalesced 16-byte stores, with the
-// rank de-interleave ((t, r) rows -> [.., C, R] elements) done on the way out.
-// ---------------------------------------------------------------------------------------
-template <int C>
-__device__ __forceinline__ uint32_t stg_off(int row, int chunk) {
-  return (uint32_t)(row * (C * 2) + ((chunk ^ (row & 7)) << 4));
-}
-template <int C>
-__device__ __forceinline__ void stage_store16(uint8_t* stg, int row, int col0, const float (&v)[16]) {
-  uint4 q0, q1;
-  q0.x = pack_bf16(v[0], v[1]); q0.y = pack_bf16(v[2], v[3]); q0.z = pack_bf16(v[4], v[5]); q0.w = pack_bf16(v[6], v[7]);
-  q1.x = pack_bf16(v[8], v[9]); q1.y = pack_bf16(v[10], v[11]); q1.z = pack_bf16(v[12], v[13]); q1.w = pack_bf16(v[14], v[15]);
-  *reinterpret_cast<uint4*>(stg + stg_off<C>(row, col0 >> 3)) = q0;
-  *reinterpret_cast<uint4*>(stg + stg_off<C>(row, (col0 >> 3) + 1)) = q1;
-}
-// Tile rows (l * R + r) -> g[(tok0 + l * H) * C * R + c * R + r], tokens t0 + l < T only.
-// One item per 16 output bytes, consecutive items -> consecutive addresses, so every store
-// instruction of a warp writes 512 contiguous bytes whatever the rank.  The ranks are interleaved
-// in registers: output word w of a token's chunk holds elements (j, r), (j, r + 1) with
-// j = 2w / R, r = 2w % R, i.e. one 16-bit half from each of two neighbouring rank rows.
-template <int R, int C>
-__device__ __forceinline__ void copy_out(const uint8_t* stg, __nv_bfloat16* g, size_t tok0, int H, int T, int t0) {
-  constexpr int LT = kRows / R, CPR = C / 8;  // source chunks per row
-#pragma unroll
-  for (int i = 0; i < LT * CPR * R / 256; ++i) {
-    const int it = threadIdx.x + 256 * i;
-    const int o = it % R, c = (it / R) % CPR, l = it / (R * CPR);
-    if (t0 + l >= T) continue;
-    uint4 q;
-    if (R == 1) {
-      q = *reinterpret_cast<const uint4*>(stg + stg_off<C>(l, c));
-    } else {
-      uint32_t w4[4];
-#pragma unroll
-      for (int wi = 0; wi < 4; ++wi) {
-        const int w = 4 * o + wi, j = (2 * w) / R, r = (2 * w) % R;
-        const uint32_t lo = *reinterpret_cast<const uint32_t*>(stg + stg_off<C>(l * R + r, c) + ((j >> 1) << 2));
-        const uint32_t hi = *reinterpret_cast<const uint32_t*>(stg + stg_off<C>(l * R + r + 1, c) + ((j >> 1) << 2));
-        w4[wi] = __byte_perm(lo, hi, (j & 1) ? 0x7632 : 0x5410);
-      }
-      q = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-    }
-    *reinterpret_cast<uint4*>(g + (tok0 + (size_t)l * H) * C * R + (size_t)c * 8 * R + (size_t)o * 8) = q;
-  }
-}
-
-// Sum over the 256 threads of the CTA; red: >= 8 floats of shared scratch.  Contains two syncs.
-__device__ __forceinline__ float cta_sum(float v, float* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float s = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) s += red[i];
-  return s;
 }
 
 // v[32] per lane -> returns on lane j the sum over the warp's lanes of v[j].
