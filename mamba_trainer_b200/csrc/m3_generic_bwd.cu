@@ -43,10 +43,11 @@ static void final_tokens(cudaStream_t st, const Dims& d, const m3_scan_desc& des
                          float* dalog, float* ddsk, const m3_scan_grads* raw) {
   const unsigned blocks = (unsigned)(((size_t)d.B * d.T * d.H + 255) / 256);
   const HeadSums hs{desc.a_log, dalog, ddsk};
-  kb_final<T><<<blocks + (hs.any() ? d.H : 0), 256, 0, st>>>(
+  const int heads = hs.any() ? d.H : 0;
+  kb_final<T><<<blocks + heads, 256, 0, st>>>(
       d, static_cast<const T*>(desc.dt), static_cast<const T*>(desc.lambda), desc.a_log, bw, (desc.h0 && !d.raw) ? 1 : 0,
       static_cast<T*>(ddt), static_cast<T*>(dlam), raw ? static_cast<T*>(raw->da_raw) : nullptr,
-      raw ? static_cast<T*>(raw->dg_raw) : nullptr, raw ? static_cast<T*>(raw->dw_raw) : nullptr, hs, (int)blocks);
+      raw ? static_cast<T*>(raw->dg_raw) : nullptr, raw ? static_cast<T*>(raw->dw_raw) : nullptr, hs, heads);
 }
 
 template <class T>

@@ -231,13 +231,13 @@ template <class T>
 __global__ void kb_final(Dims d, const T* __restrict__ dt, const T* __restrict__ lam,
                          const float* __restrict__ a_log, GenericBwdWs bw, int has_state,
                          T* __restrict__ ddt, T* __restrict__ dlam, T* __restrict__ da_raw, T* __restrict__ dg_raw,
-                         T* __restrict__ dw_raw, HeadSums hs, int token_blocks) {
-  if ((int)blockIdx.x >= token_blocks) {   // the blocks behind those of the tokens: one per head
+                         T* __restrict__ dw_raw, HeadSums hs, int head_blocks) {
+  if ((int)blockIdx.x < head_blocks) {   // the blocks ahead of those of the tokens: one per head
     __shared__ float red[8];
-    head_sums(d, blockIdx.x - token_blocks, hs, bw, red);
+    head_sums(d, blockIdx.x, hs, bw, red);
     return;
   }
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t i = (size_t)(blockIdx.x - head_blocks) * blockDim.x + threadIdx.x;
   const size_t total = (size_t)d.B * d.T * d.H;
   if (i >= total) return;
   const int h = i % d.H;

@@ -456,20 +456,23 @@ __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoin
 // ---- rotational dynamics: the later chunks' d phi on top, then per token d theta, d dt and d lambda (the arithmetic of
 // kb_final).  A warp per step, lanes over planes; a block per d.L steps, `per_seg` blocks to a segment whose sums of d phi
 // are complete within it, `nseg` of those (here the chunks; the tensor-core family's segments are longer).
-// Behind these rows of blocks, one block per head for its sums.  A warp requests eight steps before it uses the first (as a
-// loop over steps it waited for each pair of loads: float32, 8 x 1024 tokens x 16 heads, 42 us; its bytes take 15).
+// Ahead of these rows of blocks (`head_rows`), one block per head for its sums.  A warp requests its next four steps before
+// it uses the first (as a loop over steps it waited for each pair of loads), and what the per-token part needs with them:
+// float32, 8 x 1024 tokens x 16 heads, d_state 128, 42 -> 25 us; its bytes take 15.  (Eight steps, fewer blocks: 35.)
 template <class T, int N>
 __global__ void __launch_bounds__(256) k_rows_final(Dims d, m3_scan_desc in, RowsBwdWs rw, GenericBwdWs bw, int has_state,
                                                     T* __restrict__ ddt, T* __restrict__ dlam, T* __restrict__ dtheta,
-                                                    float* __restrict__ dangle0, int per_seg, int nseg, HeadSums hs) {
-  constexpr int NH = N / 2, NQ = 256 / NH, PL = NH / 32, U = 8;
+                                                    float* __restrict__ dangle0, int per_seg, int nseg, HeadSums hs, int head_rows) {
+  constexpr int NH = N / 2, NQ = 256 / NH, PL = NH / 32, U = 4;
   __shared__ float s_off[NQ][NH], s_rot[128], red[8];
-  if (blockIdx.z || (int)blockIdx.y >= d.B * d.H) {
-    const int h = ((int)blockIdx.y - (blockIdx.z ? 0 : d.B * d.H)) * (int)gridDim.x + (int)blockIdx.x;
+  if (blockIdx.z || (int)blockIdx.y < head_rows) {
+    const int h = (int)blockIdx.y * (int)gridDim.x + (int)blockIdx.x;
     if (h < d.H) head_sums(d, h, hs, bw, red);
     return;
   }
-  const Chunk c = this_chunk(d);
+  Chunk c;
+  c.k = blockIdx.x; c.bh = blockIdx.y - head_rows;
+  c.b = c.bh / d.H; c.h = c.bh - c.b * d.H; c.t0 = c.k * d.L;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const T* dt = static_cast<const T*>(in.dt);
   const T* theta = static_cast<const T*>(in.theta);
@@ -489,6 +492,18 @@ __global__ void __launch_bounds__(256) k_rows_final(Dims d, m3_scan_desc in, Row
     }
   };
   load(warp);
+  // what the per-token part at the end needs, requested with the rest
+  const int t_own = c.t0 + tid;
+  const bool own = tid < d.L && t_own < d.T && (ddt || dlam);
+  const size_t o_own = (size_t)c.bh * d.Tp + (own ? t_own : c.t0), i_own = own ? tok_index(d, c.b, t_own, c.h) : 0;
+  float own_da = 0.0f, own_gw = 0.0f, own_dwm1 = 0.0f, own_dt = 0.0f, own_lam = 0.0f;
+  if (own) {
+    own_da = bw.da[o_own];
+    own_gw = bw.dg[o_own] + bw.dw[o_own];
+    own_dwm1 = t_own > 0 ? bw.dw[o_own - 1] : 0.0f;
+    own_dt = ldf(dt, i_own);
+    own_lam = lambda_at(static_cast<const T*>(in.lambda), d.disc, i_own);
+  }
   {
     const int q = tid / NH, m = tid % NH;
     float s = 0.0f;
@@ -525,31 +540,30 @@ __global__ void __launch_bounds__(256) k_rows_final(Dims d, m3_scan_desc in, Row
     if (lane % (32 / U) == 0 && l < d.L) s_rot[l] = sum;
   }
   __syncthreads();
-  const int t = c.t0 + tid;
-  if (tid < d.L && t < d.T && (ddt || dlam)) {
-    const size_t o = (size_t)c.bh * d.Tp + t, ti = tok_index(d, c.b, t, c.h);
+  if (own) {
     const float A = -expf(in.a_log[c.h]);
-    const float vdt0 = ldf(dt, ti), vl = lambda_at(static_cast<const T*>(in.lambda), d.disc, ti);
-    const float gw = bw.dg[o] + bw.dw[o], dwm1 = t > 0 ? bw.dw[o - 1] : 0.0f;
-    float vdl = gw * vdt0 - dwm1 * vdt0;
-    float vdd = bw.da[o] * A + gw * vl + dwm1 * (1.0f - vl) + s_rot[tid];
-    if (has_state && t == 0) {
+    float vdl = own_gw * own_dt - own_dwm1 * own_dt;
+    float vdd = own_da * A + own_gw * own_lam + own_dwm1 * (1.0f - own_lam) + s_rot[tid];
+    if (has_state && t_own == 0) {
       const float ip = bw.ip0[c.bh];
-      vdl -= vdt0 * ip;
-      vdd += (1.0f - vl) * ip;
+      vdl -= own_dt * ip;
+      vdd += (1.0f - own_lam) * ip;
     }
-    if (ddt) stf(ddt, ti, vdd);
-    if (dlam) stf(dlam, ti, vdl);
+    if (ddt) stf(ddt, i_own, vdd);
+    if (dlam) stf(dlam, i_own, vdl);
   }
 }
 
 template <class T, int N>
 cudaError_t final_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const RowsBwdWs& rw, const GenericBwdWs& bw, void* ddt,
                     void* dlam, void* dtheta, float* dangle0, int per_seg, int nseg, const HeadSums& hs) {
-  const int nx = (d.T + d.L - 1) / d.L, BH = d.B * d.H, ny = BH + (hs.any() ? (d.H + nx - 1) / nx : 0);
-  const dim3 grid = ny <= 65535 ? dim3(nx, ny) : dim3(nx, BH, 2);   // (a layer of its own where the rows are used up)
+  const int nx = (d.T + d.L - 1) / d.L, BH = d.B * d.H;
+  int rows = hs.any() ? (d.H + nx - 1) / nx : 0;
+  const bool layer = BH + rows > 65535;   // (the heads' blocks in a layer of their own where the rows are used up)
+  if (layer) rows = 0;
+  const dim3 grid(nx, BH + rows, layer ? 2 : 1);
   k_rows_final<T, N><<<grid, 256, 0, st>>>(d, in, rw, bw, in.h0 ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam),
-                                                   static_cast<T*>(dtheta), dangle0, per_seg, nseg, hs);
+                                                   static_cast<T*>(dtheta), dangle0, per_seg, nseg, hs, rows);
   return cudaGetLastError();
 }
 
