@@ -198,6 +198,7 @@ __device__ __forceinline__ void act_forward(const Front& f, const FrontOut& o, i
 
 template <class T, int N, int R, int RUN>
 __global__ void __launch_bounds__(kWarps * 32, 3) k_front_fwd(Front f, FrontOut o, int nx, int nb) {
+  after_predecessor();
   using P = Place<N, R>;
   constexpr int kStage = R > 1 ? kWarps * 4 * 128 : 1;
   __shared__ __align__(16) T stage[kStage];   // ranks > 1: four steps of every warp's rows, [time lane][step][n * R + r]
@@ -385,6 +386,7 @@ __device__ __forceinline__ void act_backward(const Front& f, const FrontGrads& g
 
 template <class T, int N, int R, int RUN>
 __global__ void __launch_bounds__(kBwdWarps * 32, 3) k_front_bwd(Front f, FrontGrads gr, int nx, int nb) {
+  after_predecessor();
   using P = Place<N, R>;
   __shared__ __align__(16) float ahead[kBwdWarps][KT - 1][128];   // g of every warp's first three steps, for the warp before it
   __shared__ __align__(16) float red[kBwdWarps][128];
@@ -656,6 +658,7 @@ struct SumPlan {
 };
 __global__ void __launch_bounds__(32 * kSumRows) k_front_sums(SumPlan plan, const float* __restrict__ part, size_t pitch, int nblk,
                                                              int N) {
+  after_predecessor();
   __shared__ float red[kSumRows][33];
   int i = 0;
   while (i + 1 < plan.n && (int)blockIdx.x >= plan.r[i + 1].first_block) ++i;
@@ -745,8 +748,8 @@ cudaError_t forward_t(cudaStream_t st, const Front& f, const FrontOut& o) {
   front_tiles<N, R>(f, &nx, &nb);
   const int run = front_long(f, nx + 2 * nb) ? 16 : 4;
   const dim3 grid(nx + 2 * nb + 1, (f.T + kWarps * run - 1) / (kWarps * run), f.B);
-  if (run == 16) k_front_fwd<T, N, R, 16><<<grid, kWarps * 32, 0, st>>>(f, o, nx, nb);
-  else k_front_fwd<T, N, R, 4><<<grid, kWarps * 32, 0, st>>>(f, o, nx, nb);
+  if (run == 16) launch(k_front_fwd<T, N, R, 16>, grid, kWarps * 32, 0, st, f, o, nx, nb);
+  else launch(k_front_fwd<T, N, R, 4>, grid, kWarps * 32, 0, st, f, o, nx, nb);
   return cudaGetLastError();
 }
 template <class T, int N, int R>
@@ -755,12 +758,12 @@ cudaError_t backward_t(cudaStream_t st, const Front& f, const FrontGrads& g) {
   front_tiles<N, R>(f, &nx, &nb);
   const int steps = bwd_steps(f, nx + 2 * nb);
   const dim3 grid(nx + 2 * nb + 1, (f.T + steps - 1) / steps, f.B);
-  if (steps == kBwdWarps * 32) k_front_bwd<T, N, R, 32><<<grid, kBwdWarps * 32, 0, st>>>(f, g, nx, nb);
-  else k_front_bwd<T, N, R, 8><<<grid, kBwdWarps * 32, 0, st>>>(f, g, nx, nb);
+  if (steps == kBwdWarps * 32) launch(k_front_bwd<T, N, R, 32>, grid, kBwdWarps * 32, 0, st, f, g, nx, nb);
+  else launch(k_front_bwd<T, N, R, 8>, grid, kBwdWarps * 32, 0, st, f, g, nx, nb);
   const int nblk = (int)(grid.y * grid.z);
   const SumPlan plan = sum_plan(f, g, nblk);
   if (plan.blocks)
-    k_front_sums<<<plan.blocks, dim3(32, kSumRows), 0, st>>>(plan, g.part, part_layout(f).total, nblk, N);
+    launch(k_front_sums, plan.blocks, dim3(32, kSumRows), 0, st, plan, g.part, part_layout(f).total, nblk, N);
   return cudaGetLastError();
 }
 

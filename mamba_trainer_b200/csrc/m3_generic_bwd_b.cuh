@@ -232,6 +232,7 @@ __global__ void kb_final(Dims d, const T* __restrict__ dt, const T* __restrict__
                          const float* __restrict__ a_log, GenericBwdWs bw, int has_state,
                          T* __restrict__ ddt, T* __restrict__ dlam, T* __restrict__ da_raw, T* __restrict__ dg_raw,
                          T* __restrict__ dw_raw, HeadSums hs, int head_blocks) {
+  after_predecessor();
   if ((int)blockIdx.x < head_blocks) {   // the blocks ahead of those of the tokens: one per head
     __shared__ float red[8];
     head_sums(d, blockIdx.x, hs, bw, red);

@@ -393,6 +393,7 @@ __device__ __forceinline__ float silu_grad(float v) {
 template <class T, bool VEC>
 __global__ void k_gate_fwd(size_t ntok, int Cn, long long zs, const T* __restrict__ y, const T* __restrict__ z,
                            T* __restrict__ out) {
+  m3::after_predecessor();
   constexpr int V = VEC ? (int)(16 / sizeof(T)) : 1;
   const int per_row = Cn / V;
   const size_t n = ntok * per_row;
@@ -418,6 +419,7 @@ __global__ void k_gate_fwd(size_t ntok, int Cn, long long zs, const T* __restric
 template <class T, bool VEC>
 __global__ void k_gate_bwd(size_t ntok, int Cn, long long zs, const T* __restrict__ y, const T* __restrict__ z,
                            const T* __restrict__ dout, T* __restrict__ dy, T* __restrict__ dz) {
+  m3::after_predecessor();
   constexpr int V = VEC ? (int)(16 / sizeof(T)) : 1;
   const int per_row = Cn / V;
   const size_t n = ntok * per_row;
@@ -931,11 +933,11 @@ int m3_gate_forward(m3_ctx* ctx, const m3_gate_desc* s, void* out) {
   const unsigned grid = (unsigned)((items + 255) / 256 < 148 * 16 ? (items + 255) / 256 : 148 * 16);
   if (s->dtype == M3_BF16) {
     using T = __nv_bfloat16;
-    if (vec) k_gate_fwd<T, true><<<grid, 256, 0, ctx->stream>>>(ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<T*>(out));
-    else k_gate_fwd<T, false><<<grid, 256, 0, ctx->stream>>>(ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<T*>(out));
+    if (vec) m3::launch(k_gate_fwd<T, true>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<T*>(out));
+    else m3::launch(k_gate_fwd<T, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<T*>(out));
   } else {
-    if (vec) k_gate_fwd<float, true><<<grid, 256, 0, ctx->stream>>>(ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<float*>(out));
-    else k_gate_fwd<float, false><<<grid, 256, 0, ctx->stream>>>(ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<float*>(out));
+    if (vec) m3::launch(k_gate_fwd<float, true>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<float*>(out));
+    else m3::launch(k_gate_fwd<float, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<float*>(out));
   }
   M3_CUDA(ctx, cudaGetLastError());
   ctx->launches += 1;
@@ -956,11 +958,11 @@ int m3_gate_backward(m3_ctx* ctx, const m3_gate_desc* s, const void* dout, void*
   const unsigned grid = (unsigned)((items + 255) / 256 < 148 * 16 ? (items + 255) / 256 : 148 * 16);
   if (s->dtype == M3_BF16) {
     using T = __nv_bfloat16;
-    if (vec) k_gate_bwd<T, true><<<grid, 256, 0, ctx->stream>>>(ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<const T*>(dout), static_cast<T*>(dy), static_cast<T*>(dz));
-    else k_gate_bwd<T, false><<<grid, 256, 0, ctx->stream>>>(ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<const T*>(dout), static_cast<T*>(dy), static_cast<T*>(dz));
+    if (vec) m3::launch(k_gate_bwd<T, true>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<const T*>(dout), static_cast<T*>(dy), static_cast<T*>(dz));
+    else m3::launch(k_gate_bwd<T, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<const T*>(dout), static_cast<T*>(dy), static_cast<T*>(dz));
   } else {
-    if (vec) k_gate_bwd<float, true><<<grid, 256, 0, ctx->stream>>>(ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<const float*>(dout), static_cast<float*>(dy), static_cast<float*>(dz));
-    else k_gate_bwd<float, false><<<grid, 256, 0, ctx->stream>>>(ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<const float*>(dout), static_cast<float*>(dy), static_cast<float*>(dz));
+    if (vec) m3::launch(k_gate_bwd<float, true>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<const float*>(dout), static_cast<float*>(dy), static_cast<float*>(dz));
+    else m3::launch(k_gate_bwd<float, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<const float*>(dout), static_cast<float*>(dy), static_cast<float*>(dz));
   }
   M3_CUDA(ctx, cudaGetLastError());
   ctx->launches += 1;

@@ -14,6 +14,7 @@ namespace {
 
 template <int N, bool ROT>
 __global__ void __launch_bounds__(256) k_rows_pass_rev(Dims d, const float* __restrict__ dh, RowsWs ws, RowsBwdWs rw) {
+  after_predecessor();
   constexpr int NH = N / 2, PN = kP * N, U = 4;
   const int bh = blockIdx.y;
   const int id = blockIdx.x * 256 + threadIdx.x, m = id % NH, p = id / NH;   // planes (m, m + NH) of rows p, p + 32
@@ -58,6 +59,7 @@ __global__ void __launch_bounds__(256) k_rows_pass_rev(Dims d, const float* __re
 template <class T, int N>
 __global__ void __launch_bounds__(256) k_rows_seed(Dims d, m3_scan_desc in, RowsBwdWs rw, float* __restrict__ ip0,
                                                    float* __restrict__ dh0, float* __restrict__ dlu0) {
+  after_predecessor();
   __shared__ float red[8];
   constexpr int PN = kP * N;
   const int bh = blockIdx.x, b = bh / d.H, h = bh - b * d.H;
@@ -126,6 +128,7 @@ struct AdjOut {
 template <class T, int N, int R, bool ROT>
 __global__ void __launch_bounds__(kAdjThreads<N>, N == 64 ? 2 : 1) k_rows_adjoint(Dims d, m3_scan_desc in, const T* __restrict__ dy, RowsWs ws,
                                                           RowsBwdWs rw, AdjOut<T> out) {
+  after_predecessor();
   extern __shared__ __align__(16) unsigned char smem[];
   AdjSmem<N, R>& sm = *reinterpret_cast<AdjSmem<N, R>*>(smem);
   constexpr int NH = N / 2, PN = kP * N, LT = kRows / R, kAdj = kAdjThreads<N>;
@@ -463,6 +466,7 @@ template <class T, int N>
 __global__ void __launch_bounds__(256) k_rows_final(Dims d, m3_scan_desc in, RowsBwdWs rw, GenericBwdWs bw, int has_state,
                                                     T* __restrict__ ddt, T* __restrict__ dlam, T* __restrict__ dtheta,
                                                     float* __restrict__ dangle0, int per_seg, int nseg, HeadSums hs, int head_rows) {
+  after_predecessor();
   constexpr int NH = N / 2, NQ = 256 / NH, PL = NH / 32, U = 4;
   __shared__ float s_off[NQ][NH], s_rot[128], red[8];
   if (blockIdx.z || (int)blockIdx.y < head_rows) {
@@ -562,7 +566,7 @@ cudaError_t final_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, cons
   const bool layer = BH + rows > 65535;   // (the heads' blocks in a layer of their own where the rows are used up)
   if (layer) rows = 0;
   const dim3 grid(nx, BH + rows, layer ? 2 : 1);
-  k_rows_final<T, N><<<grid, 256, 0, st>>>(d, in, rw, bw, in.h0 ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam),
+  launch(k_rows_final<T, N>, grid, 256, 0, st, d, in, rw, bw, in.h0 ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam),
                                                    static_cast<T*>(dtheta), dangle0, per_seg, nseg, hs, rows);
   return cudaGetLastError();
 }
@@ -579,13 +583,13 @@ cudaError_t backward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, c
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_rows_adjoint<T, N, R, ROT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem<N, R>));
   if (e != cudaSuccess) return e;
-  k_rows_pass_rev<N, ROT><<<dim3(32 * (N / 2) / 256, d.B * d.H), 256, 0, st>>>(d, up.dh, ws, rw);
+  launch(k_rows_pass_rev<N, ROT>, dim3(32 * (N / 2) / 256, d.B * d.H), 256, 0, st, d, up.dh, ws, rw);
   const AdjOut<T> out{static_cast<T*>(want(M3_GRAD_X, g.dx)), static_cast<T*>(want(M3_GRAD_B, g.db)),
                       static_cast<T*>(want(M3_GRAD_C, g.dc)), bw.da, bw.dg, bw.dw, bw.partA, bw.partD,
                       d.raw ? nullptr : up.dlast_u, up.dangle};
-  k_rows_adjoint<T, N, R, ROT><<<grid, kAdjThreads<N>, sizeof(AdjSmem<N, R>), st>>>(d, in, static_cast<const T*>(up.dy), ws, rw, out);
+  launch(k_rows_adjoint<T, N, R, ROT>, grid, kAdjThreads<N>, sizeof(AdjSmem<N, R>), st, d, in, static_cast<const T*>(up.dy), ws, rw, out);
   if (has_state) {
-    k_rows_seed<T, N><<<d.B * d.H, 256, 0, st>>>(d, in, rw, bw.ip0, static_cast<float*>(want(M3_GRAD_H0, g.dh0)),
+    launch(k_rows_seed<T, N>, d.B * d.H, 256, 0, st, d, in, rw, bw.ip0, static_cast<float*>(want(M3_GRAD_H0, g.dh0)),
                                                  d.raw ? nullptr : static_cast<float*>(want(M3_GRAD_LAST_U0, g.dlast_u0)));
     n += 1;
   }

@@ -118,6 +118,7 @@ __device__ __forceinline__ void conv_step(const MixerStep& m, int b, int c, cons
 
 template <class T, int N, int R, int RPT, bool FUSED>
 __global__ void __launch_bounds__(256, 3) k_step_rows(const __grid_constant__ StepRows a) {
+  after_predecessor();
   constexpr int LPR = N / 4, RPW = 32 / LPR, PASS = 8 * RPW * RPT, NH = N / 2, JN = N / 32;
   const m3_step_desc& d = a.d;
   const m3_step_out& o = a.o;
@@ -335,7 +336,7 @@ cudaError_t step_rows_launch(cudaStream_t st, StepRows a) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<grid, 256, smem, st>>>(a);
+  launch(kern, grid, 256, smem, st, a);
   return cudaGetLastError();
 }
 template <class T, int N, bool FUSED>

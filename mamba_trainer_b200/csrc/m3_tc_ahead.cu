@@ -213,6 +213,7 @@ struct HalfAngles {
 // to rotate.
 template <int R>
 __global__ void __launch_bounds__(kThreads) k_group_angle(Dims d, m3_scan_desc in, TcAhead a, int tiles) {
+  after_predecessor();
   __shared__ float2 part[8][32];
   constexpr int LT = 2 * kRows / R;   // steps of a tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -240,6 +241,7 @@ __global__ void __launch_bounds__(kThreads) k_group_angle(Dims d, m3_scan_desc i
 template <int R, bool ROT, bool BWD, bool FULL_ANGLE>
 __global__ void __launch_bounds__(kThreads, 2) k_group_state(Dims d, m3_scan_desc in, const __nv_bfloat16* __restrict__ dy,
                                                              const float* __restrict__ ckpt_angle, TcAhead a, int tiles) {
+  after_predecessor();
   extern __shared__ __align__(128) unsigned char smem[];
   GroupSmem<R>& sm = *reinterpret_cast<GroupSmem<R>*>(smem);
   using IT = Item<R>;
@@ -411,6 +413,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_group_state(Dims d, m3_scan_des
 // ROT: the groups have angles; LOCAL: their states are those of B rotated by the angle since the group's start.
 template <bool ROT, bool BWD, bool LOCAL>
 __global__ void __launch_bounds__(256) k_group_pass(Dims d, m3_scan_desc in, const float* __restrict__ dh, TcAhead a, int count) {
+  after_predecessor();
   using T = __nv_bfloat16;
   constexpr int U = 8;
   const int bh = blockIdx.y, b = bh / d.H, h = bh - b * d.H;
@@ -477,10 +480,10 @@ cudaError_t ahead_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, cons
   const int count = (a.nseg - 1) * a.gps;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmem<R>));
   if (e != cudaSuccess) return e;
-  if (FULL_ANGLE) k_group_angle<R><<<dim3(count, d.B * d.H), kThreads, 0, st>>>(d, in, a, tc_tiles(d.T, R));
-  kern<<<dim3(count, d.B * d.H), kThreads, sizeof(GroupSmem<R>), st>>>(d, in, static_cast<const __nv_bfloat16*>(dy), ckpt_angle, a,
+  if (FULL_ANGLE) launch(k_group_angle<R>, dim3(count, d.B * d.H), kThreads, 0, st, d, in, a, tc_tiles(d.T, R));
+  launch(kern, dim3(count, d.B * d.H), kThreads, sizeof(GroupSmem<R>), st, d, in, static_cast<const __nv_bfloat16*>(dy), ckpt_angle, a,
                                                                        tc_tiles(d.T, R));
-  k_group_pass<ROT, BWD, ROT && !BWD && !FULL_ANGLE><<<dim3(32 * kNH / 256, d.B * d.H), 256, 0, st>>>(d, in, dh, a, count);
+  launch(k_group_pass<ROT, BWD, ROT && !BWD && !FULL_ANGLE>, dim3(32 * kNH / 256, d.B * d.H), 256, 0, st, d, in, dh, a, count);
   return cudaGetLastError();
 }
 

@@ -22,6 +22,7 @@
 // the tile has finished with (d x over dS, d B over the scaled copies, d C over dG).
 // The (cos, sin) table of the tile's angles is computed once, used for the rotation, and kept in 64
 // TMEM columns for the un-rotation of the gradients (its shared-memory buffer becomes M in between).
+#include "m3_internal.h"
 #include "m3_tc.h"
 #include "m3_tc_roles.cuh"
 
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = *tmem_slot;
+  after_predecessor();
 
   if (warp == kCopyWarp) {
     regs_for_helpers();
@@ -919,7 +921,7 @@ cudaError_t launch_r(cudaStream_t st, const TcBwdParams& p, bool rot) {
                           : (rot ? tc_bwd_kernel<R, true, 1> : tc_bwd_kernel<R, false, 1>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
   if (e != cudaSuccess) return e;
-  kern<<<p.grid, kCtaThreads, kSmemBytes, st>>>(p);
+  launch(kern, p.grid, kCtaThreads, kSmemBytes, st, p);
   return cudaGetLastError();
 }
 

@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_fwd_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = *tmem_slot;
+  after_predecessor();
 
   if (warp == kCopyWarp) {
     regs_for_helpers();
@@ -496,7 +497,7 @@ cudaError_t launch_r(cudaStream_t st, const TcFwdParams& p, bool rot) {
   constexpr uint32_t bytes = FwdSmem<R>::bytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e != cudaSuccess) return e;
-  kern<<<p.grid, kCtaThreads, bytes, st>>>(p);
+  launch(kern, p.grid, kCtaThreads, bytes, st, p);
   return cudaGetLastError();
 }
 
