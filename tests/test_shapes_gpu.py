@@ -373,3 +373,47 @@ def test_a_state_replaced_in_place(dtype, H, N, R, T, rot):
             assert float((torch.sin(a) - torch.sin(e)).abs().max()) <= (2e-3 if tol else 0.0)
         else:
             assert norm_rel(a.float(), e.float()) <= tol, n
+
+
+@pytest.mark.parametrize("rank,rot,seq,rev", [
+    (2, True, 1465, 1),      # 23 tiles in three segments, each way
+    (4, False, 730, 0),      # 23 tiles forward in two
+    (1, False, 1001, 0),     # rank 1, real dynamics, no multiple of eight: eight tiles, cut in the backward pass only
+])
+def test_longer_stripes_cut_in_time_equal_whole_ones(rank, rot, seq, rev):
+    """160 stripes long enough that the plan cuts them (it weighs rounds by what a tile and an item's start take)."""
+    from test_scan_gpu import test_time_segments_leave_results_unchanged
+    test_time_segments_leave_results_unchanged(rank, rot, seq, rev)
+
+
+def test_real_dynamics_of_rank_1_match_the_oracle_at_multiples_of_eight():
+    """Sequences a multiple of eight, whole stripes: more heads than are cut side by side."""
+    from test_scan_gpu import check_bf16, compare_all, small_inputs
+    t, ds = small_inputs(6, 264, 10, 64, 128, 1, False, True, seed=3)
+    for k in ("b", "c"):
+        t[k] = t[k] / 128 ** 0.5
+    t["dt"] = t["dt"] * 0.2
+    for k in ("x", "b", "c", "dt", "lam", "dy"):
+        t[k] = t[k].to(torch.bfloat16)
+    compare_all(t, 64, check_bf16, True, ds, path=2)
+
+
+def test_per_head_sums_where_the_grid_has_no_row_left():
+    """65535 stripes: the heads' blocks of the last launch, which lie ahead of the stripes' rows, get a layer of their own.
+    The sums equal those of the two halves (float32 sums of 65535 terms: 1e-4)."""
+    from _util import fused_run
+    from mamba_trainer_b200 import synthetic
+    w = synthetic.Workload("rows", 65535, 2, 1, 64, 64, 64, 1, torch.float32, Discretization.LearnedTrapezoid, True, "rms")
+    t = synthetic.make_inputs(w, seed=7)
+    _, _, g = fused_run(t, 64, False, True)
+    sums = {}
+    for lo, hi in ((0, 30000), (30000, 65535)):
+        part = {k: v if v is None or k in ("a_log", "d_skip") else v[lo:hi] for k, v in t.items()}
+        _, _, gp = fused_run(part, 64, False, True)
+        for n, v in gp.items():
+            if n in ("a_log", "d_skip"):
+                sums[n] = sums.get(n, 0) + v.double()
+            else:
+                assert torch.equal(g[n][lo:hi], v), n
+    for n, v in sums.items():
+        assert torch.allclose(g[n].double(), v, rtol=1e-4, atol=1e-3), (n, g[n], v)
