@@ -31,7 +31,6 @@ from mamba_trainer_b200 import sharding, synthetic  # noqa: E402
 # from the committed ncu captures under profiles/ (a small case of the same instantiation; traffic is
 # proportional to the token-heads a launch processes).  None where no capture was taken.
 NCU_TRAFFIC_BYTES_PER_TOKEN_HEAD = {
-    "cfg1_siso_trapezoid_bf16": 267403520 / (8 * 2048 * 12),
     # profiles/tc_fwd_bwd_kernels_cfg4.md: batch 4 x seq 4096 (whole stripes) and batch 8 x seq 4096 (stripes cut
     # into time segments, which adds the hand-over of the state between segments)
     "cfg4_mimo2_scaling_bf16": {"whole": 1722.7e6 / (4 * 4096 * 32), "split": 3560.8e6 / (8 * 4096 * 32)},
@@ -39,7 +38,7 @@ NCU_TRAFFIC_BYTES_PER_TOKEN_HEAD = {
 
 
 def traffic_per_token_head(w, sms: int):
-    """The captured DRAM traffic per (token, head) of the instantiation this shard runs: the library cuts
+    """The captured DRAM traffic per (token, head) of the instantiation this shard runs: at these lengths the library cuts
     stripes in time when there are more stripes than SMs but fewer than six per SM (tc_segment_plan)."""
     v = NCU_TRAFFIC_BYTES_PER_TOKEN_HEAD.get(w.name)
     if isinstance(v, dict):
