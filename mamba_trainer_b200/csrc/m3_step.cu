@@ -25,13 +25,15 @@ constexpr int kStepMaxRows = 64;
 // FUSED, the rotation) runs while they are under way, the update happens in place in shared memory and the new state
 // leaves by two bulk copies.  No register holds state in flight, so the number of bytes in flight is that of the
 // resident CTAs' buffers (the first version, with the state prefetched into registers, had 103 registers per thread
-// and 25 % occupancy and ran at 2.5 TB/s; batch 64 x 32 heads x 64 x 128, rank 2: 94 us -> 64 us, 69 % of the measured copy bandwidth).
+// and 25 % occupancy and ran at 2.5 TB/s; batch 64 x 32 heads x 64 x 128, rank 2: 94 us -> 64 us; 57 us with
+// the prefetch of step_ahead: 77 % of the measured copy bandwidth).
 // A step is latency bound while the grid is small (rows per CTA go down to 8: more CTAs) and HBM bound once it is
 // large (64 rows per CTA: the prologue is shared by all of them); see step_rows_per_cta.
 struct StepRows {
   m3_step_desc d;
   m3_step_out o;
   int rows;       // state rows of a CTA
+  unsigned ahead; // a CTA brings into L2 what the one this many places later will read; 0: none
   int* err;       // raised when the wait for the copies gives up
   uint32_t wait_limit;
   MixerStep mx;
@@ -116,6 +118,45 @@ __device__ __forceinline__ void conv_step(const MixerStep& m, int b, int c, cons
   for (int i = 0; i < V; ++i) out[i] = round_to(proj_row, __fdividef(acc.v[i], 1.0f + __expf(-acc.v[i])));
 }
 
+// Called by one warp: requests into L2 the state of the CTA `ahead` places later in the grid and, eight regions of four
+// 128-byte lines, what its prologue reads of its own (a longer region's rest is left; B, C and the parameters are shared by
+// CTAs and in L2 anyway).  Hints only, of addresses that the later CTA does read.
+template <class T, int N, int R, bool FUSED>
+__device__ __forceinline__ void prefetch_later(const StepRows& a) {
+  const m3_step_desc& d = a.d;
+  const MixerStep& mx = a.mx;
+  const unsigned at = blockIdx.x + blockIdx.y * gridDim.x + a.ahead;
+  if (at >= gridDim.x * gridDim.y) return;
+  constexpr int NH = N / 2, kElt = (int)sizeof(T);
+  const int P = d.head_dim, bh = (int)(at % gridDim.x), p_lo = (int)(at / gridDim.x) * a.rows, nrows = min(P - p_lo, a.rows);
+  const int lane = threadIdx.x & 31, region = lane >> 2, byte = (lane & 3) * 128;
+  if (lane < 2) m3tc::bulk_prefetch((lane ? d.last_u : d.h) + ((size_t)bh * P + p_lo) * N, (uint32_t)(nrows * N * 4));
+  const void* p = nullptr;
+  int bytes = 0;
+  if (region == 7) {
+    if (d.dynamics == M3_ROTATIONAL && d.angle) p = d.angle + (size_t)bh * NH, bytes = NH * 4;
+  } else if (FUSED) {
+    const int h = bh % d.heads, b = bh / d.heads, col = (h * P + p_lo) * R;
+    const T* pr = static_cast<const T*>(mx.proj) + (size_t)b * mx.width;
+    bytes = nrows * R * kElt;
+    if (region == 6) {
+      p = pr + mx.off_theta + h * NH, bytes = d.dynamics == M3_ROTATIONAL ? NH * kElt : 0;
+    } else if (region >= 2) {   // the carried inputs of x's channels
+      p = static_cast<const T*>(mx.conv_in) + ((size_t)b * (mx.K - 1) + region - 2) * mx.conv_channels + col;
+      if (region - 2 >= mx.K - 1) bytes = 0;
+    } else {
+      p = pr + col + (region ? mx.d_inner : 0);   // z, x
+    }
+  } else if (region == 0) {
+    p = static_cast<const T*>(d.x) + ((size_t)bh * P + p_lo) * R, bytes = nrows * R * kElt;
+  } else if (region < 3) {
+    p = static_cast<const T*>(region == 1 ? d.b : d.c) + (size_t)bh * N * R, bytes = N * R * kElt;
+  } else if (region == 3 && d.dynamics == M3_ROTATIONAL) {
+    p = static_cast<const T*>(d.theta) + (size_t)bh * NH, bytes = NH * kElt;
+  }
+  if (byte < bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(p) + byte));
+}
+
 template <class T, int N, int R, int RPT, bool FUSED>
 __global__ void __launch_bounds__(256, 3) k_step_rows(const __grid_constant__ StepRows a) {
   after_predecessor();
@@ -139,6 +180,7 @@ __global__ void __launch_bounds__(256, 3) k_step_rows(const __grid_constant__ St
     m3tc::bulk_load(s_h, d.h + slab, slab_bytes, &bar);
     m3tc::bulk_load(s_u, d.last_u + slab, slab_bytes, &bar);
   }
+  if (a.ahead && warp == 7) prefetch_later<T, N, R, FUSED>(a);
   // ---- scalars, angles -------------------------------------------------------------------------------------
   const T* pr = FUSED ? static_cast<const T*>(mx.proj) + (size_t)b * mx.width : nullptr;
   float dt, lam;
@@ -323,6 +365,13 @@ inline int step_rows_per_cta(int bh, int head_dim, int pass1) {
   return (rows + pass1 - 1) / pass1 * pass1;
 }
 
+// A grid of several waves (three CTAs per SM) is bound by the chain inside a CTA as much as by bytes: its small loads wait
+// behind the state of its neighbours.  Each CTA therefore requests into L2 what the CTA one per SM later needs.
+// Mixer steps, d_state 128, bf16, behind a flushed L2, us: 64 sequences x 32 heads of rank 1 / 2 / 4: 65.5 / 69.6 / 79.9 -> 59.4 / 63.5
+// / 75.8; 128 x 32: 114.8 -> 100.4; 256 x 24: 170 -> 137; 24 x 24: 28.7 -> 26.6. The state alone gives half of it or less (128 x 32:
+// 110.8); half a CTA per SM later is as good, two per SM 3 % worse and three 10 %: the requests take bandwidth from what is waited for.
+inline unsigned step_ahead(unsigned ctas) { return ctas > 3u * sm_count() ? (unsigned)sm_count() : 0u; }
+
 inline uint32_t step_wait_limit(const m3_ctx* ctx) { return ctx->wait_limit ? ctx->wait_limit : (1u << 18); }
 
 template <class T, int N, int R, bool FUSED>
@@ -330,6 +379,7 @@ cudaError_t step_rows_launch(cudaStream_t st, StepRows a) {
   constexpr int kPass1 = 8 * (128 / N);   // rows of a pass with one row per thread
   a.rows = step_rows_per_cta(a.d.batch * a.d.heads, a.d.head_dim, kPass1);
   const dim3 grid(a.d.batch * a.d.heads, (a.d.head_dim + a.rows - 1) / a.rows);
+  a.ahead = step_ahead(grid.x * grid.y);
   const int smem = (int)sizeof(float) * a.rows * (2 * N + 2 * R);
   auto kern = a.rows > kPass1 ? k_step_rows<T, N, R, 2, FUSED> : k_step_rows<T, N, R, 1, FUSED>;
   if (smem > 44 * 1024) {
@@ -369,7 +419,7 @@ cudaError_t mixer_step(const m3_ctx* ctx, const m3_step_desc& d, const m3_step_o
   auto ok = [](const void* p, size_t a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
   m.vec4 = m.width % 4 == 0 && m.d_inner % 4 == 0 && m.bc % 4 == 0 && (d.head_dim * d.rank) % 4 == 0 && ok(m.proj, 4 * es) &&
            ok(m.conv_in, 4 * es) && ok(m.conv_out, 4 * es) && ok(m.conv_w, 16) && ok(m.conv_b, 16);
-  return step_rows<true>(ctx->stream, StepRows{d, o, 0, ctx->dev_err, step_wait_limit(ctx), m});
+  return step_rows<true>(ctx->stream, StepRows{d, o, 0, 0, ctx->dev_err, step_wait_limit(ctx), m});
 }
 
 template <class T>
@@ -510,7 +560,7 @@ extern "C" int m3_step_forward(m3_ctx* ctx, const m3_step_desc* d, const m3_step
   cudaError_t e = cudaSetDevice(ctx->device);
   if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "cudaSetDevice");
   if (m3::step_rows_supported(d->head_dim, d->d_state, d->rank, {d->h, d->last_u, o->h, o->last_u})) {
-    e = m3::step_rows<false>(ctx->stream, m3::StepRows{*d, *o, 0, ctx->dev_err, m3::step_wait_limit(ctx), {}});
+    e = m3::step_rows<false>(ctx->stream, m3::StepRows{*d, *o, 0, 0, ctx->dev_err, m3::step_wait_limit(ctx), {}});
     if (e != cudaSuccess) return m3::cuda_fail(ctx, e, "decode step");
     ctx->launches += 1;
     return M3_OK;

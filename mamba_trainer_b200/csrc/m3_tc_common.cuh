@@ -124,6 +124,9 @@ __device__ __forceinline__ void tma_load_rows(void* dst, const void* tensor_map,
 }
 
 // The same box into L2 only, for a tma_load_rows to come.
+__device__ __forceinline__ void bulk_prefetch(const void* gmem, uint32_t bytes) {   // into L2; 16-byte address and size
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_rows(const void* tensor_map, int col, int h, int t, int b) {
   asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(tensor_map), "r"(col), "r"(h), "r"(t), "r"(b)
                : "memory");

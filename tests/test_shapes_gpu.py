@@ -39,6 +39,36 @@ def test_decode_step_matches_the_parallel_pass(dtype, B, H, P, N, R, groups, K, 
     assert ref_metric(got.float(), whole.float()) <= (2e-4 if dtype == torch.float32 else 3e-2)
 
 
+@pytest.mark.parametrize("dtype,H,P,N,R,K,rot,fused", [
+    (torch.bfloat16, 16, 64, 128, 2, 4, True, True),
+    (torch.bfloat16, 15, 96, 128, 4, 2, True, True),      # two blocks a head, the second of half the rows
+    (torch.float32, 15, 72, 64, 1, 8, False, True),       # more taps than are brought in ahead, no angles
+    (torch.float32, 16, 64, 128, 4, 4, True, False),
+    (torch.bfloat16, 17, 96, 64, 1, 4, False, False),
+])
+def test_decode_steps_of_several_waves_equal_small_ones(dtype, H, P, N, R, K, rot, fused):
+    """Grids of more than three blocks per SM bring later blocks' inputs into L2; three rows of the batch alone do not.  The
+    arithmetic is the same up to the order of a row's sums: float32 outputs within N float32 roundings, bf16 within two."""
+    from mamba_trainer_b200.nn import MixerCache, MixerCore, MixerShape
+    from mamba_trainer_b200.ssm import SsmState, mamba3_step
+    B, few = 3 * torch.cuda.get_device_properties(0).multi_processor_count // H + 2, slice(0, 3)
+    torch.manual_seed(H)
+    r = lambda *s: torch.randn(*s, device="cuda")
+    h, u, ang = r(B, H, P, N), r(B, H, P, N), r(B, H, N // 2)
+    state = lambda rows: SsmState(h[rows], u[rows], ang[rows] if rot else None)
+    if fused:
+        core = MixerCore(MixerShape(H, P, N, R, rotational=rot), conv_kernel=K, device="cuda")
+        proj, conv = r(B, 1, core.shape.in_proj_width).to(dtype), r(B, K - 1, core.shape.conv_channels).to(dtype)
+        run = lambda rows: core.forward_cached(proj[rows], MixerCache(conv[rows], state(rows)))[0]
+    else:
+        ins = [r(B, H, P, R), r(B, H, N, R), r(B, H, N, R) / N ** 0.5, r(B, H).abs(), torch.sigmoid(r(B, H))]
+        theta, a_log = r(B, H, N // 2), r(H)
+        run = lambda rows: mamba3_step(*(t[rows].to(dtype) for t in ins), a_log, theta[rows] if rot else None, None, state(rows))[0]
+    tol = N * 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -8
+    for rows in (few, slice(B - 3, B)):
+        assert norm_rel(run(slice(0, B))[rows].float(), run(rows).float()) <= tol
+
+
 @pytest.mark.parametrize("dtype,B,T,H,N,R,rot,state,rev,disc", [
     (torch.float32, 2, 64, 2, 128, 1, True, False, 0, 2),     # exactly one chunk
     (torch.float32, 1, 1, 3, 64, 1, True, True, 0, 2),        # one token
