@@ -22,7 +22,8 @@ struct Dims {
 };
 
 // First of all in a kernel that launch() starts: wait for the kernel before it on the stream (nothing of that one may be read or
-// overwritten earlier).  The kernel behind is let in when this one's blocks have ended, not sooner (griddepcontrol.
+// overwritten earlier, and no TMEM taken: that kernel need not be one of this library, and if it lets its successor in before its own
+// blocks have allocated theirs, each would wait for the other for good).  The kernel behind is let in when this one's blocks have ended, not sooner (griddepcontrol.
 // launch_dependents at the start): blocks that wait held slots the running ones could use - float32 mixer, 8 x 1024 tokens,
 // 16 heads: 1132 us without any of this, 1184 with the early start, 1103 without.
 __device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -144,13 +144,13 @@ __global__ void __launch_bounds__(kCtaThreads, 1) tc_bwd_kernel(const __grid_con
     mbar_init(&bars[3], 1);
     mbar_init(&bars[4], 1);
   }
+  after_predecessor();   // (ahead of the TMEM: see there)
   if (warp == 0) tmem_alloc(tmem_slot, TM_COLS);
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = *tmem_slot;
-  after_predecessor();
 
   if (warp == kCopyWarp) {
     regs_for_helpers();
