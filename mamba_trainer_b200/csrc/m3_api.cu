@@ -133,7 +133,7 @@ namespace {
 // bounded waits.  Within this process they are therefore chained across streams: a launch waits for the event
 // the previous one of the device recorded behind itself.  (They fill every SM anyway, so nothing is lost; launches
 // that wait on nobody - whole stripes, other libraries' kernels - finish on their own and need no such care.)
-// Streams under capture are left alone: a captured graph replays alone on its stream.
+// A graph's launches cannot be chained so - nobody here sees when or beside what it is replayed - and stay whole.
 struct SplitChain {
   std::mutex mu;
   cudaEvent_t ev[64] = {};
@@ -143,12 +143,13 @@ SplitChain& split_chain() {
   static SplitChain c;
   return c;
 }
-cudaError_t split_chain_enter(m3_ctx* ctx) {
+bool capturing(cudaStream_t st) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return cudaSuccess;
-  }
+  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+cudaError_t split_chain_enter(m3_ctx* ctx) {
   const int dev = ctx->device;
   if (dev < 0 || dev >= 64) return cudaSuccess;
   SplitChain& c = split_chain();
@@ -156,11 +157,6 @@ cudaError_t split_chain_enter(m3_ctx* ctx) {
   return c.recorded[dev] ? cudaStreamWaitEvent(ctx->stream, c.ev[dev], 0) : cudaSuccess;
 }
 void split_chain_leave(m3_ctx* ctx) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return;
-  }
   const int dev = ctx->device;
   if (dev < 0 || dev >= 64) return;
   SplitChain& c = split_chain();
@@ -174,7 +170,7 @@ void split_chain_leave(m3_ctx* ctx) {
   else cudaGetLastError();
 }
 
-// Time segments of the stripes for one launch of the role-split kernels: the plan, and - when a stripe is
+// Time segments of the stripes for one launch of the stripe kernels: the plan, and - when a stripe is
 // cut - the hand-over scratch (state, angle, flags; the flags zeroed on the stream).  `*scratch` is null
 // when nothing is handed over; the caller frees it on the stream after the launch.
 template <class Params>
@@ -182,6 +178,7 @@ cudaError_t plan_segments(m3_ctx* ctx, Params& p, int tiles, bool allow_split, b
   *scratch = nullptr;
   p.ahead = 0;
   size_t bytes = 0;
+  allow_split = allow_split && p.B * p.H > m3::sm_count() && !capturing(ctx->stream);
   m3::tc_segment_plan(p.B * p.H, tiles, allow_split, backward, rot, p.R, &p.nseg, &p.tps, &p.grid, &bytes);
   if (p.nseg == 1) return cudaSuccess;
   cudaError_t e = m3::scratch_alloc(ctx, reinterpret_cast<void**>(scratch), bytes, ctx->stream);

@@ -494,6 +494,53 @@ def test_cut_stripe_launches_on_two_streams_do_not_wait_on_each_other():
         assert torch.equal(y, alone[i % 2]), i
 
 
+@pytest.mark.parametrize("rank,rot,seq", [(1, False, 2900), (2, True, 1465)])
+def test_graphs_of_long_stripes_replay_beside_each_other(rank, rot, seq):
+    """Nobody chains the launches of graphs, so a captured call leaves its stripes whole even where an ordinary one cuts them:
+    two graphs of forward and backward passes replayed on two streams, beside ordinary calls, give the ordinary calls'
+    results, and no wait gives up."""
+    from mamba_trainer_b200.ssm.scan import Context
+    w = tc_workload(rank, rot, seq, batch=5, heads=32)
+    ctx = Context.for_device(torch.device("cuda"))
+    ctx.sync()
+
+    def make(seed):
+        t = synthetic.make_inputs(w, seed=seed, device="cuda")
+        leaves = [t[k].requires_grad_(True) for k in ("x", "b", "c", "dt", "a_log", "lam", "theta", "d_skip") if t[k] is not None]
+        inp = ScanInputs.new(t["x"], t["b"], t["c"], t["dt"], t["a_log"], t["lam"]).with_chunk_size(w.chunk)
+        inp = inp.with_skip(t["d_skip"]).with_state_output(False).with_path(2)
+        inp = inp.with_theta(t["theta"]) if rot else inp
+
+        def run():
+            y = mamba3_scan(inp).y
+            return (y.detach(),) + torch.autograd.grad(y, leaves, t["dy"])
+        return run
+
+    runs = [make(11), make(12)]
+    want = [run() for run in runs]
+    torch.cuda.synchronize()
+    graphs, streams, outs = [], [torch.cuda.Stream(), torch.cuda.Stream()], []
+    for run, st in zip(runs, streams):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], stream=st):
+            outs.append(run())
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for out in outs:
+            for v in out:
+                v.zero_()
+        torch.cuda.synchronize()
+        for g, st in zip(graphs, streams):
+            with torch.cuda.stream(st):
+                g.replay()
+        beside = runs[0]()
+        torch.cuda.synchronize()
+        ctx.sync()     # raises if a bounded wait gave up
+        for got, exp in zip(outs + [beside], want + [want[0]]):
+            for i, (a, e) in enumerate(zip(got, exp)):
+                assert torch.equal(a, e), i
+
+
 def test_misaligned_rows_take_the_generic_family():
     """The tensor-core kernels move rows as 16-byte vectors and bulk tensor copies.  An input that is not
     16-byte aligned (a view that starts one element into its buffer) is served by the generic family when the
