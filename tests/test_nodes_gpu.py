@@ -188,3 +188,49 @@ def test_traced_calls_compute():
     traced = torch.jit.trace(core, (proj,), check_trace=False)
     for a, e in zip(_gradients_alone(traced, [proj + 1], dout), _gradients_alone(core, [proj + 1], dout)):
         assert torch.equal(a, e)
+
+
+@pytest.mark.parametrize("kind,dtype,d_state,T,rank", [
+    ("step", torch.bfloat16, 128, 1, 2),       # more than three blocks per SM: with the prefetch of later blocks' inputs
+    ("window", torch.bfloat16, 128, 300, 1),   # the front, states of segments, the stripes, the gate
+    ("window", torch.float32, 64, 90, 1),
+    ("mixer", torch.bfloat16, 128, 300, 2),
+    ("mixer", torch.float32, 128, 130, 1),
+    ("mixer", torch.bfloat16, 64, 200, 1),
+])
+def test_captured_calls_replay(kind, dtype, d_state, T, rank):
+    """A graph of an inference window or a training step, whose launches are programmatic edges there, computes what the
+    calls do - from the values its inputs hold when it is replayed."""
+    from mamba_trainer_b200.nn import MixerCache
+    from mamba_trainer_b200.ssm import SsmState
+    heads, B = (32, 16) if kind == "step" else (4, 2)
+    shape = MixerShape(heads, 64, d_state, rank)
+    torch.manual_seed(7)
+    core = MixerCore(shape, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(8)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    proj, other = (r(B, T, shape.in_proj_width).to(dtype) for _ in range(2))
+    if kind == "mixer":
+        dout, leaves = r(B, T, shape.d_inner).to(dtype), [proj.requires_grad_(True)] + list(core.parameters())
+
+        def run():
+            y = core(proj)
+            return (y.detach(),) + torch.autograd.grad(y, leaves, dout)
+    else:
+        cache = MixerCache(r(B, 3, shape.conv_channels).to(dtype), SsmState(r(B, heads, 64, d_state), r(B, heads, 64, d_state),
+                                                                            r(B, heads, d_state // 2)))
+
+        def run():
+            y, c = core.forward_cached(proj, cache)
+            return y, c.conv, c.ssm.h, c.ssm.last_u, c.ssm.angle
+    run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = run()
+    for values in (other, other * 0.5):
+        with torch.no_grad():
+            proj.copy_(values)
+        graph.replay()
+        for i, (a, e) in enumerate(zip([v.clone() for v in out], run())):
+            assert torch.equal(a, e), i
