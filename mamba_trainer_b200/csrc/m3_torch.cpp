@@ -3,7 +3,10 @@
 // gradient buffer at a time - cost 120 us of a scan's forward + backward whose library calls take 26 us; the small calls
 // (a 2 x 256-token scan, a decoding step) were bound by it.
 // The arithmetic stays in libm3scan; this extension allocates with torch and enqueues on torch's current stream.
+#include <ATen/Context.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/record_function.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
@@ -71,13 +74,25 @@ void* mut(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 const float* fptr(const Tensor& t) { return static_cast<const float*>(ptr(t)); }
 float* fmut(const Tensor& t) { return static_cast<float*>(mut(t)); }
 
-// Uninitialised memory for results and scratch, straight from the allocator behind at::empty: these calls are the larger part
-// of what a small call costs the host (a decoding step makes five of them).
-Tensor fresh(at::IntArrayRef sizes, at::ScalarType el, const Tensor& like) {
-  return Tensor(at::detail::empty_cuda(sizes, el, like.device(), c10::nullopt));
-}
-Tensor fresh_like(const Tensor& t) { return fresh(t.sizes(), t.scalar_type(), t); }
-Tensor fresh_bytes(size_t n, const Tensor& like) { return fresh({static_cast<int64_t>(n)}, at::kByte, like); }
+// Uninitialised memory for results and scratch of one call, straight from the allocator behind at::empty: these calls are the
+// larger part of what a small call costs the host (a decoding step makes five of them).  What at::empty does besides is for those
+// who watch the dispatcher (modes, profilers) and for the fill that torch's deterministic algorithms ask for: they get at::empty
+// itself.
+class Fresh {
+ public:
+  Fresh()
+      : watched_(c10::impl::TorchDispatchModeTLS::any_modes_set() || at::hasCallbacks() ||
+                 (at::globalContext().deterministicAlgorithms() && at::globalContext().deterministicFillUninitializedMemory())) {}
+  Tensor operator()(at::IntArrayRef sizes, at::ScalarType el, const Tensor& device_of) const {
+    if (watched_) return at::empty(sizes, at::TensorOptions().dtype(el).device(device_of.device()));
+    return Tensor(at::detail::empty_cuda(sizes, el, device_of.device(), c10::nullopt));
+  }
+  Tensor like(const Tensor& t) const { return (*this)(t.sizes(), t.scalar_type(), t); }
+  Tensor bytes(size_t n, const Tensor& device_of) const { return (*this)({static_cast<int64_t>(n)}, at::kByte, device_of); }
+
+ private:
+  bool watched_;
+};
 
 Tensor as(const Tensor& t, at::ScalarType el) {
   if (!t.defined()) return t;
@@ -158,9 +173,10 @@ struct ScanNode : public torch::autograd::Node {
     m3_scan_desc d = desc;
     scan_inputs(d, t);
     uint32_t mask = 0;
+    const Fresh fresh;
     for (int i = 0; i < kScanInputs; ++i)
       if (in[i].present && task_should_compute_output(i)) {
-        g[i] = fresh_like(t[i]);
+        g[i] = fresh.like(t[i]);
         mask |= 1u << i;
       }
     auto dense = [](const Tensor& v) { return v.defined() ? v.contiguous() : v; };
@@ -196,7 +212,8 @@ std::vector<OptTensor> scan(uintptr_t handle, const Tensor& x0, const Tensor& b0
   d.discretization = disc; d.dynamics = t[6].defined() ? M3_ROTATIONAL : M3_REAL; d.want_state = want_state; d.path = path;
   d.reverse_heads = rev;
   scan_inputs(d, t);
-  Tensor y = fresh_like(x), h, lu, ang;
+  const Fresh fresh;
+  Tensor y = fresh.like(x), h, lu, ang;
   if (want_state) {
     h = fresh({B, H, P, N}, at::kFloat, x);
     lu = fresh({B, H, P, N}, at::kFloat, x);
@@ -282,12 +299,13 @@ struct MixerNode : public torch::autograd::Node {
     mixer_inputs(d, t[0], t + 1);
     const Tensor dout = up[0].contiguous();
     // (a gain whose norm was switched off is read by nothing: no gradient)
+    const Fresh fresh;
     for (int i = 0; i <= kMixerParams; ++i)
       if (in[i].present && (i != 1 + kNormWeight || d.has_norm) && (i != 1 + kPostWeight || d.post_norm))
-        g[i] = fresh_like(t[i]);
+        g[i] = fresh.like(t[i]);
     const m3_mixer_grads out{mut(g[0]), fmut(g[1]), fmut(g[2]), fmut(g[3]), fmut(g[4]), fmut(g[5]),
                              fmut(g[6]), fmut(g[7]), fmut(g[8]), fmut(g[9])};
-    const Tensor work = fresh_bytes(m3_mixer_backward_bytes(&d), act);
+    const Tensor work = fresh.bytes(m3_mixer_backward_bytes(&d), act);
     const Status s = locked(ctx, t[0], [&] { return m3_mixer_backward(ctx, &d, handle, ptr(act), ptr(dout), &out, mut(work)); });
     if (s.rc != M3_OK) raise_status(s);
     return g;
@@ -304,8 +322,9 @@ Tensor mixer(uintptr_t handle, const Tensor& proj0, const std::vector<OptTensor>
   refuse_tangents(&proj, 1);
   refuse_tangents(p, kMixerParams);
   const m3_mixer_desc d = mixer_desc(proj, p, spec_of(ints), eps);
+  const Fresh fresh;
   Tensor out = fresh({proj.size(0), proj.size(1), d_inner}, proj.scalar_type(), proj);
-  const Tensor act = fresh_bytes(m3_mixer_activation_bytes(&d), proj);
+  const Tensor act = fresh.bytes(m3_mixer_activation_bytes(&d), proj);
   bool track = false;
   if (at::GradMode::is_enabled()) {
     track = proj.requires_grad();
@@ -342,14 +361,15 @@ std::vector<OptTensor> window(uintptr_t handle, const Tensor& proj0, const std::
   const m3_mixer_desc d = mixer_desc(proj, p, s, eps);
   const Tensor conv = as(conv0, proj.scalar_type()), h = as(h0, at::kFloat), lu = as(lu0, at::kFloat);
   const Tensor ang = s.rotational ? as(ang0, at::kFloat) : Tensor();
-  const Tensor out = fresh({proj.size(0), proj.size(1), d_inner}, proj.scalar_type(), proj), conv2 = fresh_like(conv);
-  const Tensor h2 = fresh_like(h), lu2 = fresh_like(lu);
+  const Fresh fresh;
+  const Tensor out = fresh({proj.size(0), proj.size(1), d_inner}, proj.scalar_type(), proj), conv2 = fresh.like(conv);
+  const Tensor h2 = fresh.like(h), lu2 = fresh.like(lu);
   Tensor ang2;
   if (s.rotational) ang2 = fresh({proj.size(0), s.heads, s.d_state / 2}, at::kFloat, proj);
   const m3_mixer_window_io io{ptr(conv), fptr(h), fptr(lu), fptr(ang), mut(out), mut(conv2), fmut(h2), fmut(lu2), fmut(ang2)};
   const size_t bytes = m3_mixer_window_bytes(&d, &io);
   Tensor work;
-  if (bytes) work = fresh_bytes(bytes, proj);
+  if (bytes) work = fresh.bytes(bytes, proj);
   const Status done = locked(ctx, proj, [&] { return m3_mixer_window(ctx, &d, &io, mut(work)); });
   if (done.rc != M3_OK) raise_status(done);
   return {out, conv2, h2, lu2, ang2.defined() ? OptTensor(ang2) : OptTensor()};

@@ -234,3 +234,30 @@ def test_captured_calls_replay(kind, dtype, d_state, T, rank):
         graph.replay()
         for i, (a, e) in enumerate(zip([v.clone() for v in out], run())):
             assert torch.equal(a, e), i
+
+
+@pytest.mark.parametrize("case", ["scan_tensor_core", "mixer_bf16"])
+def test_allocations_are_seen_by_those_who_watch(case):
+    """Results and scratch come from at::empty when a dispatch mode or a profiler is active: both see them, in the forward pass
+    and in the backward pass."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Seen(TorchDispatchMode):
+        def __init__(self):
+            super().__init__()
+            self.names = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.names.append(str(func))
+            return func(*args, **(kwargs or {}))
+    f, leaves, dout = CASES[case]()
+    leaves = [t.clone().requires_grad_(True) for t in leaves]
+    out = f(*leaves)
+    with Seen() as fwd:
+        out = f(*leaves)
+    with Seen() as bwd:
+        torch.autograd.grad(out, leaves, dout)
+    assert any("empty" in n for n in fwd.names) and sum("empty" in n for n in bwd.names) >= len(leaves)
+    with torch.autograd.profiler.profile() as prof:
+        f(*leaves)
+    assert any("aten::empty" == e.key for e in prof.key_averages())
