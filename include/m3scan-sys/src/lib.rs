@@ -385,6 +385,8 @@ extern "C" {
                                   input: *const m3_scan_bwd_in, grad_mask: u32, grads: *const m3_scan_grads) -> c_int;
     pub fn m3_saved_free(ctx: *mut m3_ctx, saved: *mut m3_saved) -> c_int;
     pub fn m3_scan_scratch_bytes(desc: *const m3_scan_desc, for_backward: c_int) -> usize;
+    /// 1 whole stripes, n > 1 segments one after another, -n side by side, 0 another family's call.
+    pub fn m3_scan_segments(desc: *const m3_scan_desc, backward: c_int) -> c_int;
 
     /// ssm::mamba3_step (src/ssm/scan.rs:649-712).
     pub fn m3_step_forward(ctx: *mut m3_ctx, desc: *const m3_step_desc, out: *const m3_step_out) -> c_int;

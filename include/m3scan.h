@@ -448,6 +448,13 @@ int m3_mixer_backward(m3_ctx *ctx, const m3_mixer_desc *desc, const m3_saved *sa
  * for shapes of the tensor-core family what the generic family would need. */
 size_t m3_scan_scratch_bytes(const m3_scan_desc *desc, int for_backward);
 
+/* Into how many segments in time a call with this descriptor cuts every stripe (one batch row x head) on the current
+ * device, forward or backward: 1 whole stripes, n > 1 segments handed over one after another, -n segments that run
+ * side by side; 0 for a call that the tensor-core family does not take (absent pointers count as aligned).  A state
+ * that is replaced in place, m3_scan_forward_noalloc and calls captured into a graph may leave whole what is cut
+ * elsewhere. */
+int m3_scan_segments(const m3_scan_desc *desc, int backward);
+
 #ifdef __cplusplus
 }
 #endif

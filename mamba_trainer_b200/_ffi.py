@@ -130,6 +130,7 @@ SYMBOLS = {
                                          C.POINTER(ScanGrads)]),
     "m3_saved_free": (C.c_int, [C.c_void_p, C.c_void_p]),
     "m3_scan_scratch_bytes": (C.c_size_t, [C.POINTER(ScanDesc), C.c_int]),
+    "m3_scan_segments": (C.c_int, [C.POINTER(ScanDesc), C.c_int]),
     "m3_step_forward": (C.c_int, [C.c_void_p, C.POINTER(StepDesc), C.POINTER(StepOut)]),
     "m3_scan_forward_noalloc": (C.c_int, [C.c_void_p, C.POINTER(ScanDesc), C.POINTER(ScanOut)]),
     "m3_conv_forward": (C.c_int, [C.c_void_p, C.POINTER(ConvDesc), C.c_void_p, C.c_void_p]),

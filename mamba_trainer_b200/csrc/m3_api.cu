@@ -339,6 +339,24 @@ cudaError_t rows_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3::row
   return e;
 }
 
+// The descriptor as a query sees it: a stand-in for every pointer that the caller may not have yet (`*y` one for the output);
+// those it has decide the family by their alignment.  False: no call takes it, or there is nothing to do.
+bool query_dims(const m3_scan_desc& desc, m3_scan_desc* s, m3::Dims* d, const void** y) {
+  alignas(16) static const float dummy = 0.0f;
+  auto want = [](const auto*& p) { if (!p) p = &dummy; };
+  *s = desc;
+  want(s->x); want(s->b); want(s->c); want(s->dt); want(s->a_log);
+  if (s->discretization == M3_LEARNED_TRAPEZOID) want(s->lambda);
+  if (s->dynamics == M3_ROTATIONAL) want(s->theta);
+  s->h0 = s->last_u0 = nullptr;
+  if (s->a_raw) { want(s->g_raw); want(s->w_raw); }
+  *y = &dummy;
+  return m3::make_dims(nullptr, *s, d) == M3_OK && d->T > 0;
+}
+bool query_tensor(const m3_scan_desc& s, const m3::Dims& d) {
+  return m3::tc_supported(s) && !d.raw && s.path != M3_PATH_GENERIC;
+}
+
 }  // namespace
 
 extern "C" {
@@ -466,24 +484,28 @@ int m3_download(m3_ctx* ctx, void* dst, const void* src, size_t bytes) {
 
 size_t m3_scan_scratch_bytes(const m3_scan_desc* desc, int for_backward) {
   if (!desc) return 0;
+  m3_scan_desc s;
   m3::Dims d;
-  m3_scan_desc s = *desc;
-  // Stand in for pointers the caller may not have yet; those it has decide the family by their alignment.
-  alignas(16) static const float dummy = 0.0f;
-  auto want = [](const auto*& p) { if (!p) p = &dummy; };
-  want(s.x); want(s.b); want(s.c); want(s.dt); want(s.a_log);
-  if (s.discretization == M3_LEARNED_TRAPEZOID) want(s.lambda);
-  if (s.dynamics == M3_ROTATIONAL) want(s.theta);
-  s.h0 = s.last_u0 = nullptr;
-  if (s.a_raw) { want(s.g_raw); want(s.w_raw); }
-  if (make_dims(nullptr, s, &d) != M3_OK || d.T == 0) return 0;
-  const bool tensor = m3::tc_supported(s) && !d.raw && s.path != M3_PATH_GENERIC;
-  if (!tensor && m3::rows_supported(s, &dummy)) {
+  const void* y;
+  if (!query_dims(*desc, &s, &d, &y)) return 0;
+  if (!query_tensor(s, d) && m3::rows_supported(s, y)) {
     d = m3::rows_dims(d);
     return m3::rows_ws_layout(d, nullptr, nullptr) + (for_backward ? m3::rows_bwd_ws_layout(d, nullptr, nullptr, nullptr) : 0);
   }
   size_t n = m3::generic_ws_layout(d, nullptr, nullptr);
   if (for_backward) n += m3::generic_bwd_ws_layout(d, nullptr, nullptr);
+  return n;
+}
+
+int m3_scan_segments(const m3_scan_desc* desc, int backward) {
+  m3_scan_desc s;
+  m3::Dims d;
+  const void* y;
+  if (!desc || !query_dims(*desc, &s, &d, &y) || !query_tensor(s, d)) return 0;
+  const int BH = d.B * d.H, tiles = m3::tc_tiles(d.T, d.R);
+  int n = 1, tps, grid;
+  if (m3::tc_ahead_plan(BH, tiles, backward != 0, d.rot != 0, d.R, &n, &tps)) return -n;
+  m3::tc_segment_plan(BH, tiles, true, backward != 0, d.rot != 0, d.R, &n, &tps, &grid, nullptr);
   return n;
 }
 

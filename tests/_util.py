@@ -110,3 +110,14 @@ def reference_mode_error(t: dict, chunk: int, exact: dict, names, want_state=Fal
     d a_log, d dt_bias: sums over every token)."""
     _, _, g = oracle_run(t, chunk, want_state, torch.float32, True, matmul_narrow=torch.bfloat16)
     return {n: norm_rel(g[n].double(), exact[n]) for n in names if n in g and n in exact}
+
+
+def segments(w, batch=None, reverse_heads=0):
+    """Segments that a stripe of workload `w` is cut into (forward, backward), as m3_scan_segments has it."""
+    import ctypes as C
+    from mamba_trainer_b200 import _ffi
+    d = _ffi.ScanDesc(batch=w.batch if batch is None else batch, seq=w.seq, heads=w.heads, head_dim=w.head_dim, d_state=w.d_state,
+                      rank=w.rank, chunk=w.chunk, dtype=_ffi.F32 if w.dtype == torch.float32 else _ffi.BF16, discretization=2,
+                      dynamics=int(w.rotational), path=_ffi.PATH_AUTO, reverse_heads=reverse_heads)
+    lib = _ffi.load()
+    return lib.m3_scan_segments(C.byref(d), 0), lib.m3_scan_segments(C.byref(d), 1)

@@ -88,6 +88,20 @@ def test_scratch_size_follows_the_family():
         assert size(dtype=_ffi.BF16, d_state=128, backward=backward) == size(_ffi.PATH_GENERIC, _ffi.BF16, 128, backward=backward)
 
 
+def test_segments_query_needs_no_gpu():
+    """Few stripes side by side, more than there are SMs (148 where there is none to ask) one after another, whole where a cut
+    would not pay, and no answer for calls of other families."""
+    from mamba_trainer_b200 import synthetic
+    from tests._util import segments
+    w = synthetic.WORKLOADS[4]    # rank 2, rotational: 64 steps a tile
+    cut = lambda batch, heads, seq, v=w: segments(v.scaled(batch=batch, heads=heads, seq=seq))
+    assert all(n < -1 for n in cut(1, 4, 1000))
+    assert cut(4, 32, 1000) == (1, 1)
+    assert all(n > 1 for n in cut(5, 32, 2000))
+    assert cut(64, 32, 1000) == (1, 1)
+    assert cut(5, 32, 2000, synthetic.WORKLOADS[0]) == (0, 0)   # float32
+
+
 def test_rust_sys_source_covers_the_header():
     """include/m3scan-sys/src/lib.rs (uncompiled here: the image has no Rust toolchain) declares every function
     of the header and nothing else, and lists every structure's fields in the header's order."""

@@ -18,7 +18,7 @@ from mamba_trainer_b200.error import ConfigError, RankError, ShapeError
 from mamba_trainer_b200.ssm import Discretization, ScanInputs, SsmState, mamba3_scan
 from oracle.recurrence import Case, recurrence
 from tests._util import (allclose_excess, angle_close, fused_run, norm_rel, oracle_run, ref_metric,
-                         reference_mode_error)
+                         reference_mode_error, segments)
 
 pytestmark = pytest.mark.gpu
 
@@ -434,13 +434,22 @@ def test_tensor_core_backward(rank, rot, seq, state, disc):
     compare_all(t, w.chunk, check_bf16, True, ds, discretization=disc, path=2)
 
 
-@pytest.mark.parametrize("rank,rot,seq,rev", [(2, True, 1000, 1), (1, True, 1100, 0), (4, False, 520, 0), (2, False, 1000, 32)])
-def test_time_segments_leave_results_unchanged(rank, rot, seq, rev):
-    """With more stripes than SMs the kernels cut every stripe into time segments, possibly run by different
+@pytest.mark.parametrize("rank,rot,seq,rev,cut", [
+    (2, True, 1000, 1, "backward"), (1, True, 1100, 0, "backward"), (4, False, 520, 0, "backward"), (2, False, 1000, 32, "backward"),
+    (1, False, 1001, 0, "backward"),
+    (1, True, 850, 0, "backward"),     # seven tiles: the last segment is one of them
+    (1, True, 2000, 1, "both"), (1, False, 2900, 0, "both"), (2, True, 1465, 1, "both"), (2, False, 1465, 32, "both"),
+    (4, True, 730, 1, "both"), (4, False, 730, 0, "both"),
+])
+def test_time_segments_leave_results_unchanged(rank, rot, seq, rev, cut):
+    """With more stripes than SMs the kernels cut every stripe into time segments where that pays, possibly run by different
     CTAs, which hand the fp32 state (backward: its gradient) and the running angle over in global memory.
     The arithmetic and its order are those of whole stripes, so the results are identical: 160 stripes in one
-    call (cut) against the same rows in calls of 64 and 96 stripes (never cut)."""
+    call (cut in the backward pass or both ways) against the same rows in calls of 64 and 96 stripes (whole)."""
     w = tc_workload(rank, rot, seq, batch=5, heads=32)
+    fwd, bwd = segments(w)
+    assert bwd > 1 and (fwd > 1 if cut == "both" else fwd == 1), (fwd, bwd)
+    assert segments(w, batch=2) == segments(w, batch=3) == (1, 1)
     t = synthetic.make_inputs(w, seed=seq + rank, with_state=True)
     g = torch.Generator().manual_seed(seq)
     ds = {"h": torch.randn(w.batch, w.heads, 64, 128, generator=g) * 0.1,

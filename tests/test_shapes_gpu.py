@@ -405,17 +405,6 @@ def test_a_state_replaced_in_place(dtype, H, N, R, T, rot):
             assert norm_rel(a.float(), e.float()) <= tol, n
 
 
-@pytest.mark.parametrize("rank,rot,seq,rev", [
-    (2, True, 1465, 1),      # 23 tiles in three segments, each way
-    (4, False, 730, 0),      # 23 tiles forward in two
-    (1, False, 1001, 0),     # rank 1, real dynamics, no multiple of eight: eight tiles, cut in the backward pass only
-])
-def test_longer_stripes_cut_in_time_equal_whole_ones(rank, rot, seq, rev):
-    """160 stripes long enough that the plan cuts them (it weighs rounds by what a tile and an item's start take)."""
-    from test_scan_gpu import test_time_segments_leave_results_unchanged
-    test_time_segments_leave_results_unchanged(rank, rot, seq, rev)
-
-
 def test_real_dynamics_of_rank_1_match_the_oracle_at_multiples_of_eight():
     """Sequences a multiple of eight, whole stripes: more heads than are cut side by side."""
     from test_scan_gpu import check_bf16, compare_all, small_inputs
