@@ -315,26 +315,43 @@ def test_bf16_configs_full_size(idx):
 
 # ---- a bounded device-side wait that runs out (no fault, no hang: the kernels give up and say so) ----
 
-@pytest.mark.parametrize("idx,kw", [(4, dict(batch=1, heads=2, seq=700)), (1, dict(batch=1, heads=2, seq=512)),
-                                    (4, dict(batch=5, heads=32, seq=640))])
-def test_a_wait_that_runs_out_is_reported_and_the_context_stays_usable(idx, kw):
+@pytest.mark.parametrize("idx,kw,form", [
+    (4, dict(batch=1, heads=2, seq=700), "side by side"), (1, dict(batch=1, heads=2, seq=1100), "side by side"),
+    (4, dict(batch=4, heads=32, seq=640), "whole"), (1, dict(batch=1, heads=2, seq=512), "whole"),
+    (4, dict(batch=5, heads=32, seq=2000), "one after another"), (1, dict(batch=5, heads=32, seq=2900), "one after another"),
+])
+def test_a_wait_that_runs_out_is_reported_and_the_context_stays_usable(idx, kw, form):
     """Every device-side wait of the tensor-core kernels has an iteration limit.  With the limit set to one
     poll (m3_ctx_set_wait_limit) the first wait of every CTA gives up before its products or copies have
     finished: the kernels must return by themselves, the condition must surface as DeviceTimeout - at
     Context.sync() and, for callers that never sync, on entry to the next scan call - and once the limit
-    is back to its default the same context must compute correct results again.  Covers the role-split
-    kernels (rank 2, rotational), the direct form (rank 1, real dynamics) and stripes cut into time segments
-    (160 stripes on 148 SMs: a CTA that gave up still raises its hand-over flag, and the wait for a
-    predecessor's flag is bounded like every other)."""
+    is back to its default the same context must compute correct results again.  A forward pass alone, a backward
+    pass alone (behind a good forward pass) and both, of rank 2 rotational and rank 1 real stripes: whole, and cut into
+    time segments that run side by side or one after another (160 stripes on 148 SMs: a CTA that gave up still raises
+    its hand-over flag, and the wait for a predecessor's flag is bounded like every other)."""
     from mamba_trainer_b200.error import DeviceTimeout
     from mamba_trainer_b200.ssm import Context
     w = synthetic.WORKLOADS[idx].scaled(**kw)
+    want = {"side by side": lambda n: n < -1, "whole": lambda n: n == 1, "one after another": lambda n: n > 1}[form]
+    assert all(want(n) for n in segments(w)), segments(w)
     t = synthetic.make_inputs(w, seed=21)
     good_y, _, good_g = fused_run(t, w.chunk, False)
     ctx = Context.for_device(torch.device("cuda", torch.cuda.current_device()))
     ctx.sync()
+    leaves = {k: v.cuda().requires_grad_(True) for k, v in t.items() if v is not None and k != "dy"}
+    inp = ScanInputs.new(*(leaves[k] for k in ("x", "b", "c", "dt", "a_log", "lam"))).with_chunk_size(w.chunk)
+    inp = inp.with_skip(leaves["d_skip"]).with_state_output(False)
+    y = mamba3_scan(inp.with_theta(leaves["theta"]) if w.rotational else inp).y
+    ctx.sync()
     try:
         ctx.set_wait_limit(1)
+        torch.autograd.grad(y, list(leaves.values()), t["dy"].cuda())
+        with pytest.raises(DeviceTimeout):    # the backward pass gave up
+            ctx.sync()
+        fused_run(t, w.chunk, False, grads=False)
+        with pytest.raises(DeviceTimeout):    # the forward pass gave up
+            ctx.sync()
+        ctx.sync()                            # (reported once)
         with pytest.raises(DeviceTimeout):
             fused_run(t, w.chunk, False)      # the forward gives up; the backward call may already see it on entry
             ctx.sync()                        # ... and if it was too early for that, the sync does
