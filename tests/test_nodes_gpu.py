@@ -192,9 +192,9 @@ def test_traced_calls_compute():
 
 @pytest.mark.parametrize("kind,dtype,d_state,T,rank", [
     ("step", torch.bfloat16, 128, 1, 2),       # more than three blocks per SM: with the prefetch of later blocks' inputs
-    ("window", torch.bfloat16, 128, 300, 1),   # the front, states of segments, the stripes, the gate
+    ("window", torch.bfloat16, 128, 900, 1),   # the front, states of segments side by side, the stripes, the gate
     ("window", torch.float32, 64, 90, 1),
-    ("mixer", torch.bfloat16, 128, 300, 2),
+    ("mixer", torch.bfloat16, 128, 500, 2),    # segments side by side each way
     ("mixer", torch.float32, 128, 130, 1),
     ("mixer", torch.bfloat16, 64, 200, 1),
 ])
@@ -204,6 +204,10 @@ def test_captured_calls_replay(kind, dtype, d_state, T, rank):
     from mamba_trainer_b200.nn import MixerCache
     from mamba_trainer_b200.ssm import SsmState
     heads, B = (32, 16) if kind == "step" else (4, 2)
+    if d_state == 128 and dtype == torch.bfloat16 and T > 1:
+        from tests._util import segments
+        from tests.test_scan_gpu import tc_workload
+        assert max(segments(tc_workload(rank, True, T, B, heads))) < -1
     shape = MixerShape(heads, 64, d_state, rank)
     torch.manual_seed(7)
     core = MixerCore(shape, device="cuda")

@@ -411,8 +411,8 @@ def tc_workload(rank, rot, seq, batch=2, heads=2, disc=Discretization.LearnedTra
     (1, False, 300, True, Discretization.LearnedTrapezoid),
     (1, True, 256, False, Discretization.LearnedTrapezoid),
     (1, False, 128, False, Discretization.Euler),
-    (1, False, 200, True, Discretization.LearnedTrapezoid),    # bulk-copy path with a ragged last tile
-    (1, False, 384, False, Discretization.Trapezoid),          # bulk-copy path, three full tiles
+    (1, False, 200, True, Discretization.LearnedTrapezoid),    # a ragged last tile
+    (1, False, 384, False, Discretization.Trapezoid),          # three full tiles
     (2, True, 200, True, Discretization.LearnedTrapezoid),
     (4, True, 130, True, Discretization.Trapezoid),
     (4, False, 64, False, Discretization.LearnedTrapezoid),
@@ -434,8 +434,8 @@ def test_tensor_core_forward(rank, rot, seq, state, disc):
     (1, False, 300, True, Discretization.LearnedTrapezoid),
     (1, True, 256, False, Discretization.LearnedTrapezoid),
     (1, False, 128, False, Discretization.Euler),
-    (1, False, 200, True, Discretization.LearnedTrapezoid),    # bulk-copy path with a ragged last tile
-    (1, False, 384, False, Discretization.Trapezoid),          # bulk-copy path, three full tiles
+    (1, False, 200, True, Discretization.LearnedTrapezoid),    # a ragged last tile
+    (1, False, 384, False, Discretization.Trapezoid),          # three full tiles
     (2, True, 200, True, Discretization.LearnedTrapezoid),
     (4, True, 130, True, Discretization.Trapezoid),
     (4, False, 64, False, Discretization.LearnedTrapezoid),
@@ -498,6 +498,7 @@ def test_cut_stripe_launches_on_two_streams_do_not_wait_on_each_other():
     enqueued back to back on two streams finish without a wait giving up and equal the same scans run alone."""
     from mamba_trainer_b200.ssm.scan import Context
     w = tc_workload(2, True, 2000, batch=5, heads=32)
+    assert segments(w)[0] > 1
     ts = [synthetic.make_inputs(w, seed=s_, device="cuda") for s_ in (11, 12)]
 
     def run(t):
@@ -527,6 +528,7 @@ def test_graphs_of_long_stripes_replay_beside_each_other(rank, rot, seq):
     results, and no wait gives up."""
     from mamba_trainer_b200.ssm.scan import Context
     w = tc_workload(rank, rot, seq, batch=5, heads=32)
+    assert min(segments(w)) > 1
     ctx = Context.for_device(torch.device("cuda"))
     ctx.sync()
 

@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from _util import norm_rel, ref_metric
+from _util import norm_rel, ref_metric, segments
 from mamba_trainer_b200.ssm import Discretization
 
 pytestmark = pytest.mark.gpu
@@ -285,17 +285,21 @@ def test_mixer_front_tiles_past_the_bands_end(dtype, B, T, H, P, N, R, bidir):
 
 
 @pytest.mark.parametrize("B,H,R,rot,T,state,rev", [
-    (2, 2, 1, True, 385, True, 0),      # four tiles, the last one a single step
-    (2, 2, 1, False, 1000, True, 0),    # real dynamics: the role-split kernels instead of the direct ones
+    (2, 2, 1, True, 385, True, 0),      # four tiles, the last one a single step: cut in the backward pass only
+    (2, 2, 1, True, 769, True, 0),      # seven tiles: the fewest that are cut both ways
+    (2, 2, 1, False, 1000, True, 0),    # real dynamics of rank 1
     (2, 2, 2, True, 1000, True, 1),     # a right-to-left head, carried state and angle
     (2, 2, 2, True, 449, False, 0),     # the second half of the last tile is padding
     (2, 2, 4, True, 321, True, 0),
-    (2, 2, 4, False, 96, False, 1),     # three tiles: the fewest that are cut
+    (2, 2, 4, False, 160, False, 1),    # five tiles: the fewest of real dynamics that the backward pass cuts
+    (2, 2, 4, False, 256, False, 1),    # eight: the forward pass too
     (5, 8, 4, True, 999, True, 0),       # 32 tiles of 40 stripes: states of groups of several tiles, the last one shorter
 ])
 def test_side_by_side_segments_match_the_oracle(B, H, R, rot, T, state, rev):
     """Few stripes of the tensor-core family: segments of a stripe run at once from states worked out ahead of them."""
-    from test_scan_gpu import check_bf16, compare_all, small_inputs
+    from test_scan_gpu import check_bf16, compare_all, small_inputs, tc_workload
+    fwd, bwd = segments(tc_workload(R, rot, T, B, H))
+    assert bwd < -1 and (fwd < -1) == ((R, T) not in ((1, 385), (4, 160))), (fwd, bwd)
     t, ds = small_inputs(B, T, H, 64, 128, R, rot, state, seed=T + R)
     for k in ("b", "c"):
         t[k] = t[k] / 128 ** 0.5
@@ -316,9 +320,9 @@ def test_side_by_side_segments_match_the_oracle(B, H, R, rot, T, state, rev):
 
 @pytest.mark.parametrize("T,H,R,copies", [(1670, 4, 1, 40), (1072, 6, 2, 27)])
 def test_cut_stripes_lose_no_accuracy(T, H, R, copies):
-    """Few stripes, cut into segments, against the same stripes among copies of themselves, which run whole: d theta, where
-    the two sides of every pair of steps have to cancel, is as close to the float64 oracle (1.08: what the segments' own
-    float32 sums may move)."""
+    """Few stripes, cut into segments that run side by side, against the same stripes among copies of themselves, which run
+    whole or cut one segment after another (bit for bit the same): d theta, where the two sides of every pair of steps have
+    to cancel, is as close to the float64 oracle (1.08: what the segments' own float32 sums may move)."""
     from _util import fused_run, oracle_run
     from mamba_trainer_b200 import synthetic
     from mamba_trainer_b200.ssm import Context
@@ -330,6 +334,7 @@ def test_cut_stripes_lose_no_accuracy(T, H, R, copies):
         before = ctx.lib.m3_launch_count(ctx.handle)
         _, _, g = fused_run(v, 64, False, path=2)
         return g["theta"], ctx.lib.m3_launch_count(ctx.handle) - before
+    assert max(segments(w)) < -1 and min(segments(w, batch=copies)) >= 1
     errors = []
     for seed in range(3):
         t = synthetic.make_inputs(w, seed=seed)
@@ -352,11 +357,12 @@ def test_long_cut_stripes_match_the_oracle(T, H, R):
     from mamba_trainer_b200.ssm import Context
     w = synthetic.Workload("long", 1, T, H, 64, 128, 64, R, torch.bfloat16, Discretization.LearnedTrapezoid, True,
                            "rms" if R == 1 else "scaled")
+    assert max(segments(w)) < -1
     t = synthetic.make_inputs(w, seed=R)
     ctx = Context.for_device(torch.device("cuda"))
     before = ctx.lib.m3_launch_count(ctx.handle)
     y, _, got = fused_run(t, 64, False, path=2)
-    # group states, pass and stripe kernel each way, then the joined sums of d phi and the per-head sums
+    # group states, pass and stripe kernel each way, the angles of the forward pass, the joined sums of d phi
     assert ctx.lib.m3_launch_count(ctx.handle) - before >= 7
     ey, _, exact = oracle_run(t, 64, False)
     mode = reference_mode_error(t, 64, exact, ("theta",))
