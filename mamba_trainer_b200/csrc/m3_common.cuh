@@ -21,11 +21,11 @@ struct Dims {
   int ths;       // elements between consecutive tokens of theta and its gradient (a band of a wider row)
 };
 
-// First of all in a kernel that launch() starts: wait for the kernel before it on the stream (nothing of that one may be read or
-// overwritten earlier, and no TMEM taken: that kernel need not be one of this library, and if it lets its successor in before its own
-// blocks have allocated theirs, each would wait for the other for good).  The kernel behind is let in when this one's blocks have ended, not sooner (griddepcontrol.
-// launch_dependents at the start): blocks that wait held slots the running ones could use - float32 mixer, 8 x 1024 tokens,
-// 16 heads: 1132 us without any of this, 1184 with the early start, 1103 without.
+// First of all in a kernel that launch() starts: wait for the kernel before it on the stream.  Nothing of that one may be read or
+// overwritten earlier, and no TMEM taken: it need not be a kernel of this library, and if it lets its successor in before its
+// own blocks have allocated theirs, each would wait for the other for good.  The kernel behind is let in when this one's blocks
+// have ended, not sooner (griddepcontrol.launch_dependents at the start): blocks that wait held slots the running ones could
+// use - float32 mixer, 8 x 1024 tokens, 16 heads: 1132 us without any of this, 1184 with the early start, 1103 without.
 __device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Token-head index (row of a [B, T, H, ...] tensor) of scan position t of head h: heads that

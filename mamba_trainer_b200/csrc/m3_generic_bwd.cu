@@ -44,9 +44,10 @@ static void final_tokens(cudaStream_t st, const Dims& d, const m3_scan_desc& des
   const unsigned blocks = (unsigned)(((size_t)d.B * d.T * d.H + 255) / 256);
   const HeadSums hs{desc.a_log, dalog, ddsk};
   const int heads = hs.any() ? d.H : 0;
-  launch(kb_final<T>, blocks + heads, 256, 0, st, d, static_cast<const T*>(desc.dt), static_cast<const T*>(desc.lambda), desc.a_log, bw, (desc.h0 && !d.raw) ? 1 : 0,
-      static_cast<T*>(ddt), static_cast<T*>(dlam), raw ? static_cast<T*>(raw->da_raw) : nullptr,
-      raw ? static_cast<T*>(raw->dg_raw) : nullptr, raw ? static_cast<T*>(raw->dw_raw) : nullptr, hs, heads);
+  launch(kb_final<T>, blocks + heads, 256, 0, st, d, static_cast<const T*>(desc.dt), static_cast<const T*>(desc.lambda),
+         desc.a_log, bw, (desc.h0 && !d.raw) ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam),
+         raw ? static_cast<T*>(raw->da_raw) : nullptr, raw ? static_cast<T*>(raw->dg_raw) : nullptr,
+         raw ? static_cast<T*>(raw->dw_raw) : nullptr, hs, heads);
 }
 
 template <class T>

@@ -110,8 +110,7 @@ struct GenericBwdWs {
 
 // Per head: d a_log = A * sum da dt (A = -exp(a_log), scan.rs:470-475) and dD, summed over batch and chunks in a fixed
 // order by one block of 256 threads (red: 8 floats).  These blocks ride ahead of those of the last per-token launch (behind
-// them they would be its tail): as a
-// launch of their own they cost 2.4 us and the host 3.5 us of every backward pass.
+// them they would be its tail): as a launch of their own they cost 2.4 us and the host 3.5 us of every backward pass.
 struct HeadSums {
   const float* a_log;
   float *da_log, *dd_skip;   // NULL skips the store

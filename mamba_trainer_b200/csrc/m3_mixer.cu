@@ -931,14 +931,12 @@ int m3_gate_forward(m3_ctx* ctx, const m3_gate_desc* s, void* out) {
   const bool vec = gate_vec(s, es, zs, {s->y, s->z, out});
   const size_t items = ntok * (s->channels / (vec ? 16 / es : 1));
   const unsigned grid = (unsigned)((items + 255) / 256 < 148 * 16 ? (items + 255) / 256 : 148 * 16);
-  if (s->dtype == M3_BF16) {
-    using T = __nv_bfloat16;
-    if (vec) m3::launch(k_gate_fwd<T, true>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<T*>(out));
-    else m3::launch(k_gate_fwd<T, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<T*>(out));
-  } else {
-    if (vec) m3::launch(k_gate_fwd<float, true>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<float*>(out));
-    else m3::launch(k_gate_fwd<float, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<float*>(out));
-  }
+  auto go = [&](auto t) {
+    using T = decltype(t);
+    m3::launch(vec ? k_gate_fwd<T, true> : k_gate_fwd<T, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs,
+               static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<T*>(out));
+  };
+  if (s->dtype == M3_BF16) go(__nv_bfloat16{}); else go(float{});
   M3_CUDA(ctx, cudaGetLastError());
   ctx->launches += 1;
   return M3_OK;
@@ -956,14 +954,13 @@ int m3_gate_backward(m3_ctx* ctx, const m3_gate_desc* s, const void* dout, void*
   const bool vec = gate_vec(s, es, zs, {s->y, s->z, dout, dy, dz});
   const size_t items = ntok * (s->channels / (vec ? 16 / es : 1));
   const unsigned grid = (unsigned)((items + 255) / 256 < 148 * 16 ? (items + 255) / 256 : 148 * 16);
-  if (s->dtype == M3_BF16) {
-    using T = __nv_bfloat16;
-    if (vec) m3::launch(k_gate_bwd<T, true>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<const T*>(dout), static_cast<T*>(dy), static_cast<T*>(dz));
-    else m3::launch(k_gate_bwd<T, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<const T*>(dout), static_cast<T*>(dy), static_cast<T*>(dz));
-  } else {
-    if (vec) m3::launch(k_gate_bwd<float, true>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<const float*>(dout), static_cast<float*>(dy), static_cast<float*>(dz));
-    else m3::launch(k_gate_bwd<float, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs, static_cast<const float*>(s->y), static_cast<const float*>(s->z), static_cast<const float*>(dout), static_cast<float*>(dy), static_cast<float*>(dz));
-  }
+  auto go = [&](auto t) {
+    using T = decltype(t);
+    m3::launch(vec ? k_gate_bwd<T, true> : k_gate_bwd<T, false>, grid, 256, 0, ctx->stream, ntok, s->channels, zs,
+               static_cast<const T*>(s->y), static_cast<const T*>(s->z), static_cast<const T*>(dout), static_cast<T*>(dy),
+               static_cast<T*>(dz));
+  };
+  if (s->dtype == M3_BF16) go(__nv_bfloat16{}); else go(float{});
   M3_CUDA(ctx, cudaGetLastError());
   ctx->launches += 1;
   return M3_OK;

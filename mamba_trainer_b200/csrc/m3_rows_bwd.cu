@@ -567,7 +567,7 @@ cudaError_t final_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, cons
   if (layer) rows = 0;
   const dim3 grid(nx, BH + rows, layer ? 2 : 1);
   launch(k_rows_final<T, N>, grid, 256, 0, st, d, in, rw, bw, in.h0 ? 1 : 0, static_cast<T*>(ddt), static_cast<T*>(dlam),
-                                                   static_cast<T*>(dtheta), dangle0, per_seg, nseg, hs, rows);
+         static_cast<T*>(dtheta), dangle0, per_seg, nseg, hs, rows);
   return cudaGetLastError();
 }
 
@@ -587,10 +587,11 @@ cudaError_t backward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, c
   const AdjOut<T> out{static_cast<T*>(want(M3_GRAD_X, g.dx)), static_cast<T*>(want(M3_GRAD_B, g.db)),
                       static_cast<T*>(want(M3_GRAD_C, g.dc)), bw.da, bw.dg, bw.dw, bw.partA, bw.partD,
                       d.raw ? nullptr : up.dlast_u, up.dangle};
-  launch(k_rows_adjoint<T, N, R, ROT>, grid, kAdjThreads<N>, sizeof(AdjSmem<N, R>), st, d, in, static_cast<const T*>(up.dy), ws, rw, out);
+  launch(k_rows_adjoint<T, N, R, ROT>, grid, kAdjThreads<N>, sizeof(AdjSmem<N, R>), st, d, in,
+         static_cast<const T*>(up.dy), ws, rw, out);
   if (has_state) {
     launch(k_rows_seed<T, N>, d.B * d.H, 256, 0, st, d, in, rw, bw.ip0, static_cast<float*>(want(M3_GRAD_H0, g.dh0)),
-                                                 d.raw ? nullptr : static_cast<float*>(want(M3_GRAD_LAST_U0, g.dlast_u0)));
+           d.raw ? nullptr : static_cast<float*>(want(M3_GRAD_LAST_U0, g.dlast_u0)));
     n += 1;
   }
   void* ddt = want(M3_GRAD_DT, g.ddt);

@@ -57,8 +57,8 @@ __global__ void __launch_bounds__(256, N == 64 ? 4 : 3) k_rows_state(Dims d, m3_
 
 // ---- the pass over chunk states: a thread owns planes (m, m + NH) of two rows p, p + 32 --------------------------
 template <class T, int N, bool ROT>
-__global__ void __launch_bounds__(256) k_rows_pass(Dims d, m3_scan_desc in, RowsWs ws, float* h_out) {
-  after_predecessor();   // (h_out may be h0)
+__global__ void __launch_bounds__(256) k_rows_pass(Dims d, m3_scan_desc in, RowsWs ws, float* h_out) {   // (h_out may be h0)
+  after_predecessor();
   constexpr int NH = N / 2, PN = kP * N, U = 4;
   const int bh = blockIdx.y, b = bh / d.H, h = bh - b * d.H;
   const int id = blockIdx.x * 256 + threadIdx.x, m = id % NH, p = id / NH;   // p < 32
@@ -225,8 +225,10 @@ cudaError_t forward_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, co
   if (e == cudaSuccess) e = smem_limit(k_rows_out<T, N, R, ROT>, sizeof(OutSmem<N, R>));
   if (e != cudaSuccess) return e;
   launch(k_rows_state<T, N, R, ROT, false>, grid, 256, sizeof(StateSmem<N, R>), st, d, in, nullptr, ws, ws.hs);
-  launch(k_rows_pass<T, N, ROT>, dim3(32 * (N / 2) / 256, d.B * d.H), 256, 0, st, d, in, ws, in.want_state ? out.h : nullptr);
-  launch(k_rows_out<T, N, R, ROT>, grid, 256, sizeof(OutSmem<N, R>), st, d, in, ws, static_cast<T*>(out.y), in.want_state && !d.raw ? out.last_u : nullptr, in.want_state ? out.angle : nullptr);
+  launch(k_rows_pass<T, N, ROT>, dim3(32 * (N / 2) / 256, d.B * d.H), 256, 0, st, d, in, ws,
+         in.want_state ? out.h : nullptr);
+  launch(k_rows_out<T, N, R, ROT>, grid, 256, sizeof(OutSmem<N, R>), st, d, in, ws, static_cast<T*>(out.y),
+         in.want_state && !d.raw ? out.last_u : nullptr, in.want_state ? out.angle : nullptr);
   return cudaGetLastError();
 }
 
@@ -247,7 +249,8 @@ template <class T, int N, int R, bool ROT>
 cudaError_t dh_local_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, const void* dy, const RowsWs& ws, float* dhs) {
   cudaError_t e = smem_limit(k_rows_state<T, N, R, ROT, true>, sizeof(StateSmem<N, R>));
   if (e != cudaSuccess) return e;
-  launch(k_rows_state<T, N, R, ROT, true>, dim3(d.C, d.B * d.H), 256, sizeof(StateSmem<N, R>), st, d, in, static_cast<const T*>(dy), ws, dhs);
+  launch(k_rows_state<T, N, R, ROT, true>, dim3(d.C, d.B * d.H), 256, sizeof(StateSmem<N, R>), st, d, in,
+         static_cast<const T*>(dy), ws, dhs);
   return cudaGetLastError();
 }
 

@@ -481,8 +481,8 @@ cudaError_t ahead_t(cudaStream_t st, const Dims& d, const m3_scan_desc& in, cons
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmem<R>));
   if (e != cudaSuccess) return e;
   if (FULL_ANGLE) launch(k_group_angle<R>, dim3(count, d.B * d.H), kThreads, 0, st, d, in, a, tc_tiles(d.T, R));
-  launch(kern, dim3(count, d.B * d.H), kThreads, sizeof(GroupSmem<R>), st, d, in, static_cast<const __nv_bfloat16*>(dy), ckpt_angle, a,
-                                                                       tc_tiles(d.T, R));
+  launch(kern, dim3(count, d.B * d.H), kThreads, sizeof(GroupSmem<R>), st, d, in, static_cast<const __nv_bfloat16*>(dy),
+         ckpt_angle, a, tc_tiles(d.T, R));
   launch(k_group_pass<ROT, BWD, ROT && !BWD && !FULL_ANGLE>, dim3(32 * kNH / 256, d.B * d.H), 256, 0, st, d, in, dh, a, count);
   return cudaGetLastError();
 }
@@ -502,9 +502,8 @@ cudaError_t tc_ahead_load() {
 
 // Whether to cut `BH` stripes of `tiles` tiles into segments that run side by side, and into how many.  Microseconds,
 // measured on a B200: a tile takes tc_tile_us inside a stripe, an item about one more to start and finish; working out what
-// a tile adds to the state
-// takes about 4 per tile and SM, and the two launches and the pass some 12 more.  Beyond a third of the SMs it takes long
-// stripes to gain anything (96 stripes of 16 tiles: nothing; 64 of 248: forward + backward 3.47 -> 2.06 ms).
+// a tile adds to the state takes about 4 per tile and SM, and the two launches and the pass some 12 more.  Beyond a third of
+// the SMs it takes long stripes to gain anything (96 stripes of 16 tiles: nothing; 64 of 248: forward + backward 3.47 -> 2.06 ms).
 bool tc_ahead_plan(int BH, int tiles, bool backward, bool rot, int rank, int* nseg, int* tps) {
   const int sms = sm_count();
   if (BH > sms || tiles < (BH > sms / 3 ? 24 : 3)) return false;

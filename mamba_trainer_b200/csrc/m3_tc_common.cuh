@@ -123,10 +123,11 @@ __device__ __forceinline__ void tma_load_rows(void* dst, const void* tensor_map,
       : "memory");
 }
 
-// The same box into L2 only, for a tma_load_rows to come.
-__device__ __forceinline__ void bulk_prefetch(const void* gmem, uint32_t bytes) {   // into L2; 16-byte address and size
+// A contiguous range into L2 only; address and size are multiples of 16 bytes.
+__device__ __forceinline__ void bulk_prefetch(const void* gmem, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem), "r"(bytes) : "memory");
 }
+// The box of a tma_load_rows to come into L2 only.  `t` is not negative (the callers leave such tiles out).
 __device__ __forceinline__ void tma_prefetch_rows(const void* tensor_map, int col, int h, int t, int b) {
   asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(tensor_map), "r"(col), "r"(h), "r"(t), "r"(b)
                : "memory");

@@ -266,7 +266,7 @@ __device__ __forceinline__ void table_cos_sin(const float* tab, int l, int m0, f
   }
 }
 // Eight columns of both halves (m, m + 64) of rank r, rotated by -phi.
-template <int R, bool ROT, int NREG>
+template <int R, int NREG>
 __device__ __forceinline__ void rotate_store(uint8_t* dst, int row, int n0, const uint32_t (&v0)[NREG], const uint32_t (&v1)[NREG], int r,
                                              const float2 (&cs)[4], const float2 (&sn)[4]) {
   float2 o1[4], o2[4];
@@ -498,7 +498,7 @@ __device__ __forceinline__ void convert_bc(const uint8_t* rawB, const uint8_t* r
       for (int rr = 0; rr < R; ++rr) {
         const int r = rr ^ rot;
         if constexpr (ROT) {
-          rotate_store<R, ROT>(dst, l * R + r, n0, v[0], v[RB::NP - 1], r, cs, sn);
+          rotate_store<R>(dst, l * R + r, n0, v[0], v[RB::NP - 1], r, cs, sn);
         } else {
           float2 o[4];
 #pragma unroll
@@ -576,7 +576,7 @@ __device__ __forceinline__ void store_bc(const RawBC<R, ROT>& raw, uint8_t* sB, 
       for (int rr = 0; rr < R; ++rr) {
         const int r = rr ^ rot;
         if constexpr (ROT) {
-          rotate_store<R, ROT>(dst, l * R + r, n0, raw.v[i][which][0], raw.v[i][which][RB::NP - 1], r, cs, sn);
+          rotate_store<R>(dst, l * R + r, n0, raw.v[i][which][0], raw.v[i][which][RB::NP - 1], r, cs, sn);
         } else {
           float2 o[4];
 #pragma unroll

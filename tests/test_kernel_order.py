@@ -32,12 +32,11 @@ def test_kernels_launched_early_wait_before_they_touch_memory():
     launched = set()
     for path in CSRC.glob("*.cu"):
         s = _text(path)
-        for first in re.findall(r"\blaunch\((\w+)", s):
-            launched |= {first} & set(kernels)
-            if first == "kern":   # (chosen above the launch)
-                for choice in re.findall(r"auto kern\s*=([^;]*);", s):
-                    launched |= set(re.findall(r"\w+", choice)) & set(kernels)
-    assert {"tc_fwd_kernel", "tc_bwd_kernel", "k_step_rows", "k_group_state", "k_rows_adjoint", "k_front_bwd", "kb_final"} <= launched
+        # kernels named in the statement of a launch, or chosen for its `kern` above it
+        for text in re.findall(r"\blaunch\(([^;]*);", s) + re.findall(r"auto kern\s*=([^;]*);", s):
+            launched |= set(re.findall(r"\w+", text)) & set(kernels)
+    assert {"tc_fwd_kernel", "tc_bwd_kernel", "k_step_rows", "k_group_state", "k_rows_adjoint", "k_front_bwd", "k_gate_bwd",
+            "kb_final"} <= launched
     for name in launched:
         before, wait, _ = kernels[name].partition("after_predecessor()")
         assert wait, name
