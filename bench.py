@@ -33,18 +33,23 @@ from mamba_trainer_b200 import sharding, synthetic  # noqa: E402
 NCU_TRAFFIC_BYTES_PER_TOKEN_HEAD = {
     # profiles/tc_fwd_bwd_kernels_cfg4.md: batch 4 x seq 4096 (whole stripes) and batch 8 x seq 4096 (stripes cut
     # into time segments, which adds the hand-over of the state between segments)
-    "cfg4_mimo2_scaling_bf16": {"whole": 1722.7e6 / (4 * 4096 * 32), "split": 3560.8e6 / (8 * 4096 * 32)},
+    "cfg4_mimo2_scaling_bf16": {"whole": 1729.1e6 / (4 * 4096 * 32), "split": 3585.8e6 / (8 * 4096 * 32)},
 }
 
 
-def traffic_per_token_head(w, sms: int):
-    """The captured DRAM traffic per (token, head) of the instantiation this shard runs: at these lengths the library cuts
-    stripes in time when there are more stripes than SMs but fewer than six per SM (tc_segment_plan)."""
+def traffic_per_token_head(w):
+    """The captured DRAM traffic per (token, head) of the instantiation this shard's backward pass runs, as the library says
+    that it cuts the stripes (m3_scan_segments): whole, or segments one after another.  None for segments side by side."""
     v = NCU_TRAFFIC_BYTES_PER_TOKEN_HEAD.get(w.name)
-    if isinstance(v, dict):
-        stripes = w.batch * w.heads
-        return v["split"] if sms < stripes < 6 * sms else v["whole"]
-    return v
+    if v is None:
+        return None
+    import ctypes as C
+    from mamba_trainer_b200 import _ffi
+    d = _ffi.ScanDesc(batch=w.batch, seq=w.seq, heads=w.heads, head_dim=w.head_dim, d_state=w.d_state, rank=w.rank, chunk=w.chunk,
+                      dtype=_ffi.BF16, discretization=int(w.discretization.value), dynamics=int(w.rotational), path=_ffi.PATH_AUTO)
+    n = _ffi.load().m3_scan_segments(C.byref(d), 1)
+    return v["whole"] if n == 1 else v["split"] if n > 1 else None
+
 
 METRIC = "mamba3_ssd_scan_fwd_bwd_throughput"
 UNIT = "Mtokens/s"
@@ -539,7 +544,7 @@ def main():
         achieved = bwd_bytes / (bwd_ms * 1e-3) / 1e9
         whole = alg_bytes / (ms_step * 1e-3) / 1e9
         flops = w.flops_per_token_head() * th
-        per_th = traffic_per_token_head(w, torch.cuda.get_device_properties(dev).multi_processor_count)
+        per_th = traffic_per_token_head(w)
         cfg = workload_config(gw, world, args.config)
         cfg["batch_per_gpu"] = w.batch
         # float32 takes the chunk-parallel family
@@ -557,7 +562,7 @@ def main():
             "config": cfg,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": per_th * th if per_th else None, "peak_kind": peak_kind,
-                         "kernel": bwd_name + " (backward stripe kernel, with its two finalisation launches)",
+                         "kernel": bwd_name + " (backward pass: this kernel and the launch of the per-token and per-head sums)",
                          "ms_per_launch": bwd_ms, "algorithmic_bytes_per_launch": bwd_bytes,
                          "forward": {"kernel": fwd_name, "ms_per_launch": fwd_ms,
                                      "achieved": fwd_bytes / (fwd_ms * 1e-3) / 1e9,

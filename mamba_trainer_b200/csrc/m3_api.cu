@@ -219,7 +219,7 @@ cudaError_t plan_ahead(m3_ctx* ctx, Params& p, const m3::Dims& d, const m3_scan_
 }
 
 // Backward of a forward that ran the tensor-core family: one stripe kernel, then the shared
-// per-token / per-head finalisation.
+// per-token and per-head sums.
 int tc_backward_call(m3_ctx* ctx, const m3_saved* saved, const m3_scan_bwd_in* in, uint32_t mask,
                      const m3_scan_grads* g) {
   const m3_scan_desc& desc = saved->desc;
