@@ -182,6 +182,12 @@ cudaError_t plan_segments(m3_ctx* ctx, Params& p, int tiles, bool allow_split, b
   m3::tc_segment_plan(p.B * p.H, tiles, allow_split, backward, rot, p.R, &p.nseg, &p.tps, &p.grid, &bytes);
   if (p.nseg == 1) return cudaSuccess;
   cudaError_t e = m3::scratch_alloc(ctx, reinterpret_cast<void**>(scratch), bytes, ctx->stream);
+  if (e == cudaErrorMemoryAllocation) {   // no room for the hand-over: whole stripes need none
+    cudaGetLastError();
+    *scratch = nullptr;
+    m3::tc_segment_plan(p.B * p.H, tiles, false, backward, rot, p.R, &p.nseg, &p.tps, &p.grid, &bytes);
+    return cudaSuccess;
+  }
   if (e != cudaSuccess) return e;
   const size_t items = (size_t)p.B * p.H * p.nseg;
   p.seg_state = reinterpret_cast<float*>(*scratch);

@@ -233,3 +233,48 @@ assert torch.cuda.mem_get_info()[0] == free, (free, torch.cuda.mem_get_info()[0]
     root = Path(__file__).resolve().parent.parent
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_stripes_stay_whole_where_memory_has_run_out():
+    """In a process of its own: with no room left for the scratch that cut stripes hand their state over in, a forward pass
+    runs whole stripes, to the same results bit for bit."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    code = """
+import ctypes as C, torch
+from mamba_trainer_b200 import _ffi, synthetic
+from mamba_trainer_b200.ssm import Discretization
+from tests.test_zz_no_alloc import _desc, _outputs
+lib, ctx = _ffi.load(), C.c_void_p()
+assert lib.m3_ctx_create(0, C.byref(ctx)) == _ffi.OK
+def make(batch, seq):
+    w = synthetic.Workload('w', batch, seq, 32, 64, 128, 64, 1, torch.bfloat16, Discretization.LearnedTrapezoid, False, 'rms')
+    t = {k: (v.cuda() if v is not None else None) for k, v in synthetic.make_inputs(w, seed=1).items()}
+    d = _desc(t, w)
+    d.path = _ffi.PATH_AUTO
+    return t, d, _outputs(t, w)
+def run(c):
+    rc = lib.m3_scan_forward(ctx, C.byref(c[1]), C.byref(c[2][1]), None)
+    assert rc == _ffi.OK, lib.m3_last_error(ctx)
+    assert lib.m3_sync(ctx) == _ffi.OK
+    return [v.clone() for v in c[2][0] if v is not None]
+small, big = make(2, 300), make(5, 2900)
+assert lib.m3_scan_segments(C.byref(small[1]), 0) == 1 and lib.m3_scan_segments(C.byref(big[1]), 0) > 1
+run(small)                                  # loads the kernel of whole stripes
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+MiB = 1 << 20
+fill = torch.empty((torch.cuda.mem_get_info()[0] // (2 * MiB) - 3) * 2 * MiB, dtype=torch.uint8, device='cuda')
+assert torch.cuda.mem_get_info()[0] < 15 * MiB                        # the scratch takes 15.9
+rc = lib.m3_scan_forward(ctx, C.byref(big[1]), C.byref(big[2][1]), None)
+assert rc == _ffi.OK, lib.m3_last_error(ctx)
+assert lib.m3_sync(ctx) == _ffi.OK
+del fill
+torch.cuda.empty_cache()
+whole = [v.clone() for v in big[2][0] if v is not None]
+for a, e in zip(run(big), whole): assert torch.equal(a, e)
+"""
+    root = Path(__file__).resolve().parent.parent
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
